@@ -404,7 +404,7 @@ __device__ __forceinline__ uint32_t ld_acquire_sys(const volatile uint32_t* p) {
 // no entry for `idle_limit` polls (about a microsecond apart), or sees
 // `stop`, exits. Every wait is bounded.
 template <int NT>
-__global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* __restrict__ desc, SoloQueue* q,
+__global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* desc, SoloQueue* q,
                                                            uint32_t* head, int idle_limit, int gen) {
     __shared__ __align__(16) SoloArgs S;
     __shared__ GridParams g;
@@ -438,9 +438,13 @@ __global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* __res
         if (rec < 0) break;
         if (threadIdx.x == 0) q->live[gen][blockIdx.x] = 2u;  // 2: running a request
         {
+            // the host rewrites a record between the requests of its slot,
+            // while this kernel runs: read past L1 (a line kept from the
+            // slot's previous record would give this request that one's
+            // atom count or buffers)
             const int4* src = reinterpret_cast<const int4*>(desc + rec);
             int4* dst = reinterpret_cast<int4*>(&S);
-            for (int k = threadIdx.x; k < (int)(sizeof(SoloArgs) / sizeof(int4)); k += NT) dst[k] = src[k];
+            for (int k = threadIdx.x; k < (int)(sizeof(SoloArgs) / sizeof(int4)); k += NT) dst[k] = __ldcv(src + k);
         }
         __syncthreads();
         if (S.any_eam) solo_run<true, NT>(S, g, red, scan_sh);
