@@ -454,6 +454,45 @@ static void force_rows(const std::vector<double>& ry, const std::vector<double>&
     }
 }
 
+// The FP64 pieces the FP64 force stages evaluate, in x = r - r_n: per interval
+// W = V'r - V (cubic) and D = rho' (quadratic), then the rho and V pieces
+// themselves and r_n, from the reference's Hermite form (value, slope, a, b).
+static void rows64(const mdg_potential& p, std::vector<double>& out) {
+    const int N = p.Nr1;
+    const double h1 = 1.0 / p.dr;
+    std::vector<double> wd, rho, v;
+    auto piece = [&](const std::vector<double>& y, const std::vector<double>& z, int n, double c[4]) {
+        const double m = (y[n + 1] - y[n]) * h1;
+        const double aa = (z[n + 1] - m) - (m - z[n]);
+        const double bb = aa - (m - z[n]);
+        c[0] = y[n];
+        c[1] = z[n];
+        c[2] = -bb * h1;
+        c[3] = aa * h1 * h1;
+    };
+    for (int n = 0; n < N; ++n) {
+        double r[4], c[4];
+        const double xn = n * p.dr;
+        piece(p.Rho, p.dRho, n, r);
+        piece(p.Vpar, p.dVpar, n, c);
+        const double row[8] = {c[1] * xn - c[0], 2.0 * c[2] * xn, c[2] + 3.0 * c[3] * xn, 2.0 * c[3],
+                               r[1], 2.0 * r[2], 3.0 * r[3], 0.0};
+        wd.insert(wd.end(), row, row + 8);
+        rho.insert(rho.end(), r, r + 4);
+        v.insert(v.end(), c, c + 4);
+    }
+    out.insert(out.end(), wd.begin(), wd.end());
+    out.insert(out.end(), rho.begin(), rho.end());
+    out.insert(out.end(), v.begin(), v.end());
+    for (int n = 0; n < N; ++n) out.push_back(n * p.dr);
+}
+
+// Start of the rows64 block in d_tab64: the knots before it, rounded up to a
+// 32-byte row.
+static size_t rows64_at(const mdg_potential* p) {
+    return (4 * ((size_t)p->Nr1 + 1) + 2 * ((size_t)p->Nrh1 + 1) + 3) & ~size_t(3);
+}
+
 int pot_upload(mdg_potential* p, int device) {
     if ((p->type != POT_EAM && p->type != POT_TAB) || p->device == device) return MDG_OK;
     if (p->d_tab64) cudaFree(p->d_tab64);
@@ -462,9 +501,11 @@ int pot_upload(mdg_potential* p, int device) {
     p->d_tab32 = nullptr;
     size_t nr = (size_t)p->Nr1 + 1, nh = (size_t)p->Nrh1 + 1;
     std::vector<double> h64;
-    h64.reserve(4 * nr + 2 * nh);
+    h64.reserve(4 * nr + 2 * nh + 4 + 17 * (size_t)p->Nr1);
     for (auto* v : {&p->Rho, &p->dRho, &p->Vpar, &p->dVpar}) h64.insert(h64.end(), v->begin(), v->end());
     for (auto* v : {&p->Femb, &p->dFemb}) h64.insert(h64.end(), v->begin(), v->end());
+    h64.resize(rows64_at(p), 0.0);
+    rows64(*p, h64);
     std::vector<float4> rc, vc, fc, h32;
     cubic_coeffs(p->Rho, p->dRho, p->dr, p->Nr1, rc);
     cubic_coeffs(p->Vpar, p->dVpar, p->dr, p->Nr1, vc);
@@ -491,6 +532,7 @@ int pot_upload(mdg_potential* p, int device) {
 // `z32`, kZeroRows rows of zeros, so that no kernel load sees a null pointer.
 static void zero_tables(PotParams& P, const double* z64, const float4* z32) {
     P.Rho = P.dRho = P.Vpar = P.dVpar = P.Femb = P.dFemb = z64;
+    P.wd64 = P.rho64 = P.v64 = P.rn64 = z64;
     P.rho_c = P.v_c = P.f_c = P.rv_c = z32;
 }
 
@@ -510,6 +552,8 @@ static void fill_params(const mdg_potential* p, PotParams& P, const double* z64,
         P.lj1_f = (float)p->lj1;
         P.lj2_f = (float)p->lj2;
         P.mhf_f = (float)(-0.5 * p->factor);
+        P.mhf_lj1 = -0.5 * p->factor * p->lj1;
+        P.hf_lj2 = 0.5 * p->factor * p->lj2;
     } else if (p->type == POT_LJS) {
         P.ljs_rVr1 = p->ljs_rVr1;
         P.ljs_rVr2 = p->ljs_rVr2;
@@ -538,6 +582,10 @@ static void fill_params(const mdg_potential* p, PotParams& P, const double* z64,
         P.dVpar = p->d_tab64 + 3 * nr;
         P.Femb = p->d_tab64 + 4 * nr;
         P.dFemb = p->d_tab64 + 4 * nr + nh;
+        P.wd64 = p->d_tab64 + rows64_at(p);
+        P.rho64 = P.wd64 + 8 * (size_t)p->Nr1;
+        P.v64 = P.rho64 + 4 * (size_t)p->Nr1;
+        P.rn64 = P.v64 + 4 * (size_t)p->Nr1;
         P.rho_c = p->d_tab32;
         P.v_c = p->d_tab32 + p->Nr1;
         P.f_c = p->d_tab32 + 2 * p->Nr1;
@@ -561,7 +609,7 @@ struct SolverBlob {
     PotSet ps;
     ThermoDev th;
     alignas(32) float4 z32[2 * kZeroRows];
-    double z64[2 * kZeroRows];
+    alignas(32) double z64[2 * kZeroRows];
 };
 
 struct SolverDev {

@@ -19,13 +19,16 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "mdg_host.h"
+#include "forces64_dev.cuh"
 #include "forces_dev.cuh"
 #include "integrate_dev.cuh"
 
 namespace mdg {
 
+constexpr int kBlock64 = 128;  // threads per block of the FP64 pair passes
 
 // ---------------------------------------------------------------------------
 // FP64 spline pieces (EAM.cxx, same operation order)
@@ -140,42 +143,6 @@ __device__ __forceinline__ double lj_pref64(const PotParams& P, double r2) {
     return -0.5 * P.factor * (P.lj1 * r6inv - P.lj2) * r6inv * r2inv;
 }
 
-// Visits the listed pairs of atom i the way Pair::* + Periodic::*_one do:
-// main pass with raw differences, then the ghost pass for bc atoms.
-// fn(kj, j, dx, dy, dz, r2, ghost)
-template <bool MULTI, typename Fn>
-__device__ __forceinline__ void visit64(const FArgs& A, int i, Fn&& fn) {
-    double xi = A.rx[i], yi = A.ry[i], zi = A.rz[i];
-    int cnt = A.ncnt[i];
-    // main pass (the self entry contributes nothing: r2 < 1e-15)
-    for (int k = 0; k < cnt; ++k) {
-        uint32_t j = A.nbr[nidx(k, i, A.np)] & kJMask;
-        int kj = MULTI ? (A.kind[j] & 3) : 0;
-        double dx = A.rx[j] - xi, dy = A.ry[j] - yi, dz = A.rz[j] - zi;
-        double r2 = dx * dx + dy * dy + dz * dz;
-        fn(kj, (int)j, dx, dy, dz, r2, false);
-    }
-    if (!A.bc[i]) return;
-    double rni = A.rns[i];
-    for (int k = 0; k < cnt; ++k) {
-        uint32_t j = A.nbr[nidx(k, i, A.np)] & kJMask;
-        int kj = MULTI ? (A.kind[j] & 3) : 0;
-        double dx = A.rx[j] - xi, dy = A.ry[j] - yi, dz = A.rz[j] - zi;
-        double rnj = A.rns[j];
-        double r2rns = rnj < rni ? rni : rnj;
-        r2rns *= r2rns;
-        if (dx * dx + dy * dy + dz * dz < r2rns) continue;
-        dx = shortest1(dx, A.L[0], A.periodic[0]);
-        dy = shortest1(dy, A.L[1], A.periodic[1]);
-        dz = shortest1(dz, A.L[2], A.periodic[2]);
-        if (dx * dx + dy * dy + dz * dz > r2rns) continue;
-        // ghost copy at r_i + d, seen from r_i
-        double gx = (xi + dx) - xi, gy = (yi + dy) - yi, gz = (zi + dz) - zi;
-        double r2 = gx * gx + gy * gy + gz * gz;
-        fn(kj, (int)j, gx, gy, gz, r2, true);
-    }
-}
-
 // ---- F'(nc) of the current densities, FP64 -----------------------------------
 // The reference's force pass evaluates the embedding derivative from each
 // atom's nc as it is (EAM.cxx:465-497); the FP64 force kernel reads it from
@@ -196,158 +163,233 @@ __global__ void __launch_bounds__(kBlock) k_embed64(FArgs A, const PotSet* __res
     }
 }
 
-// ---- LJsCut / EAM forces, FP64 ------------------------------------------------
+// ---- pair and EAM forces, FP64 ------------------------------------------------
 // HALF (half lists, verlet-list.cxx:345): the pair-type potentials push the
 // pair force onto the neighbour as well (LJs-cut.cxx:57-62, pair.cxx:387-420,
 // LJs.cxx:196-222); EAM uses the atom's half alone, as EAM::force does; the
 // ghost pass acts on the atom alone (its ghost list is a full one,
 // periodic.cxx:77-88). Both sides accumulate with atomics onto the outputs
 // prepare cleared, as the reference's += does.
-template <bool MULTI, bool HALF>
-__global__ void __launch_bounds__(kBlock) k_forces64(FArgs A, const PotSet* __restrict__ ps) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.n || A.tag[i] == 0) return;
-    int ki = MULTI ? (A.kind[i] & 3) : 0;
-    double fm[3] = {0, 0, 0}, fg[3] = {0, 0, 0};
-    visit64<MULTI>(A, i, [&](int kj, int j, double dx, double dy, double dz, double r2, bool ghost) {
-        const PotParams& P = ps->p[ki][kj];
-        if (r2 > P.R2cut || r2 < 1e-15) return;
-        double pref;
-        if (P.type == 1) {
-            pref = lj_pref64(P, r2);
-        } else if (P.type == 2) {
-            double AdF = A.Fp64[(size_t)ki * A.np + j] + A.Fp64[(size_t)kj * A.np + i];
-            pref = eam_ff64(P, r2, AdF, nullptr);
-        } else if (P.type == POT_TAB) {
-            pref = tab_ff64(P, r2, nullptr);
-        } else if (P.type == POT_LJS) {
-            pref = ljs_ff64(P, r2, nullptr);
-        } else {
-            return;
-        }
-        double* f = ghost ? fg : fm;
-        f[0] += dx * pref;
-        f[1] += dy * pref;
-        f[2] += dz * pref;
-        if (HALF && !ghost && P.type != 2) {
-            atomicAdd(&A.fx[j], -(dx * pref));
-            atomicAdd(&A.fy[j], -(dy * pref));
-            atomicAdd(&A.fz[j], -(dz * pref));
-        }
-    });
-    double fx = fm[0] + fg[0], fy = fm[1] + fg[1], fz = fm[2] + fg[2];
-    if (!isfinite(fx) || !isfinite(fy) || !isfinite(fz)) atomicOr(&A.st->flags, FLAG_NONFINITE);
+// FORM: the potential of every pair where there is one (POT_LJCUT, POT_EAM;
+// Single), 0 = by kind pair. G lanes share an atom (with_lanes64).
+template <bool MULTI, int FORM, bool HALF, int G>
+__global__ void __launch_bounds__(kBlock64) k_forces64(FArgs A, const PotSet* __restrict__ ps) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % G;
+    const bool live = t / G < A.n && A.tag[t / G] != 0;
+    const int i = live ? t / G : 0;
+    double f[3] = {0, 0, 0};
+    if (live) {
+        const int ki = MULTI ? (A.kind[i] & 3) : 0;
+        walk64<MULTI, G, true>(A, ps, i, ki, lane, [](const PotParams&, int, int, bool) {},
+                         [&](const PotParams& P, int kj, uint32_t j, const Pair64& p, bool ghost) {
+            const int type = FORM ? FORM : P.type;
+            double pref, E;
+            if (type == POT_LJCUT) {
+                pref = ljcut_ff64<false>(P, p.r2, E);
+            } else if (type == POT_EAM) {
+                const double AdF = A.Fp64[(size_t)ki * A.np + j] + A.Fp64[(size_t)kj * A.np + i];
+                pref = table_ff64<true, false>(P, p.r2, AdF, E);
+            } else if (type == POT_TAB) {
+                pref = table_ff64<false, false>(P, p.r2, 0.0, E);
+            } else if (type == POT_LJS) {
+                pref = ljs_pair64<false>(P, p.r2, E);
+            } else {
+                return;
+            }
+            f[0] = fma(p.dx, pref, f[0]);
+            f[1] = fma(p.dy, pref, f[1]);
+            f[2] = fma(p.dz, pref, f[2]);
+            if (HALF && !ghost && type != POT_EAM) {
+                atomicAdd(&A.fx[j], -(p.dx * pref));
+                atomicAdd(&A.fy[j], -(p.dy * pref));
+                atomicAdd(&A.fz[j], -(p.dz * pref));
+            }
+        });
+    }
+    for (int a = 0; a < 3; ++a) f[a] = lane_sum<G>(f[a]);
+    if (!live || lane) return;
+    if (!isfinite(f[0]) || !isfinite(f[1]) || !isfinite(f[2])) atomicOr(&A.st->flags, FLAG_NONFINITE);
     if (HALF) {
-        atomicAdd(&A.fx[i], fx);
-        atomicAdd(&A.fy[i], fy);
-        atomicAdd(&A.fz[i], fz);
+        atomicAdd(&A.fx[i], f[0]);
+        atomicAdd(&A.fy[i], f[1]);
+        atomicAdd(&A.fz[i], f[2]);
     } else {
-        A.fx[i] = fx;
-        A.fy[i] = fy;
-        A.fz[i] = fz;
+        A.fx[i] = f[0];
+        A.fy[i] = f[1];
+        A.fz[i] = f[2];
     }
 }
 
 // ---- EAM density + embedding derivative, FP64 ------------------------------
-template <bool MULTI>
-__global__ void __launch_bounds__(kBlock) k_density64(FArgs A, const PotSet* __restrict__ ps) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.n) return;
-    if (A.tag[i] == 0) {
-        // untouched by the reference's charge stage; F' still defined
-        double nci = A.nc[i];
-        int ki = MULTI ? (A.kind[i] & 3) : 0;
-        for (int b = 0; b < ps->nkinds; ++b) {
-            const PotParams& P = ps->p[ki][b];
-            double EF = 0, dF = 0;
-            if (P.type == 2) eam_embed64(P, nci, &EF, &dF, A.st);
-            A.Fp64[(size_t)b * A.np + i] = dF;
-        }
-        return;
-    }
-    int ki = MULTI ? (A.kind[i] & 3) : 0;
-    double sm = 0.0, sg = 0.0;
-    visit64<MULTI>(A, i, [&](int kj, int j, double, double, double, double r2, bool ghost) {
-        const PotParams& P = ps->p[ki][kj];
-        if (P.type != 2 || r2 > P.R2cut || r2 < 1e-15) return;
-        double v = eam_rho64(P, sqrt(r2));
-        if (ghost) sg = sg + v;
-        else sm = sm + v;
-    });
-    double nci = sm + sg;
-    A.nc[i] = nci;
+template <bool MULTI, int G>
+__global__ void __launch_bounds__(kBlock64) k_density64(FArgs A, const PotSet* __restrict__ ps) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % G;
+    const bool in = t / G < A.n;
+    const int i = in ? t / G : 0;
+    const int ki = MULTI && in ? (A.kind[i] & 3) : 0;
+    const bool live = in && A.tag[i] != 0;
+    double rho = 0.0;
+    if (live)
+        walk64<MULTI, G, true>(A, ps, i, ki, lane, [](const PotParams&, int, int, bool) {},
+                         [&](const PotParams& P, int, uint32_t, const Pair64& p, bool) {
+            if (!MULTI || P.type == POT_EAM) rho += table_rho64(P, p.r2);
+        });
+    rho = lane_sum<G>(rho);
+    if (!in || lane) return;
+    // an atom with tag 0 is untouched by the reference's charge stage; its F' is still defined
+    if (live) A.nc[i] = rho;
+    else rho = A.nc[i];
     for (int b = 0; b < ps->nkinds; ++b) {
         const PotParams& P = ps->p[ki][b];
         double EF = 0, dF = 0;
-        if (P.type == 2) eam_embed64(P, nci, &EF, &dF, A.st);
+        if (P.type == POT_EAM) eam_embed64(P, rho, &EF, &dF, A.st);
         A.Fp64[(size_t)b * A.np + i] = dF;
     }
 }
 
 // ---- energies and virials, FP64 (LJs-cut.cxx:70-131, EAM.cxx:306-415,
-// pair.cxx:228-314, LJs.cxx:103-151); HALF as for the forces above.
-template <bool MULTI, bool HALF>
-__global__ void __launch_bounds__(kBlock) k_virials64(FArgs A, const PotSet* __restrict__ ps) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.n || A.tag[i] == 0) return;
-    int ki = MULTI ? (A.kind[i] & 3) : 0;
+// pair.cxx:228-314, LJs.cxx:103-151); HALF and FORM as for the forces above.
+// The virial of a pair is symmetric: six sums.
+template <bool MULTI, int FORM, bool HALF, int G>
+__global__ void __launch_bounds__(kBlock64) k_virials64(FArgs A, const PotSet* __restrict__ ps) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % G;
+    const bool live = t / G < A.n && A.tag[t / G] != 0;
+    const int i = live ? t / G : 0;
+    const int ki = MULTI && live ? (A.kind[i] & 3) : 0;
     double Ep = 0.0;
-    double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    int last_kind = -1;
-    visit64<MULTI>(A, i, [&](int kj, int j, double dx, double dy, double dz, double r2, bool ghost) {
-        const PotParams& P = ps->p[ki][kj];
-        if (P.type == 2) last_kind = kj > last_kind || ghost ? kj : last_kind;
-        if (r2 > P.R2cut || r2 < 1e-15) return;
-        double d[3] = {dx, dy, dz};
-        double E = 0.0, Mp[9];
-        if (P.type == 1) {
-            double r2inv = 1.0 / r2;
-            double r6inv = r2inv * r2inv * r2inv;
-            double pref = -0.5 * P.factor * (P.lj1 * r6inv - P.lj2) * r6inv * r2inv;
-            double tmp = P.s6 * r6inv;
-            E = 0.5 * 4 * P.a * tmp * (tmp - 1);
-            for (int c = 0; c < 3; ++c)
-                for (int r = 0; r < 3; ++r) Mp[r + 3 * c] = 0.5 * (pref * d[r]) * d[c];
-        } else if (P.type == 2) {
-            double AdF = A.Fp64[(size_t)ki * A.np + j] + A.Fp64[(size_t)kj * A.np + i];
-            double FF = eam_ff64(P, r2, AdF, &E);
-            double h = 0.5 * FF;
-            for (int c = 0; c < 3; ++c)
-                for (int r = 0; r < 3; ++r) Mp[r + 3 * c] = h * d[r] * d[c];
-        } else if (P.type == POT_TAB) {
-            double h = 0.5 * tab_ff64(P, r2, &E);
-            for (int c = 0; c < 3; ++c)
-                for (int r = 0; r < 3; ++r) Mp[r + 3 * c] = h * d[r] * d[c];
-        } else if (P.type == POT_LJS) {
-            double FF = ljs_ff64(P, r2, &E);
-            for (int c = 0; c < 3; ++c)
-                for (int r = 0; r < 3; ++r) Mp[r + 3 * c] = 0.5 * (FF * d[r]) * d[c];
-        } else {
-            return;
+    double M[6] = {0, 0, 0, 0, 0, 0};  // xx yy zz xy xz yz
+    // the kind whose embedding table gives Em: the last ghost's, else the
+    // largest listed (both among EAM pairs); -1 and (entry, kind) codes
+    int last_main = -1, last_ghost = -1;
+    constexpr int kSym[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
+    if (live)
+        walk64<MULTI, G, !MULTI>(A, ps, i, ki, lane, [&](const PotParams& P, int kj, int k, bool ghost) {
+            if (!MULTI || P.type != POT_EAM) return;
+            if (ghost) last_ghost = 4 * k + kj;
+            else last_main = max(last_main, kj);
+        }, [&](const PotParams& P, int kj, uint32_t j, const Pair64& p, bool ghost) {
+            const int type = FORM ? FORM : P.type;
+            double E = 0.0, ff;
+            if (type == POT_LJCUT) {
+                ff = ljcut_ff64<true>(P, p.r2, E);
+            } else if (type == POT_EAM) {
+                const double AdF = A.Fp64[(size_t)ki * A.np + j] + A.Fp64[(size_t)kj * A.np + i];
+                ff = table_ff64<true, true>(P, p.r2, AdF, E);
+            } else if (type == POT_TAB) {
+                ff = table_ff64<false, true>(P, p.r2, 0.0, E);
+            } else if (type == POT_LJS) {
+                ff = ljs_pair64<true>(P, p.r2, E);
+            } else {
+                return;
+            }
+            const double h = 0.5 * ff, hx = h * p.dx, hy = h * p.dy;
+            Ep += E;
+            if (HALF && !ghost && type != POT_EAM) {
+                const double m[6] = {hx * p.dx, hy * p.dy, h * p.dz * p.dz, hx * p.dy, hx * p.dz, hy * p.dz};
+                for (int q = 0; q < 6; ++q) M[q] += m[q];
+                atomicAdd(&A.Ep[j], E);
+                for (int k = 0; k < 9; ++k) atomicAdd(&A.V[k][j], m[kSym[k]]);
+            } else {
+                M[0] = fma(hx, p.dx, M[0]);
+                M[1] = fma(hy, p.dy, M[1]);
+                M[2] = fma(h * p.dz, p.dz, M[2]);
+                M[3] = fma(hx, p.dy, M[3]);
+                M[4] = fma(hx, p.dz, M[4]);
+                M[5] = fma(hy, p.dz, M[5]);
+            }
+        });
+    Ep = lane_sum<G>(Ep);
+    for (int q = 0; q < 6; ++q) M[q] = lane_sum<G>(M[q]);
+    if (MULTI) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+            last_main = max(last_main, __shfl_xor_sync(0xffffffffu, last_main, o));
+            last_ghost = max(last_ghost, __shfl_xor_sync(0xffffffffu, last_ghost, o));
         }
-        Ep += E;
-        for (int k = 0; k < 9; ++k) M[k] += Mp[k];
-        if (HALF && !ghost && P.type != 2) {
-            atomicAdd(&A.Ep[j], E);
-            for (int k = 0; k < 9; ++k) atomicAdd(&A.V[k][j], Mp[k]);
-        }
-    });
+    }
+    if (!live || lane) return;
     if (HALF) {
         atomicAdd(&A.Ep[i], Ep);
-        for (int k = 0; k < 9; ++k) atomicAdd(&A.V[k][i], M[k]);
+        for (int k = 0; k < 9; ++k) atomicAdd(&A.V[k][i], M[kSym[k]]);
     } else {
         A.Ep[i] = Ep;
-        for (int k = 0; k < 9; ++k) A.V[k][i] = M[k];
+        for (int k = 0; k < 9; ++k) A.V[k][i] = M[kSym[k]];
     }
     if (ps->any_eam) {
-        int kb = MULTI ? (last_kind >= 0 ? last_kind : ki) : 0;
+        const int last = last_ghost >= 0 ? last_ghost & 3 : last_main;
+        const int kb = MULTI ? (last >= 0 ? last : ki) : 0;
         const PotParams& P = ps->p[ki][kb];
         double EF = 0.0, dF = 0.0;
-        if (P.type == 2) {
+        if (P.type == POT_EAM) {
             eam_embed64(P, A.nc[i], &EF, &dF, A.st);
             A.Em[i] = EF;
         }
     }
+}
+
+// Lanes per atom of the FP64 passes: 32 below 12,500 atoms, 4 below 100,000,
+// else one. Fewer atoms than about 100,000 threads' worth leave SMs with too
+// few warps to keep their FP64 pipe busy; more lanes than that cost the sums
+// over lanes and lanes without a pair. Measured per FP64 step, 1 / 4 / 32
+// lanes: LJ argon 500 atoms 137 / 72 / 46 us, 4,000 atoms 140 / 62 / 51 us;
+// EAM Cu 32,000 atoms 253 / 213 / 295 us, 108,000 atoms 560 / 565 / 924 us,
+// 1,000,188 atoms 3.87 / 4.54 / 8.20 ms. (2, 8 and 16 lanes are never more
+// than 8% faster than the best of these three.)
+// Calls f(std::integral_constant<int, G>) with the G of n atoms.
+template <typename F>
+static void with_lanes64(size_t n, F&& f) {
+    if (n < 12500) f(std::integral_constant<int, 32>());
+    else if (n < 100000) f(std::integral_constant<int, 4>());
+    else f(std::integral_constant<int, 1>());
+}
+
+static void launch_density64(const FArgs& A, const PotSet* dps, const PotSet& ps, cudaStream_t st) {
+    with_lanes64(A.n, [&](auto g) {
+        constexpr int G = decltype(g)::value;
+        const int nb = (int)(((size_t)A.n * G + kBlock64 - 1) / kBlock64);
+        if (ps.multi) k_density64<true, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        else k_density64<false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+    });
+}
+
+static void launch_forces64(const FArgs& A, const PotSet* dps, const PotSet& ps, bool half, cudaStream_t st) {
+    const int only = ps.multi ? 0 : ps.any_eam ? POT_EAM : ps.any_lj ? POT_LJCUT : 0;
+    with_lanes64(A.n, [&](auto g) {
+        constexpr int G = decltype(g)::value;
+        const int nb = (int)(((size_t)A.n * G + kBlock64 - 1) / kBlock64);
+        if (half) {
+            if (ps.multi) k_forces64<true, 0, true, G><<<nb, kBlock64, 0, st>>>(A, dps);
+            else k_forces64<false, 0, true, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        } else if (ps.multi) {
+            k_forces64<true, 0, false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        } else if (only == POT_EAM) {
+            k_forces64<false, POT_EAM, false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        } else if (only == POT_LJCUT) {
+            k_forces64<false, POT_LJCUT, false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        } else {
+            k_forces64<false, 0, false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        }
+    });
+}
+
+static void launch_virials64(const FArgs& A, const PotSet* dps, const PotSet& ps, bool half, cudaStream_t st) {
+    const int only = ps.multi ? 0 : ps.any_eam ? POT_EAM : ps.any_lj ? POT_LJCUT : 0;
+    with_lanes64(A.n, [&](auto g) {
+        constexpr int G = decltype(g)::value;
+        const int nb = (int)(((size_t)A.n * G + kBlock64 - 1) / kBlock64);
+        if (half) {
+            if (ps.multi) k_virials64<true, 0, true, G><<<nb, kBlock64, 0, st>>>(A, dps);
+            else k_virials64<false, 0, true, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        } else if (ps.multi) {
+            k_virials64<true, 0, false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        } else if (only == POT_EAM) {
+            k_virials64<false, POT_EAM, false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        } else if (only == POT_LJCUT) {
+            k_virials64<false, POT_LJCUT, false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        } else {
+            k_virials64<false, 0, false, G><<<nb, kBlock64, 0, st>>>(A, dps);
+        }
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -731,8 +773,7 @@ int launch_stage(mdg_system* sys, const PotSet* dps, const PotSet& ps, int preci
     bool multi = ps.multi != 0;
     if (precision == MDG_PREC_FP64) {
         if (stage == 0) {
-            if (multi) k_density64<true><<<nb, kBlock, 0, st>>>(A, dps);
-            else k_density64<false><<<nb, kBlock, 0, st>>>(A, dps);
+            launch_density64(A, dps, ps, st);
             sys->fp_ok = 1;
         } else {
             if (ps.any_eam && !sys->fp_ok) {
@@ -741,13 +782,7 @@ int launch_stage(mdg_system* sys, const PotSet* dps, const PotSet& ps, int preci
                 MDG_LAUNCHED(ctx);
                 sys->fp_ok = 1;
             }
-            if (sys->half) {
-                if (multi) k_forces64<true, true><<<nb, kBlock, 0, st>>>(A, dps);
-                else k_forces64<false, true><<<nb, kBlock, 0, st>>>(A, dps);
-            } else {
-                if (multi) k_forces64<true, false><<<nb, kBlock, 0, st>>>(A, dps);
-                else k_forces64<false, false><<<nb, kBlock, 0, st>>>(A, dps);
-            }
+            launch_forces64(A, dps, ps, sys->half != 0, st);
         }
     } else {
         if (stage == 0) {
@@ -770,17 +805,12 @@ int launch_virials(mdg_system* sys, const PotSet* dps, const PotSet& ps) {
     mdg_ctx* ctx = sys->ctx;
     if (sys->n == 0) return MDG_OK;
     FArgs A = force_args(sys);
-    int nb = nblk(sys->n);
     if (sys->half) {
         // accumulates onto the outputs: cleared first, as prepare leaves them
         int rc = launch_zero_meas(sys);
         if (rc) return rc;
-        if (ps.multi) k_virials64<true, true><<<nb, kBlock, 0, ctx->stream>>>(A, dps);
-        else k_virials64<false, true><<<nb, kBlock, 0, ctx->stream>>>(A, dps);
-    } else {
-        if (ps.multi) k_virials64<true, false><<<nb, kBlock, 0, ctx->stream>>>(A, dps);
-        else k_virials64<false, false><<<nb, kBlock, 0, ctx->stream>>>(A, dps);
     }
+    launch_virials64(A, dps, ps, sys->half != 0, ctx->stream);
     MDG_LAUNCHED(ctx);
     return MDG_OK;
 }

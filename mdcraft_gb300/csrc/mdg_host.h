@@ -87,7 +87,7 @@ struct mdg_potential {
     double dr = 0, drh = 0, dr1 = 0, drh1 = 0;
     std::vector<double> Rho, dRho, Vpar, dVpar, Femb, dFemb;
     int device = -1;
-    double* d_tab64 = nullptr;   // Rho,dRho,Vpar,dVpar (Nr1+1 each), Femb,dFemb (Nrh1+1 each)
+    double* d_tab64 = nullptr;   // Rho,dRho,Vpar,dVpar (Nr1+1 each), Femb,dFemb (Nrh1+1 each), then rows64
     float4* d_tab32 = nullptr;   // rho_c, v_c (Nr1 each), f_c (Nrh1)
 };
 
