@@ -396,16 +396,15 @@ static void launch_virials64(const FArgs& A, const PotSet* dps, const PotSet& ps
 // mixed precision (bodies in forces_dev.cuh)
 // ---------------------------------------------------------------------------
 // Blocks of 256 threads per SM the register budget must allow, measured on
-// EAM Cu 1M atoms: the force pass is fastest at 4 (64 registers; 0.227 ms
-// against 0.237 ms at 3), the density pass at 4 (0.165 ms against 0.177 ms
-// at 5, where it spills).
+// EAM Cu 1M atoms: the force pass is fastest at 4 (64 registers; 0.229 ms
+// against 0.238 ms at 3), the density pass at 4 (0.154 ms against 0.177 ms
+// at 3, 0.195 ms at 5, where it spills).
 constexpr int kForceMinBlocks = 4;
 constexpr int kDensityMinBlocks = 4;
-// The Multi force body (per-pair kind, parameters and F' columns) spills at
-// 64 registers; three blocks per SM (up to 85 registers) measured fastest on
-// NiAl B2 1M atoms: 7.2e8 atom-steps/s against 6.4e8 at four blocks and
-// 6.2e8 at two. The Multi density body fits 64 registers without spills and
-// runs best at four blocks like the single one (7.39e8 against 7.20e8).
+// The Multi bodies spill at 64 registers; three blocks per SM (up to 85
+// registers) are fastest for two kinds (NiAl B2 1M: force pass 0.551 ms
+// against 0.638 ms at four, density 0.355 against 0.383). With more kinds the
+// density body's parameters are read per pair and four blocks do as well.
 constexpr int kMultiMinBlocks = 3;
 // MB = blocks of 256 threads per SM the register budget allows: a system's
 // launch shape (mdg_system_set_shape, chosen by the project's autotuner),
@@ -416,22 +415,23 @@ __global__ void __launch_bounds__(kBlock, MB) k_lj_mixed(FArgs A, const PotSet* 
     if (i < A.n) lj_mixed_one<MULTI, KICK>(A, ps, i);
 }
 
-template <bool MULTI, int MB>
+// KINDS: 0 Single, 2 two kinds, 4 up to four (KindPots).
+template <int KINDS, int MB>
 __global__ void __launch_bounds__(kBlock, MB) k_density_rec(FArgs A, const PotSet* __restrict__ ps) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < A.n) density_mixed_one<MULTI, true>(A, ps, i);
+    if (i < A.n) density_mixed_one<KINDS, true>(A, ps, i);
 }
 
-template <bool MULTI, int MB>
+template <int KINDS, int MB>
 __global__ void __launch_bounds__(kBlock, MB) k_density_mixed(FArgs A, const PotSet* __restrict__ ps) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < A.n) density_mixed_one<MULTI>(A, ps, i);
+    if (i < A.n) density_mixed_one<KINDS>(A, ps, i);
 }
 
-template <bool MULTI, bool KICK, int MB>
+template <int KINDS, bool KICK, int MB>
 __global__ void __launch_bounds__(kBlock, MB) k_eam_mixed(FArgs A, const PotSet* __restrict__ ps) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < A.n) eam_mixed_one<MULTI, KICK>(A, ps, i);
+    if (i < A.n) eam_mixed_one<KINDS, KICK>(A, ps, i);
 }
 
 // The blocks-per-SM budget of a pass: the system's shape if set, else the
@@ -440,36 +440,135 @@ static int force_blocks(const mdg_system* sys, bool multi) {
     return sys->shape[MDG_SHAPE_FORCE_BLOCKS_PER_SM] ? sys->shape[MDG_SHAPE_FORCE_BLOCKS_PER_SM]
                                                      : (multi ? kMultiMinBlocks : kForceMinBlocks);
 }
-static int density_blocks(const mdg_system* sys, bool multi) {
-    (void)multi;  // the Multi body fits the same budget
-    return sys->shape[MDG_SHAPE_DENSITY_BLOCKS_PER_SM] ? sys->shape[MDG_SHAPE_DENSITY_BLOCKS_PER_SM]
-                                                       : kDensityMinBlocks;
+static int density_blocks(const mdg_system* sys, const PotSet& ps) {
+    if (sys->shape[MDG_SHAPE_DENSITY_BLOCKS_PER_SM]) return sys->shape[MDG_SHAPE_DENSITY_BLOCKS_PER_SM];
+    return ps.multi && ps.nkinds <= 2 ? kMultiMinBlocks : kDensityMinBlocks;
+}
+
+template <int KINDS, bool KICK>
+static void launch_eam(int mb, const FArgs& A, const PotSet* dps, int nb, cudaStream_t st) {
+    if (mb == 3) k_eam_mixed<KINDS, KICK, 3><<<nb, kBlock, 0, st>>>(A, dps);
+    else k_eam_mixed<KINDS, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
 }
 
 template <bool MULTI, bool KICK>
-static void launch_eam_lj(bool eam, int mb, const FArgs& A, const PotSet* dps, int nb, cudaStream_t st) {
-    if (eam) {
-        if (mb == 3) k_eam_mixed<MULTI, KICK, 3><<<nb, kBlock, 0, st>>>(A, dps);
-        else k_eam_mixed<MULTI, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
-    } else {
-        if (mb == 3) k_lj_mixed<MULTI, KICK, 3><<<nb, kBlock, 0, st>>>(A, dps);
-        else k_lj_mixed<MULTI, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
-    }
+static void launch_lj(int mb, const FArgs& A, const PotSet* dps, int nb, cudaStream_t st) {
+    if (mb == 3) k_lj_mixed<MULTI, KICK, 3><<<nb, kBlock, 0, st>>>(A, dps);
+    else k_lj_mixed<MULTI, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
 }
 
-template <bool MULTI>
+template <int KINDS>
 static void launch_density(int mb, const FArgs& A, const PotSet* dps, int nb, cudaStream_t st) {
-    if (mb == 3) k_density_mixed<MULTI, 3><<<nb, kBlock, 0, st>>>(A, dps);
-    else if (mb == 5) k_density_mixed<MULTI, 5><<<nb, kBlock, 0, st>>>(A, dps);
-    else k_density_mixed<MULTI, 4><<<nb, kBlock, 0, st>>>(A, dps);
+    if (mb == 3) k_density_mixed<KINDS, 3><<<nb, kBlock, 0, st>>>(A, dps);
+    else if (mb == 5) k_density_mixed<KINDS, 5><<<nb, kBlock, 0, st>>>(A, dps);
+    else k_density_mixed<KINDS, 4><<<nb, kBlock, 0, st>>>(A, dps);
 }
 
+template <int KINDS>
+static void launch_rec(int mb, const FArgs& A, const PotSet* dps, int nb, cudaStream_t st) {
+    if (mb == 3) k_density_rec<KINDS, 3><<<nb, kBlock, 0, st>>>(A, dps);
+    else if (mb == 5) k_density_rec<KINDS, 5><<<nb, kBlock, 0, st>>>(A, dps);
+    else k_density_rec<KINDS, 4><<<nb, kBlock, 0, st>>>(A, dps);
+}
+
+// Calls f(std::integral_constant<int, KINDS>) for a solver's kinds.
+template <typename F>
+static void with_kinds(const PotSet& ps, F&& f) {
+    if (!ps.multi) f(std::integral_constant<int, 0>());
+    else if (ps.nkinds <= 2) f(std::integral_constant<int, 2>());
+    else f(std::integral_constant<int, 4>());
+}
 
 template <bool MULTI, int FORM, bool KICK>
 __global__ void __launch_bounds__(kBlock, kForceMinBlocks) k_pair_mixed(FArgs A, const PotSet* __restrict__ ps) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < A.n) pair_mixed_one<MULTI, FORM, KICK>(A, ps, i);
 }
+
+// The end of a step's force pass for atom i (k_force_step): the second
+// half-kick, and with `next` the next step's start; its rebuild test.
+__device__ __forceinline__ bool end_step(const FArgs& A, const IArgs& D, int i, bool moved, bool next,
+                                         const float f[3]) {
+    if (!next) {
+        if (moved) store_force<true>(A, i, f[0], f[1], f[2]);
+        return false;
+    }
+    if (moved) return kick_drift_mixed(D, A.gx, A.gy, A.gz, i, f[0], f[1], f[2]);
+    const double r[3] = {D.rx[i], D.ry[i], D.rz[i]};
+    return offsets_check_mixed(D, i, r);
+}
+
+// ---- eight lanes per atom: systems that do not fill the GPU ------------------
+// A block is 256 threads = 32 atoms. The pair loops run with eight lanes per
+// atom (lane_sums: the same sums in the same order as one thread's, so the
+// same bits); the sums meet in shared memory and the block's first warp does
+// the rest, a lane per atom, so that its FP64 instructions carry 32 atoms.
+constexpr int kLaneAtoms = kBlock / 8;
+
+template <typename Group>
+__device__ __forceinline__ int block_forces(const FArgs& A, const PotSet* __restrict__ ps, float f[3]) {
+    __shared__ float sh[kBlock / 32][96];
+    __shared__ float sum[3][kLaneAtoms];
+    const int a = threadIdx.x >> 3, i = blockIdx.x * kLaneAtoms + a;
+    const bool in = i < A.n;
+    lane_forces<Group>(A, ps, in, in ? i : 0, sh[threadIdx.x >> 5], f);
+    if ((threadIdx.x & 7) == 0)
+        for (int k = 0; k < 3; ++k) sum[k][a] = f[k];
+    __syncthreads();
+    if (threadIdx.x >= kLaneAtoms) return -1;
+    for (int k = 0; k < 3; ++k) f[k] = sum[k][threadIdx.x];
+    const int me = blockIdx.x * kLaneAtoms + threadIdx.x;
+    return me < A.n ? me : -1;
+}
+
+// Blocks per SM of the lane kernels: four (64 registers) but for the two-kind
+// bodies, which spill there.
+constexpr int lane_budget(int kinds) { return kinds == 2 ? 3 : 4; }
+
+template <typename Group, bool KICK, int MB>
+__global__ void __launch_bounds__(kBlock, MB) k_lane_forces(FArgs A, const PotSet* __restrict__ ps) {
+    float f[3];
+    const int i = block_forces<Group>(A, ps, f);
+    if (i >= 0 && A.tag[i] != 0) store_force<KICK>(A, i, f[0], f[1], f[2]);
+}
+
+template <int KINDS, bool REC>
+__global__ void __launch_bounds__(kBlock, lane_budget(KINDS)) k_lane_density(FArgs A, const PotSet* __restrict__ ps) {
+    __shared__ float sh[kBlock / 32][32];
+    __shared__ float sum[kLaneAtoms];
+    const int a = threadIdx.x >> 3, i = blockIdx.x * kLaneAtoms + a, w = i < A.n ? i : 0;
+    const bool live = i < A.n && A.tag[w] != 0;
+    float rho[1];
+    RhoGroup<KINDS, REC> grp(A, ps, w);
+    lane_sums<1>(A, live, w, live ? A.ncnt[w] >> 2 : 0, grp, sh[threadIdx.x >> 5], rho);
+    if ((threadIdx.x & 7) == 0) sum[a] = rho[0];
+    __syncthreads();
+    const int me = blockIdx.x * kLaneAtoms + threadIdx.x;
+    if (threadIdx.x < kLaneAtoms && me < A.n)
+        store_density<(KINDS != 0)>(A, ps, me, A.pos32[me], KINDS ? (A.kind[me] & 3) : 0, sum[threadIdx.x]);
+}
+
+// k_force_step with eight lanes per atom.
+template <int KINDS>
+__global__ void __launch_bounds__(kBlock, lane_budget(KINDS))
+    k_lane_force_step(FArgs A, IArgs D, const PotSet* __restrict__ ps, const unsigned long long* __restrict__ left) {
+    const bool next = *left > 1ull && A.st->need_rebuild == 0u;
+    float f[3];
+    const int i = block_forces<EamGroup<KINDS, true>>(A, ps, f);
+    if (threadIdx.x >= kLaneAtoms) return;
+    const bool need = i >= 0 && end_step(A, D, i, A.tag[i] != 0, next, f);
+    if (next) flag_need_next(need, A.st);
+}
+
+// Whether a system's mixed passes take eight lanes per atom: below 45,000
+// atoms with EAM tables, 24,000 without (a pair costs less there). One thread
+// per atom leaves the GPU with fewer than nine warps per SM at 45,000 atoms;
+// eight lanes cost about twice the instructions where it is full. Measured per
+// step, one thread / eight lanes: EAM Cu 4,000 atoms 51.3 / 26.8 us, 32,000
+// 51.4 / 43.3, 62,500 54.9 / 68.9; NiAl 31,094 114 / 79; LJ argon 4,000
+// 36.5 / 26.9, 32,000 41.3 / 41.1; LJ liquid 62,500 54.3 / 61.9.
+static bool lanes_mixed(size_t n, const PotSet& ps) { return n < (ps.any_eam ? 45000u : 24000u); }
+static int lane_blocks(size_t n) { return (int)((n + kLaneAtoms - 1) / kLaneAtoms); }
 
 // ---- Langevin thermostat (langevin.cxx:29-42) ----------------------------------
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11): ten rounds of two
@@ -632,13 +731,32 @@ static int launch_thermostat(mdg_system* sys, const ThermoDev* th, int precision
 }
 
 template <bool KICK>
+static void launch_lane_forces(const FArgs& A, const PotSet* dps, const PotSet& ps, int nb, cudaStream_t st) {
+    const bool multi = ps.multi != 0;
+    if (ps.any_eam) {
+        with_kinds(ps, [&](auto k) {
+            constexpr int K = decltype(k)::value;
+            k_lane_forces<EamGroup<K, false>, KICK, lane_budget(K)><<<nb, kBlock, 0, st>>>(A, dps);
+        });
+    } else if (ps.any_tab || ps.any_ljs) {
+        if (!multi && ps.any_tab) k_lane_forces<PairGroup<false, 3>, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
+        else if (!multi) k_lane_forces<PairGroup<false, 4>, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
+        else k_lane_forces<PairGroup<true, 0>, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
+    } else {
+        if (multi) k_lane_forces<LjGroup<true>, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
+        else k_lane_forces<LjGroup<false>, KICK, 4><<<nb, kBlock, 0, st>>>(A, dps);
+    }
+}
+
+template <bool KICK>
 static void launch_forces_mixed(const mdg_system* sys, const FArgs& A, const PotSet* dps, const PotSet& ps, int nb,
                                 cudaStream_t st) {
     const bool multi = ps.multi != 0;
     const int mb = force_blocks(sys, multi);
-    if (ps.any_eam) {
-        if (multi) launch_eam_lj<true, KICK>(true, mb, A, dps, nb, st);
-        else launch_eam_lj<false, KICK>(true, mb, A, dps, nb, st);
+    if (lanes_mixed(sys->n, ps)) {
+        launch_lane_forces<KICK>(A, dps, ps, lane_blocks(sys->n), st);
+    } else if (ps.any_eam) {
+        with_kinds(ps, [&](auto k) { launch_eam<decltype(k)::value, KICK>(mb, A, dps, nb, st); });
     } else if (ps.any_tab || ps.any_ljs) {
         const int kinds = ps.any_lj + ps.any_tab + ps.any_ljs;
         if (!multi && ps.any_tab) k_pair_mixed<false, 3, KICK><<<nb, kBlock, 0, st>>>(A, dps);
@@ -647,8 +765,8 @@ static void launch_forces_mixed(const mdg_system* sys, const FArgs& A, const Pot
         else if (ps.any_tab) k_pair_mixed<true, 3, KICK><<<nb, kBlock, 0, st>>>(A, dps);
         else k_pair_mixed<true, 4, KICK><<<nb, kBlock, 0, st>>>(A, dps);
     } else {
-        if (multi) launch_eam_lj<true, KICK>(false, mb, A, dps, nb, st);
-        else launch_eam_lj<false, KICK>(false, mb, A, dps, nb, st);
+        if (multi) launch_lj<true, KICK>(mb, A, dps, nb, st);
+        else launch_lj<false, KICK>(mb, A, dps, nb, st);
     }
 }
 
@@ -665,23 +783,16 @@ static void launch_forces_mixed(const mdg_system* sys, const FArgs& A, const Pot
 // neighbours only through the density pass's copies (pos32b, Fp32) and takes
 // each pair's cut decision from the density pass (cutbits), where the
 // unfused pass would settle pairs near the cutoff on the FP64 positions.
-template <bool MULTI, int MB, int NT = kBlock>
+template <int KINDS, int MB, int NT = kBlock>
 __global__ void __launch_bounds__(NT, MB)
     k_force_step(FArgs A, IArgs D, const PotSet* __restrict__ ps, const unsigned long long* __restrict__ left) {
     const bool next = *left > 1ull && A.st->need_rebuild == 0u;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     bool need = false;
     if (i < A.n) {
-        float fx, fy, fz;
-        const bool moved = eam_mixed_force<MULTI, true>(A, ps, i, fx, fy, fz);
-        if (!next) {
-            if (moved) store_force<true>(A, i, fx, fy, fz);
-        } else if (moved) {
-            need = kick_drift_mixed(D, A.gx, A.gy, A.gz, i, fx, fy, fz);
-        } else {
-            const double r[3] = {D.rx[i], D.ry[i], D.rz[i]};
-            need = offsets_check_mixed(D, i, r);
-        }
+        float f[3];
+        const bool moved = thread_forces<EamGroup<KINDS, true>>(A, ps, i, f);
+        need = end_step(A, D, i, moved, next, f);
     }
     if (next) flag_need_next(need, A.st);
 }
@@ -705,15 +816,13 @@ int launch_forces_step(mdg_system* sys, const PotSet* dps, const PotSet& ps, dou
     // 8: eight 128-thread blocks per SM (the 4-block budget in blocks half
     // the size, so the launch's last, partly filled wave is shorter)
     const int nb128 = nblk(sys->n, 128);
-    if (multi) {
-        if (mb == 3) k_force_step<true, 3><<<nb, kBlock, 0, st>>>(A, D, dps, left);
-        else if (mb == 8) k_force_step<true, 8, 128><<<nb128, 128, 0, st>>>(A, D, dps, left);
-        else k_force_step<true, 4><<<nb, kBlock, 0, st>>>(A, D, dps, left);
-    } else {
-        if (mb == 3) k_force_step<false, 3><<<nb, kBlock, 0, st>>>(A, D, dps, left);
-        else if (mb == 8) k_force_step<false, 8, 128><<<nb128, 128, 0, st>>>(A, D, dps, left);
-        else k_force_step<false, 4><<<nb, kBlock, 0, st>>>(A, D, dps, left);
-    }
+    with_kinds(ps, [&](auto k) {
+        constexpr int K = decltype(k)::value;
+        if (lanes_mixed(sys->n, ps)) k_lane_force_step<K><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, D, dps, left);
+        else if (mb == 3) k_force_step<K, 3><<<nb, kBlock, 0, st>>>(A, D, dps, left);
+        else if (mb == 8) k_force_step<K, 8, 128><<<nb128, 128, 0, st>>>(A, D, dps, left);
+        else k_force_step<K, 4><<<nb, kBlock, 0, st>>>(A, D, dps, left);
+    });
     MDG_LAUNCHED(ctx);
     return MDG_OK;
 }
@@ -731,16 +840,12 @@ int launch_density_rec(mdg_system* sys, const PotSet* dps, const PotSet& ps) {
     const int nb = nblk(sys->n);
     cudaStream_t st = sys->ctx->stream;
     const bool multi = ps.multi != 0;
-    const int mb = density_blocks(sys, multi);
-    if (multi) {
-        if (mb == 3) k_density_rec<true, 3><<<nb, kBlock, 0, st>>>(A, dps);
-        else if (mb == 5) k_density_rec<true, 5><<<nb, kBlock, 0, st>>>(A, dps);
-        else k_density_rec<true, 4><<<nb, kBlock, 0, st>>>(A, dps);
-    } else {
-        if (mb == 3) k_density_rec<false, 3><<<nb, kBlock, 0, st>>>(A, dps);
-        else if (mb == 5) k_density_rec<false, 5><<<nb, kBlock, 0, st>>>(A, dps);
-        else k_density_rec<false, 4><<<nb, kBlock, 0, st>>>(A, dps);
-    }
+    const int mb = density_blocks(sys, ps);
+    with_kinds(ps, [&](auto k) {
+        constexpr int K = decltype(k)::value;
+        if (lanes_mixed(sys->n, ps)) k_lane_density<K, true><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, dps);
+        else launch_rec<K>(mb, A, dps, nb, st);
+    });
     MDG_LAUNCHED(sys->ctx);
     sys->fp_ok = 0;  // nc rewritten (FP32 sums); Fp64 no longer matches it
     return MDG_OK;
@@ -786,8 +891,11 @@ int launch_stage(mdg_system* sys, const PotSet* dps, const PotSet& ps, int preci
         }
     } else {
         if (stage == 0) {
-            if (multi) launch_density<true>(density_blocks(sys, true), A, dps, nb, st);
-            else launch_density<false>(density_blocks(sys, false), A, dps, nb, st);
+            with_kinds(ps, [&](auto k) {
+                constexpr int K = decltype(k)::value;
+                if (lanes_mixed(sys->n, ps)) k_lane_density<K, false><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, dps);
+                else launch_density<K>(density_blocks(sys, ps), A, dps, nb, st);
+            });
             sys->fp_ok = 0;  // nc rewritten (FP32 sums); Fp64 no longer matches it
         } else if (kick_dt > 0.0 && !th) {
             A.kick_hdt = 0.5f * (float)kick_dt;

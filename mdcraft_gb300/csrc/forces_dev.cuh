@@ -70,17 +70,6 @@ __device__ __forceinline__ void store_force(const FArgs& A, int i, float fx, flo
 // ---------------------------------------------------------------------------
 // mixed precision
 // ---------------------------------------------------------------------------
-struct Kahan3 {
-    float s[3] = {0.f, 0.f, 0.f};
-    float c[3] = {0.f, 0.f, 0.f};
-    __device__ __forceinline__ void add(int k, float v) {
-        float y = v - c[k];
-        float t = s[k] + y;
-        c[k] = (t - s[k]) - y;
-        s[k] = t;
-    }
-};
-
 __device__ __forceinline__ float ksum_add(float& s, float& c, float v) {
     float y = v - c;
     float t = s + y;
@@ -148,21 +137,24 @@ __device__ __forceinline__ bool cut_in(const FArgs& A, int i, uint32_t j, float 
 // Cutoff membership from the FP32 r^2, with the rare pairs inside the
 // 1e-5 band around rc^2 (and entries that crossed a periodic face when the
 // solver has no Periodic boundary) settled exactly.
-__device__ __forceinline__ bool pair_in(const FArgs& A, int i, uint32_t e, float r2, float r2c, double R2c,
+// (R2c() gives the FP64 cutoff, read only for those).
+template <typename Cut>
+__device__ __forceinline__ bool pair_in(const FArgs& A, int i, uint32_t e, float r2, float r2c, Cut&& R2c,
                                         bool per) {
     bool in = r2 >= 1e-15f && r2 <= r2c;
-    if (fabsf(r2 - r2c) <= 1e-5f * r2c) in = cut_in(A, i, e & kJMask, r2, r2c, R2c);
+    if (fabsf(r2 - r2c) <= 1e-5f * r2c) in = cut_in(A, i, e & kJMask, r2, r2c, R2c());
     return in && (per || !(e & kWrapBit));
 }
 
 // pair_in for the density pass of a step whose force pass moves atoms: the
 // FP64 decisions of the band pairs (entry k of atom i) are also collected in
 // *bits, one bit per entry, and *band notes that the word has one.
-__device__ __forceinline__ bool pair_in_rec(const FArgs& A, int i, uint32_t e, float r2, float r2c, double R2c,
+template <typename Cut>
+__device__ __forceinline__ bool pair_in_rec(const FArgs& A, int i, uint32_t e, float r2, float r2c, Cut&& R2c,
                                             bool per, int k, uint32_t* bits, bool* band) {
     bool in = r2 >= 1e-15f && r2 <= r2c;
     if (fabsf(r2 - r2c) <= 1e-5f * r2c) {
-        in = cut_in(A, i, e & kJMask, r2, r2c, R2c);
+        in = cut_in(A, i, e & kJMask, r2, r2c, R2c());
         *bits |= (uint32_t)in << (k & 31);
         *band = true;
     }
@@ -181,27 +173,97 @@ __device__ __forceinline__ bool pair_in_bits(const FArgs& A, int i, uint32_t e, 
 
 // The pair loops below read four list entries with one 16-byte load, then
 // the four neighbour records, so the loads of a group overlap; the four
-// contributions are summed in FP32 and the group sum enters a Kahan sum.
+// contributions are summed in FP32 and the group sum enters a Kahan sum, in
+// the order of the groups. A body's state and its group are a struct
+// (LjGroup, PairGroup, RhoGroup, EamGroup), walked by one thread per atom
+// (group_sums) or by eight lanes per atom (lane_sums); both add the same
+// group sums in the same order, so they give the same bits.
 
-template <bool MULTI>
-__device__ __forceinline__ bool lj_mixed_force(const FArgs& A, const PotSet* __restrict__ ps, int i, float& out_x,
-                                             float& out_y, float& out_z) {
-    if (A.tag[i] == 0) return false;
-    const int4 pi = A.pos32[i];
-    const int ng = A.ncnt[i] >> 2;
-    const int ki = MULTI ? (A.kind[i] & 3) : 0;
-    const bool per = ps->periodic;
-    const float uf[3] = {A.uf[0], A.uf[1], A.uf[2]};
-    const PotParams& P0 = ps->p[ki][0];
-    float r2c = P0.r2cut_f, l1 = P0.lj1_f, l2 = P0.lj2_f, mh = P0.mhf_f;
-    double R2c = P0.R2cut;
-    Kahan3 acc;
+// One thread per atom: the sums of NC components over the atom's groups.
+template <int NC, typename Group>
+__device__ __forceinline__ void group_sums(const FArgs& A, int i, int ng, Group& grp, float out[NC]) {
+    float s[NC], c[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) s[k] = c[k] = 0.f;
     const uint4* row = reinterpret_cast<const uint4*>(A.nbr) + i;
     uint4 e4n = ng > 0 ? ldg_list(row) : make_uint4(0, 0, 0, 0);
     for (int g = 0; g < ng; ++g) {
         // the next group's entries are requested before this group's work
         const uint4 e4 = e4n;
         if (g + 1 < ng) e4n = ldg_list(row + (size_t)(g + 1) * A.np);
+        float f[NC];
+        grp(A, i, g, e4, f);
+#pragma unroll
+        for (int k = 0; k < NC; ++k) ksum_add(s[k], c[k], f[k]);
+        grp.word(A, i, g, ng);
+    }
+#pragma unroll
+    for (int k = 0; k < NC; ++k) out[k] = s[k];
+}
+
+// Eight lanes per atom (lane = threadIdx.x & 7; `live` false: no atom): lane l
+// evaluates groups l, l + 8, ...; after each round of eight groups lane k adds
+// the eight sums of component k in group order (through sh, 32 NC floats per
+// warp). Every lane of the warp calls this; out is the atom's sums, on all
+// eight lanes. A group's sums take about 120 instructions and the ordered
+// additions 4 a group and component, so the eight lanes run about six times
+// as fast as one where the GPU is not full.
+template <int NC, typename Group>
+__device__ __forceinline__ void lane_sums(const FArgs& A, bool live, int i, int ng, Group& grp, float* sh,
+                                          float out[NC]) {
+    const int lane = threadIdx.x & 31, sub = lane & 7;
+    if (!live) ng = 0;
+    const uint4* row = reinterpret_cast<const uint4*>(A.nbr) + i;
+    const int rounds = (__reduce_max_sync(0xffffffffu, (unsigned)ng) + 7) >> 3;
+    uint4 e4n = sub < ng ? ldg_list(row + (size_t)sub * A.np) : make_uint4(0, 0, 0, 0);
+    float s = 0.f, c = 0.f;  // component `sub` of this lane's atom
+    for (int r = 0; r < rounds; ++r) {
+        const int g = 8 * r + sub;
+        const uint4 e4 = e4n;
+        if (g + 8 < ng) e4n = ldg_list(row + (size_t)(g + 8) * A.np);
+        float f[NC];
+#pragma unroll
+        for (int k = 0; k < NC; ++k) f[k] = 0.f;
+        if (g < ng) grp(A, i, g, e4, f);
+        grp.word8(A, i, r, g < ng);
+#pragma unroll
+        for (int k = 0; k < NC; ++k) sh[32 * k + lane] = f[k];
+        __syncwarp();
+        const float4* col = reinterpret_cast<const float4*>(sh + 32 * (sub < NC ? sub : 0) + (lane & ~7));
+        const float4 lo = col[0], hi = col[1];
+        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (8 * r + q < ng) ksum_add(s, c, v[q]);
+        __syncwarp();
+    }
+#pragma unroll
+    for (int k = 0; k < NC; ++k) out[k] = __shfl_sync(0xffffffffu, s, (lane & ~7) + k);
+}
+
+template <bool MULTI>
+struct LjGroup {
+    const PotSet* ps;
+    int4 pi;
+    int ki;
+    bool per;
+    float uf[3], r2c, l1, l2, mh;
+    double R2c;
+
+    __device__ __forceinline__ LjGroup(const FArgs& A, const PotSet* __restrict__ p, int i) : ps(p) {
+        pi = A.pos32[i];
+        ki = MULTI ? (A.kind[i] & 3) : 0;
+        per = ps->periodic;
+        for (int a = 0; a < 3; ++a) uf[a] = A.uf[a];
+        if (MULTI) return;
+        const PotParams& P0 = ps->p[ki][0];
+        r2c = P0.r2cut_f;
+        l1 = P0.lj1_f;
+        l2 = P0.lj2_f;
+        mh = P0.mhf_f;
+        R2c = P0.R2cut;
+    }
+    __device__ __forceinline__ void operator()(const FArgs& A, int i, int, const uint4& e4, float f[3]) {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
@@ -209,14 +271,13 @@ __device__ __forceinline__ bool lj_mixed_force(const FArgs& A, const PotSet* __r
         float fx = 0.f, fy = 0.f, fz = 0.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            if (MULTI) {
-                const PotParams& P = ps->p[ki][pj[q].w & 3];
-                r2c = P.r2cut_f; l1 = P.lj1_f; l2 = P.lj2_f; mh = P.mhf_f; R2c = P.R2cut;
-            }
+            const PotParams* P = MULTI ? &ps->p[ki][pj[q].w & 3] : nullptr;
+            const float r2c = MULTI ? P->r2cut_f : this->r2c, l1 = MULTI ? P->lj1_f : this->l1;
+            const float l2 = MULTI ? P->lj2_f : this->l2, mh = MULTI ? P->mhf_f : this->mh;
             float dx, dy, dz;
             pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
             float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            bool in = pair_in(A, i, e[q], r2, r2c, R2c, per);
+            bool in = pair_in(A, i, e[q], r2, r2c, [&] { return MULTI ? P->R2cut : this->R2c; }, per);
             float r2inv = __fdividef(1.0f, fmaxf(r2, 1e-12f));
             float r6inv = r2inv * r2inv * r2inv;
             float pref = in ? mh * fmaf(l1, r6inv, -l2) * r6inv * r2inv : 0.f;
@@ -224,20 +285,37 @@ __device__ __forceinline__ bool lj_mixed_force(const FArgs& A, const PotSet* __r
             fy = fmaf(dy, pref, fy);
             fz = fmaf(dz, pref, fz);
         }
-        acc.add(0, fx);
-        acc.add(1, fy);
-        acc.add(2, fz);
+        f[0] = fx;
+        f[1] = fy;
+        f[2] = fz;
     }
-    out_x = acc.s[0];
-    out_y = acc.s[1];
-    out_z = acc.s[2];
+    __device__ __forceinline__ void word(const FArgs&, int, int, int) {}
+    __device__ __forceinline__ void word8(const FArgs&, int, int, bool) {}
+};
+
+// The forces of atom i by a thread of its own; false for an atom with tag 0.
+template <typename Group>
+__device__ __forceinline__ bool thread_forces(const FArgs& A, const PotSet* __restrict__ ps, int i, float f[3]) {
+    if (A.tag[i] == 0) return false;
+    Group grp(A, ps, i);
+    group_sums<3>(A, i, A.ncnt[i] >> 2, grp, f);
     return true;
+}
+
+// By eight lanes (every lane of the warp calls this; i < n where `in`).
+template <typename Group>
+__device__ __forceinline__ bool lane_forces(const FArgs& A, const PotSet* __restrict__ ps, bool in, int i, float* sh,
+                                            float f[3]) {
+    const bool live = in && A.tag[i] != 0;
+    Group grp(A, ps, i);
+    lane_sums<3>(A, live, i, live ? A.ncnt[i] >> 2 : 0, grp, sh, f);
+    return live;
 }
 
 template <bool MULTI, bool KICK = false>
 __device__ __forceinline__ void lj_mixed_one(const FArgs& A, const PotSet* __restrict__ ps, int i) {
-    float fx, fy, fz;
-    if (lj_mixed_force<MULTI>(A, ps, i, fx, fy, fz)) store_force<KICK>(A, i, fx, fy, fz);
+    float f[3];
+    if (thread_forces<LjGroup<MULTI>>(A, ps, i, f)) store_force<KICK>(A, i, f[0], f[1], f[2]);
 }
 
 // Force / r of a tabulated Pair term (pair.cxx:316-346) in FP32 from the
@@ -279,20 +357,20 @@ __device__ __forceinline__ float analytic_ff32(const PotParams& P, float r2) {
 // every pair a tabulated Pair, 4 = every pair LJs, 0 = chosen per kind pair
 // among LJsCut, Pair and LJs.
 template <bool MULTI, int FORM>
-__device__ __forceinline__ bool pair_mixed_force(const FArgs& A, const PotSet* __restrict__ ps, int i, float& out_x,
-                                             float& out_y, float& out_z) {
-    if (A.tag[i] == 0) return false;
-    const int4 pi = A.pos32[i];
-    const int ng = A.ncnt[i] >> 2;
-    const int ki = MULTI ? (A.kind[i] & 3) : 0;
-    const bool per = ps->periodic;
-    const float uf[3] = {A.uf[0], A.uf[1], A.uf[2]};
-    Kahan3 acc;
-    const uint4* row = reinterpret_cast<const uint4*>(A.nbr) + i;
-    uint4 e4n = ng > 0 ? ldg_list(row) : make_uint4(0, 0, 0, 0);
-    for (int g = 0; g < ng; ++g) {
-        const uint4 e4 = e4n;
-        if (g + 1 < ng) e4n = ldg_list(row + (size_t)(g + 1) * A.np);
+struct PairGroup {
+    const PotSet* ps;
+    int4 pi;
+    int ki;
+    bool per;
+    float uf[3];
+
+    __device__ __forceinline__ PairGroup(const FArgs& A, const PotSet* __restrict__ p, int i) : ps(p) {
+        pi = A.pos32[i];
+        ki = MULTI ? (A.kind[i] & 3) : 0;
+        per = ps->periodic;
+        for (int a = 0; a < 3; ++a) uf[a] = A.uf[a];
+    }
+    __device__ __forceinline__ void operator()(const FArgs& A, int i, int, const uint4& e4, float f[3]) {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
@@ -304,7 +382,7 @@ __device__ __forceinline__ bool pair_mixed_force(const FArgs& A, const PotSet* _
             float dx, dy, dz;
             pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
             const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            bool in = pair_in(A, i, e[q], r2, P.r2cut_f, P.R2cut, per);
+            bool in = pair_in(A, i, e[q], r2, P.r2cut_f, [&] { return P.R2cut; }, per);
             float FF;
             if (FORM == 3 || (FORM == 0 && P.type == POT_TAB)) {
                 FF = tab_ff32(P, r2, in);
@@ -319,20 +397,18 @@ __device__ __forceinline__ bool pair_mixed_force(const FArgs& A, const PotSet* _
             fy = fmaf(dy, FF, fy);
             fz = fmaf(dz, FF, fz);
         }
-        acc.add(0, fx);
-        acc.add(1, fy);
-        acc.add(2, fz);
+        f[0] = fx;
+        f[1] = fy;
+        f[2] = fz;
     }
-    out_x = acc.s[0];
-    out_y = acc.s[1];
-    out_z = acc.s[2];
-    return true;
-}
+    __device__ __forceinline__ void word(const FArgs&, int, int, int) {}
+    __device__ __forceinline__ void word8(const FArgs&, int, int, bool) {}
+};
 
 template <bool MULTI, int FORM, bool KICK = false>
 __device__ __forceinline__ void pair_mixed_one(const FArgs& A, const PotSet* __restrict__ ps, int i) {
-    float fx, fy, fz;
-    if (pair_mixed_force<MULTI, FORM>(A, ps, i, fx, fy, fz)) store_force<KICK>(A, i, fx, fy, fz);
+    float f[3];
+    if (thread_forces<PairGroup<MULTI, FORM>>(A, ps, i, f)) store_force<KICK>(A, i, f[0], f[1], f[2]);
 }
 
 __device__ __forceinline__ void embed32(const PotParams& P, float rho, float* F, float* dF,
@@ -349,68 +425,141 @@ __device__ __forceinline__ void embed32(const PotParams& P, float rho, float* F,
     *dF = dcubic(c, u) * P.inv_drh_f;
 }
 
-// REC: also record the FP64 decisions of the band pairs in A.cutbits, for a
-// force pass that moves atoms (pair_in_rec).
-template <bool MULTI, bool REC = false>
-__device__ __forceinline__ void density_mixed_one(const FArgs& A, const PotSet* __restrict__ ps, int i) {
-    const int4 pi = A.pos32[i];
-    const int ki = MULTI ? (A.kind[i] & 3) : 0;
-    const float uf[3] = {A.uf[0], A.uf[1], A.uf[2]};
-    const bool per = ps->periodic;
-    float s = 0.f, c = 0.f;
-    if (A.tag[i] != 0) {
-        const int ng = A.ncnt[i] >> 2;
-        const PotParams* P = &ps->p[ki][0];
-        float r2c = P->r2cut_f, idr = P->inv_dr_f;
-        double R2c = P->R2cut;
-        int Nr1 = P->Nr1;
-        const float4* tab = P->rho_c;
-        const uint4* row = reinterpret_cast<const uint4*>(A.nbr) + i;
-        uint4 e4n = ng > 0 ? ldg_list(row) : make_uint4(0, 0, 0, 0);
-        uint32_t bits = 0;   // FP64 cut decisions of this word's band entries, for A.cutbits
-        bool band = false;  // the word has a band entry
-        for (int g = 0; g < ng; ++g) {
-            // the next group's entries are requested before this group's work
-            const uint4 e4 = e4n;
-            if (g + 1 < ng) e4n = ldg_list(row + (size_t)(g + 1) * A.np);
-            const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
-            int4 pj[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) pj[q] = __ldg(A.pos32 + (e[q] & kJMask));
-            float part = 0.f;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                bool eam = true;
-                if (MULTI) {
-                    P = &ps->p[ki][pj[q].w & 3];  // the partner's kind rides in its offsets' w
-                    r2c = P->r2cut_f; idr = P->inv_dr_f; Nr1 = P->Nr1; tab = P->rho_c; R2c = P->R2cut;
-                    eam = P->type == 2;
-                }
-                float dx, dy, dz;
-                pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
-                float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                bool in;
-                if (REC)  // every pair's band decision, whatever its potential
-                    in = pair_in_rec(A, i, e[q], r2, r2c, R2c, per, 4 * g + q, &bits, &band) && eam;
-                else
-                    in = eam && pair_in(A, i, e[q], r2, r2c, R2c, per);
-                float t = r2 * rsqrt_nr(fmaxf(r2, 1e-12f)) * idr;
-                int nn = (int)t;
-                in = in && nn < Nr1;
-                nn = in ? nn : 0;
-                float u = t - (float)nn;
-                float v = in ? cubic(__ldg(tab + nn), u) : 0.f;
-                part += v;
-            }
-            ksum_add(s, c, part);
-            if (REC && ((g & 7) == 7 || g + 1 == ng)) {
-                if (band) A.cutbits[(size_t)(g >> 3) * A.np + i] = bits;
-                bits = 0;
-                band = false;
+// What the EAM passes need of a pair's potential, by the partner's kind.
+// KINDS = 0: Single (read once per atom); 2: two kinds, both read once per
+// atom and selected per pair; 4: read from the PotSet per pair. (The Multi
+// passes are bound by L1 as well, and the five reads per pair took as many
+// wavefronts as the pair's own gathers: NiAl B2 1M force pass 0.687 ->
+// 0.551 ms, density 0.421 -> 0.355 ms.)
+struct PairPot {
+    float r2c, idr;
+    int Nr1;
+    const float4* tab;
+    bool eam, lj;
+};
+template <int KINDS, bool FORCE>
+struct KindPots {
+    float r2c[2], idr[2];
+    int Nr1[2];
+    const float4* tab[2];
+    unsigned eam, lj;  // bit per kind
+
+    static __device__ __forceinline__ const float4* table(const PotParams& P) { return FORCE ? P.rv_c : P.rho_c; }
+    // a tabulated Pair has zero rho rows: the EAM force arithmetic reduces to
+    // its pair term exactly
+    static __device__ __forceinline__ bool is_eam(int type) {
+        return type == POT_EAM || (FORCE && type == POT_TAB);
+    }
+    static __device__ __forceinline__ bool is_lj(int type) {
+        return FORCE && (type == POT_LJCUT || type == POT_LJS);
+    }
+    __device__ __forceinline__ void set(const PotSet* ps, int ki) {
+        eam = lj = 0;
+        if (KINDS == 4) return;
+        for (int b = 0; b < (KINDS ? 2 : 1); ++b) {
+            const PotParams& P = ps->p[KINDS ? ki : 0][b];
+            r2c[b] = P.r2cut_f;
+            idr[b] = P.inv_dr_f;
+            Nr1[b] = P.Nr1;
+            tab[b] = table(P);
+            if (KINDS) {
+                eam |= is_eam(P.type) ? 1u << b : 0u;
+                lj |= is_lj(P.type) ? 1u << b : 0u;
             }
         }
     }
-    float rho = s;
+    __device__ __forceinline__ PairPot get(const PotSet* ps, int ki, int kj) const {
+        if (KINDS == 4) {
+            const PotParams& P = ps->p[ki][kj];
+            return PairPot{P.r2cut_f, P.inv_dr_f, P.Nr1, table(P), is_eam(P.type), is_lj(P.type)};
+        }
+        if (KINDS == 2) {
+            const bool one = kj & 1;  // a kind beyond the two has no potential (its bits are clear)
+            return PairPot{one ? r2c[1] : r2c[0], one ? idr[1] : idr[0], one ? Nr1[1] : Nr1[0],
+                           one ? tab[1] : tab[0], ((eam >> kj) & 1u) != 0u, FORCE && ((lj >> kj) & 1u) != 0u};
+        }
+        return PairPot{r2c[0], idr[0], Nr1[0], tab[0], true, false};
+    }
+};
+
+// REC: also record the FP64 decisions of the band pairs in A.cutbits, for a
+// force pass that moves atoms (pair_in_rec): one bit per entry, a word of 32
+// stored when it has a band pair.
+template <int KINDS, bool REC>
+struct RhoGroup {
+    static constexpr bool MULTI = KINDS != 0;
+    const PotSet* ps;
+    int4 pi;
+    int ki;
+    bool per, band = false;
+    float uf[3];
+    KindPots<KINDS, false> pots;
+    uint32_t bits = 0;  // FP64 cut decisions of this word's band entries
+
+    __device__ __forceinline__ RhoGroup(const FArgs& A, const PotSet* __restrict__ p, int i) : ps(p) {
+        pi = A.pos32[i];
+        ki = MULTI ? (A.kind[i] & 3) : 0;
+        per = ps->periodic;
+        for (int a = 0; a < 3; ++a) uf[a] = A.uf[a];
+        pots.set(ps, ki);
+    }
+    __device__ __forceinline__ void operator()(const FArgs& A, int i, int g, const uint4& e4, float f[1]) {
+        const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
+        int4 pj[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) pj[q] = __ldg(A.pos32 + (e[q] & kJMask));
+        float part = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int kj = MULTI ? pj[q].w & 3 : 0;  // the partner's kind rides in its offsets' w
+            const PairPot P = pots.get(ps, ki, kj);
+            auto R2c = [&] { return ps->p[ki][kj].R2cut; };
+            float dx, dy, dz;
+            pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
+            float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            bool in;
+            if (REC)  // every pair's band decision, whatever its potential
+                in = pair_in_rec(A, i, e[q], r2, P.r2c, R2c, per, 4 * g + q, &bits, &band) && P.eam;
+            else
+                in = P.eam && pair_in(A, i, e[q], r2, P.r2c, R2c, per);
+            float t = r2 * rsqrt_nr(fmaxf(r2, 1e-12f)) * P.idr;
+            int nn = (int)t;
+            in = in && nn < P.Nr1;
+            nn = in ? nn : 0;
+            float u = t - (float)nn;
+            float v = in ? cubic(__ldg(P.tab + nn), u) : 0.f;
+            part += v;
+        }
+        f[0] = part;
+    }
+    __device__ __forceinline__ void word(const FArgs& A, int i, int g, int ng) {
+        if (REC && ((g & 7) == 7 || g + 1 == ng)) {
+            if (band) A.cutbits[(size_t)(g >> 3) * A.np + i] = bits;
+            bits = 0;
+            band = false;
+        }
+    }
+    // eight lanes hold the word of round r
+    __device__ __forceinline__ void word8(const FArgs& A, int i, int r, bool) {
+        if (REC && __any_sync(0xffffffffu, band)) {
+            unsigned any = band;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                bits |= __shfl_xor_sync(0xffffffffu, bits, o);
+                any |= __shfl_xor_sync(0xffffffffu, any, o);
+            }
+            if (any && (threadIdx.x & 7) == 0) A.cutbits[(size_t)r * A.np + i] = bits;
+            bits = 0;
+            band = false;
+        }
+    }
+};
+
+// The atom's density rho from its sum, F'(rho) for its partners' kinds, and
+// the record the force pass gathers.
+template <bool MULTI>
+__device__ __forceinline__ void store_density(const FArgs& A, const PotSet* __restrict__ ps, int i, const int4& pi,
+                                              int ki, float rho) {
     // the atom's density as the reference's charge stage leaves it (FP32 sum here)
     if (A.tag[i] != 0) A.nc[i] = (double)rho;
     float Fp0 = 0.f;
@@ -427,41 +576,46 @@ __device__ __forceinline__ void density_mixed_one(const FArgs& A, const PotSet* 
     A.pos32b[i] = make_int4(pi.x, pi.y, pi.z, w);
 }
 
+template <int KINDS, bool REC = false>
+__device__ __forceinline__ void density_mixed_one(const FArgs& A, const PotSet* __restrict__ ps, int i) {
+    float rho[1] = {0.f};
+    RhoGroup<KINDS, REC> grp(A, ps, i);
+    if (A.tag[i] != 0) group_sums<1>(A, i, A.ncnt[i] >> 2, grp, rho);
+    store_density<(KINDS != 0)>(A, ps, i, grp.pi, grp.ki, rho[0]);
+}
+
 // BITS: a pair in the 1e-5 band around the cutoff takes the density pass's
 // FP64 decision (A.cutbits) rather than testing the FP64 positions itself;
 // the force pass then reads no FP64 position of a neighbour (what a force
 // pass that moves its atoms needs).
-template <bool MULTI, bool BITS = false>
-__device__ __forceinline__ bool eam_mixed_force(const FArgs& A, const PotSet* __restrict__ ps, int i, float& out_x,
-                                             float& out_y, float& out_z) {
-    if (A.tag[i] == 0) return false;
-    const int4 pi = A.pos32b[i];
-    const int ng = A.ncnt[i] >> 2;
-    const int ki = MULTI ? (A.kind[i] & 3) : 0;
-    const float uf[3] = {A.uf[0], A.uf[1], A.uf[2]};
-    const bool per = ps->periodic;
-    const PotParams* P = &ps->p[ki][0];
-    float r2c = P->r2cut_f, idr = P->inv_dr_f;
-    double R2c = P->R2cut;
-    int Nr1 = P->Nr1;
-    const float4* rv = P->rv_c;
-    Kahan3 acc;
+template <int KINDS, bool BITS>
+struct EamGroup {
+    static constexpr bool MULTI = KINDS != 0;
+    const PotSet* ps;
+    int4 pi;
+    int ki;
+    bool per;
+    float uf[3];
+    KindPots<KINDS, true> pots;
     // Multi: F' of atom i for the kinds 1..3 of its partners, read once (the
     // density pass's Fp32 rows; kind 0's is the record's w, with the atom's
     // kind in its two lowest bits)
     float fpi1 = 0.f, fpi2 = 0.f, fpi3 = 0.f;
-    if (MULTI) {
-        const int nk = ps->nkinds;
-        if (nk > 1) fpi1 = A.Fp32[A.np + i];
-        if (nk > 2) fpi2 = A.Fp32[2 * (size_t)A.np + i];
-        if (nk > 3) fpi3 = A.Fp32[3 * (size_t)A.np + i];
+
+    __device__ __forceinline__ EamGroup(const FArgs& A, const PotSet* __restrict__ p, int i) : ps(p) {
+        pi = A.pos32b[i];
+        ki = MULTI ? (A.kind[i] & 3) : 0;
+        per = ps->periodic;
+        for (int a = 0; a < 3; ++a) uf[a] = A.uf[a];
+        pots.set(ps, ki);
+        if (MULTI) {
+            const int nk = ps->nkinds;
+            if (nk > 1) fpi1 = A.Fp32[A.np + i];
+            if (KINDS == 4 && nk > 2) fpi2 = A.Fp32[2 * (size_t)A.np + i];
+            if (KINDS == 4 && nk > 3) fpi3 = A.Fp32[3 * (size_t)A.np + i];
+        }
     }
-    const uint4* row = reinterpret_cast<const uint4*>(A.nbr) + i;
-    uint4 e4n = ng > 0 ? ldg_list(row) : make_uint4(0, 0, 0, 0);
-    for (int g = 0; g < ng; ++g) {
-        // the next group's entries are requested before this group's work
-        const uint4 e4 = e4n;
-        if (g + 1 < ng) e4n = ldg_list(row + (size_t)(g + 1) * A.np);
+    __device__ __forceinline__ void operator()(const FArgs& A, int i, int g, const uint4& e4, float f[3]) {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
@@ -470,60 +624,54 @@ __device__ __forceinline__ bool eam_mixed_force(const FArgs& A, const PotSet* __
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             float Fpi = __int_as_float(MULTI ? pi.w & ~3 : pi.w), Fpj = __int_as_float(MULTI ? pj[q].w & ~3 : pj[q].w);
-            bool eam = true, lj = false;
+            const int kj = MULTI ? pj[q].w & 3 : 0;
+            const PairPot P = pots.get(ps, ki, kj);
             if (MULTI) {
-                uint32_t j = e[q] & kJMask;
-                const int kj = pj[q].w & 3;
-                P = &ps->p[ki][kj];
-                // a tabulated Pair has zero rho rows: the EAM arithmetic
-                // below reduces to its pair term exactly
-                eam = P->type == POT_EAM || P->type == POT_TAB;
-                lj = P->type == POT_LJCUT || P->type == POT_LJS;
-                r2c = P->r2cut_f; idr = P->inv_dr_f; Nr1 = P->Nr1; rv = P->rv_c; R2c = P->R2cut;
                 // j's F' for i's kind (kind 0's is in j's record)
-                if (ki != 0) Fpj = A.Fp32[(size_t)ki * A.np + j];
-                Fpi = kj == 0 ? Fpi : kj == 1 ? fpi1 : kj == 2 ? fpi2 : fpi3;
+                if (ki != 0) Fpj = A.Fp32[(size_t)ki * A.np + (e[q] & kJMask)];
+                Fpi = kj == 0 ? Fpi : KINDS == 2 || kj == 1 ? fpi1 : kj == 2 ? fpi2 : fpi3;
             }
             float dx, dy, dz;
             pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
             float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             bool in;
-            if (BITS) in = (eam || lj) && pair_in_bits(A, i, e[q], r2, r2c, per, 4 * g + q);
-            else in = (eam || lj) && pair_in(A, i, e[q], r2, r2c, R2c, per);
+            if (BITS)
+                in = (P.eam || P.lj) && pair_in_bits(A, i, e[q], r2, P.r2c, per, 4 * g + q);
+            else
+                in = (P.eam || P.lj) &&
+                     pair_in(A, i, e[q], r2, P.r2c, [&] { return ps->p[ki][kj].R2cut; }, per);
             // one reciprocal square root gives both r and 1/r
             float rinv = rsqrt_nr(fmaxf(r2, 1e-12f));
             float r = r2 * rinv;
-            float t = r * idr;
+            float t = r * P.idr;
             int nn = (int)t;
-            in = in && (lj || nn < Nr1);
-            nn = in && !lj ? nn : 0;
+            in = in && (P.lj || nn < P.Nr1);
+            nn = in && !P.lj ? nn : 0;
             float u = t - (float)nn;
             float4 cw, cd;
-            load_rv(rv, nn, cw, cd);
+            load_rv(P.tab, nn, cw, cd);
             // W = V'r - V and D = rho' on the interval (force_rows)
             const float W = cubic(cw, u);
             const float D = fmaf(u, fmaf(u, cd.z, cd.y), cd.x);
             float FF = fmaf(Fpi + Fpj, D, W * (rinv * rinv)) * rinv;
-            if (MULTI && lj) FF = analytic_ff32(*P, r2);
+            if (MULTI && P.lj) FF = analytic_ff32(ps->p[ki][kj], r2);
             FF = in ? FF : 0.f;
             fx = fmaf(FF, dx, fx);
             fy = fmaf(FF, dy, fy);
             fz = fmaf(FF, dz, fz);
         }
-        acc.add(0, fx);
-        acc.add(1, fy);
-        acc.add(2, fz);
+        f[0] = fx;
+        f[1] = fy;
+        f[2] = fz;
     }
-    out_x = acc.s[0];
-    out_y = acc.s[1];
-    out_z = acc.s[2];
-    return true;
-}
+    __device__ __forceinline__ void word(const FArgs&, int, int, int) {}
+    __device__ __forceinline__ void word8(const FArgs&, int, int, bool) {}
+};
 
-template <bool MULTI, bool KICK = false>
+template <int KINDS, bool KICK = false>
 __device__ __forceinline__ void eam_mixed_one(const FArgs& A, const PotSet* __restrict__ ps, int i) {
-    float fx, fy, fz;
-    if (eam_mixed_force<MULTI>(A, ps, i, fx, fy, fz)) store_force<KICK>(A, i, fx, fy, fz);
+    float f[3];
+    if (thread_forces<EamGroup<KINDS, false>>(A, ps, i, f)) store_force<KICK>(A, i, f[0], f[1], f[2]);
 }
 
 }  // namespace mdg

@@ -275,9 +275,9 @@ template <bool EAM, bool KICK, int NT>
 __device__ __forceinline__ void solo_stages(const SoloArgs& S) {
     const int t = threadIdx.x, n = S.n;
     if (EAM) {
-        for (int i = t; i < n; i += NT) density_mixed_one<false>(S.F, S.ps, i);
+        for (int i = t; i < n; i += NT) density_mixed_one<0>(S.F, S.ps, i);
         __syncthreads();
-        for (int i = t; i < n; i += NT) eam_mixed_one<false, KICK>(S.F, S.ps, i);
+        for (int i = t; i < n; i += NT) eam_mixed_one<0, KICK>(S.F, S.ps, i);
     } else {
         for (int i = t; i < n; i += NT) lj_mixed_one<false, KICK>(S.F, S.ps, i);
     }
