@@ -45,7 +45,6 @@ int launch_drift_guarded(mdg_system* sys, double dt, const unsigned long long* l
 int ensure_cutbits(mdg_system* sys);
 int launch_density_rec(mdg_system* sys, const PotSet* dps, const PotSet& ps);
 int launch_decide(mdg_system* sys);
-int launch_trig(mdg_system* sys);
 int launch_offsets(mdg_system* sys);
 int launch_force_copy(mdg_system* sys, int to64);
 int launch_zero(mdg_system* sys, int eam);
@@ -2009,7 +2008,6 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
         MDG_CUDA(cudaStreamBeginCaptureToGraph(st, pp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                                cudaStreamCaptureModeThreadLocal));
         int rc1 = nlist_enqueue(sys);
-        if (rc1 == 0) rc1 = launch_trig(sys);
         cudaGraph_t outr = nullptr;
         cudaError_t ec = cudaStreamEndCapture(st, &outr);
         if (rc1) return rc1;
@@ -2065,7 +2063,6 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
     MDG_CUDA(cudaStreamBeginCaptureToGraph(st, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                            cudaStreamCaptureModeThreadLocal));
     rc = nlist_enqueue(sys);
-    if (rc == 0) rc = launch_trig(sys);
     // the next step's half-kick and drift, which the force pass left to
     // after the rebuild (none after the last step)
     if (rc == 0 && next) rc = launch_drift_guarded(sys, dt, sys->dcounter, 2);
@@ -2213,8 +2210,6 @@ int request_begin(mdg_solver* s, mdg_system* sys, const mdg_atom* atoms, double 
     if (rc) return rc;
     sys->grid = *sys->hgrid;
     rc = nlist_enqueue(sys);
-    if (rc) return rc;
-    rc = launch_trig(sys);
     if (rc) return rc;
     sys->have_list = 1;
     sys->dirty = 0;

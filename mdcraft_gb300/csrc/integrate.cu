@@ -23,19 +23,6 @@ namespace mdg {
 
 
 
-// Launch shape of the one-thread-per-atom passes: as many threads per block as
-// spread the atoms over all SMs, up to 256. Their FP64 work (a warp
-// instruction every 16 cycles per SM) otherwise sits on n / 256 SMs.
-constexpr int kSpreadSms = 152;
-static inline int pass_threads(size_t n) {
-    const size_t per = ((n + kSpreadSms - 1) / kSpreadSms + 31) & ~size_t(31);
-    return (int)(per < 32 ? 32 : per > (size_t)kBlock ? (size_t)kBlock : per);
-}
-static inline int pass_blocks(size_t n) {
-    const size_t t = (size_t)pass_threads(n);
-    return (int)((n + t - 1) / t);
-}
-
 // step_one_coords + prepare + decide (FP64 form). drift = 0 runs only the
 // prepare + decide part (Pair::prepare called on its own).
 __global__ void k_drift64(IArgs A, int drift, int check) {
@@ -87,13 +74,6 @@ __global__ void k_drift_mixed_guarded(IArgs A, const unsigned long long* __restr
 __global__ void k_kick_mixed(IArgs A) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < A.n) kick_mixed_one(A, i);
-}
-
-// Half-skin threshold per atom for the mixed test (trig_one).
-__global__ void k_trig(int n, const double* __restrict__ saved_rns, const double* __restrict__ saved_rcut,
-                       const GridParams* __restrict__ gp, float2* __restrict__ trig) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) trig_one(i, saved_rns, saved_rcut, *gp, trig);
 }
 
 // Refresh of the fixed-point offsets from FP64 positions (after uploads).
@@ -268,8 +248,8 @@ int launch_drift(mdg_system* sys, double dt, int precision, double pot_rcut, int
     IArgs A = integrator_args(sys, dt);
     A.pot_rcut = pot_rcut;
     A.periodic_boundary = periodic_boundary;
-    if (precision == MDG_PREC_MIXED && drift) k_drift_mixed<<<pass_blocks(sys->n), pass_threads(sys->n), 0, ctx->stream>>>(A);
-    else k_drift64<<<pass_blocks(sys->n), pass_threads(sys->n), 0, ctx->stream>>>(A, drift, check);
+    if (precision == MDG_PREC_MIXED && drift) k_drift_mixed<<<spread_blocks(sys->n), spread_threads(sys->n), 0, ctx->stream>>>(A);
+    else k_drift64<<<spread_blocks(sys->n), spread_threads(sys->n), 0, ctx->stream>>>(A, drift, check);
     MDG_LAUNCHED(ctx);
     return MDG_OK;
 }
@@ -277,7 +257,7 @@ int launch_drift(mdg_system* sys, double dt, int precision, double pot_rcut, int
 int launch_drift_guarded(mdg_system* sys, double dt, const unsigned long long* left, unsigned long long min_left) {
     if (sys->n == 0) return MDG_OK;
     IArgs A = integrator_args(sys, dt);
-    k_drift_mixed_guarded<<<pass_blocks(sys->n), pass_threads(sys->n), 0, sys->ctx->stream>>>(A, left, min_left);
+    k_drift_mixed_guarded<<<spread_blocks(sys->n), spread_threads(sys->n), 0, sys->ctx->stream>>>(A, left, min_left);
     MDG_LAUNCHED(sys->ctx);
     return MDG_OK;
 }
@@ -285,7 +265,7 @@ int launch_drift_guarded(mdg_system* sys, double dt, const unsigned long long* l
 int launch_decide(mdg_system* sys) {
     if (sys->n == 0) return MDG_OK;
     IArgs A = integrator_args(sys, 0.0);
-    k_decide<<<pass_blocks(sys->n), pass_threads(sys->n), 0, sys->ctx->stream>>>(A);
+    k_decide<<<spread_blocks(sys->n), spread_threads(sys->n), 0, sys->ctx->stream>>>(A);
     MDG_LAUNCHED(sys->ctx);
     return MDG_OK;
 }
@@ -294,24 +274,16 @@ int launch_kick(mdg_system* sys, double dt, int precision) {
     if (sys->n == 0) return MDG_OK;
     mdg_ctx* ctx = sys->ctx;
     IArgs A = integrator_args(sys, dt);
-    if (precision == MDG_PREC_MIXED) k_kick_mixed<<<pass_blocks(sys->n), pass_threads(sys->n), 0, ctx->stream>>>(A);
-    else k_kick64<<<pass_blocks(sys->n), pass_threads(sys->n), 0, ctx->stream>>>(A);
+    if (precision == MDG_PREC_MIXED) k_kick_mixed<<<spread_blocks(sys->n), spread_threads(sys->n), 0, ctx->stream>>>(A);
+    else k_kick64<<<spread_blocks(sys->n), spread_threads(sys->n), 0, ctx->stream>>>(A);
     MDG_LAUNCHED(ctx);
-    return MDG_OK;
-}
-
-int launch_trig(mdg_system* sys) {
-    if (sys->n == 0) return MDG_OK;
-    k_trig<<<pass_blocks(sys->n), pass_threads(sys->n), 0, sys->ctx->stream>>>((int)sys->n, sys->saved_rns, sys->saved_rcut,
-                                                          sys->dgrid, sys->trig32);
-    MDG_LAUNCHED(sys->ctx);
     return MDG_OK;
 }
 
 int launch_offsets(mdg_system* sys) {
     if (sys->n == 0) return MDG_OK;
     int c = sys->cur;
-    k_offsets<<<pass_blocks(sys->n), pass_threads(sys->n), 0, sys->ctx->stream>>>((int)sys->n, sys->f64[RX][c], sys->f64[RY][c],
+    k_offsets<<<spread_blocks(sys->n), spread_threads(sys->n), 0, sys->ctx->stream>>>((int)sys->n, sys->f64[RX][c], sys->f64[RY][c],
                                                              sys->f64[RZ][c], sys->Rc[0], sys->Rc[1], sys->Rc[2],
                                                              sys->grid.inv_u[0], sys->grid.inv_u[1],
                                                              sys->grid.inv_u[2], sys->pos32, sys->u16[KIND][c]);
@@ -323,11 +295,11 @@ int launch_force_copy(mdg_system* sys, int to64) {
     if (sys->n == 0) return MDG_OK;
     int c = sys->cur;
     if (to64)
-        k_forces_to64<<<pass_blocks(sys->n), pass_threads(sys->n), 0, sys->ctx->stream>>>(
+        k_forces_to64<<<spread_blocks(sys->n), spread_threads(sys->n), 0, sys->ctx->stream>>>(
             (int)sys->n, sys->f32[0][c], sys->f32[1][c], sys->f32[2][c], sys->u16[TAG][c], sys->f64[FX][c],
             sys->f64[FY][c], sys->f64[FZ][c]);
     else
-        k_forces_to32<<<pass_blocks(sys->n), pass_threads(sys->n), 0, sys->ctx->stream>>>(
+        k_forces_to32<<<spread_blocks(sys->n), spread_threads(sys->n), 0, sys->ctx->stream>>>(
             (int)sys->n, sys->f64[FX][c], sys->f64[FY][c], sys->f64[FZ][c], sys->f32[0][c], sys->f32[1][c],
             sys->f32[2][c]);
     MDG_LAUNCHED(sys->ctx);

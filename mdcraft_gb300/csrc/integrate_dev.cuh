@@ -38,7 +38,7 @@ struct IArgs {
     const int4* q0;      // fixed-point offsets at the last rebuild
     double inv_u[3];     // fixed-point offset units per axis (GridParams::inv_u)
     float uf[3];         // their lengths in FP32 (cs / 2^29)
-    const float2* trig;  // (skin/2)^2 of the last rebuild (-1 when skin <= 0) and its band (trig_one)
+    const float2* trig;  // (skin/2)^2 of the last rebuild (-1 when skin <= 0) and its band (trig_of)
     DevStatus* st;
 };
 
@@ -116,7 +116,7 @@ __device__ __forceinline__ bool drift64_one(const IArgs& A, int i, int drift, in
 // VerletList::decide (verlet-list.cxx:135-154) with the FP64 result: the
 // displacement since the rebuild is first taken from the fixed-point offsets
 // (q - q0, exact up to one offset unit per axis) in FP32; only an atom whose
-// estimate lies within the proven error band around (skin/2)^2 (trig_one;
+// estimate lies within the proven error band around (skin/2)^2 (trig_of;
 // about 1e-5 of it) is tested again with the reference's FP64 arithmetic, so
 // every decision equals decide_one's on the same positions. (The size, uid,
 // rcut and rns comparisons of decide cannot change inside the step loop: the
@@ -206,17 +206,12 @@ __device__ __forceinline__ void kick_mixed_one(const IArgs& A, int i) {
 // 4 sqrt(threshold) u + 4 u^2, covers both. The threshold is FP64 (as
 // decide_one's) rounded to FP32; the band, a bound with 15% or more to
 // spare in each term, is evaluated in FP32 (FP64 square roots are slow).
-__device__ __forceinline__ void trig_one(int i, const double* __restrict__ saved_rns,
-                                         const double* __restrict__ saved_rcut, const GridParams& g,
-                                         float2* __restrict__ trig) {
-    double skin = dsub(saved_rns[i], saved_rcut[i]);
-    if (skin <= 0.0) {
-        trig[i] = make_float2(-1.0f, 0.0f);
-        return;
-    }
+__device__ __forceinline__ float2 trig_of(double rns, double rcut, const GridParams& g) {
+    double skin = dsub(rns, rcut);
+    if (skin <= 0.0) return make_float2(-1.0f, 0.0f);
     const float t = (float)dmul(dmul(0.25, skin), skin);
     const float u = fmaxf(g.csf[0], fmaxf(g.csf[1], g.csf[2])) * (1.0f / (float)kOffUnits);
-    trig[i] = make_float2(t, fmaf(1e-5f, t, fmaf(4.0f * sqrtf(t), u, 4.0f * u * u)));
+    return make_float2(t, fmaf(1e-5f, t, fmaf(4.0f * sqrtf(t), u, 4.0f * u * u)));
 }
 
 }  // namespace mdg

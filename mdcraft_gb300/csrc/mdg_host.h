@@ -258,6 +258,19 @@ const ThermoDev* thermo_of(mdg_solver* s);
 int settle_outputs(mdg_system* sys);
 // Ep and V of atoms with tag != 0 cleared (before an accumulating pass).
 int launch_zero_meas(mdg_system* sys);
+
+// Launch shape of the one-thread-per-atom passes: as many threads per block as
+// spread the atoms over all SMs, up to 256. Their FP64 work (a warp
+// instruction every 16 cycles per SM) otherwise sits on n / 256 SMs.
+constexpr size_t kSpreadSms = 152;
+inline int spread_threads(size_t n) {
+    const size_t per = ((n + kSpreadSms - 1) / kSpreadSms + 31) & ~size_t(31);
+    return (int)(per < 32 ? 32 : per > (size_t)kBlock ? (size_t)kBlock : per);
+}
+inline int spread_blocks(size_t n) {
+    const size_t t = (size_t)spread_threads(n);
+    return (int)((n + t - 1) / t);
+}
 int nlist_capacity_host(mdg_system* sys, const mdg_atom* atoms, size_t n, int half);
 // The fused one-block driver loop (solo.cu): small mixed-precision systems,
 // one request per block of a persistent kernel fed through a queue.

@@ -144,13 +144,13 @@ struct PotParams {
     const float4* v_c;
     const float4* f_c;
     const float4* rv_c;  // force rows: W(u) = V'r - V, then D(u) = rho' (2 float4 per interval)
+    float inv_dr_f, inv_drh_f, dr1_f, drh_f;
     // FP64 pieces in x = r - r_n, 32-byte aligned rows of four coefficients
     const double* wd64;   // W(x) = V'r - V, then D(x) = rho' (2 rows per interval)
     const double* rho64;  // rho(x)
     const double* v64;    // V(x)
     const double* rn64;   // r_n
     double mhf_lj1, hf_lj2;  // LJsCut: -factor lj1 / 2, factor lj2 / 2
-    float inv_dr_f, inv_drh_f, dr1_f, drh_f;
 };
 
 struct PotSet {
@@ -211,6 +211,7 @@ struct DevStatus {
     uint32_t therm_calls;   // thermostat applications so far (Philox counter word)
     uint32_t need_next;     // rebuild test of the next step's positions, from a force pass
                             // that ran the next step's first half-kick and drift
+    uint32_t arrived;       // blocks of the bounds pass done (0 between rebuilds)
 };
 
 }  // namespace mdg

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "mdg_host.h"
+#include "integrate_dev.cuh"
 #include "nlist_dev.cuh"
 
 namespace mdg {
@@ -28,75 +29,120 @@ namespace mdg {
 // grid.cxx:209-243)
 // ---------------------------------------------------------------------------
 
-__global__ void k_wrap_bounds(int n, double* __restrict__ rx, double* __restrict__ ry,
-                              double* __restrict__ rz, const double* __restrict__ rns,
-                              DomainDev d, double* __restrict__ part) {
-    __shared__ double sh[7][kBlock];
-    double lo[3] = {1.7976931348623157e308, 1.7976931348623157e308, 1.7976931348623157e308};
-    double hi[3] = {-1.7976931348623157e308, -1.7976931348623157e308, -1.7976931348623157e308};
-    double mr = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double v[3];
-        wrap_one(d, rx, ry, rz, i, v);
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fmin(lo[a], v[a]);
-            hi[a] = fmax(hi[a], v[a]);
+// Reduces the block's bounds (lo, hi, largest rns) over its threads; the
+// result is in v of thread 0.
+__device__ __forceinline__ void block_bounds(double v[7]) {
+    __shared__ double sh[kBlock / 32][7];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        for (int k = 0; k < 7; ++k) {
+            const double y = __shfl_down_sync(0xffffffffu, v[k], o);
+            v[k] = k < 3 ? fmin(v[k], y) : fmax(v[k], y);
         }
-        double q = rns[i];
-        mr = mr < q ? q : mr;
-    }
-    int t = threadIdx.x;
-    sh[0][t] = lo[0]; sh[1][t] = lo[1]; sh[2][t] = lo[2];
-    sh[3][t] = hi[0]; sh[4][t] = hi[1]; sh[5][t] = hi[2];
-    sh[6][t] = mr;
+    if (lane == 0)
+        for (int k = 0; k < 7; ++k) sh[w][k] = v[k];
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (t < s) {
-            for (int k = 0; k < 3; ++k) sh[k][t] = fmin(sh[k][t], sh[k][t + s]);
-            for (int k = 3; k < 7; ++k) sh[k][t] = fmax(sh[k][t], sh[k][t + s]);
-        }
-        __syncthreads();
+    if (w == 0) {
+        if (lane < kBlock / 32)
+            for (int k = 0; k < 7; ++k) v[k] = sh[lane][k];
+#pragma unroll
+        for (int o = kBlock / 64; o > 0; o >>= 1)
+            for (int k = 0; k < 7; ++k) {
+                const double y = __shfl_down_sync(0xffffffffu, v[k], o);
+                v[k] = k < 3 ? fmin(v[k], y) : fmax(v[k], y);
+            }
     }
-    if (t < 7) part[blockIdx.x * 8 + t] = sh[t][0];
 }
 
+__device__ __forceinline__ void no_bounds(double v[7]) {
+    for (int k = 0; k < 3; ++k) {
+        v[k] = 1.7976931348623157e308;
+        v[3 + k] = -1.7976931348623157e308;
+    }
+    v[6] = 0.0;
+}
 
-__global__ void k_grid_finalize(const double* __restrict__ part, int nparts, DomainDev d,
-                                GridParams* __restrict__ out, long long bin_cap, DevStatus* st) {
-    __shared__ double sh[7][kBlock];
-    int t = threadIdx.x;
-    double v[7] = {1.7976931348623157e308, 1.7976931348623157e308, 1.7976931348623157e308,
-                   -1.7976931348623157e308, -1.7976931348623157e308, -1.7976931348623157e308, 0.0};
-    for (int b = t; b < nparts; b += blockDim.x) {
-        for (int k = 0; k < 3; ++k) v[k] = fmin(v[k], part[b * 8 + k]);
-        for (int k = 3; k < 7; ++k) v[k] = fmax(v[k], part[b * 8 + k]);
-    }
-    for (int k = 0; k < 7; ++k) sh[k][t] = v[k];
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (t < s) {
-            for (int k = 0; k < 3; ++k) sh[k][t] = fmin(sh[k][t], sh[k][t + s]);
-            for (int k = 3; k < 7; ++k) sh[k][t] = fmax(sh[k][t], sh[k][t + s]);
+// Wraps the positions and finds their bounds, the largest rns and whether the
+// rns differ, clears the bin counts, and, in the block that finishes last,
+// computes the grid. (One launch: as passes of their own these were five
+// launches, of which a small system's rebuild has nothing but.)
+__global__ void __launch_bounds__(kBlock)
+    k_wrap_bounds(int n, double* __restrict__ rx, double* __restrict__ ry, double* __restrict__ rz,
+                  const double* __restrict__ rns, DomainDev d, double* __restrict__ part,
+                  GridParams* __restrict__ out, long long bin_cap, uint32_t* __restrict__ bin_count,
+                  DevStatus* st) {
+    const int t = threadIdx.x;
+    double v[7];
+    no_bounds(v);
+    const double r0 = n > 0 ? rns[0] : 0.0;
+    bool differ = false;
+    for (int i = blockIdx.x * kBlock + t; i < n; i += gridDim.x * kBlock) {
+        double x[3];
+        wrap_one(d, rx, ry, rz, i, x);
+        for (int a = 0; a < 3; ++a) {
+            v[a] = fmin(v[a], x[a]);
+            v[3 + a] = fmax(v[3 + a], x[a]);
         }
-        __syncthreads();
+        const double q = rns[i];
+        v[6] = v[6] < q ? q : v[6];
+        differ = differ || q != r0;
     }
-    if (t != 0) return;
-    GridParams g;
-    double lo[3] = {sh[0][0], sh[1][0], sh[2][0]}, hi[3] = {sh[3][0], sh[4][0], sh[5][0]};
-    grid_from_bounds(d, lo, hi, sh[6][0], g);
-    if (g.empty == -1) {
-        *out = g;
-        return;
+    if (bin_count)
+        for (long long b = (long long)blockIdx.x * kBlock + t; b < bin_cap; b += (long long)gridDim.x * kBlock)
+            bin_count[b] = 0u;
+    if (differ) atomicOr(&st->nonuniform, 1u);
+    block_bounds(v);
+    __shared__ bool last;
+    if (t == 0) {
+        for (int k = 0; k < 7; ++k) part[blockIdx.x * 8 + k] = v[k];
+        __threadfence();
+        last = atomicAdd(&st->arrived, 1u) == gridDim.x - 1;
     }
-    long long nb = g.nbins;
-    // the bin arrays were sized on the host; a grid that outgrew them
-    // invalidates this rebuild (every later kernel of it returns early)
-    if (g.empty == 0 && nb + 1 > bin_cap) {
-        g.empty = -3;
-        atomicOr(&st->flags, FLAG_OVERFLOW);
-        atomicOr(&st->build_flags, FLAG_OVERFLOW);
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    no_bounds(v);
+    for (int b = t; b < (int)gridDim.x; b += kBlock)
+        for (int k = 0; k < 7; ++k) {
+            const double y = __ldcg(part + b * 8 + k);
+            v[k] = k < 3 ? fmin(v[k], y) : fmax(v[k], y);
+        }
+    __syncthreads();  // block_bounds' shared array, read by the first call
+    block_bounds(v);
+    if (t >= 32) return;
+    // three lanes take an axis each
+    __shared__ GridParams g;
+    if (t == 0) memset(&g, 0, sizeof(g));
+    const double cell = __shfl_sync(0xffffffffu, v[6], 0);
+    double lo = 0.0, hi = 0.0;
+    for (int a = 0; a < 3; ++a) {
+        const double l = __shfl_sync(0xffffffffu, v[a], 0), h = __shfl_sync(0xffffffffu, v[3 + a], 0);
+        if (t == a && a < d.dim) {
+            lo = l;
+            hi = h;
+        }
     }
-    *out = g;
+    __syncwarp();
+    bool small = false, bad = false;
+    if (t < 3) grid_axis(d, lo, hi, cell, t, g, &small, &bad);
+    small = __any_sync(0xffffffffu, small);
+    bad = __any_sync(0xffffffffu, bad);
+    __syncwarp();
+    if (t == 0) {
+        st->arrived = 0;
+        grid_totals(d, cell, small, bad, g);
+        // the bin arrays were sized on the host; a grid that outgrew them
+        // invalidates this rebuild (every later kernel of it returns early)
+        if (g.empty == 0 && (long long)g.nbins + 1 > bin_cap) {
+            g.empty = -3;
+            atomicOr(&st->flags, FLAG_OVERFLOW);
+            atomicOr(&st->build_flags, FLAG_OVERFLOW);
+        }
+    }
+    __syncwarp();
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&g);
+    for (int k = t; k < (int)(sizeof(GridParams) / 4); k += 32) reinterpret_cast<uint32_t*>(out)[k] = src[k];
 }
 
 // ---------------------------------------------------------------------------
@@ -105,12 +151,12 @@ __global__ void k_grid_finalize(const double* __restrict__ part, int nparts, Dom
 
 __global__ void k_bin_count(int n, const double* __restrict__ rx, const double* __restrict__ ry,
                             const double* __restrict__ rz, const GridParams* __restrict__ gp,
-                            uint32_t* __restrict__ key, uint32_t* __restrict__ rank,
+                            uint32_t* __restrict__ key, uint32_t* __restrict__ rank, uint32_t* __restrict__ cell,
                             uint32_t* __restrict__ bin_count, DevStatus* st) {
-    const GridParams g = *gp;
+    const GridParams& g = *gp;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || g.empty) return;
-    bin_count_one(g, i, rx, ry, rz, key, rank, bin_count, st);
+    bin_count_one(g, i, rx, ry, rz, key, rank, cell, bin_count, st);
 }
 
 // Exclusive scan of nb uint32 counts into start[0..nb] (start[nb] = total),
@@ -176,54 +222,106 @@ __global__ void k_scan_final(const uint32_t* __restrict__ in, const GridParams* 
     if ((int)blockIdx.x == last && threadIdx.x == blockDim.x - 1) out[nb] = off;
 }
 
+// The same scan by one block, for up to kScanOne bins (one launch).
+constexpr int kScanOne = 16384;
+__global__ void __launch_bounds__(kScanT)
+    k_scan_one(const uint32_t* __restrict__ in, const GridParams* __restrict__ gp, uint32_t* __restrict__ out) {
+    __shared__ uint32_t sh[32];
+    const int nb = live_bins(gp), per = (nb + kScanT - 1) / kScanT;
+    const int b0 = min((int)threadIdx.x * per, nb), b1 = min(b0 + per, nb);
+    uint32_t s = 0;
+    for (int b = b0; b < b1; ++b) s += in[b];
+    uint32_t tot;
+    uint32_t off = block_excl_scan(s, sh, &tot);
+    for (int b = b0; b < b1; ++b) {
+        const uint32_t v = in[b];
+        out[b] = off;
+        off += v;
+    }
+    if (threadIdx.x == 0) out[nb] = tot;
+}
+
+// Atoms and their caller indices in arrival order, bin by bin.
 __global__ void k_scatter(int n, const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank,
-                          const uint32_t* __restrict__ start, uint32_t* __restrict__ src,
+                          const uint32_t* __restrict__ start, const uint32_t* __restrict__ orig,
+                          uint32_t* __restrict__ src, uint32_t* __restrict__ orig_at,
                           const GridParams* __restrict__ gp) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !gp->empty) src[start[key[i]] + rank[i]] = (uint32_t)i;
+    if (i >= n || gp->empty) return;
+    const uint32_t k = start[key[i]] + rank[i];
+    src[k] = (uint32_t)i;
+    orig_at[k] = orig[i];
 }
 
-// Deterministic order inside a bin: ascending caller index.
-__global__ void k_bin_sort(const GridParams* __restrict__ gp, const uint32_t* __restrict__ start,
-                           uint32_t* __restrict__ src, const uint32_t* __restrict__ orig) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= live_bins(gp)) return;
-    bin_sort_one(b, start, src, orig);
-}
-
-// Permutation of the per-atom fields: dst[k] = src_field[src[k]].
-
-template <int NF, typename T>
-__global__ void k_gather(int n, const uint32_t* __restrict__ src, GatherSet<NF, T> gs,
-                         const GridParams* __restrict__ gp) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Every per-atom field into the spare buffers, each bin ordered by caller
+// index (deterministic): thread k takes the atom that arrived k-th to its
+// slot in the bin, so both the reads and the writes of a warp stay within a
+// few bins. One pass for all fields; counting the smaller indices of the bin
+// replaces an insertion sort by a thread per bin (argon 4,000 atoms: 35 us,
+// 500 atoms in 8 cells: 116 us).
+__global__ void __launch_bounds__(kBlock)
+    k_permute(int n, const uint32_t* __restrict__ src, const uint32_t* __restrict__ orig_at,
+              const uint32_t* __restrict__ key, const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell,
+              uint32_t* __restrict__ cell_out, GatherAll G, const GridParams* __restrict__ gp) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n || gp->empty) return;
-    uint32_t s = src[k];
+    const uint32_t i = src[k];
+    const uint32_t d = sorted_slot((uint32_t)k, key[i], start, orig_at);
+    double x[12];
 #pragma unroll
-    for (int f = 0; f < NF; ++f) gs.out[f][k] = gs.in[f][s];
+    for (int f = 0; f < 12; ++f) x[f] = G.a.in[f][i];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) G.a.out[f][d] = x[f];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) x[f] = G.b.in[f][i];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) G.b.out[f][d] = x[f];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) G.fc.out[f][d] = G.fc.in[f][i];
+#pragma unroll
+    for (int f = 0; f < 2; ++f) G.u.out[f][d] = G.u.in[f][i];
+#pragma unroll
+    for (int f = 0; f < 2; ++f) G.h.out[f][d] = G.h.in[f][i];
+    cell_out[d] = cell[i];
 }
+
+struct CellOut {
+    uint32_t* cellp;
+    double *Rx, *Ry, *Rz;
+    int4 *pos32, *q0;
+    float4* o0;
+    uint32_t* slot_of;
+    float2* trig;
+};
 
 // The permuted fields back into the live buffers (so device pointers stay
-// fixed across rebuilds, as a captured graph needs).
-template <int NF, typename T>
-__global__ void k_copy(int n, GatherSet<NF, T> gs, const GridParams* __restrict__ gp) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n || gp->empty) return;
+// fixed across rebuilds, as a captured graph needs), and what follows from
+// them: cell centres, offsets, the rebuild test's thresholds.
+__global__ void __launch_bounds__(kBlock)
+    k_settle(int n, GatherAll G, const uint32_t* __restrict__ cell, CellOut C, const GridParams* __restrict__ gp) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const GridParams& g = *gp;
+    if (k >= n || g.empty) return;
+    double x[12];
 #pragma unroll
-    for (int f = 0; f < NF; ++f) gs.out[f][k] = gs.in[f][k];
-}
-
-// Cell centre, cell-relative FP32 offsets and packed cell of every atom.
-__global__ void k_cells(int n, const double* __restrict__ rx, const double* __restrict__ ry,
-                        const double* __restrict__ rz, const GridParams* __restrict__ gp,
-                        uint32_t* __restrict__ cellp, double* __restrict__ Rx, double* __restrict__ Ry,
-                        double* __restrict__ Rz, int4* __restrict__ pos32, int4* __restrict__ q0, float4* __restrict__ o0,
-                        const uint32_t* __restrict__ orig, uint32_t* __restrict__ slot_of,
-                        const uint16_t* __restrict__ kind) {
-    const GridParams g = *gp;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || g.empty) return;
-    cells_one(g, i, rx, ry, rz, cellp, Rx, Ry, Rz, pos32, q0, o0, orig, slot_of, kind);
+    for (int f = 0; f < 12; ++f) x[f] = G.b2.in[f][k];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) G.b2.out[f][k] = x[f];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) G.fc2.out[f][k] = G.fc2.in[f][k];
+    const uint32_t orig = G.u2.in[0][k];
+    G.u2.out[0][k] = orig;
+    G.u2.out[1][k] = G.u2.in[1][k];
+    const uint16_t kind = G.h2.in[0][k];
+    G.h2.out[0][k] = kind;
+    G.h2.out[1][k] = G.h2.in[1][k];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) x[f] = G.a2.in[f][k];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) G.a2.out[f][k] = x[f];
+    const double r[3] = {x[RX], x[RY], x[RZ]};
+    cells_one(g, k, r, cell[k], orig, kind, C.cellp, C.Rx, C.Ry, C.Rz, C.pos32, C.q0, C.o0, C.slot_of);
+    C.trig[k] = trig_of(x[RNS], x[RCUT], g);
 }
 
 // ---------------------------------------------------------------------------
@@ -360,23 +458,25 @@ __global__ void __launch_bounds__(kExportWarps * 32)
 // Verlet list
 // ---------------------------------------------------------------------------
 
-// Block of NW warps (cells per block: a system's launch shape, default 4),
-// a warp per bin, on grids without a periodic axis of 2 cells or fewer
-// (GridParams::small_box; those take k_nbuild_atoms). 64 registers.
+// Block of NW warps (a system's launch shape, default 4), `parts` warps per
+// bin, on grids without a periodic axis of 2 cells or fewer
+// (GridParams::small_box; those take k_nbuild_atoms).
+constexpr int kNbChunks = 8;
 template <int NW>
-__global__ void __launch_bounds__(NW * 32, 32 / NW) k_nbuild_warp(NbArgs A, const GridParams* __restrict__ gp) {
+__global__ void __launch_bounds__(NW * 32, 32 / NW)
+    k_nbuild_warp(NbArgs A, const GridParams* __restrict__ gp, int parts) {
     __shared__ GridParams g;
-    __shared__ NbWarpSmem S[NW];
+    __shared__ NbWarpSmem<kNbChunks> S[NW];
     if (threadIdx.x == 0) g = *gp;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bin = blockIdx.x * NW + warp;
+    const int w = blockIdx.x * NW + warp, bin = w / parts;
     if (g.empty || g.small_box || bin >= g.nbins) return;
-    nbuild_cell_warp(A, g, bin, lane, A.st->nonuniform == 0, S[warp]);
+    nbuild_cell_warp(A, g, bin, w - bin * parts, parts, lane, A.st->nonuniform == 0, S[warp]);
 }
 
 // The list build of grids with a periodic axis of 2 cells or fewer (a few
-// cells of many atoms): a thread per atom. Launched after k_nbuild_warp. On
+// cells of many atoms): a warp per atom. Launched after k_nbuild_warp. On
 // the other grids it returns at once, unless some atom was clamped into the
 // grid (FLAG_RANGE): those atoms' lists are built again from their
 // unclamped cells (nbuild_atom), over what the warp build wrote.
@@ -388,8 +488,9 @@ __global__ void __launch_bounds__(kBlock) k_nbuild_atoms(NbArgs A, const GridPar
     const bool clamped_only = !g.small_box;
     if (clamped_only && !(A.st->build_flags & FLAG_RANGE)) return;
     const bool uniform = A.st->nonuniform == 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (uint32_t)A.n; i += gridDim.x * blockDim.x)
-        if (!clamped_only || A.o0[i].w == 2.0f) nbuild_atom(A, g, i, uniform);
+    const uint32_t warps = gridDim.x * (kBlock / 32);
+    for (uint32_t i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); i < (uint32_t)A.n; i += warps)
+        if (!clamped_only || A.o0[i].w == 2.0f) nbuild_atom(A, g, i, threadIdx.x & 31, uniform);
 }
 
 // VerletList::optimize_search_radius (verlet-list.cxx:72-92):
@@ -412,11 +513,6 @@ __global__ void k_optimize_rns(int n, int np, double kbuf, int have_list, const 
         }
     }
     rns[i] = kbuf * hmax;
-}
-
-__global__ void k_check_rns(int n, const double* __restrict__ rns, DevStatus* st) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && rns[i] != rns[0]) atomicOr(&st->nonuniform, 1u);
 }
 
 // ---------------------------------------------------------------------------
@@ -500,9 +596,8 @@ int nlist_capacity(mdg_system* sys, int half) {
     DomainDev d = domain_dev(sys);
     int c = sys->cur;
     k_wrap_bounds<<<nparts, kBlock, 0, st>>>(n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c],
-                                             sys->f64[RNS][c], d, sys->part);
-    MDG_LAUNCHED(ctx);
-    k_grid_finalize<<<1, kBlock, 0, st>>>(sys->part, nparts, d, sys->dgrid, 1LL << 40, sys->dstat);
+                                             sys->f64[RNS][c], d, sys->part, sys->dgrid, 1LL << 40, nullptr,
+                                             sys->dstat);
     MDG_LAUNCHED(ctx);
     MDG_CUDA(cudaMemcpyAsync(sys->hgrid, sys->dgrid, sizeof(GridParams), cudaMemcpyDeviceToHost, st));
     MDG_CUDA(cudaStreamSynchronize(st));
@@ -519,9 +614,8 @@ int grid_build_only(mdg_system* sys, GridParams* out) {
     DomainDev d = domain_dev(sys);
     const int c = sys->cur;
     k_wrap_bounds<<<nparts, kBlock, 0, st>>>((int)sys->n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c],
-                                             sys->f64[RNS][c], d, sys->part);
-    MDG_LAUNCHED(ctx);
-    k_grid_finalize<<<1, kBlock, 0, st>>>(sys->part, nparts, d, sys->dgrid, 1LL << 40, sys->dstat);
+                                             sys->f64[RNS][c], d, sys->part, sys->dgrid, 1LL << 40, nullptr,
+                                             sys->dstat);
     MDG_LAUNCHED(ctx);
     MDG_CUDA(cudaMemcpyAsync(out, sys->dgrid, sizeof(GridParams), cudaMemcpyDeviceToHost, st));
     MDG_CUDA(cudaStreamSynchronize(st));
@@ -669,8 +763,35 @@ NbArgs nb_args(const mdg_system* sys) {
 
 DomainDev domain_of(const mdg_system* sys) { return domain_dev(sys); }
 
-// Lanes per cell of the list build: 16, or 32 when the cells of the last
-// sized grid hold more than 16 atoms on average.
+// Exclusive scan of the live bins' counts into out[0..nbins].
+static int launch_scan(mdg_system* sys, uint32_t* out) {
+    mdg_ctx* ctx = sys->ctx;
+    cudaStream_t st = ctx->stream;
+    if (sys->bin_cap <= (size_t)kScanOne) {
+        k_scan_one<<<1, kScanT, 0, st>>>(sys->bin_count, sys->dgrid, out);
+        MDG_LAUNCHED(ctx);
+        return MDG_OK;
+    }
+    const int nscan = (int)((sys->bin_cap + kScanT * kScanItems - 1) / (kScanT * kScanItems));
+    if (nscan > kScanT * kScanItems) {
+        set_error("too many cell bins for the scan");
+        return MDG_ERR_INVALID;
+    }
+    k_scan_partial<<<nscan, kScanT, 0, st>>>(sys->bin_count, sys->dgrid, sys->scan_tmp);
+    MDG_LAUNCHED(ctx);
+    k_scan_top<<<1, kScanT, 0, st>>>(sys->scan_tmp, sys->dgrid);
+    MDG_LAUNCHED(ctx);
+    k_scan_final<<<nscan, kScanT, 0, st>>>(sys->bin_count, sys->dgrid, sys->scan_tmp, out);
+    MDG_LAUNCHED(ctx);
+    return MDG_OK;
+}
+
+// Warps per cell of the list build: several where the cells are fewer than
+// the GPU's warp slots (whole rebuilds with 1 / 2 / 4 / 8: LJ argon 4,000
+// atoms 133 / 116 / 113 / 102 us, EAM Cu 32,000 119 / 120 / 142 / 178 us,
+// LJ argon 62,500 152 / 176 / 201 / 263 us; each repeats the candidates'
+// loads).
+static int list_parts(size_t n) { return n < 12000 ? 4 : 1; }
 
 int nlist_enqueue(mdg_system* sys) {
     mdg_ctx* ctx = sys->ctx;
@@ -683,73 +804,42 @@ int nlist_enqueue(mdg_system* sys) {
     const int c = sys->cur;
     MDG_CUDA(cudaMemsetAsync(&sys->dstat->max_count, 0, 3 * sizeof(uint32_t), st));  // max_count, nonuniform, build_flags
     k_wrap_bounds<<<nparts, kBlock, 0, st>>>(n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c],
-                                             sys->f64[RNS][c], d, sys->part);
+                                             sys->f64[RNS][c], d, sys->part, sys->dgrid, (long long)sys->bin_cap,
+                                             sys->bin_count, sys->dstat);
     MDG_LAUNCHED(ctx);
-    k_grid_finalize<<<1, kBlock, 0, st>>>(sys->part, nparts, d, sys->dgrid, (long long)sys->bin_cap, sys->dstat);
+    // the atoms' cells wait in ncnt (free until the list is built)
+    const int pt = spread_threads(n), pb = nblk(n, pt);
+    k_bin_count<<<pb, pt, 0, st>>>(n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c], sys->dgrid, sys->key,
+                                   sys->rank, sys->ncnt, sys->bin_count, sys->dstat);
     MDG_LAUNCHED(ctx);
-    k_check_rns<<<nblk(n), kBlock, 0, st>>>(n, sys->f64[RNS][c], sys->dstat);
+    int rc = launch_scan(sys, sys->bin_start);
+    if (rc) return rc;
+    // src and orig_at (in cellp, rewritten by k_settle): arrival order
+    k_scatter<<<pb, pt, 0, st>>>(n, sys->key, sys->rank, sys->bin_start, sys->u32[ORIG][c], sys->src, sys->cellp,
+                                 sys->dgrid);
     MDG_LAUNCHED(ctx);
-    MDG_CUDA(cudaMemsetAsync(sys->bin_count, 0, sys->bin_cap * sizeof(uint32_t), st));
-    k_bin_count<<<nblk(n), kBlock, 0, st>>>(n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c], sys->dgrid,
-                                            sys->key, sys->rank, sys->bin_count, sys->dstat);
+    const GatherAll G = gather_sets(sys);
+    k_permute<<<pb, pt, 0, st>>>(n, sys->src, sys->cellp, sys->key, sys->bin_start, sys->ncnt, sys->rank, G,
+                                 sys->dgrid);
     MDG_LAUNCHED(ctx);
-    int nscan = (int)((sys->bin_cap + kScanT * kScanItems - 1) / (kScanT * kScanItems));
-    if (nscan > kScanT * kScanItems) {
-        set_error("too many cell bins for the scan");
-        return MDG_ERR_INVALID;
-    }
-    k_scan_partial<<<nscan, kScanT, 0, st>>>(sys->bin_count, sys->dgrid, sys->scan_tmp);
-    MDG_LAUNCHED(ctx);
-    k_scan_top<<<1, kScanT, 0, st>>>(sys->scan_tmp, sys->dgrid);
-    MDG_LAUNCHED(ctx);
-    k_scan_final<<<nscan, kScanT, 0, st>>>(sys->bin_count, sys->dgrid, sys->scan_tmp, sys->bin_start);
-    MDG_LAUNCHED(ctx);
-    k_scatter<<<nblk(n), kBlock, 0, st>>>(n, sys->key, sys->rank, sys->bin_start, sys->src, sys->dgrid);
-    MDG_LAUNCHED(ctx);
-    k_bin_sort<<<nblk(sys->bin_cap), kBlock, 0, st>>>(sys->dgrid, sys->bin_start, sys->src, sys->u32[ORIG][c]);
-    MDG_LAUNCHED(ctx);
-    // permute every per-atom field into the spare buffers, then copy back
-    {
-        GatherAll G = gather_sets(sys);
-        auto& a = G.a; auto& b = G.b; auto& a2 = G.a2; auto& b2 = G.b2;
-        auto& fc = G.fc; auto& fc2 = G.fc2; auto& u = G.u; auto& u2 = G.u2; auto& h = G.h; auto& h2 = G.h2;
-        k_gather<12, double><<<nblk(n), kBlock, 0, st>>>(n, sys->src, a, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_gather<12, double><<<nblk(n), kBlock, 0, st>>>(n, sys->src, b, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_gather<3, float><<<nblk(n), kBlock, 0, st>>>(n, sys->src, fc, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_gather<2, uint32_t><<<nblk(n), kBlock, 0, st>>>(n, sys->src, u, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_gather<2, uint16_t><<<nblk(n), kBlock, 0, st>>>(n, sys->src, h, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_copy<12, double><<<nblk(n), kBlock, 0, st>>>(n, a2, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_copy<12, double><<<nblk(n), kBlock, 0, st>>>(n, b2, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_copy<3, float><<<nblk(n), kBlock, 0, st>>>(n, fc2, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_copy<2, uint32_t><<<nblk(n), kBlock, 0, st>>>(n, u2, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-        k_copy<2, uint16_t><<<nblk(n), kBlock, 0, st>>>(n, h2, sys->dgrid);
-        MDG_LAUNCHED(ctx);
-    }
-    k_cells<<<nblk(n), kBlock, 0, st>>>(n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c], sys->dgrid,
-                                        sys->cellp, sys->Rc[0], sys->Rc[1], sys->Rc[2], sys->pos32, sys->q0, sys->o0,
-                                        sys->u32[ORIG][c], sys->slot_of, sys->u16[KIND][c]);
+    const CellOut C = {sys->cellp, sys->Rc[0], sys->Rc[1], sys->Rc[2], sys->pos32, sys->q0, sys->o0, sys->slot_of,
+                       sys->trig32};
+    k_settle<<<pb, pt, 0, st>>>(n, G, sys->rank, C, sys->dgrid);
     MDG_LAUNCHED(ctx);
     NbArgs A = nb_args(sys);
-    // a half warp per bin of the capacity (a whole warp where cells hold more
-    // than 16 atoms on average); the live bins come from the device grid
+    // a warp per bin of the capacity; the live bins come from the device grid.
+    // Systems with fewer cells than the GPU has warp slots give each cell's
+    // atoms to several warps
     const int cpb = sys->shape[MDG_SHAPE_LIST_CELLS_PER_BLOCK] ? sys->shape[MDG_SHAPE_LIST_CELLS_PER_BLOCK] : 4;
-    const unsigned nbw = (unsigned)((sys->bin_cap + cpb - 1) / cpb);
-    if (cpb == 2) k_nbuild_warp<2><<<nbw, 2 * 32, 0, st>>>(A, sys->dgrid);
-    else if (cpb == 8) k_nbuild_warp<8><<<nbw, 8 * 32, 0, st>>>(A, sys->dgrid);
-    else k_nbuild_warp<4><<<nbw, 4 * 32, 0, st>>>(A, sys->dgrid);
+    const int parts = list_parts(sys->n);
+    const unsigned nbw = (unsigned)((sys->bin_cap * parts + cpb - 1) / cpb);
+    if (cpb == 2) k_nbuild_warp<2><<<nbw, 2 * 32, 0, st>>>(A, sys->dgrid, parts);
+    else if (cpb == 8) k_nbuild_warp<8><<<nbw, 8 * 32, 0, st>>>(A, sys->dgrid, parts);
+    else k_nbuild_warp<4><<<nbw, 4 * 32, 0, st>>>(A, sys->dgrid, parts);
     MDG_LAUNCHED(ctx);
     // a grid-stride launch of at most four blocks per SM: on the large
     // grids, where it returns at once, its blocks are few
-    k_nbuild_atoms<<<std::min(nblk(n), 4 * std::max(ctx->num_sms, 1)), kBlock, 0, st>>>(A, sys->dgrid);
+    k_nbuild_atoms<<<std::min(nblk(n, kBlock / 32), 4 * std::max(ctx->num_sms, 1)), kBlock, 0, st>>>(A, sys->dgrid);
     MDG_LAUNCHED(ctx);
     return MDG_OK;
 }
@@ -763,13 +853,8 @@ static int sort_perm_enqueue(mdg_system* sys, uint32_t* cell_start, uint32_t* pe
     // per-cell counts in x-fastest order, scanned like the bins
     k_sort_cell_counts<<<nblk((size_t)cap), kBlock, 0, st>>>(sys->dgrid, sys->bin_start, sys->bin_count, cap);
     MDG_LAUNCHED(ctx);
-    const int nscan = (int)((cap + kScanT * kScanItems - 1) / (kScanT * kScanItems));
-    k_scan_partial<<<nscan, kScanT, 0, st>>>(sys->bin_count, sys->dgrid, sys->scan_tmp);
-    MDG_LAUNCHED(ctx);
-    k_scan_top<<<1, kScanT, 0, st>>>(sys->scan_tmp, sys->dgrid);
-    MDG_LAUNCHED(ctx);
-    k_scan_final<<<nscan, kScanT, 0, st>>>(sys->bin_count, sys->dgrid, sys->scan_tmp, cell_start);
-    MDG_LAUNCHED(ctx);
+    int rc = launch_scan(sys, cell_start);
+    if (rc) return rc;
     k_sort_place<<<nblk(n), kBlock, 0, st>>>(n, sys->dgrid, sys->cellp, sys->bin_start, cell_start,
                                              sys->u32[ORIG][sys->cur], perm);
     MDG_LAUNCHED(ctx);
@@ -897,8 +982,6 @@ int nlist_export_entries(mdg_system* sys, const std::vector<uint64_t>& off, uint
     return rc;
 }
 
-int launch_trig(mdg_system* sys);
-
 // VerletList::update (verlet-list.cxx:41-55) for the API: enqueue, wait,
 // and rebuild again with larger capacities when the grid or a list outgrew
 // them.
@@ -926,8 +1009,6 @@ int nlist_build(mdg_system* sys, double kbuf, int half) {
     }
     for (int attempt = 0; attempt < 4; ++attempt) {
         rc = nlist_enqueue(sys);
-        if (rc) return rc;
-        rc = launch_trig(sys);
         if (rc) return rc;
         MDG_CUDA(cudaMemcpyAsync(sys->hstat, sys->dstat, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
         MDG_CUDA(cudaMemcpyAsync(sys->hgrid, sys->dgrid, sizeof(GridParams), cudaMemcpyDeviceToHost, st));

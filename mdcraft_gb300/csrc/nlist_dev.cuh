@@ -24,72 +24,78 @@ struct DomainDev {
     int dim;
 };
 
-// Grid::build (grid.cxx:43-95) from the reduced bounds and the largest rns;
-// shared by the device rebuild and the host-side capacity sizing, so both
-// get the same parameters bit for bit.
-__host__ __device__ inline void grid_from_bounds(const DomainDev& d, const double lo_in[3], const double hi_in[3],
-                                          double cell, GridParams& g) {
-    memset(&g, 0, sizeof(g));
+// One axis of Grid::build (grid.cxx:43-95) from its reduced bounds and the
+// largest rns (cell > 0); *small: the axis asks for the small-box build,
+// *bad: too many cells.
+__host__ __device__ inline void grid_axis(const DomainDev& d, double lo, double hi, double cell, int i,
+                                          GridParams& g, bool* small, bool* bad) {
+    g.bmin[i] = d.bmin[i];
+    g.bmax[i] = d.bmax[i];
+    g.size[i] = d.size[i];
+    g.periodic[i] = d.periodic[i];
+    g.dom_n[i] = 1;
+    g.cs[i] = d.size[i];
+    *small = *bad = false;
+    if (!(cell > 0.0)) return;
+    g.num[i] = 1;
+    g.gmin[i] = d.bmin[i];
+    if (i < d.dim) {
+        const double q = floor(d.size[i] / cell);
+        const int c = q > 1.0e9 ? 1000000000 : (int)q;
+        g.dom_n[i] = c > 1 ? c : 1;
+        g.cs[i] = d.size[i] / (double)g.dom_n[i];
+        g.offset[i] = (int)floor((lo - d.bmin[i]) / g.cs[i]);
+        const int u = (int)floor((hi - d.bmin[i]) / g.cs[i]) + 1;
+        g.num[i] = (u < g.dom_n[i] ? u : g.dom_n[i]) - g.offset[i];
+        g.gmin[i] = d.bmin[i] + g.cs[i] * g.offset[i];
+    }
+    g.bricks[i] = (g.num[i] + 3) / 4;
+    g.csf[i] = (float)g.cs[i];
+    g.Lf[i] = (float)d.size[i];
+    g.inv_u[i] = g.cs[i] > 0.0 ? kOffUnits / g.cs[i] : 0.0;
+    g.inv_cs[i] = g.cs[i] > 0.0 ? 1.0 / g.cs[i] : 0.0;
+    // A periodic axis of 3 cells keeps the fast paths: its cells are at
+    // least max rns wide (floor(L / rns) = 3), so every listed pair is
+    // nearer than L / 2 and the image of its neighbour cell is the
+    // minimum image (no per-pair adjustment, the FP32 prefilter holds).
+    // One or two cells per axis (the reference's n = 1, 2 rules), or a
+    // local grid short of the periodic box, take the per-atom body,
+    // whose prefilter takes a per-pair minimum image.
+    *small = d.periodic[i] && i < d.dim && (g.dom_n[i] <= 2 || g.offset[i] != 0 || g.num[i] != g.dom_n[i]);
+    *bad = g.num[i] < 1 || g.num[i] > 1023;
+}
+
+// The grid's totals once its axes are set (g zeroed before them).
+__host__ __device__ inline void grid_totals(const DomainDev& d, double cell, bool small, bool bad, GridParams& g) {
     g.dim = d.dim;
-    double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-    for (int i = 0; i < d.dim; ++i) {
-        lo[i] = lo_in[i];
-        hi[i] = hi_in[i];
-    }
     g.max_rns = cell;
-    for (int i = 0; i < 3; ++i) {
-        g.bmin[i] = d.bmin[i];
-        g.bmax[i] = d.bmax[i];
-        g.size[i] = d.size[i];
-        g.periodic[i] = d.periodic[i];
-        g.dom_n[i] = 1;
-        g.cs[i] = d.size[i];
-    }
     if (!(cell > 0.0)) {
         g.empty = -1;
         return;
     }
-    for (int i = 0; i < d.dim; ++i) {
-        double q = floor(d.size[i] / cell);
-        int c = q > 1.0e9 ? 1000000000 : (int)q;
-        g.dom_n[i] = c > 1 ? c : 1;
-    }
-    for (int i = 0; i < d.dim; ++i) g.cs[i] = d.size[i] / (double)g.dom_n[i];
-    int up[3] = {0, 0, 0};
-    for (int i = 0; i < d.dim; ++i) {
-        g.offset[i] = (int)floor((lo[i] - d.bmin[i]) / g.cs[i]);
-        up[i] = (int)floor((hi[i] - d.bmin[i]) / g.cs[i]);
-        int u = up[i] + 1;
-        up[i] = u < g.dom_n[i] ? u : g.dom_n[i];
-    }
-    for (int i = 0; i < 3; ++i) g.num[i] = 1;
-    for (int i = 0; i < d.dim; ++i) g.num[i] = up[i] - g.offset[i];
-    g.small_box = 0;
-    for (int i = 0; i < 3; ++i) {
-        g.gmin[i] = d.bmin[i];
-        if (i < d.dim) g.gmin[i] = d.bmin[i] + g.cs[i] * g.offset[i];
-        g.bricks[i] = (g.num[i] + 3) / 4;
-        g.csf[i] = (float)g.cs[i];
-        g.Lf[i] = (float)d.size[i];
-        g.inv_u[i] = g.cs[i] > 0.0 ? kOffUnits / g.cs[i] : 0.0;
-        g.inv_cs[i] = g.cs[i] > 0.0 ? 1.0 / g.cs[i] : 0.0;
-        // A periodic axis of 3 cells keeps the fast paths: its cells are at
-        // least max rns wide (floor(L / rns) = 3), so every listed pair is
-        // nearer than L / 2 and the image of its neighbour cell is the
-        // minimum image (no per-pair adjustment, the FP32 prefilter holds).
-        // One or two cells per axis (the reference's n = 1, 2 rules), or a
-        // local grid short of the periodic box, take the per-atom body,
-        // whose prefilter takes a per-pair minimum image.
-        if (d.periodic[i] && i < d.dim &&
-            (g.dom_n[i] <= 2 || g.offset[i] != 0 || g.num[i] != g.dom_n[i]))
-            g.small_box = 1;
-        if (g.num[i] < 1 || g.num[i] > 1023) g.empty = -2;
-    }
-    long long nc = (long long)g.num[0] * g.num[1] * g.num[2];
-    long long nb = 64LL * g.bricks[0] * g.bricks[1] * g.bricks[2];
+    g.small_box = small ? 1 : 0;
+    if (bad) g.empty = -2;
+    const long long nc = (long long)g.num[0] * g.num[1] * g.num[2];
+    const long long nb = 64LL * g.bricks[0] * g.bricks[1] * g.bricks[2];
     if (nb > (1LL << 30)) g.empty = -2;
     g.ncells = (int)nc;
     g.nbins = (int)nb;
+}
+
+// Grid::build from the reduced bounds and the largest rns; shared by the
+// device rebuild (whose axes run on three lanes) and the host-side capacity
+// sizing, so both get the same parameters bit for bit.
+__host__ __device__ inline void grid_from_bounds(const DomainDev& d, const double lo[3], const double hi[3],
+                                                 double cell, GridParams& g) {
+    memset(&g, 0, sizeof(g));
+    bool small = false, bad = false;
+    for (int i = 0; i < 3; ++i) {
+        bool s, b;
+        grid_axis(d, i < d.dim ? lo[i] : 0.0, i < d.dim ? hi[i] : 0.0, cell, i, g, &s, &b);
+        small = small || s;
+        bad = bad || b;
+    }
+    grid_totals(d, cell, small, bad, g);
 }
 
 // floor(x / cs) with the quotient correctly rounded in FP64, as the
@@ -97,13 +103,19 @@ __host__ __device__ inline void grid_from_bounds(const DomainDev& d, const doubl
 // reciprocal 1/cs (itself rounded) lies within 1.5 * 2^-52 (relative) of the
 // exact quotient, as does the rounded quotient, so the two have the same
 // floor unless an integer lies within that distance of the product. Below
-// 2^20 cells that distance is under 3.5e-10: a product within 1e-9 of an
-// integer, or beyond 2^20, takes the division instead.
+// 2^20 cells that distance is under 3.5e-10: a product within 1.1e-9 of an
+// integer, below 2^-10 or beyond 2^20 takes the division instead. The floor
+// and the fraction of the product come from its bits (FP64 comparisons and
+// conversions run at the FP64 rate, one warp instruction in 16 cycles).
 __device__ __forceinline__ int floor_div(double x, double cs, double inv_cs) {
-    const double q = dmul(x, inv_cs);
-    const double f = floor(q);
-    const double frac = dsub(q, f);  // exact: f <= q < f + 1
-    if (frac > 1e-9 && frac < 1.0 - 1e-9 && fabs(q) < 1048576.0) return (int)f;
+    const long long b = __double_as_longlong(dmul(x, inv_cs));
+    const int e = (int)(b >> 52);  // negative products: below 1013
+    if (e >= 1013 && e < 1043) {
+        const int sh = 1075 - e;   // 33 .. 62
+        const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | 0x10000000000000ull;
+        const uint32_t frac = (uint32_t)((m << (64 - sh)) >> 32);  // in units of 2^-32
+        if (frac >= 5u && frac <= 0xfffffffau) return (int)(m >> sh);
+    }
     return (int)floor(__ddiv_rn(x, cs));
 }
 
@@ -167,9 +179,12 @@ __device__ __forceinline__ void wrap_one(const DomainDev& d, double* rx, double*
     }
 }
 
-// Bin key of atom i and its arrival rank in the bin.
+// A packed cell with the atom's clamped flag in its top bit.
+constexpr uint32_t kClampedCell = 1u << 31;
+
+// Bin key of atom i, its arrival rank in the bin and its packed cell.
 __device__ __forceinline__ void bin_count_one(const GridParams& g, int i, const double* rx, const double* ry,
-                                              const double* rz, uint32_t* key, uint32_t* rank,
+                                              const double* rz, uint32_t* key, uint32_t* rank, uint32_t* cell,
                                               uint32_t* bin_count, DevStatus* st) {
     int c[3];
     bool cl;
@@ -181,54 +196,51 @@ __device__ __forceinline__ void bin_count_one(const GridParams& g, int i, const 
     uint32_t k = (uint32_t)bin_key(g, c[0], c[1], c[2]);
     key[i] = k;
     rank[i] = atomicAdd(&bin_count[k], 1u);
+    cell[i] = pack_cell(c[0], c[1], c[2]) | (cl ? kClampedCell : 0u);
 }
 
-// Deterministic order inside bin b: ascending caller index.
-__device__ __forceinline__ void bin_sort_one(int b, const uint32_t* start, uint32_t* src, const uint32_t* orig) {
-    uint32_t s = start[b], e = start[b + 1];
-    for (uint32_t k = s + 1; k < e; ++k) {
-        uint32_t v = src[k];
-        uint32_t ov = orig[v];
-        uint32_t m = k;
-        while (m > s && orig[src[m - 1]] > ov) {
-            src[m] = src[m - 1];
-            --m;
-        }
-        src[m] = v;
-    }
+// Slot of the atom that arrived k-th (src[k] = i) once every bin is ordered
+// by caller index: its bin's start plus the number of smaller caller indices
+// in the bin (orig_at: caller indices in arrival order).
+__device__ __forceinline__ uint32_t sorted_slot(uint32_t k, uint32_t bin, const uint32_t* start,
+                                                const uint32_t* orig_at) {
+    const uint32_t s = start[bin], e = start[bin + 1], o = orig_at[k];
+    uint32_t d = s;
+    for (uint32_t m = s; m < e; ++m) d += orig_at[m] < o;
+    return d;
 }
 
-// Cell centre, cell-relative FP32 offsets and packed cell of atom i.
-__device__ __forceinline__ void cells_one(const GridParams& g, int i, const double* rx, const double* ry,
-                                          const double* rz, uint32_t* cellp, double* Rx, double* Ry, double* Rz,
-                                          int4* pos32, int4* q0, float4* o0, const uint32_t* orig,
-                                          uint32_t* slot_of, const uint16_t* kind) {
-    double r[3] = {rx[i], ry[i], rz[i]};
+// Cell centre, cell-relative FP32 offsets and packed cell of the atom in slot
+// i, at r with packed cell `cell` (bin_count_one) and caller index o.
+__device__ __forceinline__ void cells_one(const GridParams& g, int i, const double r[3], uint32_t cell, uint32_t o,
+                                          uint16_t kind, uint32_t* cellp, double* Rx, double* Ry, double* Rz,
+                                          int4* pos32, int4* q0, float4* o0, uint32_t* slot_of) {
+    const bool cl = (cell & kClampedCell) != 0;
+    cell &= ~kClampedCell;
+    cellp[i] = cell;
     int c[3];
-    bool cl;
-    local_cell(g, r[0], r[1], r[2], c, cl);
-    cellp[i] = pack_cell(c[0], c[1], c[2]);
+    unpack_cell(cell, c[0], c[1], c[2]);
     double R[3];
-    float o[3];
+    float of[3];
     int q[3];
     bool outlier = cl;
     for (int a = 0; a < 3; ++a) {
         R[a] = g.gmin[a] + ((double)c[a] + 0.5) * g.cs[a];
         if (a >= g.dim) R[a] = r[a];
-        o[a] = (float)(r[a] - R[a]);
+        of[a] = (float)(r[a] - R[a]);
         q[a] = off_encode(r[a] - R[a], g.inv_u[a]);
-        if (fabsf(o[a]) > 0.75f * g.csf[a] && a < g.dim) outlier = true;
+        if (fabsf(of[a]) > 0.75f * g.csf[a] && a < g.dim) outlier = true;
     }
     Rx[i] = R[0];
     Ry[i] = R[1];
     Rz[i] = R[2];
-    pos32[i] = make_int4(q[0], q[1], q[2], kind[i] & 3);  // w: the atom's kind (Multi passes)
+    pos32[i] = make_int4(q[0], q[1], q[2], kind & 3);  // w: the atom's kind (Multi passes)
     q0[i] = make_int4(q[0], q[1], q[2], 0);
     // w: 0 exact offsets; 1 not exact (the FP32 tests send its pairs to FP64);
     // 2 clamped into the grid (also not exact: its list is walked from the
     // unclamped cell, nbuild_atom)
-    o0[i] = make_float4(o[0], o[1], o[2], cl ? 2.0f : outlier ? 1.0f : 0.0f);
-    slot_of[orig[i]] = (uint32_t)i;
+    o0[i] = make_float4(of[0], of[1], of[2], cl ? 2.0f : outlier ? 1.0f : 0.0f);
+    slot_of[o] = (uint32_t)i;
 }
 
 // Every permuted field of one rebuild: the gathers into the spare buffers
@@ -314,11 +326,13 @@ __device__ __forceinline__ float min_image_f(float d, float L) {
     return d;
 }
 
-// The list of atom i (one thread per atom, over the whole grid: used for
-// grids with a periodic axis of 2 cells or fewer, which have few cells of
-// many atoms each): its cell's 27 (or fewer, on small periodic axes)
-// neighbour cells in the reference's order, x outer, z inner, each cell's
-// atoms in slot order. The FP32 prefilter also holds on periodic axes of
+// The list of atom i by a warp, lanes over the candidates (used for grids
+// with a periodic axis of 2 cells or fewer, which have few cells of many
+// atoms each): its cell's 27 (or fewer, on small periodic axes) neighbour
+// cells in the reference's order, x outer, z inner, each cell's atoms in
+// slot order, 32 at a time; the accepted lanes append in lane order. (A
+// thread per atom walks its ~500 candidates alone: 303 us for 500 LJ atoms.)
+// The FP32 prefilter also holds on periodic axes of
 // one or two cells when the grid covers the whole box: every cell there is
 // an edge cell, so the exact test takes the minimum image, and the FP32
 // minimum image of the neighbour cell's displacement is the same distance
@@ -329,7 +343,8 @@ __device__ __forceinline__ float min_image_f(float d, float L) {
 // but, as Grid::adjacent_cells (grid.cxx:138-207) takes the cell of the
 // position itself, its own walk and edge flags come from the unclamped cell;
 // the image codes stay relative to the cell it is binned in.
-__device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g, uint32_t i, bool uniform_rns) {
+__device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g, uint32_t i, int lane,
+                                            bool uniform_rns) {
     // prefilter band: rns^2 (1 -/+ 1e-5), valid when every atom has the same rns
     const float lo2 = (float)(g.max_rns * g.max_rns * (1.0 - 1e-5));
     const float hi2 = (float)(g.max_rns * g.max_rns * (1.0 + 1e-5));
@@ -389,33 +404,39 @@ __device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g
                 // image of the neighbour cell relative to the binned cell
                 const int dl[3] = {x + shift[0], y + shift[1], z + shift[2]};
                 const float sh[3] = {(float)dl[0] * g.csf[0], (float)dl[1] * g.csf[1], (float)dl[2] * g.csf[2]};
-                for (uint32_t j = j0; j < j1; ++j) {
-                    if (j == i) continue;
-                    if (A.half && A.orig[j] < origi) continue;
-                    const float4 oj = A.o0[j];
-                    const float dx = oi.x - oj.x - sh[0];
-                    const float dy = oi.y - oj.y - sh[1];
-                    const float dz = oi.z - oj.z - sh[2];
-                    const float ex = mi[0] ? min_image_f(dx, g.Lf[0]) : dx;
-                    const float ey = mi[1] ? min_image_f(dy, g.Lf[1]) : dy;
-                    const float ez = mi[2] ? min_image_f(dz, g.Lf[2]) : dz;
-                    const float d2 = ex * ex + ey * ey + ez * ez;
-                    bool acc;
-                    if (pfi && oj.w == 0.0f && d2 < lo2) acc = true;
-                    else if (pfi && oj.w == 0.0f && d2 > hi2) acc = false;
-                    else acc = are_neibs_exact(g, xi, yi, zi, rni, A.rx[j], A.ry[j], A.rz[j], A.rns[j], edge);
-                    if (!acc) continue;
-                    // periodic image code: minimum image of j seen from i
-                    const uint32_t code = pair_image_code(g, own, lc, dl, dx, dy, dz, A.st);
-                    if (cnt < A.K) A.nbr[nidx(cnt, i, A.np)] = j | (code << kJBits);
-                    ++cnt;
+                for (uint32_t jb = j0; jb < j1; jb += 32) {
+                    const uint32_t j = jb + lane;
+                    bool acc = j < j1 && j != i && !(A.half && A.orig[j] < origi);
+                    float dx = 0.f, dy = 0.f, dz = 0.f;
+                    if (acc) {
+                        const float4 oj = A.o0[j];
+                        dx = oi.x - oj.x - sh[0];
+                        dy = oi.y - oj.y - sh[1];
+                        dz = oi.z - oj.z - sh[2];
+                        const float ex = mi[0] ? min_image_f(dx, g.Lf[0]) : dx;
+                        const float ey = mi[1] ? min_image_f(dy, g.Lf[1]) : dy;
+                        const float ez = mi[2] ? min_image_f(dz, g.Lf[2]) : dz;
+                        const float d2 = ex * ex + ey * ey + ez * ez;
+                        if (pfi && oj.w == 0.0f && d2 < lo2) acc = true;
+                        else if (pfi && oj.w == 0.0f && d2 > hi2) acc = false;
+                        else acc = are_neibs_exact(g, xi, yi, zi, rni, A.rx[j], A.ry[j], A.rz[j], A.rns[j], edge);
+                    }
+                    const unsigned m = __ballot_sync(0xffffffffu, acc);
+                    if (acc) {
+                        // periodic image code: minimum image of j seen from i
+                        const uint32_t code = pair_image_code(g, own, lc, dl, dx, dy, dz, A.st);
+                        const int k = cnt + __popc(m & ((1u << lane) - 1u));
+                        if (k < A.K) A.nbr[nidx(k, i, A.np)] = j | (code << kJBits);
+                    }
+                    cnt += __popc(m);
                 }
             }
         }
     }
     // pad to a multiple of four with self entries
     const int padded = (cnt + 3) & ~3;
-    for (int k = cnt; k < padded && k < A.K; ++k) A.nbr[nidx(k, i, A.np)] = i | kSelfCode;
+    if (cnt + lane < padded && cnt + lane < A.K) A.nbr[nidx(cnt + lane, i, A.np)] = i | kSelfCode;
+    if (lane) return;
     A.ncnt[i] = padded < A.K ? padded : A.K;
     if (cnt > A.K) {
         atomicOr(&A.st->flags, FLAG_OVERFLOW);
@@ -433,32 +454,73 @@ __device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g
 // ---- list build, a warp per cell with lanes over candidates -------------------
 // The cell's candidates are the atoms of its neighbour cells in the
 // reference's cell order (x outer, z inner), each cell's atoms in slot order.
-// Lanes take 32 consecutive candidates; the warp walks the cell's atoms, one
-// ballot per atom, so lane i ends with atom i's row of the chunk's accept
-// matrix and appends those candidates in lane order.
-// Entry order per atom is therefore the order of the per-atom loop in
-// nbuild_atom, and the lists are the same, entry for entry. Used when no
-// periodic axis has 2 cells or fewer (no minimum-image adjustment of the
-// image code, GridParams::small_box); otherwise nbuild_atom runs.
+// Lanes take 32 consecutive candidates (a chunk); the warp walks the cell's
+// atoms, one ballot per atom, so a chunk's accept matrix ends as one row per
+// atom in shared memory. After CH chunks lane i appends the accepted
+// candidates of atom i, in order. Entry order per atom is therefore the order
+// of the per-atom loop in nbuild_atom, and the lists are the same, entry for
+// entry. Used when no periodic axis has 2 cells or fewer (no minimum-image
+// adjustment of the image code, GridParams::small_box); otherwise nbuild_atom
+// runs.
+//
+// The build is bound by instruction issue, so a test is as few instructions
+// as it takes: the squared distance from the threshold mid as |b|^2 + (|a|^2 - mid) - 2 a.b, three
+// fused operations, two atoms at once in packed FP32 pairs; the rows go to
+// shared memory once per pair of atoms; and appending waits for CH chunks, as
+// the lanes' counts even out (the longest of 19 lanes then has 1.2 times the
+// mean instead of twice it). LJ liquid 500,000 atoms: 405 us with one
+// distance per atom and an append per chunk.
+template <int CH>
 struct NbWarpSmem {
+    float4 csh[27];          // cell shift (x, y, z) of the image
+    float4 oa[32];           // pairs of atoms: (-2ax0, -2ax1, -2ay0, -2ay1), (-2az0, -2az1, m0, m1), m = |a|^2 - mid
+    float4 oi[32];           // the batch's offsets
+    uint32_t row[CH][32];    // accept rows of the turn's chunks: bit = candidate, column = atom
+    uint32_t cand[CH * 32];  // the turn's list entries (slot | image code)
+    uint32_t origi[32];
     uint32_t cj0[27];        // first slot of each non-empty neighbour cell
     uint32_t cpre[28];       // candidate prefix over those cells
     uint32_t ccode[27];      // image code << kJBits
-    float4 csh[27];          // cell shift (x, y, z) of the image
-    float4 oi[32];           // the batch's offsets
-    uint32_t origi[32];
-    uint32_t cand[32];       // the chunk's list entries (slot | image code)
 };
 
-__device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridParams& g, int bin, int lane,
-                                                 bool uniform_rns, NbWarpSmem& S) {
+// Packed pairs of FP32 numbers.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+
+// The lists of part `part` of `parts` of the bin's atoms.
+template <int CH>
+__device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridParams& g, int bin, int part, int parts,
+                                                 int lane, bool uniform_rns, NbWarpSmem<CH>& S) {
     const unsigned full = 0xffffffffu;
     const float lo2 = (float)(g.max_rns * g.max_rns * (1.0 - 1e-5));
     const float hi2 = (float)(g.max_rns * g.max_rns * (1.0 + 1e-5));
-    const uint32_t s0 = A.bin_start[bin], s1 = A.bin_start[bin + 1];
+    uint32_t s0 = A.bin_start[bin], s1 = A.bin_start[bin + 1];
     if (s0 == s1) return;
     int cx, cy, cz;
     unpack_cell(A.cellp[s0], cx, cy, cz);
+    const uint32_t home0 = s0;  // the bin's first slot
+    if (parts > 1) {
+        const uint32_t per = (s1 - s0 + parts - 1) / parts;
+        s0 += part * per;
+        s1 = min(s0 + per, s1);
+        if (s0 >= s1) return;
+    }
     int gc[3] = {cx + g.offset[0], cy + g.offset[1], cz + g.offset[2]};
     if (g.dim < 3) gc[2] = 0;
     if (g.dim < 2) gc[1] = 0;
@@ -477,7 +539,7 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
         if (valid) {
             int nb[3] = {gc[0] + dl[0], gc[1] + dl[1], gc[2] + dl[2]};
             for (int a = 0; a < 3; ++a)
-                if (g.periodic[a]) nb[a] = (nb[a] + g.dom_n[a]) % g.dom_n[a];
+                if (g.periodic[a]) nb[a] = nb[a] < 0 ? nb[a] + g.dom_n[a] : nb[a] >= g.dom_n[a] ? nb[a] - g.dom_n[a] : nb[a];
             const int lc[3] = {nb[0] - g.offset[0], nb[1] - g.offset[1], nb[2] - g.offset[2]};
             if (lc[0] < 0 || lc[0] >= g.num[0] || lc[1] < 0 || lc[1] >= g.num[1] || lc[2] < 0 || lc[2] >= g.num[2]) {
                 valid = false;
@@ -514,103 +576,130 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
     // the cell itself (lane 13: offset (0, 0, 0)) among the used cells
     const int home = __popc(vm & ((1u << 13) - 1u));
     __syncwarp();
-    const float kInf = __int_as_float(0x7f800000), kNaN = __int_as_float(0x7fffffff);
+
+    // The packed test's threshold and its error: the terms are at most
+    // |b|^2 < 9.2 cs^2 (offsets within 0.75 cells, one cell apart) and each of
+    // its seven roundings adds 2^-24 of the largest partial sum, below 5e-6 cs^2
+    // in all; pairs within `half` of the middle go to the exact tests.
+    const float csm = fmaxf(g.csf[0], fmaxf(g.csf[1], g.csf[2]));
+    const float mid = 0.5f * (lo2 + hi2), half_band = fmaf(6e-6f * csm, csm, 0.5f * (hi2 - lo2));
 
     for (uint32_t base = s0; base < s1; base += 32) {
         const uint32_t ni = s1 - base < 32u ? s1 - base : 32u;
         const bool act = (uint32_t)lane < ni;
         const uint32_t me = base + lane;
+        float4 oa = make_float4(0.f, 0.f, 0.f, 0.f);
         if (act) {
-            // an atom whose offset is not exact carries NaN in z and w: its
-            // pairs fail every FP32 test (w is the flag the FP32 tests read)
-            float4 o = A.o0[me];
-            if (o.w != 0.0f) o.z = o.w = kNaN;
-            S.oi[lane] = o;
+            oa = A.o0[me];
+            S.oi[lane] = oa;
             S.origi[lane] = A.orig[me];
         }
+        // an atom whose offset is not exact takes the batch to the exact tests
+        const bool rough = __any_sync(full, oa.w != 0.0f) || !uniform_rns || A.half;
+        {
+            // columns past the batch (the second of an odd pair) accept nothing
+            const float a2 = fmaf(oa.x, oa.x, fmaf(oa.y, oa.y, oa.z * oa.z));
+            const float m = act ? a2 - mid : 3e38f;
+            float* q = reinterpret_cast<float*>(&S.oa[lane & ~1]) + (lane & 1);
+            q[0] = -2.0f * oa.x;
+            q[2] = -2.0f * oa.y;
+            q[4] = -2.0f * oa.z;
+            q[6] = m;
+        }
         // this atom's own candidate index (it is a candidate of its own cell)
-        const uint32_t self_t = act ? S.cpre[home] + (me - S.cj0[home]) : 0xffffffffu;
+        const uint32_t self_t = act ? S.cpre[home] + (me - home0) : 0xffffffffu;
         __syncwarp();
         int cnt = 0;  // list length of atom `me`
         int c = 0;    // neighbour cell of this lane's candidate
-        for (uint32_t tb = 0; tb < T; tb += 32) {
-            const uint32_t t = tb + lane;
-            const bool have = t < T;
-            uint32_t j = 0xffffffffu, origj = 0;
-            float px = 0.f, py = 0.f, pz = 0.f;
-            bool pfj = false;
-            if (have) {
-                while (S.cpre[c + 1] <= t) ++c;
-                j = S.cj0[c] + (t - S.cpre[c]);
-                const float4 oj = A.o0[j];
-                const float4 shj = S.csh[c];
+        uint32_t* dst = A.nbr + ((size_t)me << 2);
+        // the lane's candidate of the next chunk, fetched a chunk ahead
+        uint32_t jn = 0;
+        float4 on = make_float4(0.f, 0.f, 0.f, 0.f), shn = on;
+        uint32_t en = 0;
+        auto fetch = [&](uint32_t t) {
+            if (t >= T) return;
+            while (S.cpre[c + 1] <= t) ++c;
+            jn = S.cj0[c] + (t - S.cpre[c]);
+            on = A.o0[jn];
+            shn = S.csh[c];
+            en = jn | S.ccode[c];
+        };
+        fetch(lane);
+        for (uint32_t t0 = 0; t0 < T; t0 += CH * 32) {
+            const int nch = min((int)((T - t0 + 31) >> 5), CH);
+            for (int ch = 0; ch < nch; ++ch) {
+                const uint32_t t = t0 + 32 * ch + lane;
+                const bool have = t < T;
+                const uint32_t j = jn;
                 // the candidate seen from the cell: offset + image shift
-                px = oj.x + shj.x;
-                py = oj.y + shj.y;
-                pz = oj.z + shj.z;
-                pfj = uniform_rns && oj.w == 0.0f;
-                if (A.half) origj = A.orig[j];
-                S.cand[lane] = j | S.ccode[c];
+                const float px = have ? on.x + shn.x : 0.f, py = have ? on.y + shn.y : 0.f, pz = have ? on.z + shn.z : 0.f;
+                const bool pfj = on.w == 0.0f;
+                S.cand[32 * ch + lane] = en;
+                fetch(t + 32);
+                bool exact = rough || __any_sync(full, have && !pfj);
+                if (!exact) {
+                    const float b2 = have ? fmaf(px, px, fmaf(py, py, pz * pz)) : 3e38f;
+                    const unsigned long long bx = pack2(px, px), by = pack2(py, py), bz = pack2(pz, pz),
+                                             bb = pack2(b2, b2);
+                    float near = 3e38f;  // least distance from the threshold
+                    for (uint32_t ii = 0; ii < ni; ii += 2) {
+                        const ulonglong2 u = reinterpret_cast<const ulonglong2*>(S.oa)[ii];
+                        const ulonglong2 v = reinterpret_cast<const ulonglong2*>(S.oa)[ii + 1];
+                        float d0, d1;
+                        unpack2(fma2(u.x, bx, fma2(u.y, by, fma2(v.x, bz, add2(bb, v.y)))), d0, d1);
+                        const unsigned m0 = __ballot_sync(full, d0 < 0.0f), m1 = __ballot_sync(full, d1 < 0.0f);
+                        near = fminf(near, fminf(fabsf(d0), fabsf(d1)));
+                        if (lane == 0) *reinterpret_cast<uint2*>(&S.row[ch][ii]) = make_uint2(m0, m1);
+                    }
+                    exact = __any_sync(full, near <= half_band);
+                }
+                if (exact) {
+                    // pairs within 1e-5 of rns (or of atoms whose offsets are
+                    // not exact) are marked in a second row and settled in FP64
+                    __syncwarp();
+                    unsigned mine = 0, mine_x = 0;
+                    const uint32_t origj = A.half && have ? A.orig[j] : 0u;
+                    for (uint32_t ii = 0; ii < ni; ++ii) {
+                        const float4 oi = S.oi[ii];
+                        const float dx = oi.x - px, dy = oi.y - py, dz = oi.z - pz;
+                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                        const bool pf = uniform_rns && pfj && oi.w == 0.0f;
+                        const bool ok = have && j != base + ii && !(A.half && origj < S.origi[ii]);
+                        const unsigned m = __ballot_sync(full, ok && pf && d2 < lo2);
+                        const unsigned mx = __ballot_sync(full, ok && !(pf && (d2 < lo2 || d2 > hi2)));
+                        if ((uint32_t)lane == ii) {
+                            mine = m;
+                            mine_x = mx;
+                        }
+                    }
+                    while (mine_x) {
+                        const int b = __ffs(mine_x) - 1;
+                        mine_x &= mine_x - 1u;
+                        const uint32_t jb = S.cand[32 * ch + b] & kJMask;
+                        if (are_neibs_exact(g, A.rx[me], A.ry[me], A.rz[me], A.rns[me], A.rx[jb], A.ry[jb], A.rz[jb],
+                                            A.rns[jb], edge))
+                            mine |= 1u << b;
+                    }
+                    if (act) S.row[ch][lane] = mine;
+                }
             }
             __syncwarp();
-            // row ii of the chunk's accept matrix lands in lane ii; pairs
-            // within 1e-5 of rns (or of atoms whose offsets are not exact)
-            // are marked in a second row and settled in FP64 below
-            unsigned mine = 0, mine_x = 0;
-            bool exact = A.half;
-            if (!A.half) {
-                // One ballot per atom: the candidate's coordinates are +inf
-                // without a candidate and NaN when the prefilter cannot
-                // decide its pairs, so neither is ever accepted here; the
-                // atom's own slot is cleared after the loop. A pair that the
-                // prefilter cannot settle (band, NaN) sends the whole chunk
-                // to the loop below, whose rows are therefore the same.
-                const float qx = !have ? kInf : pfj ? px : kNaN;
-                bool band = false;
-#pragma unroll 2
-                for (uint32_t ii = 0; ii < ni; ++ii) {
-                    const float4 oi = S.oi[ii];
-                    const float dx = oi.x - qx, dy = oi.y - py, dz = oi.z - pz;
-                    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    const bool sure = d2 < lo2;
-                    const unsigned m = __ballot_sync(full, sure);
-                    band |= !sure && !(d2 > hi2);
-                    if ((uint32_t)lane == ii) mine = m;
-                }
-                if (self_t - tb < 32u) mine &= ~(1u << (self_t - tb));
-                exact = __any_sync(full, band);
-            }
-            if (exact) {
-                mine = 0;
-#pragma unroll 2
-                for (uint32_t ii = 0; ii < ni; ++ii) {
-                    const float4 oi = S.oi[ii];
-                    const float dx = oi.x - px, dy = oi.y - py, dz = oi.z - pz;
-                    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    const bool pf = pfj && oi.w == 0.0f;
-                    const bool ok = have && j != base + ii && !(A.half && origj < S.origi[ii]);
-                    const unsigned m = __ballot_sync(full, ok && pf && d2 < lo2);
-                    const unsigned mx = __ballot_sync(full, ok && !(pf && (d2 < lo2 || d2 > hi2)));
-                    if ((uint32_t)lane == ii) {
-                        mine = m;
-                        mine_x = mx;
-                    }
-                }
-            }
-            while (mine_x) {
-                const int b = __ffs(mine_x) - 1;
-                mine_x &= mine_x - 1u;
-                const uint32_t jb = S.cand[b] & kJMask;
-                if (are_neibs_exact(g, A.rx[me], A.ry[me], A.rz[me], A.rns[me], A.rx[jb], A.ry[jb], A.rz[jb],
-                                    A.rns[jb], edge))
-                    mine |= 1u << b;
-            }
             // append this atom's accepted candidates in candidate order
-            while (mine) {
-                const int b = __ffs(mine) - 1;
-                mine &= mine - 1u;
-                if (cnt < A.K) A.nbr[nidx(cnt, me, A.np)] = S.cand[b];
-                ++cnt;
+            if (act) {
+                unsigned w = 0;
+                for (int ch = 0;;) {
+                    while (w == 0 && ch < nch) {
+                        w = S.row[ch][lane];
+                        if (self_t - (t0 + 32 * ch) < 32u) w &= ~(1u << (self_t & 31u));
+                        ++ch;
+                    }
+                    if (w == 0) break;
+                    const int b = __ffs(w) - 1;
+                    w &= w - 1u;
+                    if (cnt < A.K) *dst = S.cand[32 * (ch - 1) + b];
+                    ++cnt;
+                    dst += (cnt & 3) ? 1 : 4 * (size_t)A.np - 3;
+                }
             }
             __syncwarp();
         }

@@ -77,6 +77,9 @@ struct alignas(16) SoloArgs {
 };
 
 constexpr int kSoloMaxAtoms = 65536;
+// Chunks per turn of the list build here: few, as its shared memory is taken
+// from the L1 that the force passes gather through.
+constexpr int kSoloChunks = 4;
 
 template <int NT>
 __device__ __forceinline__ void gather_block(const GatherAll& G, const uint32_t* src, int n) {
@@ -172,7 +175,7 @@ __device__ __noinline__ bool solo_rebuild(const SoloArgs& S, GridParams& g, doub
     const int nb = g.nbins;
     for (long long b = t; b < S.bin_cap; b += NT) S.bin_count[b] = 0;
     __syncthreads();
-    for (int i = t; i < n; i += NT) bin_count_one(g, i, S.rx, S.ry, S.rz, S.key, S.rank, S.bin_count, S.st);
+    for (int i = t; i < n; i += NT) bin_count_one(g, i, S.rx, S.ry, S.rz, S.key, S.rank, S.N.ncnt, S.bin_count, S.st);
     __syncthreads();
     // exclusive scan: each thread a contiguous chunk of the bins
     {
@@ -190,16 +193,29 @@ __device__ __noinline__ bool solo_rebuild(const SoloArgs& S, GridParams& g, doub
         if (t == 0) S.bin_start[nb] = tot;
     }
     __syncthreads();
-    for (int i = t; i < n; i += NT) S.src[S.bin_start[S.key[i]] + S.rank[i]] = (uint32_t)i;
+    // arrival order (the atoms' cells wait in ncnt, their caller indices in
+    // arrival order in cellp), then each bin by caller index (into rank)
+    for (int i = t; i < n; i += NT) {
+        const uint32_t k = S.bin_start[S.key[i]] + S.rank[i];
+        S.src[k] = (uint32_t)i;
+        S.cellp[k] = S.orig[i];
+    }
     __syncthreads();
-    for (int b = t; b < nb; b += NT) bin_sort_one(b, S.bin_start, S.src, S.orig);
+    for (int k = t; k < n; k += NT) {
+        const uint32_t i = S.src[k];
+        S.rank[sorted_slot(k, S.key[i], S.bin_start, S.cellp)] = i;
+    }
     __syncthreads();
-    gather_block<NT>(S.G, S.src, n);
+    gather_block<NT>(S.G, S.rank, n);
+    for (int k = t; k < n; k += NT) S.src[k] = S.N.ncnt[S.rank[k]];
     __syncthreads();
     copy_back_block<NT>(S.G, n);
     __syncthreads();
-    for (int i = t; i < n; i += NT)
-        cells_one(g, i, S.rx, S.ry, S.rz, S.cellp, S.Rx, S.Ry, S.Rz, S.pos32, S.q0, S.o0, S.orig, S.slot_of, S.F.kind);
+    for (int i = t; i < n; i += NT) {
+        const double r[3] = {S.rx[i], S.ry[i], S.rz[i]};
+        cells_one(g, i, r, S.src[i], S.orig[i], S.F.kind[i], S.cellp, S.Rx, S.Ry, S.Rz, S.pos32, S.q0, S.o0,
+                  S.slot_of);
+    }
     __syncthreads();
     {
         const bool uniform = S.st->nonuniform == 0;
@@ -208,20 +224,20 @@ __device__ __noinline__ bool solo_rebuild(const SoloArgs& S, GridParams& g, doub
             // build's body); its per-warp state is the launch's dynamic
             // shared memory
             extern __shared__ __align__(16) unsigned char solo_dyn[];
-            NbWarpSmem* nbs = reinterpret_cast<NbWarpSmem*>(solo_dyn);
-            for (int b = w; b < nb; b += NT / 32) nbuild_cell_warp(S.N, g, b, lane, uniform, nbs[w]);
+            NbWarpSmem<kSoloChunks>* nbs = reinterpret_cast<NbWarpSmem<kSoloChunks>*>(solo_dyn);
+            for (int b = w; b < nb; b += NT / 32) nbuild_cell_warp(S.N, g, b, 0, 1, lane, uniform, nbs[w]);
         } else {
-            // a few cells of many atoms: a thread per atom
-            for (int i = t; i < n; i += NT) nbuild_atom(S.N, g, (uint32_t)i, uniform);
+            // a few cells of many atoms: a warp per atom
+            for (int i = w; i < n; i += NT / 32) nbuild_atom(S.N, g, (uint32_t)i, lane, uniform);
         }
         __syncthreads();
         // atoms clamped into the grid: their own lists from their unclamped cells
         if (!g.small_box && (S.st->build_flags & FLAG_RANGE))
-            for (int i = t; i < n; i += NT)
-                if (S.N.o0[i].w == 2.0f) nbuild_atom(S.N, g, (uint32_t)i, uniform);
+            for (int i = w; i < n; i += NT / 32)
+                if (S.N.o0[i].w == 2.0f) nbuild_atom(S.N, g, (uint32_t)i, lane, uniform);
     }
     __syncthreads();
-    for (int i = t; i < n; i += NT) trig_one(i, S.saved_rns, S.saved_rcut, g, S.trig);
+    for (int i = t; i < n; i += NT) S.trig[i] = trig_of(S.saved_rns[i], S.saved_rcut[i], g);
     __syncthreads();
     bool ok = !(S.st->build_flags & FLAG_OVERFLOW);
     __syncthreads();
@@ -530,7 +546,7 @@ int solo_out_read(const void* out_host, uint32_t* done, unsigned long long* left
 }
 
 // Dynamic shared memory of a launch: the list build's state, one per warp.
-static size_t solo_dyn_bytes(int threads) { return (size_t)(threads / 32) * sizeof(NbWarpSmem); }
+static size_t solo_dyn_bytes(int threads) { return (size_t)(threads / 32) * sizeof(NbWarpSmem<kSoloChunks>); }
 
 // The launch's dynamic shared memory exceeds the default 48 KB at 1024
 // threads; the attribute is per device, so it is set once per device.
