@@ -177,22 +177,24 @@ __global__ void k_measure2(MArgs A, const double* __restrict__ com) {
     if (threadIdx.x == 0) A.part[blockIdx.x * 8 + 7] = sh[0];
 }
 
-__global__ void k_measure_final(const double* __restrict__ part, int nparts, int stage, double* __restrict__ out) {
-    // one thread, fixed order: deterministic
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// The blocks' partial sums in one block: a thread per eight columns' worth of
+// rows, then a tree (a fixed order, so deterministic). One thread's chain of
+// nparts FP64 additions took 90 us at 432 parts.
+__global__ void __launch_bounds__(kBlock)
+    k_measure_final(const double* __restrict__ part, int nparts, int stage, double* __restrict__ out) {
+    __shared__ double sh[7 * kBlock];
+    double v[7] = {0, 0, 0, 0, 0, 0, 0};
+    const int nv = stage == 1 ? 7 : 1, at = stage == 1 ? 0 : 7;
+    for (int b = threadIdx.x; b < nparts; b += kBlock)
+        for (int k = 0; k < nv; ++k) v[k] += part[b * 8 + at + k];
+    block_sum(sh, v, nv);
+    if (threadIdx.x != 0) return;
     if (stage == 1) {
-        double s[7] = {0, 0, 0, 0, 0, 0, 0};
-        for (int b = 0; b < nparts; ++b)
-            for (int k = 0; k < 7; ++k) s[k] += part[b * 8 + k];
-        for (int k = 0; k < 7; ++k) out[k] = s[k];
-        double tm = s[6];
-        out[8] = tm > 0.0 ? s[3] / tm : 0.0;
-        out[9] = tm > 0.0 ? s[4] / tm : 0.0;
-        out[10] = tm > 0.0 ? s[5] / tm : 0.0;
+        for (int k = 0; k < 7; ++k) out[k] = sh[k * kBlock];
+        const double tm = out[6];
+        for (int k = 0; k < 3; ++k) out[8 + k] = tm > 0.0 ? out[3 + k] / tm : 0.0;
     } else {
-        double ke = 0.0;
-        for (int b = 0; b < nparts; ++b) ke += part[b * 8 + 7];
-        out[7] = ke;
+        out[7] = sh[0];
     }
 }
 
@@ -372,11 +374,11 @@ int launch_measure(mdg_system* sys, double out[11]) {
     A.part = sys->part;
     k_measure1<<<nparts, kBlock, 0, st>>>(A);
     MDG_LAUNCHED(ctx);
-    k_measure_final<<<1, 32, 0, st>>>(sys->part, nparts, 1, sys->red);
+    k_measure_final<<<1, kBlock, 0, st>>>(sys->part, nparts, 1, sys->red);
     MDG_LAUNCHED(ctx);
     k_measure2<<<nparts, kBlock, 0, st>>>(A, sys->red + 8);
     MDG_LAUNCHED(ctx);
-    k_measure_final<<<1, 32, 0, st>>>(sys->part, nparts, 2, sys->red);
+    k_measure_final<<<1, kBlock, 0, st>>>(sys->part, nparts, 2, sys->red);
     MDG_LAUNCHED(ctx);
     MDG_CUDA(cudaMemcpyAsync(sys->hred, sys->red, 11 * sizeof(double), cudaMemcpyDeviceToHost, st));
     MDG_CUDA(cudaStreamSynchronize(st));

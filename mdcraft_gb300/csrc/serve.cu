@@ -123,7 +123,7 @@ struct mdg_server {
     int threads = 512, blocks = 0; // persistent kernel shape
     SoloQueue* q = nullptr;        // host-mapped request queue
     SoloQueue* q_dev = nullptr;
-    uint32_t* head = nullptr;      // next entry to claim (device)
+    uint32_t* head = nullptr;      // next entry to claim, requests running (device)
     uint32_t published = 0;
     std::deque<AllocGroup> alloc_groups;
     std::vector<cudaEvent_t> free_events;
@@ -678,8 +678,10 @@ int mdg_server_create(int device, const mdg_server_config* cfg, mdg_server** out
             if (e == cudaSuccess) e = cudaHostAlloc((void**)&sv->q, sizeof(SoloQueue), cudaHostAllocMapped);
             if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&sv->q_dev, sv->q, 0);
             if (e == cudaSuccess) memset((void*)sv->q, 0, sizeof(SoloQueue));
-            if (e == cudaSuccess) e = cudaMalloc(&sv->head, sizeof(uint32_t));
-            if (e == cudaSuccess) e = cudaMemset(sv->head, 0, sizeof(uint32_t));
+            if (e == cudaSuccess) e = cudaMalloc(&sv->head, 2 * sizeof(uint32_t));
+            if (e == cudaSuccess) e = cudaMemset(sv->head, 0, 2 * sizeof(uint32_t));
+            // done before a kernel on another (non-blocking) stream reads it
+            if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
             if (e != cudaSuccess) rc = cuda_status(e, "server queue");
         }
         // persistent kernel: block size, and as many blocks as fit on the GPU

@@ -415,10 +415,18 @@ __device__ __forceinline__ uint32_t ld_acquire_sys(const volatile uint32_t* p) {
     return v;
 }
 
+// Polls without an entry after which a block exits when no block is running a
+// request (about 0.1 ms). While some are, it waits on for idle_limit polls,
+// so that the next request finds it. (With idle_limit alone, 100,000 polls,
+// a batch's blocks held every SM for 0.23 s after its last result, which any
+// other kernel, or a caller that waits for the device, sat through.)
+constexpr int kQuietPolls = 64;
+
 // Persistent consumer of the request queue: each block claims the next
 // published entry, runs that request, and claims again; a block that finds
-// no entry for `idle_limit` polls (about a microsecond apart), or sees
-// `stop`, exits. Every wait is bounded.
+// no entry for `idle_limit` polls (about a microsecond apart), or for
+// kQuietPolls with no request running, or sees `stop`, exits. Every wait is
+// bounded. head[0]: the next entry to claim; head[1]: requests running.
 template <int NT>
 __global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* desc, SoloQueue* q,
                                                            uint32_t* head, int idle_limit, int gen) {
@@ -433,18 +441,21 @@ __global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* desc,
     if (threadIdx.x == 0) q->live[gen][blockIdx.x] = 1u;
     for (;;) {
         if (threadIdx.x == 0) {
-            int rec = -1;
+            int rec = -1, quiet = 0;
             for (int it = 0; it < idle_limit; ++it) {
                 const uint32_t tl = ld_acquire_sys(&q->tail);
                 const uint32_t h = *(volatile uint32_t*)head;
                 if (h < tl) {
                     if (atomicCAS(head, h, h + 1) == h) {
+                        atomicAdd(head + 1, 1u);
                         rec = ((volatile int*)q->ring)[h % kSoloRing];
                         break;
                     }
                     continue;
                 }
                 if (q->stop) break;
+                quiet = *(volatile uint32_t*)(head + 1) ? 0 : quiet + 1;
+                if (quiet >= kQuietPolls) break;
                 __nanosleep(1000);
             }
             s_rec = rec;
@@ -465,7 +476,10 @@ __global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* desc,
         __syncthreads();
         if (S.any_eam) solo_run<true, NT>(S, g, red, scan_sh);
         else solo_run<false, NT>(S, g, red, scan_sh);
-        if (threadIdx.x == 0) q->live[gen][blockIdx.x] = 1u;  // 1: waiting for the next entry
+        if (threadIdx.x == 0) {
+            q->live[gen][blockIdx.x] = 1u;  // 1: waiting for the next entry
+            atomicSub(head + 1, 1u);
+        }
     }
     if (threadIdx.x == 0) {
         __threadfence_system();
