@@ -345,6 +345,8 @@ void system_free(mdg_system* sys) {
     sys_free(sys, sys->bin_count, sys->bin_cap * sizeof(uint32_t));
     sys_free(sys, sys->bin_start, sys->bin_cap * sizeof(uint32_t));
     sys_free(sys, sys->scan_tmp, sys->scan_cap * sizeof(uint32_t));
+    sys_free(sys, sys->team_word, sizeof(unsigned long long));
+    sys->team_word = nullptr;
     sys_free(sys, sys->part, sys->part_cap * 8 * sizeof(double));
     sys_free(sys, sys->nbr, (size_t)sys->K * sys->np * sizeof(uint32_t));
     sys_free(sys, sys->cutbits, (size_t)sys->cut_words * sys->np * sizeof(uint32_t));
@@ -2175,6 +2177,65 @@ static int graph_prologue(mdg_solver* s, mdg_system* sys) {
     return MDG_OK;
 }
 
+// The device's view of a page-locked host array; null when it has none.
+static double* locked_view(const double* p) {
+    cudaPointerAttributes a;
+    if (!p || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return a.type == cudaMemoryTypeHost ? (double*)a.devicePointer : nullptr;
+}
+
+// Largest system whose host arrays the team kernel reads and writes itself.
+constexpr size_t kTeamDirect = 16384;
+
+// Host arrays of a run whose transfers are the team kernel's own.
+struct TeamIo {
+    const double *pos = nullptr, *vel = nullptr;
+    double *opos = nullptr, *ovel = nullptr, *oforce = nullptr;
+};
+
+// `steps` steps by a grid's team (team_eligible), waited for; a rebuild that
+// outgrew its capacities ends the kernel early: grown here, and resumed. *io
+// (optional): *done tells whether the results went to its arrays.
+static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, double dt, long steps, const TeamIo* io,
+                    bool* done) {
+    int rc = graph_prologue(s, sys);
+    if (rc) return rc;
+    if (!sys->dcounter) {
+        rc = sys_malloc(sys, (void**)&sys->dcounter, sizeof(unsigned long long));
+        if (rc) return rc;
+    }
+    if (!sys->hcounter) MDG_CUDA(cudaMallocHost((void**)&sys->hcounter, sizeof(unsigned long long)));
+    if (done) *done = false;
+    long left = steps;
+    for (int round = 0; left > 0 && round < 64; ++round) {
+        const bool whole = io && round == 0;
+        rc = team_launch(sys, ext(s)->d.dev, thermo_of(s), ps.any_eam, s->precision == MDG_PREC_MIXED,
+                         pot_rcut_of(s), s->periodic, dt, left, whole ? io->pos : nullptr, whole ? io->vel : nullptr,
+                         whole ? io->opos : nullptr, whole ? io->ovel : nullptr, whole ? io->oforce : nullptr);
+        if (rc) return rc;
+        MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
+        sys->fp_ok = 0;
+        sys->force_prec = s->precision;
+        if (sys->hstat->pad[1]) {
+            set_error("the step loop's blocks did not meet at a barrier in time");
+            return MDG_ERR_TIMEOUT;
+        }
+        sys->rebuilds += sys->hstat->pad[0];
+        left = (long)*sys->hcounter;
+        if (sys->hstat->build_flags & FLAG_OVERFLOW) {
+            sys->rebuilds--;
+            rc = nlist_build(sys, -1.0, sys->half);
+            if (rc && rc != MDG_ERR_RANGE) return rc;
+        } else if (whole && done) {
+            *done = left == 0;
+        }
+    }
+    return left > 0 ? MDG_ERR_OVERFLOW : MDG_OK;
+}
+
 int run_async_begin(mdg_solver* s, mdg_system* sys, double dt, long steps) {
     PotSet ps;
     int rc = check_ready(s, sys, &ps);
@@ -2500,6 +2561,7 @@ int mdg_run(mdg_solver* s, mdg_system* sys, double dt, long steps) {
     if (rc) return rc;
     if (steps <= 0) return MDG_OK;
     mark_stepped(s, sys, ps);
+    if (team_eligible(s, sys)) return run_team(s, sys, ps, dt, steps, nullptr, nullptr);
     if (!sys->ctx->timing && sys->n > 0 && !sys->half) {
         rc = graph_prologue(s, sys);
         if (rc) return rc;
@@ -2585,6 +2647,32 @@ done:
 int mdg_run_host(mdg_solver* s, mdg_system* sys, double dt, long steps, double* pos, double* vel, double* force) {
     if (!s || !sys || !pos || !vel) return MDG_ERR_INVALID;
     PotSet ps;
+    if (steps > 0 && sys->n > 0 && !sys->half && !sys->ctx->timing && check_ready(s, sys, &ps) == MDG_OK &&
+        team_eligible(s, sys)) {
+        MDG_CUDA(cudaSetDevice(sys->ctx->device));
+        mark_stepped(s, sys, ps);
+        // page-locked arrays of a small system are read and written by the
+        // kernel itself: one launch, no copies
+        TeamIo io;
+        io.pos = io.opos = locked_view(pos);
+        io.vel = io.ovel = locked_view(vel);
+        io.oforce = locked_view(force);
+        const bool direct = sys->n <= kTeamDirect && io.pos && io.vel && (!force || io.oforce);
+        int rc = MDG_OK;
+        bool done = false;
+        if (!direct) {
+            rc = vec_io(sys, pos, RX, 1, 0);
+            if (!rc) rc = vec_io(sys, vel, VX, 1, 0);
+        }
+        if (!rc) rc = run_team(s, sys, ps, dt, steps, direct ? &io : nullptr, &done);
+        if (rc || done) return rc;
+        rc = vec_io(sys, pos, RX, 0, 0);
+        if (!rc) rc = vec_io(sys, vel, VX, 0, 0);
+        if (!rc && force) rc = vec_io(sys, force, FX, 0, 0);
+        if (rc) return rc;
+        MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
+        return MDG_OK;
+    }
     if (steps == 1 && !sys->ctx->timing && sys->n > 0 && !sys->half && check_ready(s, sys, &ps) == MDG_OK &&
         page_locked(pos) && page_locked(vel) && page_locked(force)) {
         MDG_CUDA(cudaSetDevice(sys->ctx->device));

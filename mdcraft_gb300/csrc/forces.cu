@@ -25,6 +25,7 @@
 #include "forces64_dev.cuh"
 #include "forces_dev.cuh"
 #include "integrate_dev.cuh"
+#include "thermo_dev.cuh"
 
 namespace mdg {
 
@@ -46,34 +47,6 @@ __device__ __forceinline__ double eam_rho64(const PotParams& P, double R1) {
         return P.Rho[N1] + RN * (P.dRho[N1] + DV * (DV * aa - bb));
     }
     return 0.0;
-}
-
-__device__ __forceinline__ void eam_embed64(const PotParams& P, double nr, double* EF, double* dF,
-                                            DevStatus* st) {
-    double RN = nr * P.drh1;
-    int N1 = (int)trunc(RN);
-    double dF0 = 0.0;  // the reference's output array is zero-initialised
-    if (RN >= 0.0 && N1 < P.Nrh1) {
-        if (N1 == P.Nrh1 - 1) atomicOr(&st->flags, FLAG_TABLE);
-        double VR = N1;
-        double DV = RN - VR;
-        RN = nr - VR * P.drh;
-        VR = (P.Femb[N1 + 1] - P.Femb[N1]) * P.drh1;
-        double aa = (P.dFemb[N1 + 1] - VR) - (VR - P.dFemb[N1]);
-        double bb = aa - (VR - P.dFemb[N1]);
-        aa = aa * DV;
-        *EF = P.Femb[N1] + RN * (P.dFemb[N1] + DV * (aa - bb));
-        *dF = P.dFemb[N1] + 2.0 * DV * (1.5 * aa - bb);
-    } else {
-        atomicOr(&st->flags, FLAG_TABLE);
-        if (N1 >= P.Nrh1) {
-            *EF = P.Femb[P.Nrh1] + P.dFemb[P.Nrh1] * (dF0 - P.Nrh1 * P.drh);
-            *dF = P.dFemb[P.Nrh1];
-        } else {
-            *EF = P.Femb[0] - P.dFemb[0] * dF0;
-            *dF = P.dFemb[0];
-        }
-    }
 }
 
 // Force(r)/r of one pair and the pair energy term V(r) (EAM.cxx:417-463).
@@ -177,38 +150,9 @@ __global__ void __launch_bounds__(kBlock64) k_forces64(FArgs A, const PotSet* __
     const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % G;
     const bool live = t / G < A.n && A.tag[t / G] != 0;
     const int i = live ? t / G : 0;
-    double f[3] = {0, 0, 0};
-    if (live) {
-        const int ki = MULTI ? (A.kind[i] & 3) : 0;
-        walk64<MULTI, G, true>(A, ps, i, ki, lane, [](const PotParams&, int, int, bool) {},
-                         [&](const PotParams& P, int kj, uint32_t j, const Pair64& p, bool ghost) {
-            const int type = FORM ? FORM : P.type;
-            double pref, E;
-            if (type == POT_LJCUT) {
-                pref = ljcut_ff64<false>(P, p.r2, E);
-            } else if (type == POT_EAM) {
-                const double AdF = A.Fp64[(size_t)ki * A.np + j] + A.Fp64[(size_t)kj * A.np + i];
-                pref = table_ff64<true, false>(P, p.r2, AdF, E);
-            } else if (type == POT_TAB) {
-                pref = table_ff64<false, false>(P, p.r2, 0.0, E);
-            } else if (type == POT_LJS) {
-                pref = ljs_pair64<false>(P, p.r2, E);
-            } else {
-                return;
-            }
-            f[0] = fma(p.dx, pref, f[0]);
-            f[1] = fma(p.dy, pref, f[1]);
-            f[2] = fma(p.dz, pref, f[2]);
-            if (HALF && !ghost && type != POT_EAM) {
-                atomicAdd(&A.fx[j], -(p.dx * pref));
-                atomicAdd(&A.fy[j], -(p.dy * pref));
-                atomicAdd(&A.fz[j], -(p.dz * pref));
-            }
-        });
-    }
-    for (int a = 0; a < 3; ++a) f[a] = lane_sum<G>(f[a]);
+    double f[3];
+    forces64_lanes<MULTI, FORM, HALF, G>(A, ps, live, i, lane, f);
     if (!live || lane) return;
-    if (!isfinite(f[0]) || !isfinite(f[1]) || !isfinite(f[2])) atomicOr(&A.st->flags, FLAG_NONFINITE);
     if (HALF) {
         atomicAdd(&A.fx[i], f[0]);
         atomicAdd(&A.fy[i], f[1]);
@@ -223,28 +167,8 @@ __global__ void __launch_bounds__(kBlock64) k_forces64(FArgs A, const PotSet* __
 // ---- EAM density + embedding derivative, FP64 ------------------------------
 template <bool MULTI, int G>
 __global__ void __launch_bounds__(kBlock64) k_density64(FArgs A, const PotSet* __restrict__ ps) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % G;
-    const bool in = t / G < A.n;
-    const int i = in ? t / G : 0;
-    const int ki = MULTI && in ? (A.kind[i] & 3) : 0;
-    const bool live = in && A.tag[i] != 0;
-    double rho = 0.0;
-    if (live)
-        walk64<MULTI, G, true>(A, ps, i, ki, lane, [](const PotParams&, int, int, bool) {},
-                         [&](const PotParams& P, int, uint32_t, const Pair64& p, bool) {
-            if (!MULTI || P.type == POT_EAM) rho += table_rho64(P, p.r2);
-        });
-    rho = lane_sum<G>(rho);
-    if (!in || lane) return;
-    // an atom with tag 0 is untouched by the reference's charge stage; its F' is still defined
-    if (live) A.nc[i] = rho;
-    else rho = A.nc[i];
-    for (int b = 0; b < ps->nkinds; ++b) {
-        const PotParams& P = ps->p[ki][b];
-        double EF = 0, dF = 0;
-        if (P.type == POT_EAM) eam_embed64(P, rho, &EF, &dF, A.st);
-        A.Fp64[(size_t)b * A.np + i] = dF;
-    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    density64_lanes<MULTI, G>(A, ps, t / G < A.n, t / G, t % G);
 }
 
 // ---- energies and virials, FP64 (LJs-cut.cxx:70-131, EAM.cxx:306-415,
@@ -263,7 +187,7 @@ __global__ void __launch_bounds__(kBlock64) k_virials64(FArgs A, const PotSet* _
     int last_main = -1, last_ghost = -1;
     constexpr int kSym[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
     if (live)
-        walk64<MULTI, G, !MULTI>(A, ps, i, ki, lane, [&](const PotParams& P, int kj, int k, bool ghost) {
+        walk64<MULTI, G, !MULTI, true>(A, ps, i, ki, lane, [&](const PotParams& P, int kj, int k, bool ghost) {
             if (!MULTI || P.type != POT_EAM) return;
             if (ghost) last_ghost = 4 * k + kj;
             else last_main = max(last_main, kj);
@@ -419,13 +343,13 @@ __global__ void __launch_bounds__(kBlock, MB) k_lj_mixed(FArgs A, const PotSet* 
 template <int KINDS, int MB>
 __global__ void __launch_bounds__(kBlock, MB) k_density_rec(FArgs A, const PotSet* __restrict__ ps) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < A.n) density_mixed_one<KINDS, true>(A, ps, i);
+    if (i < A.n) density_one<RhoGroup<KINDS, true>>(A, ps, i);
 }
 
 template <int KINDS, int MB>
 __global__ void __launch_bounds__(kBlock, MB) k_density_mixed(FArgs A, const PotSet* __restrict__ ps) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < A.n) density_mixed_one<KINDS>(A, ps, i);
+    if (i < A.n) density_one<RhoGroup<KINDS, false>>(A, ps, i);
 }
 
 template <int KINDS, bool KICK, int MB>
@@ -493,7 +417,7 @@ __device__ __forceinline__ bool end_step(const FArgs& A, const IArgs& D, int i, 
         if (moved) store_force<true>(A, i, f[0], f[1], f[2]);
         return false;
     }
-    if (moved) return kick_drift_mixed(D, A.gx, A.gy, A.gz, i, f[0], f[1], f[2]);
+    if (moved) return kick_drift_mixed(D, D, A.gx, A.gy, A.gz, i, f[0], f[1], f[2]);
     const double r[3] = {D.rx[i], D.ry[i], D.rz[i]};
     return offsets_check_mixed(D, i, r);
 }
@@ -570,81 +494,11 @@ __global__ void __launch_bounds__(kBlock, lane_budget(KINDS))
 static bool lanes_mixed(size_t n, const PotSet& ps) { return n < (ps.any_eam ? 45000u : 24000u); }
 static int lane_blocks(size_t n) { return (int)((n + kLaneAtoms - 1) / kLaneAtoms); }
 
-// ---- Langevin thermostat (langevin.cxx:29-42) ----------------------------------
-// Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11): ten rounds of two
-// 32x32->64 multiplications, key bumped by the Weyl constants.
-__device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint2 k) {
-#pragma unroll
-    for (int r = 0; r < 10; ++r) {
-        if (r > 0) {
-            k.x += 0x9E3779B9u;
-            k.y += 0xBB67AE85u;
-        }
-        const uint32_t lo0 = 0xD2511F53u * c.x, hi0 = __umulhi(0xD2511F53u, c.x);
-        const uint32_t lo1 = 0xCD9E8D57u * c.z, hi1 = __umulhi(0xCD9E8D57u, c.z);
-        c = make_uint4(hi1 ^ c.y ^ k.x, lo1, hi0 ^ c.w ^ k.y, lo0);
-    }
-    return c;
-}
-
-struct ThermoArgs {
-    int n;
-    const double *rx, *vx, *vy, *vz, *m;
-    const uint32_t* orig;
-    double *fx, *fy, *fz;  // FP64 form
-    float *gx, *gy, *gz;   // mixed form
-    const DevStatus* st;
-};
-
-// f += heat * (sqrt(m) * sigma * z - (v - U) * beta * m) for every term whose
-// x range holds the atom; z = three Box-Muller normals of one Philox block
-// with counter {caller index, call number, term, 0}.
+// ---- Langevin thermostat (thermo_dev.cuh) -------------------------------------
 template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_langevin(ThermoArgs A, const ThermoDev* __restrict__ th) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.n) return;
-    const int nt = th->n;
-    if (nt == 0) return;
-    const uint32_t call = A.st->therm_calls;
-    const double x = A.rx[i], m = A.m[i];
-    const double v[3] = {A.vx[i], A.vy[i], A.vz[i]};
-    const double sqrt_mass = sqrt(m);
-    double f[3] = {0.0, 0.0, 0.0};
-    if (!MIXED) {
-        f[0] = A.fx[i];
-        f[1] = A.fy[i];
-        f[2] = A.fz[i];
-    }
-    const uint32_t atom = A.orig[i];
-    for (int q = 0; q < nt && q < kMaxThermo; ++q) {
-        const LangevinTerm& L = th->t[q];
-        if (x < L.xmin || x > L.xmax) continue;
-        const uint4 b = philox4x32_10(make_uint4(atom, call, (uint32_t)q, 0u),
-                                      make_uint2((uint32_t)L.seed, (uint32_t)(L.seed >> 32)));
-        const double k32 = 2.3283064365386962890625e-10;  // 2^-32
-        const double two_pi = 6.283185307179586476925;
-        const double ra = sqrt(-2.0 * log(((double)b.x + 0.5) * k32));
-        const double rb = sqrt(-2.0 * log(((double)b.z + 0.5) * k32));
-        const double a1 = two_pi * (((double)b.y + 0.5) * k32);
-        const double a3 = two_pi * (((double)b.w + 0.5) * k32);
-        const double z[3] = {ra * cos(a1), ra * sin(a1), rb * cos(a3)};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            double tf = __dmul_rn(__dadd_rn(__dmul_rn(z[k], L.sigma), 0.0), sqrt_mass);
-            tf = __dsub_rn(tf, __dmul_rn(__dmul_rn(__dsub_rn(v[k], L.U[k]), L.beta), m));
-            tf = __dmul_rn(tf, L.heat[k]);
-            f[k] = __dadd_rn(f[k], tf);
-        }
-    }
-    if (MIXED) {
-        A.gx[i] += (float)f[0];
-        A.gy[i] += (float)f[1];
-        A.gz[i] += (float)f[2];
-    } else {
-        A.fx[i] = f[0];
-        A.fy[i] = f[1];
-        A.fz[i] = f[2];
-    }
+    if (i < A.n) langevin_one<MIXED>(A, th, i, A.st->therm_calls);
 }
 
 __global__ void k_thermo_tick(DevStatus* st) {
@@ -700,12 +554,8 @@ FArgs force_args(mdg_system* sys) {
     return A;
 }
 
-// Thermostat pass after the force stage (pair.cxx:81), then the call
-// counter's increment.
-static int launch_thermostat(mdg_system* sys, const ThermoDev* th, int precision) {
-    mdg_ctx* ctx = sys->ctx;
-    cudaStream_t st = ctx->stream;
-    int c = sys->cur;
+ThermoArgs thermo_args(mdg_system* sys) {
+    const int c = sys->cur;
     ThermoArgs T;
     T.n = (int)sys->n;
     T.rx = sys->f64[RX][c];
@@ -721,9 +571,18 @@ static int launch_thermostat(mdg_system* sys, const ThermoDev* th, int precision
     T.gy = sys->f32[1][c];
     T.gz = sys->f32[2][c];
     T.st = sys->dstat;
-    int nb = nblk(sys->n);
-    if (precision == MDG_PREC_FP64) k_langevin<false><<<nb, kBlock, 0, st>>>(T, th);
-    else k_langevin<true><<<nb, kBlock, 0, st>>>(T, th);
+    return T;
+}
+
+// Thermostat pass after the force stage (pair.cxx:81), then the call
+// counter's increment.
+static int launch_thermostat(mdg_system* sys, const ThermoDev* th, int precision) {
+    mdg_ctx* ctx = sys->ctx;
+    cudaStream_t st = ctx->stream;
+    const ThermoArgs T = thermo_args(sys);
+    const int nb = spread_blocks(sys->n), nt = spread_threads(sys->n);
+    if (precision == MDG_PREC_FP64) k_langevin<false><<<nb, nt, 0, st>>>(T, th);
+    else k_langevin<true><<<nb, nt, 0, st>>>(T, th);
     MDG_LAUNCHED(ctx);
     k_thermo_tick<<<1, 32, 0, st>>>(sys->dstat);
     MDG_LAUNCHED(ctx);

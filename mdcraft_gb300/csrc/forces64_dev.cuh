@@ -238,7 +238,7 @@ struct Screen64 {
 // the cutoff both can count.
 // For every visit: seen(P, kj, k, ghost) (without SCREEN, which skips
 // visits); for those inside the cutoff: use(P, kj, j, pair, ghost).
-template <bool MULTI, int G, bool SCREEN, typename Seen, typename Use>
+template <bool MULTI, int G, bool SCREEN, bool RO, typename Seen, typename Use>
 __device__ __forceinline__ void walk64(const FArgs& A, const PotSet* __restrict__ ps, int i, int ki, int lane,
                                        Seen&& seen, Use&& use) {
     const double xi = A.rx[i], yi = A.ry[i], zi = A.rz[i];
@@ -256,10 +256,10 @@ __device__ __forceinline__ void walk64(const FArgs& A, const PotSet* __restrict_
             todo = 0;
 #pragma unroll 4
             for (int m = 0; m < turn; ++m) {
-                const uint32_t j = __ldg(A.nbr + nidx(k0 + m * G, i, A.np)) & kJMask;
-                float dx = screen_float(__ldg(A.rx + j)) - S.x;
-                float dy = screen_float(__ldg(A.ry + j)) - S.y;
-                float dz = screen_float(__ldg(A.rz + j)) - S.z;
+                const uint32_t j = ld_ro<RO>(A.nbr + nidx(k0 + m * G, i, A.np)) & kJMask;
+                float dx = screen_float(ld_ro<RO>(A.rx + j)) - S.x;
+                float dy = screen_float(ld_ro<RO>(A.ry + j)) - S.y;
+                float dz = screen_float(ld_ro<RO>(A.rz + j)) - S.z;
                 dx = fmaf(-S.L[0], rintf(dx * S.il[0]), dx);
                 dy = fmaf(-S.L[1], rintf(dy * S.il[1]), dy);
                 dz = fmaf(-S.L[2], rintf(dz * S.il[2]), dz);
@@ -270,11 +270,11 @@ __device__ __forceinline__ void walk64(const FArgs& A, const PotSet* __restrict_
         while (todo) {
             const int k = k0 + (__ffsll((long long)todo) - 1) * G;
             todo &= todo - 1ull;
-            const uint32_t j = __ldg(A.nbr + nidx(k, i, A.np)) & kJMask;
+            const uint32_t j = ld_ro<RO>(A.nbr + nidx(k, i, A.np)) & kJMask;
             const int kj = MULTI ? (A.kind[j] & 3) : 0;
             const PotParams& P = ps->p[ki][kj];
             Pair64 p, s;
-            const double xj = __ldg(A.rx + j), yj = __ldg(A.ry + j), zj = __ldg(A.rz + j);
+            const double xj = ld_ro<RO>(A.rx + j), yj = ld_ro<RO>(A.ry + j), zj = ld_ro<RO>(A.rz + j);
             p.dx = xj - xi;
             p.dy = yj - yi;
             p.dz = zj - zi;
@@ -326,6 +326,101 @@ __device__ __forceinline__ double lane_sum(double v) {
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+__device__ __forceinline__ void eam_embed64(const PotParams& P, double nr, double* EF, double* dF,
+                                            DevStatus* st) {
+    double RN = nr * P.drh1;
+    int N1 = (int)trunc(RN);
+    double dF0 = 0.0;  // the reference's output array is zero-initialised
+    if (RN >= 0.0 && N1 < P.Nrh1) {
+        if (N1 == P.Nrh1 - 1) atomicOr(&st->flags, FLAG_TABLE);
+        double VR = N1;
+        double DV = RN - VR;
+        RN = nr - VR * P.drh;
+        VR = (P.Femb[N1 + 1] - P.Femb[N1]) * P.drh1;
+        double aa = (P.dFemb[N1 + 1] - VR) - (VR - P.dFemb[N1]);
+        double bb = aa - (VR - P.dFemb[N1]);
+        aa = aa * DV;
+        *EF = P.Femb[N1] + RN * (P.dFemb[N1] + DV * (aa - bb));
+        *dF = P.dFemb[N1] + 2.0 * DV * (1.5 * aa - bb);
+    } else {
+        atomicOr(&st->flags, FLAG_TABLE);
+        if (N1 >= P.Nrh1) {
+            *EF = P.Femb[P.Nrh1] + P.dFemb[P.Nrh1] * (dF0 - P.Nrh1 * P.drh);
+            *dF = P.dFemb[P.Nrh1];
+        } else {
+            *EF = P.Femb[0] - P.dFemb[0] * dF0;
+            *dF = P.dFemb[0];
+        }
+    }
+}
+
+// The force of atom i by G lanes (every lane of a warp calls this; `live`
+// false: none); on all of them. FORM: the potential of every pair where there
+// is one (POT_LJCUT, POT_EAM; Single), 0 = by kind pair. HALF also pushes the
+// pair-type terms onto the neighbours.
+template <bool MULTI, int FORM, bool HALF, int G, bool RO = true>
+__device__ __forceinline__ void forces64_lanes(const FArgs& A, const PotSet* __restrict__ ps, bool live, int i,
+                                               int lane, double f[3]) {
+    f[0] = f[1] = f[2] = 0.0;
+    if (live) {
+        const int ki = MULTI ? (A.kind[i] & 3) : 0;
+        walk64<MULTI, G, true, RO>(A, ps, i, ki, lane, [](const PotParams&, int, int, bool) {},
+                         [&](const PotParams& P, int kj, uint32_t j, const Pair64& p, bool ghost) {
+            const int type = FORM ? FORM : P.type;
+            double pref, E;
+            if (type == POT_LJCUT) {
+                pref = ljcut_ff64<false>(P, p.r2, E);
+            } else if (type == POT_EAM) {
+                const double AdF = A.Fp64[(size_t)ki * A.np + j] + A.Fp64[(size_t)kj * A.np + i];
+                pref = table_ff64<true, false>(P, p.r2, AdF, E);
+            } else if (type == POT_TAB) {
+                pref = table_ff64<false, false>(P, p.r2, 0.0, E);
+            } else if (type == POT_LJS) {
+                pref = ljs_pair64<false>(P, p.r2, E);
+            } else {
+                return;
+            }
+            f[0] = fma(p.dx, pref, f[0]);
+            f[1] = fma(p.dy, pref, f[1]);
+            f[2] = fma(p.dz, pref, f[2]);
+            if (HALF && !ghost && type != POT_EAM) {
+                atomicAdd(&A.fx[j], -(p.dx * pref));
+                atomicAdd(&A.fy[j], -(p.dy * pref));
+                atomicAdd(&A.fz[j], -(p.dz * pref));
+            }
+        });
+    }
+    for (int a = 0; a < 3; ++a) f[a] = lane_sum<G>(f[a]);
+    if (live && lane == 0 && !(isfinite(f[0]) && isfinite(f[1]) && isfinite(f[2])))
+        atomicOr(&A.st->flags, FLAG_NONFINITE);
+}
+
+// The EAM density of atom i (where `in`) by G lanes, and F' of it.
+template <bool MULTI, int G, bool RO = true>
+__device__ __forceinline__ void density64_lanes(const FArgs& A, const PotSet* __restrict__ ps, bool in, int i,
+                                                int lane) {
+    if (!in) i = 0;
+    const int ki = MULTI && in ? (A.kind[i] & 3) : 0;
+    const bool live = in && A.tag[i] != 0;
+    double rho = 0.0;
+    if (live)
+        walk64<MULTI, G, true, RO>(A, ps, i, ki, lane, [](const PotParams&, int, int, bool) {},
+                         [&](const PotParams& P, int, uint32_t, const Pair64& p, bool) {
+            if (!MULTI || P.type == POT_EAM) rho += table_rho64(P, p.r2);
+        });
+    rho = lane_sum<G>(rho);
+    if (!in || lane) return;
+    // an atom with tag 0 is untouched by the reference's charge stage; its F' is still defined
+    if (live) A.nc[i] = rho;
+    else rho = A.nc[i];
+    for (int b = 0; b < ps->nkinds; ++b) {
+        const PotParams& P = ps->p[ki][b];
+        double EF = 0, dF = 0;
+        if (P.type == POT_EAM) eam_embed64(P, rho, &EF, &dF, A.st);
+        A.Fp64[(size_t)b * A.np + i] = dF;
+    }
 }
 
 }  // namespace mdg

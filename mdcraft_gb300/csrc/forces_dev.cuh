@@ -16,12 +16,25 @@ namespace mdg {
 
 // A group of four list entries: streamed once per pass, so kept out of L1
 // (the gathers of neighbour records and table rows keep it).
+// RO (here and below): the data is read-only while the kernel runs, so the
+// read-only path may serve it; the fused loops (solo.cu), whose own passes
+// write it, take ordinary loads.
+template <bool RO>
 __device__ __forceinline__ uint4 ldg_list(const uint4* p) {
     uint4 v;
-    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
+    if (RO)
+        asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+            : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+            : "l"(p));
+    else
+        asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "l"(p));
     return v;
+}
+template <bool RO, typename T>
+__device__ __forceinline__ T ld_ro(const T* p) {
+    return RO ? __ldg(p) : *p;
 }
 
 
@@ -167,7 +180,7 @@ __device__ __forceinline__ bool pair_in_rec(const FArgs& A, int i, uint32_t e, f
 __device__ __forceinline__ bool pair_in_bits(const FArgs& A, int i, uint32_t e, float r2, float r2c, bool per,
                                              int k) {
     bool in = r2 >= 1e-15f && r2 <= r2c;
-    if (fabsf(r2 - r2c) <= 1e-5f * r2c) in = (__ldg(A.cutbits + (size_t)(k >> 5) * A.np + i) >> (k & 31)) & 1u;
+    if (fabsf(r2 - r2c) <= 1e-5f * r2c) in = (A.cutbits[(size_t)(k >> 5) * A.np + i] >> (k & 31)) & 1u;
     return in && (per || !(e & kWrapBit));
 }
 
@@ -186,11 +199,11 @@ __device__ __forceinline__ void group_sums(const FArgs& A, int i, int ng, Group&
 #pragma unroll
     for (int k = 0; k < NC; ++k) s[k] = c[k] = 0.f;
     const uint4* row = reinterpret_cast<const uint4*>(A.nbr) + i;
-    uint4 e4n = ng > 0 ? ldg_list(row) : make_uint4(0, 0, 0, 0);
+    uint4 e4n = ng > 0 ? ldg_list<Group::kRO>(row) : make_uint4(0, 0, 0, 0);
     for (int g = 0; g < ng; ++g) {
         // the next group's entries are requested before this group's work
         const uint4 e4 = e4n;
-        if (g + 1 < ng) e4n = ldg_list(row + (size_t)(g + 1) * A.np);
+        if (g + 1 < ng) e4n = ldg_list<Group::kRO>(row + (size_t)(g + 1) * A.np);
         float f[NC];
         grp(A, i, g, e4, f);
 #pragma unroll
@@ -215,12 +228,12 @@ __device__ __forceinline__ void lane_sums(const FArgs& A, bool live, int i, int 
     if (!live) ng = 0;
     const uint4* row = reinterpret_cast<const uint4*>(A.nbr) + i;
     const int rounds = (__reduce_max_sync(0xffffffffu, (unsigned)ng) + 7) >> 3;
-    uint4 e4n = sub < ng ? ldg_list(row + (size_t)sub * A.np) : make_uint4(0, 0, 0, 0);
+    uint4 e4n = sub < ng ? ldg_list<Group::kRO>(row + (size_t)sub * A.np) : make_uint4(0, 0, 0, 0);
     float s = 0.f, c = 0.f;  // component `sub` of this lane's atom
     for (int r = 0; r < rounds; ++r) {
         const int g = 8 * r + sub;
         const uint4 e4 = e4n;
-        if (g + 8 < ng) e4n = ldg_list(row + (size_t)(g + 8) * A.np);
+        if (g + 8 < ng) e4n = ldg_list<Group::kRO>(row + (size_t)(g + 8) * A.np);
         float f[NC];
 #pragma unroll
         for (int k = 0; k < NC; ++k) f[k] = 0.f;
@@ -241,8 +254,9 @@ __device__ __forceinline__ void lane_sums(const FArgs& A, bool live, int i, int 
     for (int k = 0; k < NC; ++k) out[k] = __shfl_sync(0xffffffffu, s, (lane & ~7) + k);
 }
 
-template <bool MULTI>
+template <bool MULTI, bool RO = true>
 struct LjGroup {
+    static constexpr bool kRO = RO;
     const PotSet* ps;
     int4 pi;
     int ki;
@@ -267,7 +281,7 @@ struct LjGroup {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pj[q] = __ldg(A.pos32 + (e[q] & kJMask));
+        for (int q = 0; q < 4; ++q) pj[q] = ld_ro<RO>(A.pos32 + (e[q] & kJMask));
         float fx = 0.f, fy = 0.f, fz = 0.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -356,8 +370,9 @@ __device__ __forceinline__ float analytic_ff32(const PotParams& P, float r2) {
 // Pair-type forces (no EAM term) beyond the plain LJsCut kernel: FORM 3 =
 // every pair a tabulated Pair, 4 = every pair LJs, 0 = chosen per kind pair
 // among LJsCut, Pair and LJs.
-template <bool MULTI, int FORM>
+template <bool MULTI, int FORM, bool RO = true>
 struct PairGroup {
+    static constexpr bool kRO = RO;
     const PotSet* ps;
     int4 pi;
     int ki;
@@ -374,7 +389,7 @@ struct PairGroup {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pj[q] = __ldg(A.pos32 + (e[q] & kJMask));
+        for (int q = 0; q < 4; ++q) pj[q] = ld_ro<RO>(A.pos32 + (e[q] & kJMask));
         float fx = 0.f, fy = 0.f, fz = 0.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -485,8 +500,9 @@ struct KindPots {
 // REC: also record the FP64 decisions of the band pairs in A.cutbits, for a
 // force pass that moves atoms (pair_in_rec): one bit per entry, a word of 32
 // stored when it has a band pair.
-template <int KINDS, bool REC>
+template <int KINDS, bool REC, bool RO = true>
 struct RhoGroup {
+    static constexpr bool kRO = RO;
     static constexpr bool MULTI = KINDS != 0;
     const PotSet* ps;
     int4 pi;
@@ -507,7 +523,7 @@ struct RhoGroup {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pj[q] = __ldg(A.pos32 + (e[q] & kJMask));
+        for (int q = 0; q < 4; ++q) pj[q] = ld_ro<RO>(A.pos32 + (e[q] & kJMask));
         float part = 0.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -576,20 +592,21 @@ __device__ __forceinline__ void store_density(const FArgs& A, const PotSet* __re
     A.pos32b[i] = make_int4(pi.x, pi.y, pi.z, w);
 }
 
-template <int KINDS, bool REC = false>
-__device__ __forceinline__ void density_mixed_one(const FArgs& A, const PotSet* __restrict__ ps, int i) {
+template <typename Group>
+__device__ __forceinline__ void density_one(const FArgs& A, const PotSet* __restrict__ ps, int i) {
     float rho[1] = {0.f};
-    RhoGroup<KINDS, REC> grp(A, ps, i);
+    Group grp(A, ps, i);
     if (A.tag[i] != 0) group_sums<1>(A, i, A.ncnt[i] >> 2, grp, rho);
-    store_density<(KINDS != 0)>(A, ps, i, grp.pi, grp.ki, rho[0]);
+    store_density<Group::MULTI>(A, ps, i, grp.pi, grp.ki, rho[0]);
 }
 
 // BITS: a pair in the 1e-5 band around the cutoff takes the density pass's
 // FP64 decision (A.cutbits) rather than testing the FP64 positions itself;
 // the force pass then reads no FP64 position of a neighbour (what a force
 // pass that moves its atoms needs).
-template <int KINDS, bool BITS>
+template <int KINDS, bool BITS, bool RO = true>
 struct EamGroup {
+    static constexpr bool kRO = RO;
     static constexpr bool MULTI = KINDS != 0;
     const PotSet* ps;
     int4 pi;
@@ -619,7 +636,7 @@ struct EamGroup {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pj[q] = __ldg(A.pos32b + (e[q] & kJMask));
+        for (int q = 0; q < 4; ++q) pj[q] = ld_ro<RO>(A.pos32b + (e[q] & kJMask));
         float fx = 0.f, fy = 0.f, fz = 0.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {

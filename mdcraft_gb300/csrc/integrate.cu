@@ -27,7 +27,7 @@ namespace mdg {
 // prepare + decide part (Pair::prepare called on its own).
 __global__ void k_drift64(IArgs A, int drift, int check) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool need = i < A.n ? drift64_one(A, i, drift, check) : false;
+    bool need = i < A.n ? drift64_one(A, A, i, drift, check) : false;
     if (check) flag_need(need, A.st);
 }
 
@@ -42,20 +42,13 @@ __global__ void k_decide(IArgs A) {
 // step_one_velocities (verlet.cxx:80-85), FP64 form.
 __global__ void k_kick64(IArgs A) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.n || A.tag[i] == 0) return;
-    const double m = A.m[i], rm = __drcp_rn(m);
-    double* v[3] = {A.vx, A.vy, A.vz};
-    const double* f[3] = {A.fx, A.fy, A.fz};
-    for (int k = 0; k < 3; ++k) {
-        double a = div_rm(f[k][i], m, rm);
-        v[k][i] = dadd(v[k][i], dmul(dmul(a, 0.5), A.dt));
-    }
+    if (i < A.n) kick64_one(A, i);
 }
 
 // Mixed form: kick + drift, cell-offset refresh, half-skin test.
 __global__ void k_drift_mixed(IArgs A) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool need = i < A.n ? drift_mixed_one(A, i) : false;
+    bool need = i < A.n ? drift_mixed_one(A, A, i) : false;
     flag_need(need, A.st);
 }
 
@@ -67,7 +60,7 @@ __global__ void k_drift_mixed_guarded(IArgs A, const unsigned long long* __restr
                                       unsigned long long min_left) {
     if (*left < min_left || (A.st->build_flags & FLAG_OVERFLOW)) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool need = i < A.n ? drift_mixed_one(A, i) : false;
+    bool need = i < A.n ? drift_mixed_one(A, A, i) : false;
     flag_need(need, A.st);
 }
 

@@ -78,8 +78,10 @@ __device__ __forceinline__ double div_rm(double f, double m, double rm) {
 }
 
 // step_one_coords + prepare + decide, FP64 form (drift = 0: the prepare
-// part alone, Pair::prepare called on its own).
-__device__ __forceinline__ bool drift64_one(const IArgs& A, int i, int drift, int check) {
+// part alone, Pair::prepare called on its own). The new position goes to
+// `to`'s arrays: A's own, or others (a step loop whose force passes still
+// read A's).
+__device__ __forceinline__ bool drift64_one(const IArgs& A, const IArgs& to, int i, int drift, int check) {
     bool need = false;
     {
         double r[3] = {A.rx[i], A.ry[i], A.rz[i]};
@@ -93,8 +95,10 @@ __device__ __forceinline__ bool drift64_one(const IArgs& A, int i, int drift, in
                 v[k] = dadd(v[k], dmul(dmul(a, A.dt), 0.5));
                 r[k] = dadd(r[k], dmul(v[k], A.dt));
             }
-            A.rx[i] = r[0]; A.ry[i] = r[1]; A.rz[i] = r[2];
+            to.rx[i] = r[0]; to.ry[i] = r[1]; to.rz[i] = r[2];
             A.vx[i] = v[0]; A.vy[i] = v[1]; A.vz[i] = v[2];
+        } else if (to.rx != A.rx) {
+            to.rx[i] = r[0]; to.ry[i] = r[1]; to.rz[i] = r[2];
         }
         if (tg != 0 && A.pot_rcut >= 0.0) A.rcut[i] = A.pot_rcut;
         uint8_t bc = 0;
@@ -110,6 +114,18 @@ __device__ __forceinline__ bool drift64_one(const IArgs& A, int i, int drift, in
         if (check) need = decide_one(A, i, r[0], r[1], r[2]);
     }
     return need;
+}
+
+// step_one_velocities (verlet.cxx:80-85), FP64 form.
+__device__ __forceinline__ void kick64_one(const IArgs& A, int i) {
+    if (A.tag[i] == 0) return;
+    const double m = A.m[i], rm = __drcp_rn(m);
+    double* v[3] = {A.vx, A.vy, A.vz};
+    const double* f[3] = {A.fx, A.fy, A.fz};
+    for (int k = 0; k < 3; ++k) {
+        double a = div_rm(f[k][i], m, rm);
+        v[k][i] = dadd(v[k][i], dmul(dmul(a, 0.5), A.dt));
+    }
 }
 
 // Mixed form: kick + drift, cell-offset refresh, and the half-skin test of
@@ -144,9 +160,10 @@ __device__ __forceinline__ bool offsets_check_mixed(const IArgs& A, int i, const
     return skin <= 0.0 || sq3_exact(ex, ey, ez) > dmul(dmul(0.25, skin), skin);
 }
 
-__device__ __forceinline__ bool drift_mixed_one(const IArgs& A, int i) {
+__device__ __forceinline__ bool drift_mixed_one(const IArgs& A, const IArgs& to, int i) {
     double r[3] = {A.rx[i], A.ry[i], A.rz[i]};
-    if (A.tag[i] != 0) {
+    const bool moves = A.tag[i] != 0;
+    if (moves) {
         float hm = (0.5f * (float)A.dt) * __frcp_rn((float)A.m[i]);
         float g[3] = {A.gx[i], A.gy[i], A.gz[i]};
         double* v[3] = {A.vx, A.vy, A.vz};
@@ -155,9 +172,11 @@ __device__ __forceinline__ bool drift_mixed_one(const IArgs& A, int i) {
             v[k][i] = vk;
             r[k] = fma(vk, A.dt, r[k]);
         }
-        A.rx[i] = r[0]; A.ry[i] = r[1]; A.rz[i] = r[2];
     }
-    return offsets_check_mixed(A, i, r);
+    if (moves || to.rx != A.rx) {
+        to.rx[i] = r[0]; to.ry[i] = r[1]; to.rz[i] = r[2];
+    }
+    return offsets_check_mixed(to, i, r);
 }
 
 // Per-atom fields read once per step (cell centres, rebuild-time offsets
@@ -170,8 +189,8 @@ __device__ __forceinline__ bool drift_mixed_one(const IArgs& A, int i) {
 // kick_mixed_one followed by drift_mixed_one, operation for operation
 // (the same FP32 increment added to v twice, r advanced by fma(v, dt, r)).
 // Returns the rebuild test of the new position.
-__device__ __forceinline__ bool kick_drift_mixed(const IArgs& A, float* gx, float* gy, float* gz, int i, float fx,
-                                                 float fy, float fz) {
+__device__ __forceinline__ bool kick_drift_mixed(const IArgs& A, const IArgs& to, float* gx, float* gy, float* gz,
+                                                 int i, float fx, float fy, float fz) {
     gx[i] = fx;
     gy[i] = fy;
     gz[i] = fz;
@@ -185,8 +204,8 @@ __device__ __forceinline__ bool kick_drift_mixed(const IArgs& A, float* gx, floa
         v[k][i] = vk;
         r[k] = fma(vk, A.dt, r[k]);
     }
-    A.rx[i] = r[0]; A.ry[i] = r[1]; A.rz[i] = r[2];
-    return offsets_check_mixed(A, i, r);
+    to.rx[i] = r[0]; to.ry[i] = r[1]; to.rz[i] = r[2];
+    return offsets_check_mixed(to, i, r);
 }
 
 __device__ __forceinline__ void kick_mixed_one(const IArgs& A, int i) {

@@ -182,7 +182,7 @@ struct mdg_system {
     int run_rebuild_kernels = 0;
     int run_pre_kernels = 0;                 // kernels of the graph's prefix
     double graph_build_s = 0.0;              // host seconds spent building run graphs
-    int solo_threads = 0;                    // > 0: run loops as one block of this many threads (solo.cu)
+    unsigned long long* team_word = nullptr; // barrier word of the team kernel (solo.cu)
 
     // device status + grid
     mdg::DevStatus* dstat = nullptr;
@@ -290,6 +290,11 @@ struct SoloQueue {              // host-mapped
     // yet resident count), 2 running a request
     volatile uint32_t live[kSoloGens][kSoloMaxBlocks];
 };
+// The step loop of a small system by a grid of blocks (solo.cu).
+bool team_eligible(const mdg_solver* s, const mdg_system* sys);
+int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam, int mixed, double pot_rcut,
+                int periodic, double dt, long steps, const double* hpos, const double* hvel, double* opos,
+                double* ovel, double* oforce);
 int solo_eligible(const mdg_solver* s, const mdg_system* sys);
 size_t solo_args_bytes();
 size_t solo_out_bytes();

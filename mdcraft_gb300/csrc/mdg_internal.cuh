@@ -212,6 +212,7 @@ struct DevStatus {
     uint32_t need_next;     // rebuild test of the next step's positions, from a force pass
                             // that ran the next step's first half-kick and drift
     uint32_t arrived;       // blocks of the bounds pass done (0 between rebuilds)
+    uint32_t team_done;     // blocks of the team kernel done (solo.cu; 0 between launches)
 };
 
 }  // namespace mdg

@@ -30,37 +30,20 @@ namespace mdg {
 // ---------------------------------------------------------------------------
 
 // Reduces the block's bounds (lo, hi, largest rns) over its threads; the
-// result is in v of thread 0.
-__device__ __forceinline__ void block_bounds(double v[7]) {
-    __shared__ double sh[kBlock / 32][7];
+// result is in v of warp 0's first lane.
+__device__ __forceinline__ void block_bounds(long long v[7]) {
+    __shared__ long long sh[kBlock / 32][7];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        for (int k = 0; k < 7; ++k) {
-            const double y = __shfl_down_sync(0xffffffffu, v[k], o);
-            v[k] = k < 3 ? fmin(v[k], y) : fmax(v[k], y);
-        }
+    warp_bounds<7>(v);
     if (lane == 0)
         for (int k = 0; k < 7; ++k) sh[w][k] = v[k];
     __syncthreads();
     if (w == 0) {
+        no_bounds<7>(v);
         if (lane < kBlock / 32)
             for (int k = 0; k < 7; ++k) v[k] = sh[lane][k];
-#pragma unroll
-        for (int o = kBlock / 64; o > 0; o >>= 1)
-            for (int k = 0; k < 7; ++k) {
-                const double y = __shfl_down_sync(0xffffffffu, v[k], o);
-                v[k] = k < 3 ? fmin(v[k], y) : fmax(v[k], y);
-            }
+        warp_bounds<7>(v);
     }
-}
-
-__device__ __forceinline__ void no_bounds(double v[7]) {
-    for (int k = 0; k < 3; ++k) {
-        v[k] = 1.7976931348623157e308;
-        v[3 + k] = -1.7976931348623157e308;
-    }
-    v[6] = 0.0;
 }
 
 // Wraps the positions and finds their bounds, the largest rns and whether the
@@ -73,19 +56,15 @@ __global__ void __launch_bounds__(kBlock)
                   GridParams* __restrict__ out, long long bin_cap, uint32_t* __restrict__ bin_count,
                   DevStatus* st) {
     const int t = threadIdx.x;
-    double v[7];
-    no_bounds(v);
+    long long v[7];
+    no_bounds<7>(v);
     const double r0 = n > 0 ? rns[0] : 0.0;
     bool differ = false;
     for (int i = blockIdx.x * kBlock + t; i < n; i += gridDim.x * kBlock) {
         double x[3];
         wrap_one(d, rx, ry, rz, i, x);
-        for (int a = 0; a < 3; ++a) {
-            v[a] = fmin(v[a], x[a]);
-            v[3 + a] = fmax(v[3 + a], x[a]);
-        }
         const double q = rns[i];
-        v[6] = v[6] < q ? q : v[6];
+        add_bounds(v, x, q);
         differ = differ || q != r0;
     }
     if (bin_count)
@@ -95,18 +74,18 @@ __global__ void __launch_bounds__(kBlock)
     block_bounds(v);
     __shared__ bool last;
     if (t == 0) {
-        for (int k = 0; k < 7; ++k) part[blockIdx.x * 8 + k] = v[k];
+        for (int k = 0; k < 7; ++k) part[blockIdx.x * 8 + k] = __longlong_as_double(v[k]);
         __threadfence();
         last = atomicAdd(&st->arrived, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    no_bounds(v);
+    no_bounds<7>(v);
     for (int b = t; b < (int)gridDim.x; b += kBlock)
         for (int k = 0; k < 7; ++k) {
-            const double y = __ldcg(part + b * 8 + k);
-            v[k] = k < 3 ? fmin(v[k], y) : fmax(v[k], y);
+            const long long y = __ldcg(reinterpret_cast<const long long*>(part) + b * 8 + k);
+            v[k] = k < 3 ? min(v[k], y) : max(v[k], y);
         }
     __syncthreads();  // block_bounds' shared array, read by the first call
     block_bounds(v);
@@ -114,10 +93,11 @@ __global__ void __launch_bounds__(kBlock)
     // three lanes take an axis each
     __shared__ GridParams g;
     if (t == 0) memset(&g, 0, sizeof(g));
-    const double cell = __shfl_sync(0xffffffffu, v[6], 0);
+    const double cell = key_double(__shfl_sync(0xffffffffu, v[6], 0));
     double lo = 0.0, hi = 0.0;
     for (int a = 0; a < 3; ++a) {
-        const double l = __shfl_sync(0xffffffffu, v[a], 0), h = __shfl_sync(0xffffffffu, v[3 + a], 0);
+        const double l = key_double(__shfl_sync(0xffffffffu, v[a], 0));
+        const double h = key_double(__shfl_sync(0xffffffffu, v[3 + a], 0));
         if (t == a && a < d.dim) {
             lo = l;
             hi = h;
@@ -267,32 +247,9 @@ __global__ void __launch_bounds__(kBlock)
     if (k >= n || gp->empty) return;
     const uint32_t i = src[k];
     const uint32_t d = sorted_slot((uint32_t)k, key[i], start, orig_at);
-    double x[12];
-#pragma unroll
-    for (int f = 0; f < 12; ++f) x[f] = G.a.in[f][i];
-#pragma unroll
-    for (int f = 0; f < 12; ++f) G.a.out[f][d] = x[f];
-#pragma unroll
-    for (int f = 0; f < 12; ++f) x[f] = G.b.in[f][i];
-#pragma unroll
-    for (int f = 0; f < 12; ++f) G.b.out[f][d] = x[f];
-#pragma unroll
-    for (int f = 0; f < 3; ++f) G.fc.out[f][d] = G.fc.in[f][i];
-#pragma unroll
-    for (int f = 0; f < 2; ++f) G.u.out[f][d] = G.u.in[f][i];
-#pragma unroll
-    for (int f = 0; f < 2; ++f) G.h.out[f][d] = G.h.in[f][i];
+    permute_one(G, i, d);
     cell_out[d] = cell[i];
 }
-
-struct CellOut {
-    uint32_t* cellp;
-    double *Rx, *Ry, *Rz;
-    int4 *pos32, *q0;
-    float4* o0;
-    uint32_t* slot_of;
-    float2* trig;
-};
 
 // The permuted fields back into the live buffers (so device pointers stay
 // fixed across rebuilds, as a captured graph needs), and what follows from
@@ -301,27 +258,7 @@ __global__ void __launch_bounds__(kBlock)
     k_settle(int n, GatherAll G, const uint32_t* __restrict__ cell, CellOut C, const GridParams* __restrict__ gp) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const GridParams& g = *gp;
-    if (k >= n || g.empty) return;
-    double x[12];
-#pragma unroll
-    for (int f = 0; f < 12; ++f) x[f] = G.b2.in[f][k];
-#pragma unroll
-    for (int f = 0; f < 12; ++f) G.b2.out[f][k] = x[f];
-#pragma unroll
-    for (int f = 0; f < 3; ++f) G.fc2.out[f][k] = G.fc2.in[f][k];
-    const uint32_t orig = G.u2.in[0][k];
-    G.u2.out[0][k] = orig;
-    G.u2.out[1][k] = G.u2.in[1][k];
-    const uint16_t kind = G.h2.in[0][k];
-    G.h2.out[0][k] = kind;
-    G.h2.out[1][k] = G.h2.in[1][k];
-#pragma unroll
-    for (int f = 0; f < 12; ++f) x[f] = G.a2.in[f][k];
-#pragma unroll
-    for (int f = 0; f < 12; ++f) G.a2.out[f][k] = x[f];
-    const double r[3] = {x[RX], x[RY], x[RZ]};
-    cells_one(g, k, r, cell[k], orig, kind, C.cellp, C.Rx, C.Ry, C.Rz, C.pos32, C.q0, C.o0, C.slot_of);
-    C.trig[k] = trig_of(x[RNS], x[RCUT], g);
+    if (k < n && !g.empty) settle_one(g, G, k, cell[k], C);
 }
 
 // ---------------------------------------------------------------------------
@@ -458,39 +395,41 @@ __global__ void __launch_bounds__(kExportWarps * 32)
 // Verlet list
 // ---------------------------------------------------------------------------
 
-// Block of NW warps (a system's launch shape, default 4), `parts` warps per
-// bin, on grids without a periodic axis of 2 cells or fewer
-// (GridParams::small_box; those take k_nbuild_atoms).
+// Block of NW warps (a system's launch shape, default 4), a warp per bin, on
+// grids without a periodic axis of 2 cells or fewer (GridParams::small_box;
+// those take k_nbuild_atoms, as do systems below kAtomBuildMost atoms).
 constexpr int kNbChunks = 8;
 template <int NW>
-__global__ void __launch_bounds__(NW * 32, 32 / NW)
-    k_nbuild_warp(NbArgs A, const GridParams* __restrict__ gp, int parts) {
+__global__ void __launch_bounds__(NW * 32, 32 / NW) k_nbuild_warp(NbArgs A, const GridParams* __restrict__ gp) {
     __shared__ GridParams g;
     __shared__ NbWarpSmem<kNbChunks> S[NW];
     if (threadIdx.x == 0) g = *gp;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int w = blockIdx.x * NW + warp, bin = w / parts;
+    const int bin = blockIdx.x * NW + warp;
     if (g.empty || g.small_box || bin >= g.nbins) return;
-    nbuild_cell_warp(A, g, bin, w - bin * parts, parts, lane, A.st->nonuniform == 0, S[warp]);
+    nbuild_cell_warp(A, g, bin, lane, A.st->nonuniform == 0, S[warp]);
 }
 
-// The list build of grids with a periodic axis of 2 cells or fewer (a few
-// cells of many atoms): a warp per atom. Launched after k_nbuild_warp. On
-// the other grids it returns at once, unless some atom was clamped into the
-// grid (FLAG_RANGE): those atoms' lists are built again from their
-// unclamped cells (nbuild_atom), over what the warp build wrote.
+// The list build by a warp per atom: of grids with a periodic axis of 2 cells
+// or fewer (a few cells of many atoms), of small systems (every grid), and of
+// atoms that were clamped into the grid (FLAG_RANGE), whose lists are built
+// again from their unclamped cells (nbuild_atom), over what the other builds
+// wrote. On other grids it returns at once.
 __global__ void __launch_bounds__(kBlock) k_nbuild_atoms(NbArgs A, const GridParams* __restrict__ gp) {
     __shared__ GridParams g;
     if (threadIdx.x == 0) g = *gp;
     __syncthreads();
     if (g.empty) return;
-    const bool clamped_only = !g.small_box;
-    if (clamped_only && !(A.st->build_flags & FLAG_RANGE)) return;
+    const bool few = A.n < kAtomBuildMost && !g.small_box, clamped = (A.st->build_flags & FLAG_RANGE) != 0;
+    if (!g.small_box && !few && !clamped) return;
     const bool uniform = A.st->nonuniform == 0;
+    const int lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (kBlock / 32);
-    for (uint32_t i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); i < (uint32_t)A.n; i += warps)
-        if (!clamped_only || A.o0[i].w == 2.0f) nbuild_atom(A, g, i, threadIdx.x & 31, uniform);
+    for (uint32_t i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); i < (uint32_t)A.n; i += warps) {
+        if (g.small_box || A.o0[i].w == 2.0f) nbuild_atom(A, g, i, lane, uniform);
+        else if (few) nbuild_atom_cells(A, g, i, lane, uniform);
+    }
 }
 
 // VerletList::optimize_search_radius (verlet-list.cxx:72-92):
@@ -570,7 +509,8 @@ static int nparts_of(const mdg_system* sys) {
 }
 
 static int ensure_parts(mdg_system* sys) {
-    int nparts = nparts_of(sys);
+    // a row per block of the bounds pass, or of a grid's team (one per SM)
+    int nparts = std::max(nparts_of(sys), sys->ctx->num_sms);
     if ((size_t)nparts > sys->part_cap) {
         sys_free(sys, sys->part, sys->part_cap * 8 * sizeof(double));
         sys->part = nullptr;
@@ -763,6 +703,11 @@ NbArgs nb_args(const mdg_system* sys) {
 
 DomainDev domain_of(const mdg_system* sys) { return domain_dev(sys); }
 
+CellOut cell_out(const mdg_system* sys) {
+    return CellOut{sys->cellp, sys->Rc[0], sys->Rc[1], sys->Rc[2], sys->pos32, sys->q0, sys->o0, sys->slot_of,
+                   sys->trig32};
+}
+
 // Exclusive scan of the live bins' counts into out[0..nbins].
 static int launch_scan(mdg_system* sys, uint32_t* out) {
     mdg_ctx* ctx = sys->ctx;
@@ -785,13 +730,6 @@ static int launch_scan(mdg_system* sys, uint32_t* out) {
     MDG_LAUNCHED(ctx);
     return MDG_OK;
 }
-
-// Warps per cell of the list build: several where the cells are fewer than
-// the GPU's warp slots (whole rebuilds with 1 / 2 / 4 / 8: LJ argon 4,000
-// atoms 133 / 116 / 113 / 102 us, EAM Cu 32,000 119 / 120 / 142 / 178 us,
-// LJ argon 62,500 152 / 176 / 201 / 263 us; each repeats the candidates'
-// loads).
-static int list_parts(size_t n) { return n < 12000 ? 4 : 1; }
 
 int nlist_enqueue(mdg_system* sys) {
     mdg_ctx* ctx = sys->ctx;
@@ -822,21 +760,18 @@ int nlist_enqueue(mdg_system* sys) {
     k_permute<<<pb, pt, 0, st>>>(n, sys->src, sys->cellp, sys->key, sys->bin_start, sys->ncnt, sys->rank, G,
                                  sys->dgrid);
     MDG_LAUNCHED(ctx);
-    const CellOut C = {sys->cellp, sys->Rc[0], sys->Rc[1], sys->Rc[2], sys->pos32, sys->q0, sys->o0, sys->slot_of,
-                       sys->trig32};
-    k_settle<<<pb, pt, 0, st>>>(n, G, sys->rank, C, sys->dgrid);
+    k_settle<<<pb, pt, 0, st>>>(n, G, sys->rank, cell_out(sys), sys->dgrid);
     MDG_LAUNCHED(ctx);
     NbArgs A = nb_args(sys);
-    // a warp per bin of the capacity; the live bins come from the device grid.
-    // Systems with fewer cells than the GPU has warp slots give each cell's
-    // atoms to several warps
-    const int cpb = sys->shape[MDG_SHAPE_LIST_CELLS_PER_BLOCK] ? sys->shape[MDG_SHAPE_LIST_CELLS_PER_BLOCK] : 4;
-    const int parts = list_parts(sys->n);
-    const unsigned nbw = (unsigned)((sys->bin_cap * parts + cpb - 1) / cpb);
-    if (cpb == 2) k_nbuild_warp<2><<<nbw, 2 * 32, 0, st>>>(A, sys->dgrid, parts);
-    else if (cpb == 8) k_nbuild_warp<8><<<nbw, 8 * 32, 0, st>>>(A, sys->dgrid, parts);
-    else k_nbuild_warp<4><<<nbw, 4 * 32, 0, st>>>(A, sys->dgrid, parts);
-    MDG_LAUNCHED(ctx);
+    // a warp per bin of the capacity; the live bins come from the device grid
+    if (n >= kAtomBuildMost) {
+        const int cpb = sys->shape[MDG_SHAPE_LIST_CELLS_PER_BLOCK] ? sys->shape[MDG_SHAPE_LIST_CELLS_PER_BLOCK] : 4;
+        const unsigned nbw = (unsigned)((sys->bin_cap + cpb - 1) / cpb);
+        if (cpb == 2) k_nbuild_warp<2><<<nbw, 2 * 32, 0, st>>>(A, sys->dgrid);
+        else if (cpb == 8) k_nbuild_warp<8><<<nbw, 8 * 32, 0, st>>>(A, sys->dgrid);
+        else k_nbuild_warp<4><<<nbw, 4 * 32, 0, st>>>(A, sys->dgrid);
+        MDG_LAUNCHED(ctx);
+    }
     // a grid-stride launch of at most four blocks per SM: on the large
     // grids, where it returns at once, its blocks are few
     k_nbuild_atoms<<<std::min(nblk(n, kBlock / 32), 4 * std::max(ctx->num_sms, 1)), kBlock, 0, st>>>(A, sys->dgrid);

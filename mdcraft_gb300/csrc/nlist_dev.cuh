@@ -13,6 +13,8 @@
 #include <cmath>
 #include <cstring>
 
+#include "integrate_dev.cuh"
+#include "mdg_host.h"
 #include "mdg_internal.cuh"
 
 namespace mdg {
@@ -179,6 +181,49 @@ __device__ __forceinline__ void wrap_one(const DomainDev& d, double* rx, double*
     }
 }
 
+// Bounds as integers that order like the doubles: a reduction over them runs
+// on the integer pipe (FP64 minima and maxima, 7 values over 5 levels in every
+// warp, took 7 to 13 us of a rebuild).
+__device__ __forceinline__ long long double_key(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double key_double(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
+// No atoms: +max, -max per axis, rns 0 (and a flag word, N = 8).
+template <int N>
+__device__ __forceinline__ void no_bounds(long long v[N]) {
+    for (int k = 0; k < 3; ++k) {
+        v[k] = double_key(1.7976931348623157e308);
+        v[3 + k] = double_key(-1.7976931348623157e308);
+    }
+    for (int k = 6; k < N; ++k) v[k] = 0;
+}
+// An atom's position and rns; NaN counts for nothing, as in fmin and fmax.
+__device__ __forceinline__ void add_bounds(long long* v, const double x[3], double rns) {
+    const long long inf = 0x7ff0000000000000LL;
+    for (int a = 0; a < 3; ++a) {
+        const long long b = __double_as_longlong(x[a]);
+        if ((b & 0x7fffffffffffffffLL) > inf) continue;
+        const long long k = double_key(x[a]);
+        v[a] = min(v[a], k);
+        v[3 + a] = max(v[3 + a], k);
+    }
+    const long long q = double_key(rns);
+    if (q <= inf) v[6] = max(v[6], q);
+}
+template <int N>
+__device__ __forceinline__ void warp_bounds(long long v[N]) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const long long y = __shfl_down_sync(0xffffffffu, v[k], o);
+            v[k] = k < 3 ? min(v[k], y) : max(v[k], y);
+        }
+}
+
 // A packed cell with the atom's clamped flag in its top bit.
 constexpr uint32_t kClampedCell = 1u << 31;
 
@@ -252,6 +297,64 @@ struct GatherAll {
     GatherSet<2, uint16_t> h, h2;
 };
 
+// Every permuted field of atom i into slot d of the spare buffers.
+__device__ __forceinline__ void permute_one(const GatherAll& G, uint32_t i, uint32_t d) {
+    double x[12];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) x[f] = G.a.in[f][i];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) G.a.out[f][d] = x[f];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) x[f] = G.b.in[f][i];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) G.b.out[f][d] = x[f];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) G.fc.out[f][d] = G.fc.in[f][i];
+#pragma unroll
+    for (int f = 0; f < 2; ++f) G.u.out[f][d] = G.u.in[f][i];
+#pragma unroll
+    for (int f = 0; f < 2; ++f) G.h.out[f][d] = G.h.in[f][i];
+}
+
+struct CellOut {
+    uint32_t* cellp;
+    double *Rx, *Ry, *Rz;
+    int4 *pos32, *q0;
+    float4* o0;
+    uint32_t* slot_of;
+    float2* trig;
+};
+
+// The permuted fields of slot k back into the live buffers, and what follows
+// from them.
+__device__ __forceinline__ void settle_one(const GridParams& g, const GatherAll& G, int k, uint32_t cell,
+                                           const CellOut& C) {
+    double x[12];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) x[f] = G.b2.in[f][k];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) G.b2.out[f][k] = x[f];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) G.fc2.out[f][k] = G.fc2.in[f][k];
+    const uint32_t orig = G.u2.in[0][k];
+    G.u2.out[0][k] = orig;
+    G.u2.out[1][k] = G.u2.in[1][k];
+    const uint16_t kind = G.h2.in[0][k];
+    G.h2.out[0][k] = kind;
+    G.h2.out[1][k] = G.h2.in[1][k];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) x[f] = G.a2.in[f][k];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) G.a2.out[f][k] = x[f];
+    const double r[3] = {x[RX], x[RY], x[RZ]};
+    cells_one(g, k, r, cell, orig, kind, C.cellp, C.Rx, C.Ry, C.Rz, C.pos32, C.q0, C.o0, C.slot_of);
+    C.trig[k] = trig_of(x[RNS], x[RCUT], g);
+}
+
+// Systems (exclusive) whose lists are built by a warp per atom on every grid
+// (nbuild_atom_cells).
+constexpr int kAtomBuildMost = 8000;
+
 struct NbArgs {
     int n, np, K, half;
     const double *rx, *ry, *rz, *rns, *rcut;
@@ -324,6 +427,26 @@ __device__ __forceinline__ float min_image_f(float d, float L) {
     if (d > half) return d - L;
     if (d < -half) return d + L;
     return d;
+}
+
+// The end of atom i's list of cnt entries, by a warp: padding to a multiple of
+// four with self entries, the counts and the rebuild snapshot.
+__device__ __forceinline__ void end_list(const NbArgs& A, uint32_t i, int lane, int cnt) {
+    const int padded = (cnt + 3) & ~3;
+    if (cnt + lane < padded && cnt + lane < A.K) A.nbr[nidx(cnt + lane, i, A.np)] = i | kSelfCode;
+    if (lane) return;
+    A.ncnt[i] = padded < A.K ? padded : A.K;
+    if (cnt > A.K) {
+        atomicOr(&A.st->flags, FLAG_OVERFLOW);
+        atomicOr(&A.st->build_flags, FLAG_OVERFLOW);
+    }
+    atomicMax(&A.st->max_count, (uint32_t)cnt);
+    A.r0x[i] = A.rx[i];
+    A.r0y[i] = A.ry[i];
+    A.r0z[i] = A.rz[i];
+    A.saved_rcut[i] = A.rcut[i];
+    A.saved_rns[i] = A.rns[i];
+    A.saved_uid[i] = A.uid[i];
 }
 
 // The list of atom i by a warp, lanes over the candidates (used for grids
@@ -433,22 +556,92 @@ __device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g
             }
         }
     }
-    // pad to a multiple of four with self entries
-    const int padded = (cnt + 3) & ~3;
-    if (cnt + lane < padded && cnt + lane < A.K) A.nbr[nidx(cnt + lane, i, A.np)] = i | kSelfCode;
-    if (lane) return;
-    A.ncnt[i] = padded < A.K ? padded : A.K;
-    if (cnt > A.K) {
-        atomicOr(&A.st->flags, FLAG_OVERFLOW);
-        atomicOr(&A.st->build_flags, FLAG_OVERFLOW);
+    end_list(A, i, lane, cnt);
+}
+
+// The neighbour cell of lane t < 27, (t / 9 - 1, t / 3 % 3 - 1, t % 3 - 1)
+// from the cell at global index gc (local own): its first slot and count (0:
+// none, or outside the grid), image code and shift. For grids whose periodic
+// axes have 3 cells or more.
+__device__ __forceinline__ void neighbour_cell(const GridParams& g, const uint32_t* bin_start, const int gc[3],
+                                               const int own[3], int t, uint32_t& j0, uint32_t& count, uint32_t& code,
+                                               float4& sh) {
+    j0 = count = code = 0;
+    sh = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t >= 27) return;
+    const int dl[3] = {t / 9 - 1, (t / 3) % 3 - 1, t % 3 - 1};
+    int lc[3];
+    for (int a = 0; a < 3; ++a) {
+        if (g.periodic[a] && ((g.dom_n[a] == 1 && dl[a] != 0) || (g.dom_n[a] == 2 && dl[a] == 1))) return;
+        int nb = gc[a] + dl[a];
+        if (g.periodic[a]) nb = nb < 0 ? nb + g.dom_n[a] : nb >= g.dom_n[a] ? nb - g.dom_n[a] : nb;
+        lc[a] = nb - g.offset[a];
+        if (lc[a] < 0 || lc[a] >= g.num[a]) return;
     }
-    atomicMax(&A.st->max_count, (uint32_t)cnt);
-    A.r0x[i] = xi;
-    A.r0y[i] = yi;
-    A.r0z[i] = zi;
-    A.saved_rcut[i] = A.rcut[i];
-    A.saved_rns[i] = rni;
-    A.saved_uid[i] = A.uid[i];
+    const int bk = bin_key(g, lc[0], lc[1], lc[2]);
+    j0 = bin_start[bk];
+    count = bin_start[bk + 1] - j0;
+    sh = make_float4((float)dl[0] * g.csf[0], (float)dl[1] * g.csf[1], (float)dl[2] * g.csf[2], 0.f);
+    for (int a = 0; a < 3; ++a) {
+        code |= (uint32_t)(dl[a] + 1) << (2 * a);
+        if (dl[a] != lc[a] - own[a]) code |= 1u << 6;  // the image crossed a periodic face
+    }
+}
+
+// The list of atom i by a warp on such grids (an atom clamped into the grid
+// excepted): 27 lanes fetch the neighbour cells, then the cells in order, 32
+// candidates at a time. Some five times the instructions per atom of the
+// warp-per-cell build below, but a warp per atom: for systems of so few cells
+// that most SMs have none (LJ argon 4,000 atoms has 125: 42 us by cells in
+// four parts each, 13 us by atoms).
+__device__ __forceinline__ void nbuild_atom_cells(const NbArgs& A, const GridParams& g, uint32_t i, int lane,
+                                                  bool uniform_rns) {
+    const unsigned full = 0xffffffffu;
+    const float lo2 = (float)(g.max_rns * g.max_rns * (1.0 - 1e-5));
+    const float hi2 = (float)(g.max_rns * g.max_rns * (1.0 + 1e-5));
+    int own[3];
+    unpack_cell(A.cellp[i], own[0], own[1], own[2]);
+    int gc[3] = {own[0] + g.offset[0], own[1] + g.offset[1], own[2] + g.offset[2]};
+    if (g.dim < 3) gc[2] = 0;
+    if (g.dim < 2) gc[1] = 0;
+    uint32_t j0, count, code;
+    float4 sh;
+    neighbour_cell(g, A.bin_start, gc, own, lane, j0, count, code, sh);
+    const float4 oi = A.o0[i];
+    const bool pfi = uniform_rns && oi.w == 0.0f;
+    const uint32_t origi = A.half ? A.orig[i] : 0u;
+    int cnt = 0;
+    for (unsigned left = __ballot_sync(full, count > 0); left; left &= left - 1u) {
+        const int c = __ffs(left) - 1;
+        const uint32_t c0 = __shfl_sync(full, j0, c), c1 = c0 + __shfl_sync(full, count, c);
+        const uint32_t img = __shfl_sync(full, code, c) << kJBits;
+        const float sx = __shfl_sync(full, sh.x, c), sy = __shfl_sync(full, sh.y, c), sz = __shfl_sync(full, sh.z, c);
+        for (uint32_t jb = c0; jb < c1; jb += 32) {
+            const uint32_t j = jb + lane;
+            bool acc = j < c1 && j != i && !(A.half && A.orig[j] < origi);
+            if (acc) {
+                const float4 oj = A.o0[j];
+                const float dx = oi.x - (oj.x + sx), dy = oi.y - (oj.y + sy), dz = oi.z - (oj.z + sz);
+                const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                const bool pf = pfi && oj.w == 0.0f;
+                if (pf && d2 < lo2) {
+                    acc = true;
+                } else if (pf && d2 > hi2) {
+                    acc = false;
+                } else {
+                    bool edge[3] = {false, false, false};
+                    for (int a = 0; a < g.dim; ++a) edge[a] = gc[a] == 0 || gc[a] == g.num[a] - 1;
+                    acc = are_neibs_exact(g, A.rx[i], A.ry[i], A.rz[i], A.rns[i], A.rx[j], A.ry[j], A.rz[j], A.rns[j],
+                                          edge);
+                }
+            }
+            const unsigned m = __ballot_sync(full, acc);
+            const int k = cnt + __popc(m & ((1u << lane) - 1u));
+            if (acc && k < A.K) A.nbr[nidx(k, i, A.np)] = j | img;
+            cnt += __popc(m);
+        }
+    }
+    end_list(A, i, lane, cnt);
 }
 
 // ---- list build, a warp per cell with lanes over candidates -------------------
@@ -474,10 +667,8 @@ template <int CH>
 struct NbWarpSmem {
     float4 csh[27];          // cell shift (x, y, z) of the image
     float4 oa[32];           // pairs of atoms: (-2ax0, -2ax1, -2ay0, -2ay1), (-2az0, -2az1, m0, m1), m = |a|^2 - mid
-    float4 oi[32];           // the batch's offsets
     uint32_t row[CH][32];    // accept rows of the turn's chunks: bit = candidate, column = atom
     uint32_t cand[CH * 32];  // the turn's list entries (slot | image code)
-    uint32_t origi[32];
     uint32_t cj0[27];        // first slot of each non-empty neighbour cell
     uint32_t cpre[28];       // candidate prefix over those cells
     uint32_t ccode[27];      // image code << kJBits
@@ -503,60 +694,27 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
 
-// The lists of part `part` of `parts` of the bin's atoms.
 template <int CH>
-__device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridParams& g, int bin, int part, int parts,
-                                                 int lane, bool uniform_rns, NbWarpSmem<CH>& S) {
+__device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridParams& g, int bin, int lane,
+                                                 bool uniform_rns, NbWarpSmem<CH>& S) {
     const unsigned full = 0xffffffffu;
     const float lo2 = (float)(g.max_rns * g.max_rns * (1.0 - 1e-5));
     const float hi2 = (float)(g.max_rns * g.max_rns * (1.0 + 1e-5));
-    uint32_t s0 = A.bin_start[bin], s1 = A.bin_start[bin + 1];
+    const uint32_t s0 = A.bin_start[bin], s1 = A.bin_start[bin + 1];
     if (s0 == s1) return;
     int cx, cy, cz;
     unpack_cell(A.cellp[s0], cx, cy, cz);
-    const uint32_t home0 = s0;  // the bin's first slot
-    if (parts > 1) {
-        const uint32_t per = (s1 - s0 + parts - 1) / parts;
-        s0 += part * per;
-        s1 = min(s0 + per, s1);
-        if (s0 >= s1) return;
-    }
     int gc[3] = {cx + g.offset[0], cy + g.offset[1], cz + g.offset[2]};
     if (g.dim < 3) gc[2] = 0;
     if (g.dim < 2) gc[1] = 0;
     bool edge[3] = {false, false, false};
     for (int a = 0; a < g.dim; ++a) edge[a] = gc[a] == 0 || gc[a] == g.num[a] - 1;
 
-    // lane t < 27: neighbour cell (t / 9 - 1, t / 3 % 3 - 1, t % 3 - 1)
-    bool valid = false;
-    uint32_t j0 = 0, ncand = 0, code = 0;
-    float4 sh = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (lane < 27) {
-        const int dl[3] = {lane / 9 - 1, (lane / 3) % 3 - 1, lane % 3 - 1};
-        valid = true;
-        for (int a = 0; a < 3; ++a)
-            if (g.periodic[a] && ((g.dom_n[a] == 1 && dl[a] != 0) || (g.dom_n[a] == 2 && dl[a] == 1))) valid = false;
-        if (valid) {
-            int nb[3] = {gc[0] + dl[0], gc[1] + dl[1], gc[2] + dl[2]};
-            for (int a = 0; a < 3; ++a)
-                if (g.periodic[a]) nb[a] = nb[a] < 0 ? nb[a] + g.dom_n[a] : nb[a] >= g.dom_n[a] ? nb[a] - g.dom_n[a] : nb[a];
-            const int lc[3] = {nb[0] - g.offset[0], nb[1] - g.offset[1], nb[2] - g.offset[2]};
-            if (lc[0] < 0 || lc[0] >= g.num[0] || lc[1] < 0 || lc[1] >= g.num[1] || lc[2] < 0 || lc[2] >= g.num[2]) {
-                valid = false;
-            } else {
-                const int bk = bin_key(g, lc[0], lc[1], lc[2]);
-                j0 = A.bin_start[bk];
-                ncand = A.bin_start[bk + 1] - j0;
-                sh = make_float4((float)dl[0] * g.csf[0], (float)dl[1] * g.csf[1], (float)dl[2] * g.csf[2], 0.f);
-                const int own[3] = {cx, cy, cz};
-                for (int a = 0; a < 3; ++a) {
-                    code |= (uint32_t)(dl[a] + 1) << (2 * a);
-                    if (dl[a] != lc[a] - own[a]) code |= 1u << 6;  // the image crossed a periodic face
-                }
-            }
-        }
-    }
-    const bool use = valid && ncand > 0;
+    uint32_t j0, ncand, code;
+    float4 sh;
+    const int own[3] = {cx, cy, cz};
+    neighbour_cell(g, A.bin_start, gc, own, lane, j0, ncand, code, sh);
+    const bool use = ncand > 0;
     const unsigned vm = __ballot_sync(full, use);
     const int slot = __popc(vm & ((1u << lane) - 1u));
     const int nc = __popc(vm);
@@ -591,8 +749,6 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
         float4 oa = make_float4(0.f, 0.f, 0.f, 0.f);
         if (act) {
             oa = A.o0[me];
-            S.oi[lane] = oa;
-            S.origi[lane] = A.orig[me];
         }
         // an atom whose offset is not exact takes the batch to the exact tests
         const bool rough = __any_sync(full, oa.w != 0.0f) || !uniform_rns || A.half;
@@ -607,7 +763,7 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
             q[6] = m;
         }
         // this atom's own candidate index (it is a candidate of its own cell)
-        const uint32_t self_t = act ? S.cpre[home] + (me - home0) : 0xffffffffu;
+        const uint32_t self_t = act ? S.cpre[home] + (me - s0) : 0xffffffffu;
         __syncwarp();
         int cnt = 0;  // list length of atom `me`
         int c = 0;    // neighbour cell of this lane's candidate
@@ -660,11 +816,11 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
                     unsigned mine = 0, mine_x = 0;
                     const uint32_t origj = A.half && have ? A.orig[j] : 0u;
                     for (uint32_t ii = 0; ii < ni; ++ii) {
-                        const float4 oi = S.oi[ii];
+                        const float4 oi = A.o0[base + ii];
                         const float dx = oi.x - px, dy = oi.y - py, dz = oi.z - pz;
                         const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
                         const bool pf = uniform_rns && pfj && oi.w == 0.0f;
-                        const bool ok = have && j != base + ii && !(A.half && origj < S.origi[ii]);
+                        const bool ok = have && j != base + ii && !(A.half && origj < A.orig[base + ii]);
                         const unsigned m = __ballot_sync(full, ok && pf && d2 < lo2);
                         const unsigned mx = __ballot_sync(full, ok && !(pf && (d2 < lo2 || d2 > hi2)));
                         if ((uint32_t)lane == ii) {
@@ -734,4 +890,5 @@ namespace mdg {
 GatherAll gather_sets(const mdg_system* sys);
 NbArgs nb_args(const mdg_system* sys);
 DomainDev domain_of(const mdg_system* sys);
+CellOut cell_out(const mdg_system* sys);
 }  // namespace mdg

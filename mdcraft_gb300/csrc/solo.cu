@@ -1,27 +1,37 @@
-// solo.cu — the whole driver loop of one small system in one thread block.
+// solo.cu — the whole driver loop of one small system in one kernel.
 //
-// For the serving loop's systems (hundreds to tens of thousands of atoms) a
-// step is a few microseconds of work spread over a few SMs, so launching its
-// stages as separate kernels (or graph nodes) costs more than the work. Here
-// one block owns one system and runs `steps` iterations of the driver loop
-// of the reference (test/python/solver/test-EAM.py:158-200: make_step, then
-// decide() and update(-1)) with block barriers between the passes:
+// For small systems (hundreds to tens of thousands of atoms) a step is a few
+// microseconds of work, so launching its stages as separate kernels (or graph
+// nodes) costs more than the work. Here a team of blocks owns one system and
+// runs `steps` iterations of the driver loop of the reference
+// (test/python/solver/test-EAM.py:158-200: make_step, then decide() and
+// update(-1)) with barriers between the passes:
 //   drift + half-skin test -> [EAM density ->] forces -> kick
 //   -> if any atom moved half a skin: the rebuild (wrap + bounds, grid,
-//      bin count, scan, scatter, in-bin sort, permutation of every field,
-//      cell offsets, list build) -> next step.
+//      bin count, scan, scatter, permutation of every field, cell offsets,
+//      list build) -> next step.
 // Every pass calls the same per-atom (or per-bin) device code as the
 // per-stage kernels, in the same order, so a system gives the same bits
-// here as through mdg_run. Many systems run at once, one block each, in
-// shared launches. Nothing in the loop waits on another block.
+// here as through the graph of mdg_run. Two teams:
+//
+//  - one block (the serving loop): a persistent kernel's block takes a whole
+//    request from a queue; many systems run at once, a block each, and no
+//    block waits on another.
+//  - a grid of one block per SM, launched cooperatively (mdg_run and
+//    mdg_run_host of a small system): the blocks share the system's atoms and
+//    meet at barriers in global memory. Every wait is bounded.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cstring>
 
+#include "forces64_dev.cuh"
 #include "forces_dev.cuh"
 #include "integrate_dev.cuh"
 #include "mdg_host.h"
 #include "nlist_dev.cuh"
+#include "thermo_dev.cuh"
 
 namespace mdg {
 
@@ -49,21 +59,16 @@ struct alignas(16) SoloArgs {
     NbArgs N;
     GatherAll G;
     DomainDev D;
+    CellOut C;
     const PotSet* ps;
     int n;
     double *rx, *ry, *rz;
     const double* rns;
     uint32_t *key, *rank, *src, *bin_count, *bin_start;
     const uint32_t* orig;
-    uint32_t* cellp;
-    double *Rx, *Ry, *Rz;
-    int4 *pos32, *q0;
-    float4* o0;
-    uint32_t* slot_of;
-    const double *saved_rns, *saved_rcut;
-    float2* trig;
     GridParams* dgrid;
     long long bin_cap;
+    long long* part;              // a grid's team: 8 words per block
     DevStatus* st;
     long long steps;              // steps to run
     uint32_t seq;                 // completion value written to out->done
@@ -79,112 +84,194 @@ struct alignas(16) SoloArgs {
 constexpr int kSoloMaxAtoms = 65536;
 // Chunks per turn of the list build here: few, as its shared memory is taken
 // from the L1 that the force passes gather through.
-constexpr int kSoloChunks = 4;
+constexpr int kSoloChunks = 2;
+
+// Polls (each an L2 round trip) after which a team's barrier gives up: ten
+// seconds or more, against rebuild phases of microseconds.
+constexpr int kTeamPolls = 1 << 23;
+
+// The blocks that run one system together and this thread's share of it:
+// atoms a0 .. a1 of the block, thread gt of gn, warp gw of nw. WIDE: a grid of
+// blocks; else one block.
+//
+// The grid's barrier is one 64-bit word: arrivals in its low half, votes in
+// two counters above it, for barriers of even and odd number (a block may
+// stand at the next barrier when a slow one reads the word, but never
+// further). A block's first thread adds and polls. (A word per block that
+// every block reads took 4 to 6 us against 2 here: 143 x 143 polls.)
+template <int NT, bool WIDE>
+struct Team {
+    int t, lane, w, rank, size, a0, a1, gt, gn, gw, nw;
+    bool dead = false;  // a barrier gave up; the run is void
+    uint32_t epoch = 0;             // barriers passed
+    uint32_t cast[2] = {0, 0};      // votes counted so far at even and odd barriers
+    unsigned long long* word;       // zero at the kernel's start
+    int* said;                      // shared: bit 0 the vote, bit 1 a wait ran out
+
+    __device__ __forceinline__ Team(unsigned long long* wd, int* flag, int n, int per) : word(wd), said(flag) {
+        t = threadIdx.x;
+        lane = t & 31;
+        w = t >> 5;
+        rank = WIDE ? (int)blockIdx.x : 0;
+        size = WIDE ? (int)gridDim.x : 1;
+        a0 = WIDE ? min(rank * per, n) : 0;
+        a1 = WIDE ? min(a0 + per, n) : n;
+        gt = rank * NT + t;
+        gn = size * NT;
+        gw = w * size + rank;  // neighbouring tasks on different blocks
+        nw = size * (NT / 32);
+    }
+    // Every block's writes before are visible to every block after; whether
+    // any thread of the team has `vote` set.
+    __device__ __forceinline__ bool any(bool vote) {
+        const int mine = __syncthreads_or(vote);
+        if (!WIDE || dead) return mine != 0;
+        ++epoch;
+        if (t == 0) {
+            const int odd = epoch & 1, at = 32 + 16 * odd;
+            __threadfence();
+            atomicAdd(word, 1ull + ((unsigned long long)(mine ? 1 : 0) << at));
+            const uint32_t target = epoch * (uint32_t)size;
+            unsigned long long v;
+            int polls = 0;
+            do {
+                v = *(volatile unsigned long long*)word;
+            } while ((int)((uint32_t)v - target) < 0 && ++polls < kTeamPolls);
+            __threadfence();
+            const uint32_t sum = (uint32_t)(v >> at) & 0xffffu;
+            *said = (sum != cast[odd] ? 1 : 0) | ((int)((uint32_t)v - target) < 0 ? 2 : 0);
+            cast[odd] = sum;
+        }
+        __syncthreads();
+        const int s = *said;
+        dead = (s & 2) != 0;
+        return (s & 1) != 0;
+    }
+    __device__ __forceinline__ void sync() {
+        if (WIDE) any(false);
+        else __syncthreads();
+    }
+};
 
 template <int NT>
-__device__ __forceinline__ void gather_block(const GatherAll& G, const uint32_t* src, int n) {
-    for (int k = threadIdx.x; k < n; k += NT) {
-        uint32_t s = src[k];
-#pragma unroll
-        for (int f = 0; f < 12; ++f) G.a.out[f][k] = G.a.in[f][s];
-#pragma unroll
-        for (int f = 0; f < 12; ++f) G.b.out[f][k] = G.b.in[f][s];
-#pragma unroll
-        for (int f = 0; f < 3; ++f) G.fc.out[f][k] = G.fc.in[f][s];
-#pragma unroll
-        for (int f = 0; f < 2; ++f) G.u.out[f][k] = G.u.in[f][s];
-#pragma unroll
-        for (int f = 0; f < 2; ++f) G.h.out[f][k] = G.h.in[f][s];
+struct SoloShared {
+    long long red[8][NT / 32];
+    uint32_t scan[32];
+    int differ, said;
+};
+// The eight-lane passes' exchange (the grid's team only: a request's block
+// leaves its shared memory to L1).
+template <int NT>
+struct LaneShared {
+    float part[NT / 32][96];  // lane_sums
+    float sum[3][NT / 8];
+};
+
+// Reduces the bounds (BoundKeys) of the block's threads; `busy` false: the
+// whole warp has none. The result is in sh.red[k][0] after a __syncthreads by
+// the caller.
+template <int NT>
+__device__ __forceinline__ void block_bounds8(long long v[8], bool busy, SoloShared<NT>& sh) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (busy) warp_bounds<8>(v);
+    if (lane == 0)
+        for (int k = 0; k < 8; ++k) sh.red[k][w] = v[k];
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        const int k = threadIdx.x;
+        long long x = sh.red[k][0];
+        for (int q = 1; q < NT / 32; ++q) x = k < 3 ? min(x, sh.red[k][q]) : max(x, sh.red[k][q]);
+        sh.red[k][0] = x;
     }
 }
 
-template <int NT>
-__device__ __forceinline__ void copy_back_block(const GatherAll& G, int n) {
-    for (int k = threadIdx.x; k < n; k += NT) {
-#pragma unroll
-        for (int f = 0; f < 12; ++f) G.a2.out[f][k] = G.a2.in[f][k];
-#pragma unroll
-        for (int f = 0; f < 12; ++f) G.b2.out[f][k] = G.b2.in[f][k];
-#pragma unroll
-        for (int f = 0; f < 3; ++f) G.fc2.out[f][k] = G.fc2.in[f][k];
-#pragma unroll
-        for (int f = 0; f < 2; ++f) G.u2.out[f][k] = G.u2.in[f][k];
-#pragma unroll
-        for (int f = 0; f < 2; ++f) G.h2.out[f][k] = G.h2.in[f][k];
-    }
-}
-
-// One rebuild by the whole block (the pipeline of nlist_enqueue + trig).
-// Block-uniform result: false when a capacity overflowed (the loop stops and
-// the host grows the capacities).
-template <int NT>
-__device__ __noinline__ bool solo_rebuild(const SoloArgs& S, GridParams& g, double (*red)[NT / 32], uint32_t* scan_sh) {
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5, n = S.n;
-    if (t == 0) {
+// One rebuild by the team (the pipeline of nlist_enqueue). Team-uniform
+// result: false when a capacity overflowed (the loop stops and the host grows
+// the capacities).
+template <int NT, bool WIDE>
+__device__ __noinline__ bool solo_rebuild(Team<NT, WIDE>& tm, const SoloArgs& S, GridParams& g, SoloShared<NT>& sh) {
+    const int t = tm.t, n = S.n;
+    if (tm.gt == 0) {
         S.st->max_count = 0;
-        S.st->nonuniform = 0;
         S.st->build_flags = 0;
     }
     // wrap + bounds (min/max are exact, so the order of the reduction is free)
-    double v7[7] = {1.7976931348623157e308, 1.7976931348623157e308, 1.7976931348623157e308,
-                    -1.7976931348623157e308, -1.7976931348623157e308, -1.7976931348623157e308, 0.0};
-    for (int i = t; i < n; i += NT) {
-        double v[3];
-        wrap_one(S.D, S.rx, S.ry, S.rz, i, v);
-        for (int a = 0; a < 3; ++a) {
-            v7[a] = fmin(v7[a], v[a]);
-            v7[3 + a] = fmax(v7[3 + a], v[a]);
-        }
-        double q = S.rns[i];
-        v7[6] = v7[6] < q ? q : v7[6];
+    long long v[8];
+    no_bounds<8>(v);
+    const double r0 = S.rns[0];
+    for (int i = tm.a0 + t; i < tm.a1; i += NT) {
+        double x[3];
+        wrap_one(S.D, S.rx, S.ry, S.rz, i, x);
+        const double q = S.rns[i];
+        add_bounds(v, x, q);
+        if (q != r0) v[7] = 1;
     }
-    for (int o = 16; o > 0; o >>= 1)
-        for (int k = 0; k < 7; ++k) {
-            double y = __shfl_down_sync(0xffffffffu, v7[k], o);
-            v7[k] = k < 3 ? fmin(v7[k], y) : fmax(v7[k], y);
-        }
-    if (lane == 0)
-        for (int k = 0; k < 7; ++k) red[k][w] = v7[k];
+    for (long long b = tm.gt; b < S.bin_cap; b += tm.gn) S.bin_count[b] = 0;
+    block_bounds8<NT>(v, tm.a0 + (t & ~31) < tm.a1, sh);
     __syncthreads();
-    if (t == 0) {
-        for (int q = 1; q < NT / 32; ++q)
-            for (int k = 0; k < 7; ++k) red[k][0] = k < 3 ? fmin(red[k][0], red[k][q]) : fmax(red[k][0], red[k][q]);
-        double lo[3] = {red[0][0], red[1][0], red[2][0]}, hi[3] = {red[3][0], red[4][0], red[5][0]};
-        GridParams gg;
-        grid_from_bounds(S.D, lo, hi, red[6][0], gg);
-        if (gg.empty == 0 && (long long)gg.nbins + 1 > S.bin_cap) {
-            gg.empty = -3;
-            atomicOr(&S.st->flags, FLAG_OVERFLOW);
-            atomicOr(&S.st->build_flags, FLAG_OVERFLOW);
-        }
-        g = gg;
-        *S.dgrid = gg;
+    if (WIDE) {
+        if (t < 8) S.part[tm.rank * 8 + t] = sh.red[t][0];
+        tm.sync();
+        if (tm.dead) return false;
+        no_bounds<8>(v);
+        for (int b = t; b < tm.size; b += NT)
+            for (int k = 0; k < 8; ++k) {
+                const long long y = __ldcg(S.part + b * 8 + k);
+                v[k] = k < 3 ? min(v[k], y) : max(v[k], y);
+            }
+        block_bounds8<NT>(v, (t & ~31) < tm.size, sh);
+        __syncthreads();
     }
-    // nonuniform rns (the list's FP32 prefilter needs one rns for all)
-    {
-        double r0 = S.rns[0];
-        for (int i = t; i < n; i += NT)
-            if (S.rns[i] != r0) atomicOr(&S.st->nonuniform, 1u);
+    // the grid, by every block: three lanes take an axis each
+    if (t < 32) {
+        const double cell = key_double(sh.red[6][0]);
+        if (t == 0) {
+            memset(&g, 0, sizeof(g));
+            sh.differ = sh.red[7][0] == 1;
+        }
+        __syncwarp();
+        bool small = false, bad = false;
+        if (t < 3)
+            grid_axis(S.D, t < S.D.dim ? key_double(sh.red[t][0]) : 0.0, t < S.D.dim ? key_double(sh.red[3 + t][0]) : 0.0,
+                      cell, t, g, &small, &bad);
+        small = __any_sync(0xffffffffu, small);
+        bad = __any_sync(0xffffffffu, bad);
+        __syncwarp();
+        if (t == 0) {
+            grid_totals(S.D, cell, small, bad, g);
+            if (g.empty == 0 && (long long)g.nbins + 1 > S.bin_cap) {
+                g.empty = -3;
+                if (tm.rank == 0) {
+                    atomicOr(&S.st->flags, FLAG_OVERFLOW);
+                    atomicOr(&S.st->build_flags, FLAG_OVERFLOW);
+                }
+            }
+            if (tm.rank == 0) {
+                *S.dgrid = g;
+                S.st->nonuniform = sh.differ;
+            }
+        }
     }
     __syncthreads();
     if (g.empty) {
-        bool ok = g.empty != -3;
-        __syncthreads();
+        const bool ok = g.empty != -3;
+        tm.sync();
         return ok;
     }
     const int nb = g.nbins;
-    for (long long b = t; b < S.bin_cap; b += NT) S.bin_count[b] = 0;
-    __syncthreads();
-    for (int i = t; i < n; i += NT) bin_count_one(g, i, S.rx, S.ry, S.rz, S.key, S.rank, S.N.ncnt, S.bin_count, S.st);
-    __syncthreads();
-    // exclusive scan: each thread a contiguous chunk of the bins
-    {
+    // (the bins were cleared before the last barrier)
+    for (int i = tm.a0 + t; i < tm.a1; i += NT)
+        bin_count_one(g, i, S.rx, S.ry, S.rz, S.key, S.rank, S.N.ncnt, S.bin_count, S.st);
+    tm.sync();
+    if (tm.dead) return false;
+    // exclusive scan, by one block: each thread a contiguous chunk of the bins
+    if (tm.rank == 0) {
         const int chunk = (nb + NT - 1) / NT;
         const int b0 = min(t * chunk, nb), b1 = min(b0 + chunk, nb);
         uint32_t sum = 0;
         for (int b = b0; b < b1; ++b) sum += S.bin_count[b];
         uint32_t tot;
-        uint32_t off = block_excl_scan(sum, scan_sh, &tot);
+        uint32_t off = block_excl_scan(sum, sh.scan, &tot);
         for (int b = b0; b < b1; ++b) {
             uint32_t c = S.bin_count[b];
             S.bin_start[b] = off;
@@ -192,56 +279,56 @@ __device__ __noinline__ bool solo_rebuild(const SoloArgs& S, GridParams& g, doub
         }
         if (t == 0) S.bin_start[nb] = tot;
     }
-    __syncthreads();
+    tm.sync();
+    if (tm.dead) return false;
     // arrival order (the atoms' cells wait in ncnt, their caller indices in
-    // arrival order in cellp), then each bin by caller index (into rank)
-    for (int i = t; i < n; i += NT) {
+    // arrival order in cellp), then each bin by caller index
+    for (int i = tm.a0 + t; i < tm.a1; i += NT) {
         const uint32_t k = S.bin_start[S.key[i]] + S.rank[i];
         S.src[k] = (uint32_t)i;
-        S.cellp[k] = S.orig[i];
+        S.C.cellp[k] = S.orig[i];
     }
-    __syncthreads();
-    for (int k = t; k < n; k += NT) {
+    tm.sync();
+    if (tm.dead) return false;
+    for (int k = tm.a0 + t; k < tm.a1; k += NT) {
         const uint32_t i = S.src[k];
-        S.rank[sorted_slot(k, S.key[i], S.bin_start, S.cellp)] = i;
+        const uint32_t d = sorted_slot((uint32_t)k, S.key[i], S.bin_start, S.C.cellp);
+        permute_one(S.G, i, d);
+        S.rank[d] = S.N.ncnt[i];
     }
-    __syncthreads();
-    gather_block<NT>(S.G, S.rank, n);
-    for (int k = t; k < n; k += NT) S.src[k] = S.N.ncnt[S.rank[k]];
-    __syncthreads();
-    copy_back_block<NT>(S.G, n);
-    __syncthreads();
-    for (int i = t; i < n; i += NT) {
-        const double r[3] = {S.rx[i], S.ry[i], S.rz[i]};
-        cells_one(g, i, r, S.src[i], S.orig[i], S.F.kind[i], S.cellp, S.Rx, S.Ry, S.Rz, S.pos32, S.q0, S.o0,
-                  S.slot_of);
-    }
-    __syncthreads();
+    tm.sync();
+    if (tm.dead) return false;
+    for (int k = tm.a0 + t; k < tm.a1; k += NT) settle_one(g, S.G, k, S.rank[k], S.C);
+    tm.sync();
+    if (tm.dead) return false;
     {
-        const bool uniform = S.st->nonuniform == 0;
-        if (!g.small_box) {
+        const bool uniform = sh.differ == 0;
+        if (!g.small_box && WIDE && n < kAtomBuildMost) {
+            for (int i = tm.gw; i < n; i += tm.nw) nbuild_atom_cells(S.N, g, (uint32_t)i, tm.lane, uniform);
+        } else if (!g.small_box) {
             // a warp per cell, lanes over candidates (the per-stage list
             // build's body); its per-warp state is the launch's dynamic
             // shared memory
             extern __shared__ __align__(16) unsigned char solo_dyn[];
             NbWarpSmem<kSoloChunks>* nbs = reinterpret_cast<NbWarpSmem<kSoloChunks>*>(solo_dyn);
-            for (int b = w; b < nb; b += NT / 32) nbuild_cell_warp(S.N, g, b, 0, 1, lane, uniform, nbs[w]);
+            for (int b = tm.gw; b < nb; b += tm.nw)
+                nbuild_cell_warp(S.N, g, b, tm.lane, uniform, nbs[tm.w]);
         } else {
             // a few cells of many atoms: a warp per atom
-            for (int i = w; i < n; i += NT / 32) nbuild_atom(S.N, g, (uint32_t)i, lane, uniform);
+            for (int i = tm.gw; i < n; i += tm.nw) nbuild_atom(S.N, g, (uint32_t)i, tm.lane, uniform);
         }
-        __syncthreads();
+        tm.sync();
+        if (tm.dead) return false;
         // atoms clamped into the grid: their own lists from their unclamped cells
-        if (!g.small_box && (S.st->build_flags & FLAG_RANGE))
-            for (int i = w; i < n; i += NT / 32)
-                if (S.N.o0[i].w == 2.0f) nbuild_atom(S.N, g, (uint32_t)i, lane, uniform);
+        if (!g.small_box && (__ldcg(&S.st->build_flags) & FLAG_RANGE)) {
+            for (int i = tm.gw; i < n; i += tm.nw)
+                if (S.N.o0[i].w == 2.0f) nbuild_atom(S.N, g, (uint32_t)i, tm.lane, uniform);
+            tm.sync();
+        }
     }
+    const bool ok = !(__ldcg(&S.st->build_flags) & FLAG_OVERFLOW);
     __syncthreads();
-    for (int i = t; i < n; i += NT) S.trig[i] = trig_of(S.saved_rns[i], S.saved_rcut[i], g);
-    __syncthreads();
-    bool ok = !(S.st->build_flags & FLAG_OVERFLOW);
-    __syncthreads();
-    return ok;
+    return ok && !tm.dead;
 }
 
 // The input records (mdg_system_upload_atoms' scatter) from host memory.
@@ -250,7 +337,7 @@ __device__ __noinline__ void solo_read_atoms(const SoloArgs& S) {
     const GatherAll& G = S.G;
     for (int k = threadIdx.x; k < S.n; k += NT) {
         const mdg_atom& a = S.atoms_in[k];
-        const uint32_t s = S.slot_of[k];
+        const uint32_t s = S.C.slot_of[k];
         for (int c = 0; c < 3; ++c) {
             G.a2.out[RX + c][s] = a.r[c];
             G.a2.out[VX + c][s] = a.v[c];
@@ -285,17 +372,22 @@ __device__ __forceinline__ void solo_zero_one(const SoloArgs& S, int i) {
     }
 }
 
-// The force stages; with KICK the second half-kick rides in the force body
-// (the step loop), without it the forces alone (the set-up's initial forces).
+// The force stages of one block; with KICK the second half-kick rides in the
+// force body (the step loop), without it the forces alone (the set-up's
+// initial forces).
 template <bool EAM, bool KICK, int NT>
 __device__ __forceinline__ void solo_stages(const SoloArgs& S) {
     const int t = threadIdx.x, n = S.n;
     if (EAM) {
-        for (int i = t; i < n; i += NT) density_mixed_one<0>(S.F, S.ps, i);
+        for (int i = t; i < n; i += NT) density_one<RhoGroup<0, false, false>>(S.F, S.ps, i);
         __syncthreads();
-        for (int i = t; i < n; i += NT) eam_mixed_one<0, KICK>(S.F, S.ps, i);
-    } else {
-        for (int i = t; i < n; i += NT) lj_mixed_one<false, KICK>(S.F, S.ps, i);
+    }
+    for (int i = t; i < n; i += NT) {
+        float f[3];
+        bool live;
+        if (EAM) live = thread_forces<EamGroup<0, false, false>>(S.F, S.ps, i, f);
+        else live = thread_forces<LjGroup<false, false>>(S.F, S.ps, i, f);
+        if (live) store_force<KICK>(S.F, i, f[0], f[1], f[2]);
     }
 }
 
@@ -303,33 +395,33 @@ __device__ __forceinline__ void solo_stages(const SoloArgs& S) {
 // (upload, prepare, update(-1), offsets, prepare, stages). False when the
 // first list outgrew the capacities sized on the host.
 template <bool EAM, int NT>
-__device__ __noinline__ bool solo_setup(const SoloArgs& S, GridParams& g, double (*red)[NT / 32], uint32_t* scan_sh) {
+__device__ __noinline__ bool solo_setup(Team<NT, false>& tm, const SoloArgs& S, GridParams& g, SoloShared<NT>& sh) {
     const int t = threadIdx.x, n = S.n;
     // the fresh system's buffers (what system_alloc clears on a stream)
     for (int k = t; k < S.np; k += NT) {
         S.G.u2.out[0][k] = (uint32_t)k;  // caller index of slot k
-        S.slot_of[k] = (uint32_t)k;
+        S.C.slot_of[k] = (uint32_t)k;
         S.N.ncnt[k] = 0;
         S.bc[k] = 0;
-        S.trig[k] = make_float2(0.0f, 0.0f);
-        S.Rx[k] = 0.0;
-        S.Ry[k] = 0.0;
-        S.Rz[k] = 0.0;
+        S.C.trig[k] = make_float2(0.0f, 0.0f);
+        S.C.Rx[k] = 0.0;
+        S.C.Ry[k] = 0.0;
+        S.C.Rz[k] = 0.0;
         for (int q = 0; q < kMaxKinds; ++q) S.F.Fp64[(size_t)q * S.np + k] = 0.0;
     }
     if (t == 0) memset(S.st, 0, sizeof(DevStatus));
     __syncthreads();
     solo_read_atoms<NT>(S);
     __syncthreads();
-    for (int i = t; i < n; i += NT) drift64_one(S.I, i, 0, 0);
+    for (int i = t; i < n; i += NT) drift64_one(S.I, S.I, i, 0, 0);
     __syncthreads();
-    if (!solo_rebuild<NT>(S, g, red, scan_sh)) return false;
+    if (!solo_rebuild<NT, false>(tm, S, g, sh)) return false;
     for (int i = t; i < n; i += NT)
-        S.pos32[i] = make_int4(off_encode(S.rx[i] - S.Rx[i], g.inv_u[0]), off_encode(S.ry[i] - S.Ry[i], g.inv_u[1]),
-                               off_encode(S.rz[i] - S.Rz[i], g.inv_u[2]), S.F.kind[i] & 3);
+        S.C.pos32[i] = make_int4(off_encode(S.rx[i] - S.C.Rx[i], g.inv_u[0]), off_encode(S.ry[i] - S.C.Ry[i], g.inv_u[1]),
+                                 off_encode(S.rz[i] - S.C.Rz[i], g.inv_u[2]), S.F.kind[i] & 3);
     for (int i = t; i < n; i += NT) solo_zero_one(S, i);
     __syncthreads();
-    for (int i = t; i < n; i += NT) drift64_one(S.I, i, 0, 0);
+    for (int i = t; i < n; i += NT) drift64_one(S.I, S.I, i, 0, 0);
     __syncthreads();
     solo_stages<EAM, false, NT>(S);
     __syncthreads();
@@ -342,7 +434,7 @@ template <int NT>
 __device__ __noinline__ void solo_write_atoms(const SoloArgs& S) {
     const GatherAll& G = S.G;
     for (int k = threadIdx.x; k < S.n; k += NT) {
-        const uint32_t s = S.slot_of[k];
+        const uint32_t s = S.C.slot_of[k];
         mdg_atom a;
         const bool live = G.h.in[1][s] != 0;  // tag
         for (int c = 0; c < 3; ++c) {
@@ -369,28 +461,29 @@ __device__ __noinline__ void solo_write_atoms(const SoloArgs& S) {
 // One request by the whole block: set-up, the loop, the result records and
 // the completion record (last, after a system-scope fence).
 template <bool EAM, int NT>
-__device__ void solo_run(SoloArgs& S, GridParams& g, double (*red)[NT / 32], uint32_t* scan_sh) {
+__device__ void solo_run(SoloArgs& S, GridParams& g, SoloShared<NT>& sh) {
     const int t = threadIdx.x, n = S.n;
+    Team<NT, false> tm(nullptr, nullptr, n, n);
     long long left = S.steps;
     uint32_t rebuilds = 0;
     bool ok = true;
     unsigned long long t_start = 0;
     if (t == 0) t_start = global_ns();
-    if (S.setup) ok = solo_setup<EAM, NT>(S, g, red, scan_sh);
+    if (S.setup) ok = solo_setup<EAM, NT>(tm, S, g, sh);
     if (t == 0) {
         S.st->need_rebuild = 0;
         S.st->build_flags = 0;
     }
     while (ok && left > 0) {
         bool need = false;
-        for (int i = t; i < n; i += NT) need |= drift_mixed_one(S.I, i);
+        for (int i = t; i < n; i += NT) need |= drift_mixed_one(S.I, S.I, i);
         const int any = __syncthreads_or(need);
         solo_stages<EAM, true, NT>(S);
         __syncthreads();
         --left;
         if (any) {
             ++rebuilds;
-            ok = solo_rebuild<NT>(S, g, red, scan_sh);
+            ok = solo_rebuild<NT, false>(tm, S, g, sh);
         }
     }
     if (ok && left == 0) solo_write_atoms<NT>(S);
@@ -432,8 +525,7 @@ __global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* desc,
                                                            uint32_t* head, int idle_limit, int gen) {
     __shared__ __align__(16) SoloArgs S;
     __shared__ GridParams g;
-    __shared__ double red[7][NT / 32];
-    __shared__ uint32_t scan_sh[32];
+    __shared__ SoloShared<NT> sh;
     __shared__ int s_rec;
     // liveness for the host (which set 1 before the launch), so that it tops
     // up the kernel with a further launch when blocks have gone idle and
@@ -474,8 +566,8 @@ __global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* desc,
             for (int k = threadIdx.x; k < (int)(sizeof(SoloArgs) / sizeof(int4)); k += NT) dst[k] = __ldcv(src + k);
         }
         __syncthreads();
-        if (S.any_eam) solo_run<true, NT>(S, g, red, scan_sh);
-        else solo_run<false, NT>(S, g, red, scan_sh);
+        if (S.any_eam) solo_run<true, NT>(S, g, sh);
+        else solo_run<false, NT>(S, g, sh);
         if (threadIdx.x == 0) {
             q->live[gen][blockIdx.x] = 1u;  // 1: waiting for the next entry
             atomicSub(head + 1, 1u);
@@ -487,6 +579,253 @@ __global__ void __launch_bounds__(NT, 1) k_solo_persistent(const SoloArgs* desc,
     }
 }
 
+// ---- a grid's team: the step loop of mdg_run for small systems ------------------
+// A step of a 4,000-atom system is some 5 us of work on the whole GPU, but as
+// graph nodes it took 21 us (LJ) to 27 us (EAM): five nodes, each with its
+// launch and drain. Here a barrier over the blocks costs about 1.5 us. With
+// page-locked host arrays the call's transfers are the kernel's own reads and
+// writes over the host link, so a one-step call is one launch.
+struct TeamRun {
+    const double *hpos, *hvel;      // caller-order positions and velocities to start from (host), or null
+    double *opos, *ovel, *oforce;   // caller-order results (host), or null
+    const ThermoDev* th;            // thermostat, or null
+    ThermoArgs T;
+    // the same with the positions' (and LJ offsets') second buffers
+    IArgs I1;
+    FArgs F1;
+    ThermoArgs T1;
+    unsigned long long* left_dev;
+    unsigned long long* left_host;  // steps left and status at the end (pinned)
+    DevStatus* st_host;
+    unsigned long long* word;       // the barriers' word
+    int per;                        // atoms per block
+};
+
+constexpr int kTeamThreads = 768;
+
+// A step's passes by the team: the forces, the thermostat, the second
+// half-kick and, with `next`, the next step's first half-kick and drift;
+// whether that leaves a thread's atom due for a rebuild. The drift writes
+// positions (and the offsets the LJ pass reads) to the buffers that this
+// step's force pass does not read (flips), so blocks that are still in it
+// may lag by a barrier; the EAM force pass reads its neighbours only through
+// the density pass's copies and takes its cut decisions (k_force_step), so
+// the drift stays in place there. One barrier a step, two with EAM.
+template <bool EAM, bool MIXED>
+constexpr bool kFlips = !(EAM && MIXED);
+
+template <bool EAM, bool MIXED, int NT>
+__device__ __forceinline__ bool team_step(Team<NT, true>& tm, const SoloArgs& S, const TeamRun& R, LaneShared<NT>& sh,
+                                          int p, bool next, uint32_t call) {
+    const IArgs& I = p ? R.I1 : S.I;
+    const IArgs& to = !kFlips<EAM, MIXED> ? I : p ? S.I : R.I1;
+    const FArgs& F = p ? R.F1 : S.F;
+    const ThermoArgs& T = p ? R.T1 : R.T;
+    bool need = false;
+    if (!MIXED) {
+        // 16 lanes per atom, NT / 16 atoms at a time
+        const int sub = tm.t >> 4, lane = tm.t & 15;
+        if (EAM) {
+            for (int base = tm.a0; base < tm.a1; base += NT / 16)
+                density64_lanes<false, 16, false>(F, S.ps, base + sub < tm.a1, base + sub, lane);
+            tm.sync();
+            if (tm.dead) return false;
+        }
+        for (int base = tm.a0; base < tm.a1; base += NT / 16) {
+            const bool live = base + sub < tm.a1 && F.tag[base + sub] != 0;
+            const int i = live ? base + sub : tm.a0;
+            double f[3];
+            forces64_lanes<false, EAM ? POT_EAM : POT_LJCUT, false, 16, false>(F, S.ps, live, i, lane, f);
+            if (live && lane == 0) {
+                F.fx[i] = f[0];
+                F.fy[i] = f[1];
+                F.fz[i] = f[2];
+            }
+        }
+        __syncthreads();
+        for (int i = tm.a0 + tm.t; i < tm.a1; i += NT) {
+            if (R.th) langevin_one<false>(T, R.th, i, call);
+            kick64_one(I, i);
+            if (next) need |= drift64_one(I, to, i, 1, 1);
+        }
+        return need;
+    }
+    // eight lanes per atom, NT / 8 atoms at a time; the sums meet in shared
+    // memory and the first warps finish them, a lane per atom
+    const int sub = tm.t >> 3;
+    if (EAM) {
+        for (int base = tm.a0; base < tm.a1; base += NT / 8) {
+            const int i = base + sub;
+            const bool in = i < tm.a1, live = in && F.tag[i] != 0;
+            float rho[1];
+            RhoGroup<0, true, false> grp(F, S.ps, in ? i : tm.a0);
+            lane_sums<1>(F, live, in ? i : tm.a0, live ? F.ncnt[i] >> 2 : 0, grp, sh.part[tm.w], rho);
+            if ((tm.t & 7) == 0) sh.sum[0][sub] = rho[0];
+            __syncthreads();
+            const int me = base + tm.t;
+            if (tm.t < NT / 8 && me < tm.a1) store_density<false>(F, S.ps, me, F.pos32[me], 0, sh.sum[0][tm.t]);
+            __syncthreads();
+        }
+        tm.sync();
+        if (tm.dead) return false;
+    }
+    for (int base = tm.a0; base < tm.a1; base += NT / 8) {
+        const int i = base + sub;
+        const bool in = i < tm.a1;
+        float f[3];
+        if (EAM) lane_forces<EamGroup<0, true, false>>(F, S.ps, in, in ? i : tm.a0, sh.part[tm.w], f);
+        else lane_forces<LjGroup<false, false>>(F, S.ps, in, in ? i : tm.a0, sh.part[tm.w], f);
+        if ((tm.t & 7) == 0)
+            for (int k = 0; k < 3; ++k) sh.sum[k][sub] = f[k];
+        __syncthreads();
+        const int me = base + tm.t;
+        if (tm.t < NT / 8 && me < tm.a1) {
+            const bool live = F.tag[me] != 0;
+            const float fx = sh.sum[0][tm.t], fy = sh.sum[1][tm.t], fz = sh.sum[2][tm.t];
+            if (R.th) {
+                if (live) store_force<false>(F, me, fx, fy, fz);
+                langevin_one<true>(T, R.th, me, call);
+                kick_mixed_one(I, me);
+                if (next) need |= drift_mixed_one(I, to, me);
+            } else if (live && next) {
+                need |= kick_drift_mixed(I, to, F.gx, F.gy, F.gz, me, fx, fy, fz);
+            } else if (live) {
+                store_force<true>(F, me, fx, fy, fz);
+            } else if (next) {
+                need |= drift_mixed_one(I, to, me);  // tag 0: the offsets and the test alone
+            }
+        }
+        __syncthreads();
+    }
+    return need;
+}
+
+// The offsets of the block's atoms (launch_offsets).
+template <int NT>
+__device__ __forceinline__ void team_offsets(const Team<NT, true>& tm, const SoloArgs& S) {
+    for (int i = tm.a0 + tm.t; i < tm.a1; i += NT)
+        S.C.pos32[i] = make_int4(off_encode(S.rx[i] - S.C.Rx[i], S.I.inv_u[0]), off_encode(S.ry[i] - S.C.Ry[i], S.I.inv_u[1]),
+                                 off_encode(S.rz[i] - S.C.Rz[i], S.I.inv_u[2]), S.F.kind[i] & 3);
+}
+
+template <bool EAM, bool MIXED>
+__global__ void __launch_bounds__(kTeamThreads, 1)
+    k_team_run(const __grid_constant__ SoloArgs S, const __grid_constant__ TeamRun R) {
+    constexpr int NT = kTeamThreads;
+    __shared__ GridParams g;
+    __shared__ SoloShared<NT> sh;
+    __shared__ LaneShared<NT> lanes;
+    Team<NT, true> tm(R.word, &sh.said, S.n, R.per);
+    const int t = tm.t;
+    if (tm.gt == 0) {
+        S.st->build_flags = 0;  // (written by others only after a barrier)
+        S.st->pad[0] = 0;
+    }
+    if (R.hpos) {
+        for (int i = tm.a0 + t; i < tm.a1; i += NT) {
+            const size_t o = 3 * (size_t)S.orig[i];
+            S.I.rx[i] = R.hpos[o];
+            S.I.ry[i] = R.hpos[o + 1];
+            S.I.rz[i] = R.hpos[o + 2];
+            S.I.vx[i] = R.hvel[o];
+            S.I.vy[i] = R.hvel[o + 1];
+            S.I.vz[i] = R.hvel[o + 2];
+        }
+        if (!MIXED) team_offsets<NT>(tm, S);  // as a set of the positions does (mixed: below)
+    }
+    long long left = S.steps;
+    uint32_t rebuilds = 0, call = S.st->therm_calls;
+    bool ok = true;
+    if (MIXED) {
+        // the graph's prefix: rcut and boundary flags, a rebuild when an
+        // upload moved atoms past the half skin, the offsets
+        bool need = false;
+        for (int i = tm.a0 + t; i < tm.a1; i += NT) need |= drift64_one(S.I, S.I, i, 0, 1);
+        if (tm.any(need)) {
+            ++rebuilds;
+            ok = solo_rebuild<NT, true>(tm, S, g, sh);
+        }
+        team_offsets<NT>(tm, S);
+    }
+    // a step's first half-kick and drift as a pass of its own, in place;
+    // whether a rebuild is due after it
+    auto drift = [&] {
+        bool need = false;
+        for (int i = tm.a0 + t; i < tm.a1; i += NT)
+            need |= MIXED ? drift_mixed_one(S.I, S.I, i) : drift64_one(S.I, S.I, i, 1, 1);
+        return tm.any(need);
+    };
+    int p = 0;  // the buffers that hold the positions
+    bool due = ok && left > 0 && drift();
+    while (ok && left > 0 && !tm.dead) {
+        const bool next = left > 1 && !due;
+        const bool need = team_step<EAM, MIXED, NT>(tm, S, R, lanes, p, next, call);
+        bool due_next = false;
+        if (left > 1 || due) due_next = tm.any(need);
+        if (tm.dead) break;
+        --left;
+        ++call;
+        if (next) {
+            if (kFlips<EAM, MIXED>) p ^= 1;
+            due = due_next;
+            continue;
+        }
+        // the last step, or a rebuild: positions back in their own buffers
+        if (p) {
+            for (int i = tm.a0 + t; i < tm.a1; i += NT) {
+                S.I.rx[i] = R.I1.rx[i];
+                S.I.ry[i] = R.I1.ry[i];
+                S.I.rz[i] = R.I1.rz[i];
+                if (MIXED) S.I.pos32[i] = R.I1.pos32[i];
+            }
+            p = 0;
+        }
+        if (due) {
+            ++rebuilds;
+            ok = solo_rebuild<NT, true>(tm, S, g, sh);
+        }
+        due = ok && left > 0 && drift();
+    }
+    if (left == 0 && R.opos) {
+        for (int i = tm.a0 + t; i < tm.a1; i += NT) {
+            const size_t o = 3 * (size_t)S.orig[i];
+            R.opos[o] = S.rx[i];
+            R.opos[o + 1] = S.ry[i];
+            R.opos[o + 2] = S.rz[i];
+            R.ovel[o] = S.I.vx[i];
+            R.ovel[o + 1] = S.I.vy[i];
+            R.ovel[o + 2] = S.I.vz[i];
+            if (R.oforce) {
+                const bool live = !MIXED || S.F.tag[i] == 0;
+                R.oforce[o] = live ? S.F.fx[i] : (double)S.F.gx[i];
+                R.oforce[o + 1] = live ? S.F.fy[i] : (double)S.F.gy[i];
+                R.oforce[o + 2] = live ? S.F.fz[i] : (double)S.F.gz[i];
+            }
+        }
+    }
+    // the block that ends last reports, and leaves the barriers' word at zero
+    if (tm.gt == 0) {
+        S.st->pad[0] = rebuilds;
+        if (R.th) S.st->therm_calls = call;
+        *R.left_dev = (unsigned long long)left;
+    }
+    __syncthreads();
+    if (t == 0) {
+        if (tm.dead) atomicOr(&S.st->pad[1], 1u);
+        __threadfence();
+        if (atomicAdd(&S.st->team_done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            S.st->team_done = 0;
+            *R.word = 0;
+            const volatile uint32_t* from = reinterpret_cast<const volatile uint32_t*>(S.st);
+            uint32_t* to = reinterpret_cast<uint32_t*>(R.st_host);
+            for (int k = 0; k < (int)(sizeof(DevStatus) / 4); ++k) to[k] = from[k];
+            S.st->pad[1] = 0;
+            *R.left_host = *(volatile unsigned long long*)R.left_dev;
+        }
+    }
+}
+
 int solo_eligible(const mdg_solver* s, const mdg_system* sys) {
     if (s->precision != MDG_PREC_MIXED || s->multi || s->nstages < 1 || s->thermo) return 0;
     // the fused loop carries the LJsCut and EAM bodies only
@@ -495,23 +834,27 @@ int solo_eligible(const mdg_solver* s, const mdg_system* sys) {
     return 1;
 }
 
-void solo_fill(void* args, mdg_system* sys, const PotSet* dps, int any_eam, double pot_rcut, int periodic,
-               double dt, long steps, const void* atoms_in_dev, void* out_dev, void* atoms_out_dev, uint32_t seq) {
-    SoloArgs& S = *reinterpret_cast<SoloArgs*>(args);
+// Dynamic shared memory of a launch: the list build's state, one per warp.
+static size_t solo_dyn_bytes(int threads) { return (size_t)(threads / 32) * sizeof(NbWarpSmem<kSoloChunks>); }
+
+// Largest systems (exclusive) whose runs go to a grid's team.
+constexpr size_t kTeamMost64 = 12500, kTeamMostLj = 24000, kTeamMostEam = 45000;
+
+// What both teams need of a system.
+static void fill_system(SoloArgs& S, mdg_system* sys, const PotSet* dps, int any_eam, double pot_rcut, int periodic,
+                        double dt, long steps) {
     memset(&S, 0, sizeof(S));
     S.I = integrator_args(sys, dt);
     S.I.pot_rcut = pot_rcut;
     S.I.periodic_boundary = periodic;
-    S.setup = 1;
-    S.seq = seq;
     S.np = (int)sys->np;
     S.any_eam = any_eam;
-    S.atoms_in = reinterpret_cast<const mdg_atom*>(atoms_in_dev);
     S.F = force_args(sys);
     S.F.kick_hdt = 0.5f * (float)dt;  // the step loop's second half-kick, in the force body
     S.N = nb_args(sys);
     S.G = gather_sets(sys);
     S.D = domain_of(sys);
+    S.C = cell_out(sys);
     S.ps = dps;
     S.n = (int)sys->n;
     const int c = sys->cur;
@@ -525,24 +868,98 @@ void solo_fill(void* args, mdg_system* sys, const PotSet* dps, int any_eam, doub
     S.bin_count = sys->bin_count;
     S.bin_start = sys->bin_start;
     S.orig = sys->u32[ORIG][c];
-    S.cellp = sys->cellp;
-    S.Rx = sys->Rc[0];
-    S.Ry = sys->Rc[1];
-    S.Rz = sys->Rc[2];
-    S.pos32 = sys->pos32;
-    S.q0 = sys->q0;
-    S.o0 = sys->o0;
-    S.slot_of = sys->slot_of;
-    S.saved_rns = sys->saved_rns;
-    S.saved_rcut = sys->saved_rcut;
-    S.trig = sys->trig32;
     S.dgrid = sys->dgrid;
     S.bin_cap = (long long)sys->bin_cap;
     S.st = sys->dstat;
     S.steps = steps;
     S.bc = sys->bc;
+}
+
+void solo_fill(void* args, mdg_system* sys, const PotSet* dps, int any_eam, double pot_rcut, int periodic,
+               double dt, long steps, const void* atoms_in_dev, void* out_dev, void* atoms_out_dev, uint32_t seq) {
+    SoloArgs& S = *reinterpret_cast<SoloArgs*>(args);
+    fill_system(S, sys, dps, any_eam, pot_rcut, periodic, dt, steps);
+    S.setup = 1;
+    S.seq = seq;
+    S.atoms_in = reinterpret_cast<const mdg_atom*>(atoms_in_dev);
     S.out = reinterpret_cast<SoloOut*>(out_dev);
     S.atoms_out = reinterpret_cast<mdg_atom*>(atoms_out_dev);
+}
+
+// Whether a run of this solver on this system goes to a grid's team: LJsCut
+// or EAM, Single, full lists, and few enough atoms that the graph's launches
+// are a good part of a step.
+bool team_eligible(const mdg_solver* s, const mdg_system* sys) {
+    if (s->multi || s->nstages < 1 || !s->pot[0][0] || sys->half || sys->pool || sys->ctx->timing) return false;
+    const int type = s->pot[0][0]->type;
+    if (type != POT_LJCUT && type != POT_EAM) return false;
+    if (!sys->cap_ready || sys->n < 1 || !sys->ctx->num_sms) return false;
+    return sys->n < (s->precision == MDG_PREC_FP64 ? kTeamMost64 : type == POT_EAM ? kTeamMostEam : kTeamMostLj);
+}
+
+// Enqueues `steps` steps by a grid's team (any host arrays page-locked); the
+// steps left and the status words arrive in hcounter and hstat.
+int ensure_cutbits(mdg_system* sys);
+
+int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam, int mixed, double pot_rcut,
+                int periodic, double dt, long steps, const double* hpos, const double* hvel, double* opos,
+                double* ovel, double* oforce) {
+    mdg_ctx* ctx = sys->ctx;
+    SoloArgs S;
+    fill_system(S, sys, dps, eam, pot_rcut, periodic, dt, steps);
+    TeamRun R;
+    memset(&R, 0, sizeof(R));
+    R.hpos = hpos;
+    R.hvel = hvel;
+    R.opos = opos;
+    R.ovel = ovel;
+    R.oforce = oforce;
+    R.th = th;
+    R.T = thermo_args(sys);
+    if (eam && mixed) {
+        int rc = ensure_cutbits(sys);
+        if (rc) return rc;
+        S.F.cutbits = sys->cutbits;
+    }
+    // the second buffers: the rebuild's spare position arrays and, for LJ, the
+    // offsets' second half (the EAM records)
+    R.I1 = S.I;
+    R.F1 = S.F;
+    R.T1 = R.T;
+    R.I1.rx = sys->f64[RX][sys->cur ^ 1];
+    R.I1.ry = sys->f64[RY][sys->cur ^ 1];
+    R.I1.rz = sys->f64[RZ][sys->cur ^ 1];
+    R.F1.rx = R.T1.rx = R.I1.rx;
+    R.F1.ry = R.I1.ry;
+    R.F1.rz = R.I1.rz;
+    if (!eam) R.F1.pos32 = R.I1.pos32 = sys->pos32 + sys->np;
+    R.left_dev = sys->dcounter;
+    R.left_host = sys->hcounter;
+    R.st_host = sys->hstat;
+    // whole warps of eight-lane (mixed) or 32-lane (FP64) atoms, and at least
+    // four a block
+    const int n = (int)sys->n, least = mixed ? 8 : 4;
+    R.per = std::max(least, ((n + ctx->num_sms - 1) / ctx->num_sms + 3) & ~3);
+    const int blocks = (n + R.per - 1) / R.per;
+    const void* fn = eam ? (mixed ? (const void*)k_team_run<true, true> : (const void*)k_team_run<true, false>)
+                         : (mixed ? (const void*)k_team_run<false, true> : (const void*)k_team_run<false, false>);
+    if ((size_t)blocks > sys->part_cap) {
+        set_error("the list was not sized for the step loop");
+        return MDG_ERR_STATE;
+    }
+    S.part = reinterpret_cast<long long*>(sys->part);
+    if (!sys->team_word) {
+        int rc = sys_malloc(sys, (void**)&sys->team_word, sizeof(unsigned long long));
+        if (rc) return rc;
+        MDG_CUDA(cudaMemsetAsync(sys->team_word, 0, sizeof(unsigned long long), ctx->stream));
+    }
+    R.word = sys->team_word;
+    const size_t dyn = solo_dyn_bytes(kTeamThreads);
+    MDG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    void* args[2] = {&S, &R};
+    MDG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kTeamThreads), args, dyn, ctx->stream));
+    MDG_LAUNCHED(ctx);
+    return MDG_OK;
 }
 
 size_t solo_args_bytes() { return sizeof(SoloArgs); }
@@ -558,9 +975,6 @@ int solo_out_read(const void* out_host, uint32_t* done, unsigned long long* left
     if (service_s) *service_s = o->t_end > o->t_start ? (double)(o->t_end - o->t_start) * 1e-9 : 0.0;
     return MDG_OK;
 }
-
-// Dynamic shared memory of a launch: the list build's state, one per warp.
-static size_t solo_dyn_bytes(int threads) { return (size_t)(threads / 32) * sizeof(NbWarpSmem<kSoloChunks>); }
 
 // The launch's dynamic shared memory exceeds the default 48 KB at 1024
 // threads; the attribute is per device, so it is set once per device.
