@@ -2196,11 +2196,15 @@ struct TeamIo {
     double *opos = nullptr, *ovel = nullptr, *oforce = nullptr;
 };
 
-// `steps` steps by a grid's team (team_eligible), waited for; a rebuild that
-// outgrew its capacities ends the kernel early: grown here, and resumed. *io
-// (optional): *done tells whether the results went to its arrays.
-static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, double dt, long steps, const TeamIo* io,
-                    bool* done) {
+// Steps of one launch of the team kernel (3 to 15 ms).
+constexpr long kTeamSteps = 256;
+
+// `steps` steps by a grid's team (team_eligible), waited for; the graph takes
+// over once something else is in flight on the device. A rebuild that outgrew
+// its capacities ends a launch early: grown here, and resumed. *io (optional):
+// *done tells whether the results went to its arrays.
+static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, const DeviceUse& use, double dt, long steps,
+                    const TeamIo* io, bool* done) {
     int rc = graph_prologue(s, sys);
     if (rc) return rc;
     if (!sys->dcounter) {
@@ -2210,11 +2214,15 @@ static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, double dt,
     if (!sys->hcounter) MDG_CUDA(cudaMallocHost((void**)&sys->hcounter, sizeof(unsigned long long)));
     if (done) *done = false;
     long left = steps;
-    for (int round = 0; left > 0 && round < 64; ++round) {
-        const bool whole = io && round == 0;
+    int grown = 0;
+    for (bool first = true; left > 0 && grown < 64; first = false) {
+        if (!first && !use.alone()) return run_graph(s, sys, ps, dt, left);
+        const long part = std::min(left, kTeamSteps);
+        const bool last = part == left;
         rc = team_launch(sys, ext(s)->d.dev, thermo_of(s), ps.any_eam, s->precision == MDG_PREC_MIXED,
-                         pot_rcut_of(s), s->periodic, dt, left, whole ? io->pos : nullptr, whole ? io->vel : nullptr,
-                         whole ? io->opos : nullptr, whole ? io->ovel : nullptr, whole ? io->oforce : nullptr);
+                         pot_rcut_of(s), s->periodic, dt, part, io && first ? io->pos : nullptr,
+                         io && first ? io->vel : nullptr, io && last ? io->opos : nullptr,
+                         io && last ? io->ovel : nullptr, io && last ? io->oforce : nullptr);
         if (rc) return rc;
         MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
         sys->fp_ok = 0;
@@ -2224,12 +2232,13 @@ static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, double dt,
             return MDG_ERR_TIMEOUT;
         }
         sys->rebuilds += sys->hstat->pad[0];
-        left = (long)*sys->hcounter;
+        left -= part - (long)*sys->hcounter;
         if (sys->hstat->build_flags & FLAG_OVERFLOW) {
+            ++grown;
             sys->rebuilds--;
             rc = nlist_build(sys, -1.0, sys->half);
             if (rc && rc != MDG_ERR_RANGE) return rc;
-        } else if (whole && done) {
+        } else if (io && io->opos && last && done) {
             *done = left == 0;
         }
     }
@@ -2561,7 +2570,8 @@ int mdg_run(mdg_solver* s, mdg_system* sys, double dt, long steps) {
     if (rc) return rc;
     if (steps <= 0) return MDG_OK;
     mark_stepped(s, sys, ps);
-    if (team_eligible(s, sys)) return run_team(s, sys, ps, dt, steps, nullptr, nullptr);
+    const DeviceUse use(sys->ctx->device);
+    if (use.alone() && team_eligible(s, sys)) return run_team(s, sys, ps, use, dt, steps, nullptr, nullptr);
     if (!sys->ctx->timing && sys->n > 0 && !sys->half) {
         rc = graph_prologue(s, sys);
         if (rc) return rc;
@@ -2647,8 +2657,9 @@ done:
 int mdg_run_host(mdg_solver* s, mdg_system* sys, double dt, long steps, double* pos, double* vel, double* force) {
     if (!s || !sys || !pos || !vel) return MDG_ERR_INVALID;
     PotSet ps;
+    const DeviceUse use(sys->ctx->device);
     if (steps > 0 && sys->n > 0 && !sys->half && !sys->ctx->timing && check_ready(s, sys, &ps) == MDG_OK &&
-        team_eligible(s, sys)) {
+        use.alone() && team_eligible(s, sys)) {
         MDG_CUDA(cudaSetDevice(sys->ctx->device));
         mark_stepped(s, sys, ps);
         // page-locked arrays of a small system are read and written by the
@@ -2664,7 +2675,7 @@ int mdg_run_host(mdg_solver* s, mdg_system* sys, double dt, long steps, double* 
             rc = vec_io(sys, pos, RX, 1, 0);
             if (!rc) rc = vec_io(sys, vel, VX, 1, 0);
         }
-        if (!rc) rc = run_team(s, sys, ps, dt, steps, direct ? &io : nullptr, &done);
+        if (!rc) rc = run_team(s, sys, ps, use, dt, steps, direct ? &io : nullptr, &done);
         if (rc || done) return rc;
         rc = vec_io(sys, pos, RX, 0, 0);
         if (!rc) rc = vec_io(sys, vel, VX, 0, 0);

@@ -251,24 +251,18 @@ __global__ void __launch_bounds__(kBlock64) k_virials64(FArgs A, const PotSet* _
     }
 }
 
-// Lanes per atom of the FP64 passes: 32 below 12,500 atoms, 4 below 100,000,
-// else one. Fewer atoms than about 100,000 threads' worth leave SMs with too
-// few warps to keep their FP64 pipe busy; more lanes than that cost the sums
-// over lanes and lanes without a pair. Measured per FP64 step, 1 / 4 / 32
-// lanes: LJ argon 500 atoms 137 / 72 / 46 us, 4,000 atoms 140 / 62 / 51 us;
-// EAM Cu 32,000 atoms 253 / 213 / 295 us, 108,000 atoms 560 / 565 / 924 us,
-// 1,000,188 atoms 3.87 / 4.54 / 8.20 ms. (2, 8 and 16 lanes are never more
-// than 8% faster than the best of these three.)
-// Calls f(std::integral_constant<int, G>) with the G of n atoms.
+// Calls f(std::integral_constant<int, G>) with the lanes per atom of n atoms
+// (kFewAtoms64).
 template <typename F>
-static void with_lanes64(size_t n, F&& f) {
-    if (n < 12500) f(std::integral_constant<int, 32>());
+static void with_lanes64(size_t n, bool eam, F&& f) {
+    if (n < kFewAtoms64) f(std::integral_constant<int, 32>());
+    else if (n < some_atoms64(eam)) f(std::integral_constant<int, 16>());
     else if (n < 100000) f(std::integral_constant<int, 4>());
     else f(std::integral_constant<int, 1>());
 }
 
 static void launch_density64(const FArgs& A, const PotSet* dps, const PotSet& ps, cudaStream_t st) {
-    with_lanes64(A.n, [&](auto g) {
+    with_lanes64(A.n, ps.any_eam != 0, [&](auto g) {
         constexpr int G = decltype(g)::value;
         const int nb = (int)(((size_t)A.n * G + kBlock64 - 1) / kBlock64);
         if (ps.multi) k_density64<true, G><<<nb, kBlock64, 0, st>>>(A, dps);
@@ -278,7 +272,7 @@ static void launch_density64(const FArgs& A, const PotSet* dps, const PotSet& ps
 
 static void launch_forces64(const FArgs& A, const PotSet* dps, const PotSet& ps, bool half, cudaStream_t st) {
     const int only = ps.multi ? 0 : ps.any_eam ? POT_EAM : ps.any_lj ? POT_LJCUT : 0;
-    with_lanes64(A.n, [&](auto g) {
+    with_lanes64(A.n, ps.any_eam != 0, [&](auto g) {
         constexpr int G = decltype(g)::value;
         const int nb = (int)(((size_t)A.n * G + kBlock64 - 1) / kBlock64);
         if (half) {
@@ -298,7 +292,7 @@ static void launch_forces64(const FArgs& A, const PotSet* dps, const PotSet& ps,
 
 static void launch_virials64(const FArgs& A, const PotSet* dps, const PotSet& ps, bool half, cudaStream_t st) {
     const int only = ps.multi ? 0 : ps.any_eam ? POT_EAM : ps.any_lj ? POT_LJCUT : 0;
-    with_lanes64(A.n, [&](auto g) {
+    with_lanes64(A.n, ps.any_eam != 0, [&](auto g) {
         constexpr int G = decltype(g)::value;
         const int nb = (int)(((size_t)A.n * G + kBlock64 - 1) / kBlock64);
         if (half) {
@@ -698,7 +692,6 @@ int launch_density_rec(mdg_system* sys, const PotSet* dps, const PotSet& ps) {
     A.cutbits = sys->cutbits;
     const int nb = nblk(sys->n);
     cudaStream_t st = sys->ctx->stream;
-    const bool multi = ps.multi != 0;
     const int mb = density_blocks(sys, ps);
     with_kinds(ps, [&](auto k) {
         constexpr int K = decltype(k)::value;

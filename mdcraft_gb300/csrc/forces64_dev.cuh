@@ -16,7 +16,7 @@
 //  - a pair across a periodic face takes its image by one addition per axis,
 //    in the one walk over the list;
 //  - G lanes share an atom's list where one thread per atom would leave SMs
-//    without work (with_lanes64).
+//    without work (kFewAtoms64).
 // EAM Cu 389,344 atoms: force pass 0.90 ms (27 FP64 operations per in-range
 // pair, FP64 pipe 86% active), density 0.65 ms (18, 83%). EAM Cu 1,000,188
 // atoms: 13.1 -> 3.87 ms per step; LJ argon 4,000 atoms 0.45 -> 0.05 ms.
@@ -27,6 +27,19 @@
 #include "forces_dev.cuh"
 
 namespace mdg {
+
+// Lanes per atom of the FP64 passes, launched (with_lanes64) or by a grid's
+// team, whose sums over lanes then have the same order: 32 below 2,000 atoms,
+// 16 below 12,500 with EAM tables and 24,000 without, 4 below 100,000, else
+// one. Fewer atoms than about 100,000 threads' worth leave SMs with too few
+// warps to keep their FP64 pipe busy; more lanes than that cost the sums over
+// lanes and lanes without a pair. Measured per launched FP64 step, 4 / 16 / 32
+// lanes: LJ argon 500 atoms - / 30.3 / 26.4 us, 8,788 74 / 62 / 72, 19,652
+// 118 / 101 / 126; EAM Cu 500 - / 42.1 / 32.9, 8,788 - / 98.7 / 103.9, 13,500
+// 113 / 131 / 141; 1 / 4 lanes: EAM Cu 108,000 560 / 565, 1,000,188 3,870 /
+// 4,540.
+constexpr size_t kFewAtoms64 = 2000;
+inline size_t some_atoms64(bool eam) { return eam ? 12500 : 24000; }
 
 // The FP32 number nearest below a positive double (2^-126 <= x), by integer
 // operations; beyond FP32's range it saturates. NaN gives a finite number.
@@ -174,6 +187,9 @@ __device__ __forceinline__ float screen_float(double x) {
 struct Pair64 {
     double dx, dy, dz, r2;
 };
+// (Where a sum of products could be contracted in more than one way, these
+// passes spell the fma out: a grid's team gives the launched passes' bits.)
+__device__ __forceinline__ double norm64(double x, double y, double z) { return fma(x, x, fma(y, y, z * z)); }
 
 // The Periodic boundary's ghost of a listed pair (boundary/periodic.cxx:
 // 36-102), for an atom near a periodic face: a pair whose raw distance is at
@@ -187,7 +203,7 @@ __device__ __forceinline__ bool ghost64(const FArgs& A, double rni, uint32_t j, 
     q.dx = shortest1(p.dx, A.L[0], A.periodic[0]);
     q.dy = shortest1(p.dy, A.L[1], A.periodic[1]);
     q.dz = shortest1(p.dz, A.L[2], A.periodic[2]);
-    q.r2 = q.dx * q.dx + q.dy * q.dy + q.dz * q.dz;
+    q.r2 = norm64(q.dx, q.dy, q.dz);
     return !(q.r2 > r2rns);
 }
 
@@ -296,7 +312,7 @@ __device__ __forceinline__ void walk64(const FArgs& A, const PotSet* __restrict_
                     }
                 }
             }
-            p.r2 = p.dx * p.dx + p.dy * p.dy + p.dz * p.dz;
+            p.r2 = norm64(p.dx, p.dy, p.dz);
             if (!SCREEN) seen(P, kj, k, false);
             bool in = in_cut64(p.r2, P.R2cut), both = false;
             if (exact && __double_as_longlong(p.r2) >= rni2 && ghost64(A, rni, j, p, s)) {
@@ -337,13 +353,12 @@ __device__ __forceinline__ void eam_embed64(const PotParams& P, double nr, doubl
         if (N1 == P.Nrh1 - 1) atomicOr(&st->flags, FLAG_TABLE);
         double VR = N1;
         double DV = RN - VR;
-        RN = nr - VR * P.drh;
+        RN = fma(-VR, P.drh, nr);
         VR = (P.Femb[N1 + 1] - P.Femb[N1]) * P.drh1;
-        double aa = (P.dFemb[N1 + 1] - VR) - (VR - P.dFemb[N1]);
-        double bb = aa - (VR - P.dFemb[N1]);
-        aa = aa * DV;
-        *EF = P.Femb[N1] + RN * (P.dFemb[N1] + DV * (aa - bb));
-        *dF = P.dFemb[N1] + 2.0 * DV * (1.5 * aa - bb);
+        const double aa = (P.dFemb[N1 + 1] - VR) - (VR - P.dFemb[N1]);
+        const double bb = aa - (VR - P.dFemb[N1]);
+        *EF = fma(RN, fma(DV, fma(aa, DV, -bb), P.dFemb[N1]), P.Femb[N1]);
+        *dF = fma(2.0 * DV, fma(1.5 * aa, DV, -bb), P.dFemb[N1]);
     } else {
         atomicOr(&st->flags, FLAG_TABLE);
         if (N1 >= P.Nrh1) {

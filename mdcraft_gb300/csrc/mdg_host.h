@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -290,6 +291,28 @@ struct SoloQueue {              // host-mapped
     // yet resident count), 2 running a request
     volatile uint32_t live[kSoloGens][kSoloMaxBlocks];
 };
+// A run or a served request that is in flight on a device, for as long as the
+// object lives. A team of blocks (solo.cu) holds the GPU for its steps, so it
+// takes a run only where nothing else is in flight, a thousandth of a second
+// or a few at a time; a mixed or FP64 step gives the same bits either way. Eight
+// threads with an LJ argon system of 4,000 atoms each, us per step and system:
+// teams in turn 12.5, graphs side by side 4.4.
+class DeviceUse {
+public:
+    explicit DeviceUse(int device) : n_(count(device)) { n_.fetch_add(1); }
+    ~DeviceUse() { n_.fetch_sub(1); }
+    DeviceUse(const DeviceUse&) = delete;
+    DeviceUse& operator=(const DeviceUse&) = delete;
+    bool alone() const { return n_.load() == 1; }
+
+private:
+    static std::atomic<int>& count(int device) {
+        static std::atomic<int> in_flight[64];
+        return in_flight[device & 63];
+    }
+    std::atomic<int>& n_;
+};
+
 // The step loop of a small system by a grid of blocks (solo.cu).
 bool team_eligible(const mdg_solver* s, const mdg_system* sys);
 int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam, int mixed, double pot_rcut,

@@ -39,6 +39,7 @@
 #include <cmath>
 #include <cstring>
 #include <deque>
+#include <optional>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -52,6 +53,7 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 struct Request {
+    std::optional<DeviceUse> use;  // from submission to completion
     uint64_t id = 0;
     mdg_solver* solver = nullptr;
     mdg_domain dom{};
@@ -208,6 +210,7 @@ void finish(mdg_server* sv, Request* r, int status) {
     // graph mode: from admission to completion (host clock); a repeat on the
     // checked path adds its own span
     if (r->t_graph_start > 0.0) r->info.service_s += r->info.t_done - r->t_graph_start;
+    r->use.reset();
     sv->finished.push_back(r->id);
     sv->nfinished++;
 }
@@ -763,6 +766,7 @@ int mdg_server_submit(mdg_server* srv, mdg_solver* solver, const mdg_domain* dom
     r->precision = solver->precision;
     r->footprint = fp;
     r->info.t_submit = srv->now();
+    r->use.emplace(srv->device);
     srv->reqs[r->id] = r;
     *id = r->id;
     if (n == 0 || steps == 0) {

@@ -97,7 +97,9 @@ constexpr int kTeamPolls = 1 << 23;
 // The grid's barrier is one 64-bit word: arrivals in its low half, votes in
 // two counters above it, for barriers of even and odd number (a block may
 // stand at the next barrier when a slow one reads the word, but never
-// further). A block's first thread adds and polls. (A word per block that
+// further). A block's first thread adds and polls. No field may carry into
+// the next one: counts are compared without the field's top bit, and the
+// first block takes that bit out once it is set. (A word per block that
 // every block reads took 4 to 6 us against 2 here: 143 x 143 polls.)
 template <int NT, bool WIDE>
 struct Team {
@@ -134,13 +136,17 @@ struct Team {
             const uint32_t target = epoch * (uint32_t)size;
             unsigned long long v;
             int polls = 0;
+            bool wait;
             do {
                 v = *(volatile unsigned long long*)word;
-            } while ((int)((uint32_t)v - target) < 0 && ++polls < kTeamPolls);
+                wait = (((uint32_t)v - target) & 0x7fffffffu) >= 0x40000000u;
+            } while (wait && ++polls < kTeamPolls);
             __threadfence();
-            const uint32_t sum = (uint32_t)(v >> at) & 0xffffu;
-            *said = (sum != cast[odd] ? 1 : 0) | ((int)((uint32_t)v - target) < 0 ? 2 : 0);
+            const uint32_t sum = (uint32_t)(v >> at) & 0x7fffu;
+            *said = (sum != cast[odd] ? 1 : 0) | (wait ? 2 : 0);
             cast[odd] = sum;
+            const unsigned long long top = v & 0x8000800080000000ull;
+            if (rank == 0 && top) atomicAdd(word, 0ull - top);
         }
         __syncthreads();
         const int s = *said;
@@ -614,7 +620,7 @@ constexpr int kTeamThreads = 768;
 template <bool EAM, bool MIXED>
 constexpr bool kFlips = !(EAM && MIXED);
 
-template <bool EAM, bool MIXED, int NT>
+template <bool EAM, bool MIXED, int NT, int G>
 __device__ __forceinline__ bool team_step(Team<NT, true>& tm, const SoloArgs& S, const TeamRun& R, LaneShared<NT>& sh,
                                           int p, bool next, uint32_t call) {
     const IArgs& I = p ? R.I1 : S.I;
@@ -623,19 +629,19 @@ __device__ __forceinline__ bool team_step(Team<NT, true>& tm, const SoloArgs& S,
     const ThermoArgs& T = p ? R.T1 : R.T;
     bool need = false;
     if (!MIXED) {
-        // 16 lanes per atom, NT / 16 atoms at a time
-        const int sub = tm.t >> 4, lane = tm.t & 15;
+        // G lanes per atom, NT / G atoms at a time
+        const int sub = tm.t / G, lane = tm.t % G;
         if (EAM) {
-            for (int base = tm.a0; base < tm.a1; base += NT / 16)
-                density64_lanes<false, 16, false>(F, S.ps, base + sub < tm.a1, base + sub, lane);
+            for (int base = tm.a0; base < tm.a1; base += NT / G)
+                density64_lanes<false, G, false>(F, S.ps, base + sub < tm.a1, base + sub, lane);
             tm.sync();
             if (tm.dead) return false;
         }
-        for (int base = tm.a0; base < tm.a1; base += NT / 16) {
+        for (int base = tm.a0; base < tm.a1; base += NT / G) {
             const bool live = base + sub < tm.a1 && F.tag[base + sub] != 0;
             const int i = live ? base + sub : tm.a0;
             double f[3];
-            forces64_lanes<false, EAM ? POT_EAM : POT_LJCUT, false, 16, false>(F, S.ps, live, i, lane, f);
+            forces64_lanes<false, EAM ? POT_EAM : POT_LJCUT, false, G, false>(F, S.ps, live, i, lane, f);
             if (live && lane == 0) {
                 F.fx[i] = f[0];
                 F.fy[i] = f[1];
@@ -708,7 +714,8 @@ __device__ __forceinline__ void team_offsets(const Team<NT, true>& tm, const Sol
                                  off_encode(S.rz[i] - S.C.Rz[i], S.I.inv_u[2]), S.F.kind[i] & 3);
 }
 
-template <bool EAM, bool MIXED>
+// G: lanes per atom of the FP64 passes.
+template <bool EAM, bool MIXED, int G>
 __global__ void __launch_bounds__(kTeamThreads, 1)
     k_team_run(const __grid_constant__ SoloArgs S, const __grid_constant__ TeamRun R) {
     constexpr int NT = kTeamThreads;
@@ -759,7 +766,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     bool due = ok && left > 0 && drift();
     while (ok && left > 0 && !tm.dead) {
         const bool next = left > 1 && !due;
-        const bool need = team_step<EAM, MIXED, NT>(tm, S, R, lanes, p, next, call);
+        const bool need = team_step<EAM, MIXED, NT, G>(tm, S, R, lanes, p, next, call);
         bool due_next = false;
         if (left > 1 || due) due_next = tm.any(need);
         if (tm.dead) break;
@@ -837,8 +844,16 @@ int solo_eligible(const mdg_solver* s, const mdg_system* sys) {
 // Dynamic shared memory of a launch: the list build's state, one per warp.
 static size_t solo_dyn_bytes(int threads) { return (size_t)(threads / 32) * sizeof(NbWarpSmem<kSoloChunks>); }
 
-// Largest systems (exclusive) whose runs go to a grid's team.
-constexpr size_t kTeamMost64 = 12500, kTeamMostLj = 24000, kTeamMostEam = 45000;
+// Systems (exclusive) whose runs go to a grid's team: below these sizes it
+// beats the graph. A block's 768 threads take 96 atoms at a time, so 152 SMs
+// take 29,184 atoms in two rounds and 43,776 in three. Per step, graph / team:
+// LJ argon mixed 4,000 atoms 20.3 / 12.7 us, 27,436 34.2 / 25.1, 32,000
+// 35.4 / 32.1, 42,592 38.2 / 36.4, 48,668 39.1 / 44.1; EAM Cu mixed 4,000
+// 24.2 / 17.4, 27,436 40.9 / 33.7, 32,000 41.8 / 42.6, 37,044 45.4 / 45.5; FP64
+// (to where 16 lanes per atom end) argon 500 26.4 / 19.2, 4,000 42.4 / 32.2,
+// 19,652 100.9 / 98.7; FP64 Cu 500 32.9 / 27.8, 4,000 62.0 / 51.2, 8,788
+// 98.7 / 96.8.
+constexpr size_t kTeamMostLj = 43776, kTeamMostEam = 30000;
 
 // What both teams need of a system.
 static void fill_system(SoloArgs& S, mdg_system* sys, const PotSet* dps, int any_eam, double pot_rcut, int periodic,
@@ -894,7 +909,8 @@ bool team_eligible(const mdg_solver* s, const mdg_system* sys) {
     const int type = s->pot[0][0]->type;
     if (type != POT_LJCUT && type != POT_EAM) return false;
     if (!sys->cap_ready || sys->n < 1 || !sys->ctx->num_sms) return false;
-    return sys->n < (s->precision == MDG_PREC_FP64 ? kTeamMost64 : type == POT_EAM ? kTeamMostEam : kTeamMostLj);
+    if (s->precision == MDG_PREC_FP64) return sys->n < some_atoms64(type == POT_EAM);
+    return sys->n < (type == POT_EAM ? kTeamMostEam : kTeamMostLj);
 }
 
 // Enqueues `steps` steps by a grid's team (any host arrays page-locked); the
@@ -941,8 +957,10 @@ int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam
     const int n = (int)sys->n, least = mixed ? 8 : 4;
     R.per = std::max(least, ((n + ctx->num_sms - 1) / ctx->num_sms + 3) & ~3);
     const int blocks = (n + R.per - 1) / R.per;
-    const void* fn = eam ? (mixed ? (const void*)k_team_run<true, true> : (const void*)k_team_run<true, false>)
-                         : (mixed ? (const void*)k_team_run<false, true> : (const void*)k_team_run<false, false>);
+    const bool few = sys->n < kFewAtoms64;
+    const void* fn = mixed ? (eam ? (const void*)k_team_run<true, true, 8> : (const void*)k_team_run<false, true, 8>)
+                     : eam ? (few ? (const void*)k_team_run<true, false, 32> : (const void*)k_team_run<true, false, 16>)
+                           : (few ? (const void*)k_team_run<false, false, 32> : (const void*)k_team_run<false, false, 16>);
     if ((size_t)blocks > sys->part_cap) {
         set_error("the list was not sized for the step loop");
         return MDG_ERR_STATE;
