@@ -613,6 +613,9 @@ struct SolverBlob {
     alignas(32) double z64[2 * kZeroRows];
 };
 
+static_assert((offsetof(SolverBlob, th) + offsetof(ThermoDev, tab) + offsetof(ThermoTables, cs)) % 16 == 0,
+              "the thermostat's table of the circle is read by 16-byte words");
+
 struct SolverDev {
     PotSet host;
     PotSet* dev = nullptr;  // start of the SolverBlob
@@ -1589,11 +1592,32 @@ int mdg_solver_set_thermostat(mdg_solver* s, mdg_thermostat* t) {
     return MDG_OK;
 }
 
+// The thermostat's tables (ThermoTables): nodes of the logarithm, and of the
+// circle by its first eighth, so that axis points are exact.
+static ThermoTables thermo_tables() {
+    ThermoTables T;
+    for (int j = 0; j < kThermoNodes; ++j) {
+        const double c = 1.0 + j / 128.0;
+        T.inv[j] = 1.0 / c;
+        // of the rounded reciprocal itself, the half taken off before rounding
+        T.log[j] = (double)(-std::log((long double)T.inv[j]) - (j >= 53 ? 0.693147180559945309417232121458176568L : 0.0L));
+        const int o = j % 32, q = j / 32;  // quarter turn and the angle in it
+        const long double step = 2.0L * 3.141592653589793238462643383279502884L / 128.0L;
+        const double a = (double)(o <= 16 ? std::cos(step * o) : std::sin(step * (32 - o)));
+        const double b = (double)(o <= 16 ? std::sin(step * o) : std::cos(step * (32 - o)));
+        T.cs[j][0] = q == 0 ? a : q == 1 ? -b : q == 2 ? -a : b;
+        T.cs[j][1] = q == 0 ? b : q == 1 ? a : q == 2 ? -b : -a;
+    }
+    return T;
+}
+
 static int thermo_sync(mdg_solver* s) {
     if (!s->thermo) return MDG_OK;
     mdg_solver_ext* e = ext(s);
+    static const ThermoTables tables = thermo_tables();
     ThermoDev h;
     memset(&h, 0, sizeof(h));
+    h.tab = tables;
     int rc = thermo_flatten(s->thermo, h, 0);
     if (rc) return rc;
     if (e->d.th_valid && memcmp(&h, &e->d.th_host, sizeof(h)) == 0) return MDG_OK;

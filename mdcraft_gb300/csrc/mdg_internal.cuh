@@ -176,10 +176,19 @@ struct LangevinTerm {
     double xmin, xmax;
     unsigned long long seed;
 };
+// Nodes of the tables by which the thermostat takes logarithms, sines and
+// cosines (thermo_dev.cuh), filled on the host (thermo_tables).
+constexpr int kThermoNodes = 128;
+struct ThermoTables {
+    double inv[kThermoNodes];      // 1 / (1 + j / 128)
+    double log[kThermoNodes];      // log(1 + j / 128), log(that / 2) from sqrt(2) up
+    alignas(16) double cs[kThermoNodes][2];  // cos, sin of 2 pi j / 128, read as one word
+};
 struct ThermoDev {
     int n;
     int pad;
     LangevinTerm t[kMaxThermo];
+    ThermoTables tab;
 };
 
 // Exact FP64 arithmetic without contraction, for bit-for-bit parity with
