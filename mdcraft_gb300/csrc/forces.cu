@@ -319,10 +319,9 @@ static void launch_virials64(const FArgs& A, const PotSet* dps, const PotSet& ps
 // at 3, 0.195 ms at 5, where it spills).
 constexpr int kForceMinBlocks = 4;
 constexpr int kDensityMinBlocks = 4;
-// The Multi bodies spill at 64 registers; three blocks per SM (up to 85
-// registers) are fastest for two kinds (NiAl B2 1M: force pass 0.551 ms
-// against 0.638 ms at four, density 0.355 against 0.383). With more kinds the
-// density body's parameters are read per pair and four blocks do as well.
+// The Multi force bodies spill at 64 registers; three blocks per SM (up to 85
+// registers) are fastest (NiAl B2 1M: 0.497 ms against 0.715 at four), while
+// the density's fit (0.313 ms at four, 0.349 at three).
 constexpr int kMultiMinBlocks = 3;
 // MB = blocks of 256 threads per SM the register budget allows: a system's
 // launch shape (mdg_system_set_shape, chosen by the project's autotuner),
@@ -358,9 +357,9 @@ static int force_blocks(const mdg_system* sys, bool multi) {
     return sys->shape[MDG_SHAPE_FORCE_BLOCKS_PER_SM] ? sys->shape[MDG_SHAPE_FORCE_BLOCKS_PER_SM]
                                                      : (multi ? kMultiMinBlocks : kForceMinBlocks);
 }
-static int density_blocks(const mdg_system* sys, const PotSet& ps) {
+static int density_blocks(const mdg_system* sys) {
     if (sys->shape[MDG_SHAPE_DENSITY_BLOCKS_PER_SM]) return sys->shape[MDG_SHAPE_DENSITY_BLOCKS_PER_SM];
-    return ps.multi && ps.nkinds <= 2 ? kMultiMinBlocks : kDensityMinBlocks;
+    return kDensityMinBlocks;
 }
 
 template <int KINDS, bool KICK>
@@ -692,7 +691,7 @@ int launch_density_rec(mdg_system* sys, const PotSet* dps, const PotSet& ps) {
     A.cutbits = sys->cutbits;
     const int nb = nblk(sys->n);
     cudaStream_t st = sys->ctx->stream;
-    const int mb = density_blocks(sys, ps);
+    const int mb = density_blocks(sys);
     with_kinds(ps, [&](auto k) {
         constexpr int K = decltype(k)::value;
         if (lanes_mixed(sys->n, ps)) k_lane_density<K, true><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, dps);
@@ -746,7 +745,7 @@ int launch_stage(mdg_system* sys, const PotSet* dps, const PotSet& ps, int preci
             with_kinds(ps, [&](auto k) {
                 constexpr int K = decltype(k)::value;
                 if (lanes_mixed(sys->n, ps)) k_lane_density<K, false><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, dps);
-                else launch_density<K>(density_blocks(sys, ps), A, dps, nb, st);
+                else launch_density<K>(density_blocks(sys), A, dps, nb, st);
             });
             sys->fp_ok = 0;  // nc rewritten (FP32 sums); Fp64 no longer matches it
         } else if (kick_dt > 0.0 && !th) {

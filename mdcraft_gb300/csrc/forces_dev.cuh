@@ -91,22 +91,74 @@ __device__ __forceinline__ float ksum_add(float& s, float& c, float v) {
     return s;
 }
 
-// Pair vector r_j - r_i of a list entry from the fixed-point cell-centred
-// offsets: an exact integer difference (modulo 2^32; the true value is
-// within +-2^31 units), one rounding to FP32, one scaling by the unit.
-__device__ __forceinline__ void pair_vec32(uint32_t e, const int4& pi, const int4& pj, const float uf[3],
-                                           float& dx, float& dy, float& dz) {
-    dx = __int2float_rn((int)((uint32_t)pj.x - (uint32_t)pi.x + image_units(e, 0))) * uf[0];
-    dy = __int2float_rn((int)((uint32_t)pj.y - (uint32_t)pi.y + image_units(e, 1))) * uf[1];
-    dz = __int2float_rn((int)((uint32_t)pj.z - (uint32_t)pi.z + image_units(e, 2))) * uf[2];
+// The pair vectors r_j - r_i of N list entries and their
+// squares: from the fixed-point cell-centred offsets an exact integer
+// difference (modulo 2^32; the true value is within +-2^31 units), one
+// rounding to FP32, one scaling by the unit. The passes are bound by the
+// instructions they issue (LJ liquid: 79% of the slots) or, with tables, by L1
+// and those; so the FP32 arithmetic takes two pairs an instruction (the same
+// roundings), and the own offsets come with one cell less (own_units), which
+// makes an entry's image one shifted and masked word. With the cut test's one
+// branch for several pairs (cut_pairs) and the bare hardware estimates
+// (rcp_approx, rsqrt_approx): LJ liquid 4,000,000 atoms 0.675 -> 0.525 ms,
+// EAM Cu 1,000,188 density 0.153 -> 0.135 and force 0.224 -> 0.228, NiAl
+// 1,018,880 density 0.356 -> 0.332 and force 0.551 -> 0.506.
+template <int N>
+struct PairVecs {
+    float x[N], y[N], z[N], r2[N];
+};
+__device__ __forceinline__ int4 own_units(const int4& p) {
+    const uint32_t cell = 1u << kOffBits;
+    return make_int4((int)((uint32_t)p.x + cell), (int)((uint32_t)p.y + cell), (int)((uint32_t)p.z + cell), p.w);
+}
+template <int N>
+__device__ __forceinline__ PairVecs<N> pair_vecs(const uint32_t e[N], const int4& pi, const int4 pj[N],
+                                                 const float uf[3]) {
+    PairVecs<N> v;
+#pragma unroll
+    for (int q = 0; q < N; q += 2) {
+        unsigned long long d[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const uint32_t i = a == 0 ? pi.x : a == 1 ? pi.y : pi.z;
+            const uint32_t j0 = a == 0 ? pj[q].x : a == 1 ? pj[q].y : pj[q].z;
+            const uint32_t j1 = a == 0 ? pj[q + 1].x : a == 1 ? pj[q + 1].y : pj[q + 1].z;
+            d[a] = mul2(pack2(__int2float_rn((int)(j0 - i + image_units(e[q], a))),
+                              __int2float_rn((int)(j1 - i + image_units(e[q + 1], a)))),
+                        pack2(uf[a], uf[a]));
+        }
+        unpack2(d[0], v.x[q], v.x[q + 1]);
+        unpack2(d[1], v.y[q], v.y[q + 1]);
+        unpack2(d[2], v.z[q], v.z[q + 1]);
+        unpack2(fma2(d[0], d[0], fma2(d[1], d[1], mul2(d[2], d[2]))), v.r2[q], v.r2[q + 1]);
+    }
+    return v;
 }
 
-// 1/sqrt(x) for x > 0: the hardware estimate refined by one Newton step, so
+// Hardware estimates of 1/x and 1/sqrt(x), x a normal number: all that a
+// squared distance of at least 1e-12 needs (__fdividef and rsqrtf, the same
+// bits there, also carry subnormal numbers).
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// 1/sqrt(x) for x >= 1e-12: the hardware estimate refined by one Newton step, so
 // r = x * rinv and 1/r are nearly correctly rounded (pair forces near an
 // equilibrium lattice cancel, which magnifies their relative errors).
 __device__ __forceinline__ float rsqrt_nr(float x) {
-    const float y = rsqrtf(x);
+    const float y = rsqrt_approx(x);
     return y * fmaf(-0.5f * x * y, y, 1.5f);
+}
+// Of a pair of numbers.
+__device__ __forceinline__ unsigned long long rsqrt_nr2(unsigned long long x, unsigned long long y) {
+    return mul2(y, fma2(mul2(mul2(pack2(-0.5f, -0.5f), x), y), y, pack2(1.5f, 1.5f)));
 }
 
 // Both force rows (W, D) of one interval: 32 bytes, one 256-bit load
@@ -182,6 +234,34 @@ __device__ __forceinline__ bool pair_in_bits(const FArgs& A, int i, uint32_t e, 
     bool in = r2 >= 1e-15f && r2 <= r2c;
     if (fabsf(r2 - r2c) <= 1e-5f * r2c) in = (A.cutbits[(size_t)(k >> 5) * A.np + i] >> (k & 31)) & 1u;
     return in && (per || !(e & kWrapBit));
+}
+
+// pair_in of N pairs of one potential, with one branch for the
+// rare band pairs: exact(q) settles pair q. [lo, hi] are the FP32 numbers
+// within 1e-5 of rc^2 (cut_band).
+__device__ __forceinline__ void cut_band(float r2c, float& lo, float& hi) {
+    const float band = 1e-5f * r2c;
+    lo = fminf(__fsub_ru(r2c, band), r2c);
+    hi = __fadd_rd(r2c, band);
+}
+template <int N, typename Exact>
+__device__ __forceinline__ void cut_pairs(const uint32_t e[N], const float r2[N], float lo, float hi, bool per,
+                                          bool in[N], Exact&& exact) {
+    bool band = false;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        in[q] = r2[q] >= 1e-15f && r2[q] < lo;
+        band = band || (r2[q] >= lo && r2[q] <= hi);
+    }
+    if (band) {
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+            if (r2[q] >= lo && r2[q] <= hi) in[q] = exact(q);
+    }
+    if (!per) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) in[q] = in[q] && !(e[q] & kWrapBit);
+    }
 }
 
 // The pair loops below read four list entries with one 16-byte load, then
@@ -261,47 +341,60 @@ struct LjGroup {
     int4 pi;
     int ki;
     bool per;
-    float uf[3], r2c, l1, l2, mh;
-    double R2c;
+    float uf[3], lo, hi;
+    unsigned long long l1, ml2, mh;  // Single: the potential's constants, twice each
 
     __device__ __forceinline__ LjGroup(const FArgs& A, const PotSet* __restrict__ p, int i) : ps(p) {
-        pi = A.pos32[i];
+        pi = own_units(A.pos32[i]);
         ki = MULTI ? (A.kind[i] & 3) : 0;
         per = ps->periodic;
         for (int a = 0; a < 3; ++a) uf[a] = A.uf[a];
         if (MULTI) return;
         const PotParams& P0 = ps->p[ki][0];
-        r2c = P0.r2cut_f;
-        l1 = P0.lj1_f;
-        l2 = P0.lj2_f;
-        mh = P0.mhf_f;
-        R2c = P0.R2cut;
+        cut_band(P0.r2cut_f, lo, hi);
+        l1 = pack2(P0.lj1_f, P0.lj1_f);
+        ml2 = pack2(-P0.lj2_f, -P0.lj2_f);
+        mh = pack2(P0.mhf_f, P0.mhf_f);
     }
     __device__ __forceinline__ void operator()(const FArgs& A, int i, int, const uint4& e4, float f[3]) {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) pj[q] = ld_ro<RO>(A.pos32 + (e[q] & kJMask));
-        float fx = 0.f, fy = 0.f, fz = 0.f;
+        const PairVecs<4> v = pair_vecs<4>(e, pi, pj, uf);
+        float pref[4];
+        if (MULTI) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const PotParams& P = ps->p[ki][pj[q].w & 3];
+                const bool in = pair_in(A, i, e[q], v.r2[q], P.r2cut_f, [&] { return P.R2cut; }, per);
+                const float r2inv = rcp_approx(fmaxf(v.r2[q], 1e-12f));
+                const float r6inv = r2inv * r2inv * r2inv;
+                pref[q] = in ? P.mhf_f * fmaf(P.lj1_f, r6inv, -P.lj2_f) * r6inv * r2inv : 0.f;
+            }
+        } else {
+            bool in[4];
+            cut_pairs<4>(e, v.r2, lo, hi, per, in, [&](int q) {
+                const PotParams& P = ps->p[0][0];
+                return cut_in(A, i, e[q] & kJMask, v.r2[q], P.r2cut_f, P.R2cut);
+            });
+#pragma unroll
+            for (int q = 0; q < 4; q += 2) {
+                const unsigned long long r2inv =
+                    pack2(rcp_approx(fmaxf(v.r2[q], 1e-12f)), rcp_approx(fmaxf(v.r2[q + 1], 1e-12f)));
+                const unsigned long long r6inv = mul2(mul2(r2inv, r2inv), r2inv);
+                unpack2(mul2(mul2(mul2(mh, fma2(l1, r6inv, ml2)), r6inv), r2inv), pref[q], pref[q + 1]);
+                pref[q] = in[q] ? pref[q] : 0.f;
+                pref[q + 1] = in[q + 1] ? pref[q + 1] : 0.f;
+            }
+        }
+        f[0] = f[1] = f[2] = 0.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const PotParams* P = MULTI ? &ps->p[ki][pj[q].w & 3] : nullptr;
-            const float r2c = MULTI ? P->r2cut_f : this->r2c, l1 = MULTI ? P->lj1_f : this->l1;
-            const float l2 = MULTI ? P->lj2_f : this->l2, mh = MULTI ? P->mhf_f : this->mh;
-            float dx, dy, dz;
-            pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
-            float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            bool in = pair_in(A, i, e[q], r2, r2c, [&] { return MULTI ? P->R2cut : this->R2c; }, per);
-            float r2inv = __fdividef(1.0f, fmaxf(r2, 1e-12f));
-            float r6inv = r2inv * r2inv * r2inv;
-            float pref = in ? mh * fmaf(l1, r6inv, -l2) * r6inv * r2inv : 0.f;
-            fx = fmaf(dx, pref, fx);
-            fy = fmaf(dy, pref, fy);
-            fz = fmaf(dz, pref, fz);
+            f[0] = fmaf(v.x[q], pref[q], f[0]);
+            f[1] = fmaf(v.y[q], pref[q], f[1]);
+            f[2] = fmaf(v.z[q], pref[q], f[2]);
         }
-        f[0] = fx;
-        f[1] = fy;
-        f[2] = fz;
     }
     __device__ __forceinline__ void word(const FArgs&, int, int, int) {}
     __device__ __forceinline__ void word8(const FArgs&, int, int, bool) {}
@@ -349,7 +442,7 @@ __device__ __forceinline__ float tab_ff32(const PotParams& P, float r2, bool& in
 }
 
 __device__ __forceinline__ float lj_ff32(const PotParams& P, float r2) {
-    const float r2inv = __fdividef(1.0f, fmaxf(r2, 1e-12f));
+    const float r2inv = rcp_approx(fmaxf(r2, 1e-12f));
     const float r6inv = r2inv * r2inv * r2inv;
     return P.mhf_f * fmaf(P.lj1_f, r6inv, -P.lj2_f) * r6inv * r2inv;
 }
@@ -357,7 +450,7 @@ __device__ __forceinline__ float lj_ff32(const PotParams& P, float r2) {
 // Force / r of an LJs pair (LJs.cxx:153-166) in FP32.
 __device__ __forceinline__ float ljs_ff32(const PotParams& P, float r2) {
     const float XX = fmaf(P.ljs_rVr1_f, r2, -1.2599210498948732f);
-    const float FV = P.ljs_rVr2_f * __fdividef(1.0f, fmaxf(r2, 1e-12f));
+    const float FV = P.ljs_rVr2_f * rcp_approx(fmaxf(r2, 1e-12f));
     const float Ur = FV * FV * FV;
     return P.ljs_aVr2_f * fmaf(Ur * (Ur - 0.5f), FV, fmaf(P.ljs_bLJ_f, XX, P.ljs_aLJ_f) * XX);
 }
@@ -380,7 +473,7 @@ struct PairGroup {
     float uf[3];
 
     __device__ __forceinline__ PairGroup(const FArgs& A, const PotSet* __restrict__ p, int i) : ps(p) {
-        pi = A.pos32[i];
+        pi = own_units(A.pos32[i]);
         ki = MULTI ? (A.kind[i] & 3) : 0;
         per = ps->periodic;
         for (int a = 0; a < 3; ++a) uf[a] = A.uf[a];
@@ -390,13 +483,12 @@ struct PairGroup {
         int4 pj[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) pj[q] = ld_ro<RO>(A.pos32 + (e[q] & kJMask));
+        const PairVecs<4> v = pair_vecs<4>(e, pi, pj, uf);
         float fx = 0.f, fy = 0.f, fz = 0.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const PotParams& P = ps->p[ki][MULTI ? (pj[q].w & 3) : 0];
-            float dx, dy, dz;
-            pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
-            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            const float dx = v.x[q], dy = v.y[q], dz = v.z[q], r2 = v.r2[q];
             bool in = pair_in(A, i, e[q], r2, P.r2cut_f, [&] { return P.R2cut; }, per);
             float FF;
             if (FORM == 3 || (FORM == 0 && P.type == POT_TAB)) {
@@ -508,43 +600,63 @@ struct RhoGroup {
     int4 pi;
     int ki;
     bool per, band = false;
-    float uf[3];
+    float uf[3], lo, hi;
     KindPots<KINDS, false> pots;
     uint32_t bits = 0;  // FP64 cut decisions of this word's band entries
 
     __device__ __forceinline__ RhoGroup(const FArgs& A, const PotSet* __restrict__ p, int i) : ps(p) {
-        pi = A.pos32[i];
+        pi = own_units(A.pos32[i]);
         ki = MULTI ? (A.kind[i] & 3) : 0;
         per = ps->periodic;
         for (int a = 0; a < 3; ++a) uf[a] = A.uf[a];
         pots.set(ps, ki);
+        if (!MULTI) cut_band(pots.r2c[0], lo, hi);
     }
     __device__ __forceinline__ void operator()(const FArgs& A, int i, int g, const uint4& e4, float f[1]) {
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
         int4 pj[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) pj[q] = ld_ro<RO>(A.pos32 + (e[q] & kJMask));
+        const PairVecs<4> v = pair_vecs<4>(e, pi, pj, uf);
+        bool in[4];
+        if (!MULTI)
+            cut_pairs<4>(e, v.r2, lo, hi, per, in, [&](int q) {
+                const PotParams& P = ps->p[0][0];
+                const bool settled = cut_in(A, i, e[q] & kJMask, v.r2[q], P.r2cut_f, P.R2cut);
+                if (REC) {
+                    bits |= (uint32_t)settled << ((4 * g + q) & 31);
+                    band = true;
+                }
+                return settled;
+            });
         float part = 0.f;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int kj = MULTI ? pj[q].w & 3 : 0;  // the partner's kind rides in its offsets' w
-            const PairPot P = pots.get(ps, ki, kj);
-            auto R2c = [&] { return ps->p[ki][kj].R2cut; };
-            float dx, dy, dz;
-            pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
-            float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            bool in;
-            if (REC)  // every pair's band decision, whatever its potential
-                in = pair_in_rec(A, i, e[q], r2, P.r2c, R2c, per, 4 * g + q, &bits, &band) && P.eam;
-            else
-                in = P.eam && pair_in(A, i, e[q], r2, P.r2c, R2c, per);
-            float t = r2 * rsqrt_nr(fmaxf(r2, 1e-12f)) * P.idr;
-            int nn = (int)t;
-            in = in && nn < P.Nr1;
-            nn = in ? nn : 0;
-            float u = t - (float)nn;
-            float v = in ? cubic(__ldg(P.tab + nn), u) : 0.f;
-            part += v;
+        for (int q = 0; q < 4; q += 2) {
+            float t[2];
+            if (!MULTI) {
+                const float x0 = fmaxf(v.r2[q], 1e-12f), x1 = fmaxf(v.r2[q + 1], 1e-12f);
+                const unsigned long long rinv = rsqrt_nr2(pack2(x0, x1), pack2(rsqrt_approx(x0), rsqrt_approx(x1)));
+                unpack2(mul2(mul2(pack2(v.r2[q], v.r2[q + 1]), rinv), pack2(pots.idr[0], pots.idr[0])), t[0], t[1]);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int o = q + h;
+                const int kj = MULTI ? pj[o].w & 3 : 0;  // the partner's kind rides in its offsets' w
+                const PairPot P = pots.get(ps, ki, kj);
+                if (MULTI) {
+                    auto R2c = [&] { return ps->p[ki][kj].R2cut; };
+                    if (REC)  // every pair's band decision, whatever its potential
+                        in[o] = pair_in_rec(A, i, e[o], v.r2[o], P.r2c, R2c, per, 4 * g + o, &bits, &band) && P.eam;
+                    else
+                        in[o] = P.eam && pair_in(A, i, e[o], v.r2[o], P.r2c, R2c, per);
+                    t[h] = v.r2[o] * rsqrt_nr(fmaxf(v.r2[o], 1e-12f)) * P.idr;
+                }
+                int nn = (int)t[h];
+                in[o] = in[o] && nn < P.Nr1;
+                nn = in[o] ? nn : 0;
+                const float u = t[h] - (float)nn;
+                part += in[o] ? cubic(__ldg(P.tab + nn), u) : 0.f;
+            }
         }
         f[0] = part;
     }
@@ -597,7 +709,7 @@ __device__ __forceinline__ void density_one(const FArgs& A, const PotSet* __rest
     float rho[1] = {0.f};
     Group grp(A, ps, i);
     if (A.tag[i] != 0) group_sums<1>(A, i, A.ncnt[i] >> 2, grp, rho);
-    store_density<Group::MULTI>(A, ps, i, grp.pi, grp.ki, rho[0]);
+    store_density<Group::MULTI>(A, ps, i, A.pos32[i], grp.ki, rho[0]);
 }
 
 // BITS: a pair in the 1e-5 band around the cutoff takes the density pass's
@@ -612,7 +724,7 @@ struct EamGroup {
     int4 pi;
     int ki;
     bool per;
-    float uf[3];
+    float uf[3], lo, hi;
     KindPots<KINDS, true> pots;
     // Multi: F' of atom i for the kinds 1..3 of its partners, read once (the
     // density pass's Fp32 rows; kind 0's is the record's w, with the atom's
@@ -620,11 +732,12 @@ struct EamGroup {
     float fpi1 = 0.f, fpi2 = 0.f, fpi3 = 0.f;
 
     __device__ __forceinline__ EamGroup(const FArgs& A, const PotSet* __restrict__ p, int i) : ps(p) {
-        pi = A.pos32b[i];
+        pi = own_units(A.pos32b[i]);
         ki = MULTI ? (A.kind[i] & 3) : 0;
         per = ps->periodic;
         for (int a = 0; a < 3; ++a) uf[a] = A.uf[a];
         pots.set(ps, ki);
+        if (!MULTI) cut_band(pots.r2c[0], lo, hi);
         if (MULTI) {
             const int nk = ps->nkinds;
             if (nk > 1) fpi1 = A.Fp32[A.np + i];
@@ -639,43 +752,64 @@ struct EamGroup {
         for (int q = 0; q < 4; ++q) pj[q] = ld_ro<RO>(A.pos32b + (e[q] & kJMask));
         float fx = 0.f, fy = 0.f, fz = 0.f;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            float Fpi = __int_as_float(MULTI ? pi.w & ~3 : pi.w), Fpj = __int_as_float(MULTI ? pj[q].w & ~3 : pj[q].w);
-            const int kj = MULTI ? pj[q].w & 3 : 0;
-            const PairPot P = pots.get(ps, ki, kj);
-            if (MULTI) {
-                // j's F' for i's kind (kind 0's is in j's record)
-                if (ki != 0) Fpj = A.Fp32[(size_t)ki * A.np + (e[q] & kJMask)];
-                Fpi = kj == 0 ? Fpi : KINDS == 2 || kj == 1 ? fpi1 : kj == 2 ? fpi2 : fpi3;
-            }
-            float dx, dy, dz;
-            pair_vec32(e[q], pi, pj[q], uf, dx, dy, dz);
-            float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            bool in;
-            if (BITS)
-                in = (P.eam || P.lj) && pair_in_bits(A, i, e[q], r2, P.r2c, per, 4 * g + q);
-            else
-                in = (P.eam || P.lj) &&
-                     pair_in(A, i, e[q], r2, P.r2c, [&] { return ps->p[ki][kj].R2cut; }, per);
+        for (int q = 0; q < 4; q += 2) {
+            const PairVecs<2> v = pair_vecs<2>(e + q, pi, pj + q, uf);
+            bool in[2];
+            if (!MULTI)
+                cut_pairs<2>(e + q, v.r2, lo, hi, per, in, [&](int h) {
+                    const int k = 4 * g + q + h;
+                    if (BITS) return ((A.cutbits[(size_t)(k >> 5) * A.np + i] >> (k & 31)) & 1u) != 0u;
+                    const PotParams& P = ps->p[0][0];
+                    return cut_in(A, i, e[q + h] & kJMask, v.r2[h], P.r2cut_f, P.R2cut);
+                });
             // one reciprocal square root gives both r and 1/r
-            float rinv = rsqrt_nr(fmaxf(r2, 1e-12f));
-            float r = r2 * rinv;
-            float t = r * P.idr;
-            int nn = (int)t;
-            in = in && (P.lj || nn < P.Nr1);
-            nn = in && !P.lj ? nn : 0;
-            float u = t - (float)nn;
-            float4 cw, cd;
-            load_rv(P.tab, nn, cw, cd);
-            // W = V'r - V and D = rho' on the interval (force_rows)
-            const float W = cubic(cw, u);
-            const float D = fmaf(u, fmaf(u, cd.z, cd.y), cd.x);
-            float FF = fmaf(Fpi + Fpj, D, W * (rinv * rinv)) * rinv;
-            if (MULTI && P.lj) FF = analytic_ff32(ps->p[ki][kj], r2);
-            FF = in ? FF : 0.f;
-            fx = fmaf(FF, dx, fx);
-            fy = fmaf(FF, dy, fy);
-            fz = fmaf(FF, dz, fz);
+            const float x0 = fmaxf(v.r2[0], 1e-12f), x1 = fmaxf(v.r2[1], 1e-12f);
+            const unsigned long long rinv = rsqrt_nr2(pack2(x0, x1), pack2(rsqrt_approx(x0), rsqrt_approx(x1)));
+            const unsigned long long r = mul2(pack2(v.r2[0], v.r2[1]), rinv);
+            float t[2], W[2], D[2], Fp[2], FF[2];
+            if (MULTI) unpack2(r, t[0], t[1]);
+            else unpack2(mul2(r, pack2(pots.idr[0], pots.idr[0])), t[0], t[1]);
+            bool lj[2] = {false, false};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int o = q + h;
+                float Fpi = __int_as_float(MULTI ? pi.w & ~3 : pi.w), Fpj = __int_as_float(MULTI ? pj[o].w & ~3 : pj[o].w);
+                const int kj = MULTI ? pj[o].w & 3 : 0;
+                const PairPot P = pots.get(ps, ki, kj);
+                if (MULTI) {
+                    // j's F' for i's kind (kind 0's is in j's record)
+                    if (ki != 0) Fpj = A.Fp32[(size_t)ki * A.np + (e[o] & kJMask)];
+                    Fpi = kj == 0 ? Fpi : KINDS == 2 || kj == 1 ? fpi1 : kj == 2 ? fpi2 : fpi3;
+                    if (BITS)
+                        in[h] = (P.eam || P.lj) && pair_in_bits(A, i, e[o], v.r2[h], P.r2c, per, 4 * g + o);
+                    else
+                        in[h] = (P.eam || P.lj) &&
+                                pair_in(A, i, e[o], v.r2[h], P.r2c, [&] { return ps->p[ki][kj].R2cut; }, per);
+                    t[h] *= P.idr;
+                    lj[h] = P.lj;
+                }
+                int nn = (int)t[h];
+                in[h] = in[h] && (P.lj || nn < P.Nr1);
+                nn = in[h] && !P.lj ? nn : 0;
+                const float u = t[h] - (float)nn;
+                float4 cw, cd;
+                load_rv(P.tab, nn, cw, cd);
+                // W = V'r - V and D = rho' on the interval (force_rows)
+                W[h] = cubic(cw, u);
+                D[h] = fmaf(u, fmaf(u, cd.z, cd.y), cd.x);
+                Fp[h] = Fpi + Fpj;
+            }
+            unpack2(mul2(fma2(pack2(Fp[0], Fp[1]), pack2(D[0], D[1]), mul2(pack2(W[0], W[1]), mul2(rinv, rinv))), rinv),
+                    FF[0], FF[1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int o = q + h;
+                if (MULTI && lj[h]) FF[h] = analytic_ff32(ps->p[ki][pj[o].w & 3], v.r2[h]);
+                FF[h] = in[h] ? FF[h] : 0.f;
+                fx = fmaf(FF[h], v.x[h], fx);
+                fy = fmaf(FF[h], v.y[h], fy);
+                fz = fmaf(FF[h], v.z[h], fz);
+            }
         }
         f[0] = fx;
         f[1] = fy;

@@ -105,11 +105,37 @@ __host__ __device__ inline size_t nidx(int k, size_t i, size_t np) {
 }
 constexpr uint32_t kSelfCode = 0x15u << kJBits;  // image (0,0,0)
 
-// Image offset encoded in a list entry (2 bits per axis, value+1), in
-// fixed-point offset units (-2^29, 0, 2^29; modulo 2^32).
-__device__ inline uint32_t image_units(uint32_t e, int axis) {
-    uint32_t b = (e >> (kJBits + 2 * axis)) & 3u;  // 0, 1, 2 for -1, 0, +1 cells
-    return (b - 1u) << kOffBits;
+// Image offset encoded in a list entry (2 bits per axis, value + 1: 0, 1, 2 for
+// -1, 0, +1 cells), in fixed-point offset units, plus one cell (2^29): 0,
+// 2^29 or 2^30. The pair vector's other term carries the cell less.
+__device__ __forceinline__ uint32_t image_units(uint32_t e, int axis) {
+    return e << (kOffBits - kJBits - 2 * axis) & 3u << kOffBits;
+}
+static_assert(kOffBits - kJBits == 4, "axis 2's image lies in its place already");
+
+// Packed pairs of FP32 numbers.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
 
 // Potential types: LJsCut and the tabulated Pair are the reference's

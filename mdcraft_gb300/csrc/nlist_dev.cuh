@@ -674,26 +674,6 @@ struct NbWarpSmem {
     uint32_t ccode[27];      // image code << kJBits
 };
 
-// Packed pairs of FP32 numbers.
-__device__ __forceinline__ unsigned long long pack2(float a, float b) {
-    unsigned long long v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-    return v;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-    unsigned long long v;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-    return v;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long v;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
-    return v;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-
 template <int CH>
 __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridParams& g, int bin, int lane,
                                                  bool uniform_rns, NbWarpSmem<CH>& S) {
