@@ -196,16 +196,17 @@ def _pinned(x):
 
 
 @pytest.mark.parametrize("kind", ["lj", "eam"])
-@pytest.mark.parametrize("n", [500, 16384, 16385])
+@pytest.mark.parametrize("n,steps", [(500, 30), (16385, 30), (27999, 1), (28000, 1), (28000, 2)])
 @pytest.mark.parametrize("force", [False, True])
-def test_host_arrays(kind, n, force):
-    """Page-locked host arrays, which the kernel reads and writes itself up to
-    16,384 atoms, against a run and its downloads."""
+def test_host_arrays(kind, n, steps, force):
+    """Page-locked host arrays, which the kernel reads and writes itself (and
+    28,000 atoms' one-step calls the overlapped step), against a run and its
+    downloads."""
     a, b = _Run(kind, n, "mixed", tag0=11), _Run(kind, n, "mixed", tag0=11)
-    a.steps(30, True)
+    a.steps(steps, True)
     ref = a.sys.download()
     pos, vel, frc = _pinned(b.atoms["r"]), _pinned(b.atoms["v"]), _pinned(np.zeros_like(b.atoms["r"]))
-    b.verlet.run_host(b.sys, b.dt, 30, pos.numpy(), vel.numpy(), frc.numpy() if force else None)
+    b.verlet.run_host(b.sys, b.dt, steps, pos.numpy(), vel.numpy(), frc.numpy() if force else None)
     assert np.array_equal(pos.numpy(), ref["r"])
     assert np.array_equal(vel.numpy(), ref["v"])
     assert np.array_equal(frc.numpy() if force else b.sys.forces(), ref["f"])
