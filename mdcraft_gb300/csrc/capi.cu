@@ -1914,9 +1914,14 @@ namespace mdg {
 // After a step's force pass: the rebuild test of this step's positions
 // chooses the rebuild; the test of the next step's positions, when the force
 // pass already ran that step's drift, becomes the current one.
-__global__ void k_rebuild_cond(cudaGraphConditionalHandle h, DevStatus* st) {
+// A step with a thermostat counts its call here; one whose force pass moved
+// the atoms to the other set of arrays (k_lj_step) makes that the current one.
+enum : int { STEP_PLAIN = 0, STEP_THERMO = 1, STEP_FLIPS = 2 };
+__global__ void k_rebuild_cond(cudaGraphConditionalHandle h, DevStatus* st, const unsigned long long* left, int step) {
     if (threadIdx.x != 0) return;
     unsigned need = st->need_rebuild;
+    if (step == STEP_THERMO) st->therm_calls += 1u;
+    if (step == STEP_FLIPS && !need && *left > 1ull) st->flip ^= 1u;
     st->need_rebuild = st->need_next;
     st->need_next = 0;
     if (need) st->pad[0] += 1;  // rebuilds done inside graphs
@@ -1944,6 +1949,7 @@ __global__ void k_loop_start(cudaGraphConditionalHandle h, const unsigned long l
 __global__ void k_set_counter(unsigned long long* counter, unsigned long long v, DevStatus* st) {
     if (threadIdx.x == 0) {
         *counter = v;
+        st->flip = 0;
         st->need_rebuild = 0;
         st->need_next = 0;
         st->build_flags = 0;
@@ -1972,6 +1978,11 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
         int rc = ensure_cutbits(sys);
         if (rc) return rc;
     }
+    // a mixed step whose last pass also starts the next one: the EAM force
+    // pass, the LJ one (between two sets of arrays) or the thermostat's
+    const bool mixed = prec == MDG_PREC_MIXED, thermo = mixed && s->thermo;
+    const bool flips = mixed && !s->thermo && lj_starts_next(sys, ps);
+    const bool next = starts_next_step(s, ps, prec) || flips || thermo;
     cudaGraph_t g = nullptr;
     MDG_CUDA(cudaGraphCreate(&g, 0));
     sys->run_graph = g;
@@ -2010,7 +2021,7 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
         if (prec == MDG_PREC_MIXED) {
             rc0 = launch_drift(sys, 0.0, MDG_PREC_FP64, s->multi ? -1.0 : s->pot[0][0]->rcut, s->periodic, 0, 1);
             if (rc0 == 0) {
-                k_rebuild_cond<<<1, 32, 0, st>>>(hpre, sys->dstat);
+                k_rebuild_cond<<<1, 32, 0, st>>>(hpre, sys->dstat, nullptr, STEP_PLAIN);
                 ctx->launches++;
                 pp.type = cudaGraphNodeTypeConditional;
                 pp.conditional.handle = hpre;
@@ -2021,7 +2032,7 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
             if (rc0 == 0 && e == cudaSuccess) rc0 = launch_offsets(sys);
             // the first step's half-kick and drift (later steps start in the
             // force pass before them)
-            if (rc0 == 0 && e == cudaSuccess && starts_next_step(s, ps, prec))
+            if (rc0 == 0 && e == cudaSuccess && next)
                 rc0 = launch_drift_guarded(sys, dt, sys->dcounter, 1);
         }
         if (rc0 == 0 && e == cudaSuccess) {
@@ -2032,6 +2043,7 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
             wp.conditional.type = cudaGraphCondTypeWhile;
             wp.conditional.size = 1;
             e = add_cond(wp);
+            if (e == cudaSuccess && flips) rc0 = launch_flip_back(sys);
         }
         cudaGraph_t outp = nullptr;
         cudaError_t ec = cudaStreamEndCapture(st, &outp);
@@ -2054,16 +2066,24 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
 
     l0 = ctx->launches;
     MDG_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    const bool next = starts_next_step(s, ps, prec);
     int rc = MDG_OK;
-    if (next) {
+    if (starts_next_step(s, ps, prec)) {
         rc = step_stages_next(s, sys, ps, dt);
+    } else if (flips) {
+        rc = launch_lj_step(sys, ext(s)->d.dev, ps, dt, sys->dcounter);
+        sys->force_prec = MDG_PREC_MIXED;
+    } else if (thermo) {
+        for (int q = 0; q < s->nstages && rc == 0; ++q)
+            rc = launch_stage(sys, ext(s)->d.dev, ps, prec, s->stages[q], nullptr, 0.0);
+        if (rc == 0) rc = launch_thermo_step(sys, thermo_of(s), dt, sys->dcounter);
+        sys->force_prec = MDG_PREC_MIXED;
     } else {
         rc = launch_drift(sys, dt, prec, s->multi ? -1.0 : s->pot[0][0]->rcut, s->periodic, 1, 1);
         if (rc == 0) rc = step_stages(s, sys, ps, prec, dt);
     }
     if (rc == 0) {
-        k_rebuild_cond<<<1, 32, 0, st>>>(hrb, sys->dstat);
+        k_rebuild_cond<<<1, 32, 0, st>>>(hrb, sys->dstat, sys->dcounter,
+                                         thermo ? STEP_THERMO : flips ? STEP_FLIPS : STEP_PLAIN);
         ctx->launches++;
     }
     cudaStreamCaptureStatus cs;
@@ -2098,7 +2118,7 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
     l0 = ctx->launches;
     MDG_CUDA(cudaStreamBeginCaptureToGraph(st, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                            cudaStreamCaptureModeThreadLocal));
-    rc = nlist_enqueue(sys);
+    rc = nlist_enqueue(sys, flips);
     // the next step's half-kick and drift, which the force pass left to
     // after the rebuild (none after the last step)
     if (rc == 0 && next) rc = launch_drift_guarded(sys, dt, sys->dcounter, 2);

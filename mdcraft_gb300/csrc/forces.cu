@@ -404,15 +404,14 @@ __global__ void __launch_bounds__(kBlock, kForceMinBlocks) k_pair_mixed(FArgs A,
 
 // The end of a step's force pass for atom i (k_force_step): the second
 // half-kick, and with `next` the next step's start; its rebuild test.
-__device__ __forceinline__ bool end_step(const FArgs& A, const IArgs& D, int i, bool moved, bool next,
-                                         const float f[3]) {
+__device__ __forceinline__ bool end_step(const FArgs& A, const IArgs& D, const IArgs& to, int i, bool moved,
+                                         bool next, const float f[3]) {
     if (!next) {
         if (moved) store_force<true>(A, i, f[0], f[1], f[2]);
         return false;
     }
-    if (moved) return kick_drift_mixed(D, D, A.gx, A.gy, A.gz, i, f[0], f[1], f[2]);
-    const double r[3] = {D.rx[i], D.ry[i], D.rz[i]};
-    return offsets_check_mixed(D, i, r);
+    if (moved) return kick_drift_mixed(D, to, A.gx, A.gy, A.gz, i, f[0], f[1], f[2]);
+    return drift_mixed_one(D, to, i);  // tag 0: the offsets and the test
 }
 
 // ---- eight lanes per atom: systems that do not fill the GPU ------------------
@@ -473,7 +472,7 @@ __global__ void __launch_bounds__(kBlock, lane_budget(KINDS))
     float f[3];
     const int i = block_forces<EamGroup<KINDS, true>>(A, ps, f);
     if (threadIdx.x >= kLaneAtoms) return;
-    const bool need = i >= 0 && end_step(A, D, i, A.tag[i] != 0, next, f);
+    const bool need = i >= 0 && end_step(A, D, D, i, A.tag[i] != 0, next, f);
     if (next) flag_need_next(need, A.st);
 }
 
@@ -644,9 +643,95 @@ __global__ void __launch_bounds__(NT, MB)
     if (i < A.n) {
         float f[3];
         const bool moved = thread_forces<EamGroup<KINDS, true>>(A, ps, i, f);
-        need = end_step(A, D, i, moved, next, f);
+        need = end_step(A, D, D, i, moved, next, f);
     }
     if (next) flag_need_next(need, A.st);
+}
+
+// The LJ force pass of such a step. It reads its neighbours' own offsets (and
+// the FP64 positions of pairs near the cutoff), so the moved atoms go to the
+// other of two sets of arrays, which the loop's control kernel then takes for
+// the current one (DevStatus::flip). The drift as a pass of its own read and
+// wrote 190 bytes an atom again: LJ liquid 4,000,000 atoms 956 -> 877 us a
+// step, 256,000 86.5 -> 81.0, the rebuilds' share included.
+template <bool MULTI, int MB>
+__global__ void __launch_bounds__(kBlock, MB)
+    k_lj_step(FArgs A, IArgs D, const PosSet other, const PotSet* __restrict__ ps,
+              const unsigned long long* __restrict__ left) {
+    const bool next = *left > 1ull && A.st->need_rebuild == 0u;
+    IArgs to = D;
+    if (A.st->flip) {
+        A.pos32 = other.pos32;
+        A.rx = D.rx = other.rx;
+        A.ry = D.ry = other.ry;
+        A.rz = D.rz = other.rz;
+    } else {
+        to.pos32 = other.pos32;
+        to.rx = other.rx;
+        to.ry = other.ry;
+        to.rz = other.rz;
+    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool need = false;
+    if (i < A.n) {
+        float f[3];
+        const bool moved = thread_forces<LjGroup<MULTI>>(A, ps, i, f);
+        need = end_step(A, D, to, i, moved, next, f);
+    }
+    if (next) flag_need_next(need, A.st);
+}
+
+// The rest of a mixed step with a thermostat, after its force pass: the
+// thermostat, the second half-kick and, as above, the next step's start. (As
+// three passes, and one to count the call: EAM Cu 32,000 atoms 57.0 us a step,
+// 54.0 as one.)
+__global__ void __launch_bounds__(kBlock)
+    k_thermo_step(ThermoArgs T, const ThermoDev* __restrict__ th, IArgs D, const unsigned long long* __restrict__ left) {
+    const bool next = *left > 1ull && D.st->need_rebuild == 0u;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool need = false;
+    if (i < T.n) {
+        langevin_one<true>(T, th, i, T.st->therm_calls);
+        kick_mixed_one(D, i);
+        if (next) need = drift_mixed_one(D, D, i);
+    }
+    if (next) flag_need_next(need, D.st);
+}
+
+int launch_thermo_step(mdg_system* sys, const ThermoDev* th, double dt, const unsigned long long* left) {
+    if (sys->n == 0) return MDG_OK;
+    k_thermo_step<<<spread_blocks(sys->n), spread_threads(sys->n), 0, sys->ctx->stream>>>(
+        thermo_args(sys), th, integrator_args(sys, dt), left);
+    MDG_LAUNCHED(sys->ctx);
+    return MDG_OK;
+}
+
+PosSet other_positions(mdg_system* sys) {
+    const int o = sys->cur ^ 1;
+    return PosSet{sys->f64[RX][o], sys->f64[RY][o], sys->f64[RZ][o], sys->pos32 + sys->np};
+}
+
+// Whether a step loop's LJ pass starts the next step: LJsCut alone, one thread
+// per atom.
+bool lj_starts_next(const mdg_system* sys, const PotSet& ps) {
+    return ps.any_lj && !ps.any_eam && !ps.any_tab && !ps.any_ljs && !lanes_mixed(sys->n, ps);
+}
+
+int launch_lj_step(mdg_system* sys, const PotSet* dps, const PotSet& ps, double dt, const unsigned long long* left) {
+    if (sys->n == 0) return MDG_OK;
+    FArgs A = force_args(sys);
+    A.kick_hdt = 0.5f * (float)dt;
+    const IArgs D = integrator_args(sys, dt);
+    const PosSet other = other_positions(sys);
+    const int nb = nblk(sys->n);
+    cudaStream_t st = sys->ctx->stream;
+    const bool three = force_blocks(sys, ps.multi != 0) == 3;
+    if (ps.multi && three) k_lj_step<true, 3><<<nb, kBlock, 0, st>>>(A, D, other, dps, left);
+    else if (ps.multi) k_lj_step<true, 4><<<nb, kBlock, 0, st>>>(A, D, other, dps, left);
+    else if (three) k_lj_step<false, 3><<<nb, kBlock, 0, st>>>(A, D, other, dps, left);
+    else k_lj_step<false, 4><<<nb, kBlock, 0, st>>>(A, D, other, dps, left);
+    MDG_LAUNCHED(sys->ctx);
+    return MDG_OK;
 }
 
 int launch_forces_step(mdg_system* sys, const PotSet* dps, const PotSet& ps, double dt,

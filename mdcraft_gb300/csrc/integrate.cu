@@ -64,6 +64,24 @@ __global__ void k_drift_mixed_guarded(IArgs A, const unsigned long long* __restr
     flag_need(need, A.st);
 }
 
+// The end of a loop whose force pass moves atoms between two sets of arrays
+// (k_lj_step): the positions and offsets back in the first, if they are not.
+__global__ void k_flip_back(int n, PosSet main, PosSet other, DevStatus* st) {
+    if (!st->flip) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        main.rx[i] = other.rx[i];
+        main.ry[i] = other.ry[i];
+        main.rz[i] = other.rz[i];
+        main.pos32[i] = other.pos32[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&st->arrived, 1u) == gridDim.x - 1) st->arrived = st->flip = 0;
+    }
+}
+
 __global__ void k_kick_mixed(IArgs A) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < A.n) kick_mixed_one(A, i);
@@ -253,6 +271,16 @@ int launch_drift_guarded(mdg_system* sys, double dt, const unsigned long long* l
     if (sys->n == 0) return MDG_OK;
     IArgs A = integrator_args(sys, dt);
     k_drift_mixed_guarded<<<spread_blocks(sys->n), spread_threads(sys->n), 0, sys->ctx->stream>>>(A, left, min_left);
+    MDG_LAUNCHED(sys->ctx);
+    return MDG_OK;
+}
+
+int launch_flip_back(mdg_system* sys) {
+    if (sys->n == 0) return MDG_OK;
+    const int c = sys->cur;
+    const PosSet main{sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c], sys->pos32};
+    k_flip_back<<<spread_blocks(sys->n), spread_threads(sys->n), 0, sys->ctx->stream>>>((int)sys->n, main,
+                                                                                      other_positions(sys), sys->dstat);
     MDG_LAUNCHED(sys->ctx);
     return MDG_OK;
 }

@@ -362,7 +362,15 @@ int grid_build_only(mdg_system* sys, GridParams* out);
 int nlist_export_offsets(mdg_system* sys, std::vector<uint64_t>& off);
 int nlist_export_entries(mdg_system* sys, const std::vector<uint64_t>& off, uint64_t* idx);
 int nlist_capacity(mdg_system* sys, int half);
-int nlist_enqueue(mdg_system* sys);
+// flips: the positions may be in a step loop's second buffers (DevStatus::flip).
+int nlist_enqueue(mdg_system* sys, bool flips = false);
+// A step loop's passes that start the next step, and its end (forces.cu,
+// integrate.cu).
+PosSet other_positions(mdg_system* sys);
+bool lj_starts_next(const mdg_system* sys, const PotSet& ps);
+int launch_lj_step(mdg_system* sys, const PotSet* dps, const PotSet& ps, double dt, const unsigned long long* left);
+int launch_thermo_step(mdg_system* sys, const ThermoDev* th, double dt, const unsigned long long* left);
+int launch_flip_back(mdg_system* sys);
 int potset_build(mdg_solver* s, mdg_system* sys, PotSet* out);
 int pot_upload(mdg_potential* p, int device);
 int run_prepare(mdg_solver* s, mdg_system* sys, const PotSet& ps, int check_rcut);

@@ -236,6 +236,13 @@ __device__ __forceinline__ double shortest1(double v, double L, int periodic) {
 }
 
 // Device-side status words of one system.
+// Position and offset arrays of a step loop that moves atoms from one set to
+// the other (k_lj_step).
+struct PosSet {
+    double *rx, *ry, *rz;
+    int4* pos32;
+};
+
 struct DevStatus {
     uint32_t flags;         // FLAG_* accumulated until read by mdg_system_flags
     uint32_t need_rebuild;  // rebuild test of the current step
@@ -248,6 +255,7 @@ struct DevStatus {
                             // that ran the next step's first half-kick and drift
     uint32_t arrived;       // blocks of the bounds pass done (0 between rebuilds)
     uint32_t team_done;     // blocks of the team kernel done (solo.cu; 0 between launches)
+    uint32_t flip;          // 1: the positions and offsets are in their second buffers (k_lj_step)
 };
 
 }  // namespace mdg

@@ -48,20 +48,27 @@ __device__ __forceinline__ void block_bounds(long long v[7]) {
 
 // Wraps the positions and finds their bounds, the largest rns and whether the
 // rns differ, clears the bin counts, and, in the block that finishes last,
-// computes the grid. (One launch: as passes of their own these were five
+// computes the grid. `other`: where a step loop may have left the positions
+// (DevStatus::flip); null arrays: nowhere. (One launch: as passes of their own these were five
 // launches, of which a small system's rebuild has nothing but.)
 __global__ void __launch_bounds__(kBlock)
     k_wrap_bounds(int n, double* __restrict__ rx, double* __restrict__ ry, double* __restrict__ rz,
                   const double* __restrict__ rns, DomainDev d, double* __restrict__ part,
                   GridParams* __restrict__ out, long long bin_cap, uint32_t* __restrict__ bin_count,
-                  DevStatus* st) {
+                  DevStatus* st, const PosSet other) {
     const int t = threadIdx.x;
+    const bool flip = other.rx && st->flip;
     long long v[7];
     no_bounds<7>(v);
     const double r0 = n > 0 ? rns[0] : 0.0;
     bool differ = false;
     for (int i = blockIdx.x * kBlock + t; i < n; i += gridDim.x * kBlock) {
         double x[3];
+        if (flip) {
+            rx[i] = other.rx[i];
+            ry[i] = other.ry[i];
+            rz[i] = other.rz[i];
+        }
         wrap_one(d, rx, ry, rz, i, x);
         const double q = rns[i];
         add_bounds(v, x, q);
@@ -111,6 +118,7 @@ __global__ void __launch_bounds__(kBlock)
     __syncwarp();
     if (t == 0) {
         st->arrived = 0;
+        if (other.rx) st->flip = 0;
         grid_totals(d, cell, small, bad, g);
         // the bin arrays were sized on the host; a grid that outgrew them
         // invalidates this rebuild (every later kernel of it returns early)
@@ -537,7 +545,7 @@ int nlist_capacity(mdg_system* sys, int half) {
     int c = sys->cur;
     k_wrap_bounds<<<nparts, kBlock, 0, st>>>(n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c],
                                              sys->f64[RNS][c], d, sys->part, sys->dgrid, 1LL << 40, nullptr,
-                                             sys->dstat);
+                                             sys->dstat, PosSet{});
     MDG_LAUNCHED(ctx);
     MDG_CUDA(cudaMemcpyAsync(sys->hgrid, sys->dgrid, sizeof(GridParams), cudaMemcpyDeviceToHost, st));
     MDG_CUDA(cudaStreamSynchronize(st));
@@ -555,7 +563,7 @@ int grid_build_only(mdg_system* sys, GridParams* out) {
     const int c = sys->cur;
     k_wrap_bounds<<<nparts, kBlock, 0, st>>>((int)sys->n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c],
                                              sys->f64[RNS][c], d, sys->part, sys->dgrid, 1LL << 40, nullptr,
-                                             sys->dstat);
+                                             sys->dstat, PosSet{});
     MDG_LAUNCHED(ctx);
     MDG_CUDA(cudaMemcpyAsync(out, sys->dgrid, sizeof(GridParams), cudaMemcpyDeviceToHost, st));
     MDG_CUDA(cudaStreamSynchronize(st));
@@ -731,7 +739,7 @@ static int launch_scan(mdg_system* sys, uint32_t* out) {
     return MDG_OK;
 }
 
-int nlist_enqueue(mdg_system* sys) {
+int nlist_enqueue(mdg_system* sys, bool flips) {
     mdg_ctx* ctx = sys->ctx;
     sys->fp_ok = 0;  // the atoms are permuted; Fp64 is per slot
     cudaStream_t st = ctx->stream;
@@ -743,7 +751,8 @@ int nlist_enqueue(mdg_system* sys) {
     MDG_CUDA(cudaMemsetAsync(&sys->dstat->max_count, 0, 3 * sizeof(uint32_t), st));  // max_count, nonuniform, build_flags
     k_wrap_bounds<<<nparts, kBlock, 0, st>>>(n, sys->f64[RX][c], sys->f64[RY][c], sys->f64[RZ][c],
                                              sys->f64[RNS][c], d, sys->part, sys->dgrid, (long long)sys->bin_cap,
-                                             sys->bin_count, sys->dstat);
+                                             sys->bin_count, sys->dstat,
+                                             flips ? other_positions(sys) : PosSet{});
     MDG_LAUNCHED(ctx);
     // the atoms' cells wait in ncnt (free until the list is built)
     const int pt = spread_threads(n), pb = nblk(n, pt);
