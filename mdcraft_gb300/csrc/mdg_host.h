@@ -304,6 +304,7 @@ public:
     DeviceUse(const DeviceUse&) = delete;
     DeviceUse& operator=(const DeviceUse&) = delete;
     bool alone() const { return n_.load() == 1; }
+    static int in_flight(int device) { return count(device).load(); }
 
 private:
     static std::atomic<int>& count(int device) {
@@ -318,6 +319,11 @@ bool team_eligible(const mdg_solver* s, const mdg_system* sys);
 int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam, int mixed, double pot_rcut,
                 int periodic, double dt, long steps, const double* hpos, const double* hvel, double* opos,
                 double* ovel, double* oforce);
+size_t request_team_scratch(int blocks);
+int request_team_prepare(mdg_system* sys, int eam);
+int request_team_launch(const void* args, mdg_system* sys, int blocks, unsigned long long* scratch,
+                        cudaStream_t stream);
+bool solo_out_started(const void* out_host, uint32_t seq);
 int solo_eligible(const mdg_solver* s, const mdg_system* sys);
 size_t solo_args_bytes();
 size_t solo_out_bytes();

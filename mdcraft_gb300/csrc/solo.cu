@@ -41,7 +41,7 @@ struct SoloOut {
     unsigned long long left;
     DevStatus st;
     volatile uint32_t done;
-    uint32_t pad;
+    volatile uint32_t started;  // a request's team: seq, once its blocks run
     // GPU clock (%globaltimer, ns): the block starts on the request / has
     // written the result records (service time = end - start)
     unsigned long long t_start, t_end;
@@ -338,10 +338,10 @@ __device__ __noinline__ bool solo_rebuild(Team<NT, WIDE>& tm, const SoloArgs& S,
 }
 
 // The input records (mdg_system_upload_atoms' scatter) from host memory.
-template <int NT>
-__device__ __noinline__ void solo_read_atoms(const SoloArgs& S) {
+template <int NT, bool WIDE>
+__device__ __noinline__ void solo_read_atoms(const Team<NT, WIDE>& tm, const SoloArgs& S) {
     const GatherAll& G = S.G;
-    for (int k = threadIdx.x; k < S.n; k += NT) {
+    for (int k = tm.gt; k < S.n; k += tm.gn) {
         const mdg_atom& a = S.atoms_in[k];
         const uint32_t s = S.C.slot_of[k];
         for (int c = 0; c < 3; ++c) {
@@ -378,17 +378,16 @@ __device__ __forceinline__ void solo_zero_one(const SoloArgs& S, int i) {
     }
 }
 
-// The force stages of one block; with KICK the second half-kick rides in the
-// force body (the step loop), without it the forces alone (the set-up's
-// initial forces).
-template <bool EAM, bool KICK, int NT>
-__device__ __forceinline__ void solo_stages(const SoloArgs& S) {
-    const int t = threadIdx.x, n = S.n;
+// The force stages, a thread per atom; with KICK the second half-kick rides in
+// the force body (the step loop of one block), without it the forces alone
+// (the set-up's initial forces).
+template <bool EAM, bool KICK, int NT, bool WIDE>
+__device__ __forceinline__ void solo_stages(Team<NT, WIDE>& tm, const SoloArgs& S) {
     if (EAM) {
-        for (int i = t; i < n; i += NT) density_one<RhoGroup<0, false, false>>(S.F, S.ps, i);
-        __syncthreads();
+        for (int i = tm.a0 + tm.t; i < tm.a1; i += NT) density_one<RhoGroup<0, false, false>>(S.F, S.ps, i);
+        tm.sync();
     }
-    for (int i = t; i < n; i += NT) {
+    for (int i = tm.a0 + tm.t; i < tm.a1; i += NT) {
         float f[3];
         bool live;
         if (EAM) live = thread_forces<EamGroup<0, false, false>>(S.F, S.ps, i, f);
@@ -400,11 +399,11 @@ __device__ __forceinline__ void solo_stages(const SoloArgs& S) {
 // The set-up of a fresh system, in the order of the host calls it replaces
 // (upload, prepare, update(-1), offsets, prepare, stages). False when the
 // first list outgrew the capacities sized on the host.
-template <bool EAM, int NT>
-__device__ __noinline__ bool solo_setup(Team<NT, false>& tm, const SoloArgs& S, GridParams& g, SoloShared<NT>& sh) {
-    const int t = threadIdx.x, n = S.n;
+template <bool EAM, int NT, bool WIDE>
+__device__ __noinline__ bool solo_setup(Team<NT, WIDE>& tm, const SoloArgs& S, GridParams& g, SoloShared<NT>& sh) {
+    const int a0 = tm.a0 + tm.t, a1 = tm.a1;  // this thread's atoms: a0, a0 + NT, ...
     // the fresh system's buffers (what system_alloc clears on a stream)
-    for (int k = t; k < S.np; k += NT) {
+    for (int k = tm.gt; k < S.np; k += tm.gn) {
         S.G.u2.out[0][k] = (uint32_t)k;  // caller index of slot k
         S.C.slot_of[k] = (uint32_t)k;
         S.N.ncnt[k] = 0;
@@ -415,31 +414,31 @@ __device__ __noinline__ bool solo_setup(Team<NT, false>& tm, const SoloArgs& S, 
         S.C.Rz[k] = 0.0;
         for (int q = 0; q < kMaxKinds; ++q) S.F.Fp64[(size_t)q * S.np + k] = 0.0;
     }
-    if (t == 0) memset(S.st, 0, sizeof(DevStatus));
+    if (tm.gt == 0) memset(S.st, 0, sizeof(DevStatus));
+    tm.sync();
+    solo_read_atoms<NT, WIDE>(tm, S);
+    tm.sync();
+    for (int i = a0; i < a1; i += NT) drift64_one(S.I, S.I, i, 0, 0);
     __syncthreads();
-    solo_read_atoms<NT>(S);
-    __syncthreads();
-    for (int i = t; i < n; i += NT) drift64_one(S.I, S.I, i, 0, 0);
-    __syncthreads();
-    if (!solo_rebuild<NT, false>(tm, S, g, sh)) return false;
-    for (int i = t; i < n; i += NT)
+    if (!solo_rebuild<NT, WIDE>(tm, S, g, sh)) return false;
+    for (int i = a0; i < a1; i += NT)
         S.C.pos32[i] = make_int4(off_encode(S.rx[i] - S.C.Rx[i], g.inv_u[0]), off_encode(S.ry[i] - S.C.Ry[i], g.inv_u[1]),
                                  off_encode(S.rz[i] - S.C.Rz[i], g.inv_u[2]), S.F.kind[i] & 3);
-    for (int i = t; i < n; i += NT) solo_zero_one(S, i);
+    for (int i = a0; i < a1; i += NT) solo_zero_one(S, i);
     __syncthreads();
-    for (int i = t; i < n; i += NT) drift64_one(S.I, S.I, i, 0, 0);
-    __syncthreads();
-    solo_stages<EAM, false, NT>(S);
-    __syncthreads();
-    return true;
+    for (int i = a0; i < a1; i += NT) drift64_one(S.I, S.I, i, 0, 0);
+    tm.sync();
+    solo_stages<EAM, false>(tm, S);
+    tm.sync();
+    return !tm.dead;
 }
 
 // The result records (mdg_system_download_atoms' layout) straight into host
 // memory; mixed forces are widened to FP64 as the download does.
-template <int NT>
-__device__ __noinline__ void solo_write_atoms(const SoloArgs& S) {
+template <int NT, bool WIDE>
+__device__ __noinline__ void solo_write_atoms(const Team<NT, WIDE>& tm, const SoloArgs& S) {
     const GatherAll& G = S.G;
-    for (int k = threadIdx.x; k < S.n; k += NT) {
+    for (int k = tm.gt; k < S.n; k += tm.gn) {
         const uint32_t s = S.C.slot_of[k];
         mdg_atom a;
         const bool live = G.h.in[1][s] != 0;  // tag
@@ -475,7 +474,7 @@ __device__ void solo_run(SoloArgs& S, GridParams& g, SoloShared<NT>& sh) {
     bool ok = true;
     unsigned long long t_start = 0;
     if (t == 0) t_start = global_ns();
-    if (S.setup) ok = solo_setup<EAM, NT>(tm, S, g, sh);
+    if (S.setup) ok = solo_setup<EAM>(tm, S, g, sh);
     if (t == 0) {
         S.st->need_rebuild = 0;
         S.st->build_flags = 0;
@@ -484,7 +483,7 @@ __device__ void solo_run(SoloArgs& S, GridParams& g, SoloShared<NT>& sh) {
         bool need = false;
         for (int i = t; i < n; i += NT) need |= drift_mixed_one(S.I, S.I, i);
         const int any = __syncthreads_or(need);
-        solo_stages<EAM, true, NT>(S);
+        solo_stages<EAM, true>(tm, S);
         __syncthreads();
         --left;
         if (any) {
@@ -492,7 +491,7 @@ __device__ void solo_run(SoloArgs& S, GridParams& g, SoloShared<NT>& sh) {
             ok = solo_rebuild<NT, false>(tm, S, g, sh);
         }
     }
-    if (ok && left == 0) solo_write_atoms<NT>(S);
+    if (ok && left == 0) solo_write_atoms(tm, S);
     __syncthreads();
     if (t == 0) {
         S.st->need_rebuild = 0;
@@ -714,6 +713,55 @@ __device__ __forceinline__ void team_offsets(const Team<NT, true>& tm, const Sol
                                  off_encode(S.rz[i] - S.C.Rz[i], S.I.inv_u[2]), S.F.kind[i] & 3);
 }
 
+// The step loop of a team whose positions are in their first buffers, where
+// they are at the end; `ok` false, or a rebuild that outgrew its capacities,
+// ends it with steps left.
+template <bool EAM, bool MIXED, int NT, int G>
+__device__ __forceinline__ void team_steps(Team<NT, true>& tm, const SoloArgs& S, const TeamRun& R, GridParams& g,
+                                           SoloShared<NT>& sh, LaneShared<NT>& lanes, bool& ok, long long& left,
+                                           uint32_t& rebuilds, uint32_t& call) {
+    const int t = tm.t;
+    // a step's first half-kick and drift as a pass of its own, in place;
+    // whether a rebuild is due after it
+    auto drift = [&] {
+        bool need = false;
+        for (int i = tm.a0 + t; i < tm.a1; i += NT)
+            need |= MIXED ? drift_mixed_one(S.I, S.I, i) : drift64_one(S.I, S.I, i, 1, 1);
+        return tm.any(need);
+    };
+    int p = 0;  // the buffers that hold the positions
+    bool due = ok && left > 0 && drift();
+    while (ok && left > 0 && !tm.dead) {
+        const bool next = left > 1 && !due;
+        const bool need = team_step<EAM, MIXED, NT, G>(tm, S, R, lanes, p, next, call);
+        bool due_next = false;
+        if (left > 1 || due) due_next = tm.any(need);
+        if (tm.dead) break;
+        --left;
+        ++call;
+        if (next) {
+            if (kFlips<EAM, MIXED>) p ^= 1;
+            due = due_next;
+            continue;
+        }
+        // the last step, or a rebuild: positions back in their own buffers
+        if (p) {
+            for (int i = tm.a0 + t; i < tm.a1; i += NT) {
+                S.I.rx[i] = R.I1.rx[i];
+                S.I.ry[i] = R.I1.ry[i];
+                S.I.rz[i] = R.I1.rz[i];
+                if (MIXED) S.I.pos32[i] = R.I1.pos32[i];
+            }
+            p = 0;
+        }
+        if (due) {
+            ++rebuilds;
+            ok = solo_rebuild<NT, true>(tm, S, g, sh);
+        }
+        due = ok && left > 0 && drift();
+    }
+}
+
 // G: lanes per atom of the FP64 passes.
 template <bool EAM, bool MIXED, int G>
 __global__ void __launch_bounds__(kTeamThreads, 1)
@@ -754,45 +802,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         }
         team_offsets<NT>(tm, S);
     }
-    // a step's first half-kick and drift as a pass of its own, in place;
-    // whether a rebuild is due after it
-    auto drift = [&] {
-        bool need = false;
-        for (int i = tm.a0 + t; i < tm.a1; i += NT)
-            need |= MIXED ? drift_mixed_one(S.I, S.I, i) : drift64_one(S.I, S.I, i, 1, 1);
-        return tm.any(need);
-    };
-    int p = 0;  // the buffers that hold the positions
-    bool due = ok && left > 0 && drift();
-    while (ok && left > 0 && !tm.dead) {
-        const bool next = left > 1 && !due;
-        const bool need = team_step<EAM, MIXED, NT, G>(tm, S, R, lanes, p, next, call);
-        bool due_next = false;
-        if (left > 1 || due) due_next = tm.any(need);
-        if (tm.dead) break;
-        --left;
-        ++call;
-        if (next) {
-            if (kFlips<EAM, MIXED>) p ^= 1;
-            due = due_next;
-            continue;
-        }
-        // the last step, or a rebuild: positions back in their own buffers
-        if (p) {
-            for (int i = tm.a0 + t; i < tm.a1; i += NT) {
-                S.I.rx[i] = R.I1.rx[i];
-                S.I.ry[i] = R.I1.ry[i];
-                S.I.rz[i] = R.I1.rz[i];
-                if (MIXED) S.I.pos32[i] = R.I1.pos32[i];
-            }
-            p = 0;
-        }
-        if (due) {
-            ++rebuilds;
-            ok = solo_rebuild<NT, true>(tm, S, g, sh);
-        }
-        due = ok && left > 0 && drift();
-    }
+    team_steps<EAM, MIXED, NT, G>(tm, S, R, g, sh, lanes, ok, left, rebuilds, call);
     if (left == 0 && R.opos) {
         for (int i = tm.a0 + t; i < tm.a1; i += NT) {
             const size_t o = 3 * (size_t)S.orig[i];
@@ -829,6 +839,58 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             for (int k = 0; k < (int)(sizeof(DevStatus) / 4); ++k) to[k] = from[k];
             S.st->pad[1] = 0;
             *R.left_host = *(volatile unsigned long long*)R.left_dev;
+        }
+    }
+}
+
+// A served request by a team of its own, while there are fewer requests than
+// SMs: what solo_run does, with the result records written by all blocks and
+// the completion record by the one that ends last.
+template <bool EAM>
+__global__ void __launch_bounds__(kTeamThreads, 1)
+    k_team_request(const __grid_constant__ SoloArgs S, const __grid_constant__ TeamRun R) {
+    constexpr int NT = kTeamThreads;
+    __shared__ GridParams g;
+    __shared__ SoloShared<NT> sh;
+    __shared__ LaneShared<NT> lanes;
+    Team<NT, true> tm(R.word, &sh.said, S.n, R.per);
+    if (tm.gt == 0) {
+        S.out->t_start = global_ns();
+        S.out->started = S.seq;
+    }
+    bool ok = solo_setup<EAM>(tm, S, g, sh);
+    if (ok && tm.gt == 0) {  // (after a failure other blocks may still read the flags)
+        S.st->need_rebuild = 0;
+        S.st->build_flags = 0;
+    }
+    long long left = S.steps;
+    uint32_t rebuilds = 0, call = 0;
+    team_steps<EAM, true, NT, 8>(tm, S, R, g, sh, lanes, ok, left, rebuilds, call);
+    ok = ok && left == 0 && !tm.dead;
+    tm.sync();  // every block's atoms are final
+    if (ok) solo_write_atoms(tm, S);
+    if (tm.gt == 0) {
+        S.st->pad[0] = rebuilds;
+        *R.left_dev = (unsigned long long)left;
+    }
+    __threadfence_system();
+    __syncthreads();
+    if (tm.t == 0) {
+        if (tm.dead) atomicOr(&S.st->pad[1], 1u);
+        __threadfence();
+        if (atomicAdd(&S.st->team_done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            S.st->team_done = 0;
+            *R.word = 0;
+            const volatile uint32_t* from = reinterpret_cast<const volatile uint32_t*>(S.st);
+            uint32_t* to = reinterpret_cast<uint32_t*>(&S.out->st);
+            for (int k = 0; k < (int)(sizeof(DevStatus) / 4); ++k) to[k] = from[k];
+            const unsigned long long rest = *(volatile unsigned long long*)R.left_dev;
+            S.out->left = rest;
+            if (rest != 0) S.out->st.pad[1] = 1;  // void: a list outgrew its capacities
+            S.out->t_end = global_ns();
+            __threadfence_system();
+            S.out->done = S.seq;
         }
     }
 }
@@ -917,6 +979,21 @@ bool team_eligible(const mdg_solver* s, const mdg_system* sys) {
 // steps left and the status words arrive in hcounter and hstat.
 int ensure_cutbits(mdg_system* sys);
 
+static void second_buffers(mdg_system* sys, const SoloArgs& S, TeamRun& R, int eam) {
+    // the second buffers: the rebuild's spare position arrays and, for LJ, the
+    // offsets' second half (the EAM records)
+    R.I1 = S.I;
+    R.F1 = S.F;
+    R.T1 = R.T;
+    R.I1.rx = sys->f64[RX][sys->cur ^ 1];
+    R.I1.ry = sys->f64[RY][sys->cur ^ 1];
+    R.I1.rz = sys->f64[RZ][sys->cur ^ 1];
+    R.F1.rx = R.T1.rx = R.I1.rx;
+    R.F1.ry = R.I1.ry;
+    R.F1.rz = R.I1.rz;
+    if (!eam) R.F1.pos32 = R.I1.pos32 = sys->pos32 + sys->np;
+}
+
 int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam, int mixed, double pot_rcut,
                 int periodic, double dt, long steps, const double* hpos, const double* hvel, double* opos,
                 double* ovel, double* oforce) {
@@ -937,18 +1014,7 @@ int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam
         if (rc) return rc;
         S.F.cutbits = sys->cutbits;
     }
-    // the second buffers: the rebuild's spare position arrays and, for LJ, the
-    // offsets' second half (the EAM records)
-    R.I1 = S.I;
-    R.F1 = S.F;
-    R.T1 = R.T;
-    R.I1.rx = sys->f64[RX][sys->cur ^ 1];
-    R.I1.ry = sys->f64[RY][sys->cur ^ 1];
-    R.I1.rz = sys->f64[RZ][sys->cur ^ 1];
-    R.F1.rx = R.T1.rx = R.I1.rx;
-    R.F1.ry = R.I1.ry;
-    R.F1.rz = R.I1.rz;
-    if (!eam) R.F1.pos32 = R.I1.pos32 = sys->pos32 + sys->np;
+    second_buffers(sys, S, R, eam);
     R.left_dev = sys->dcounter;
     R.left_host = sys->hcounter;
     R.st_host = sys->hstat;
@@ -978,6 +1044,41 @@ int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam
     MDG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kTeamThreads), args, dyn, ctx->stream));
     MDG_LAUNCHED(ctx);
     return MDG_OK;
+}
+
+// Device scratch of a request's team: the barriers' word, the steps left and 8
+// words of bounds per block.
+size_t request_team_scratch(int blocks) { return (2 + 8 * (size_t)blocks) * sizeof(unsigned long long); }
+
+// What a system needs before its request's team (allocated on its stream).
+int request_team_prepare(mdg_system* sys, int eam) { return eam ? ensure_cutbits(sys) : MDG_OK; }
+
+// The request whose argument record (solo_fill) is `args`, by a team of up to
+// `blocks` blocks on `stream`; scratch: request_team_scratch(blocks), word 0
+// zero.
+int request_team_launch(const void* args, mdg_system* sys, int blocks, unsigned long long* scratch,
+                        cudaStream_t stream) {
+    SoloArgs S = *reinterpret_cast<const SoloArgs*>(args);
+    TeamRun R;
+    memset(&R, 0, sizeof(R));
+    R.T = thermo_args(sys);
+    if (S.any_eam) S.F.cutbits = sys->cutbits;
+    second_buffers(sys, S, R, S.any_eam);
+    R.word = scratch;
+    R.left_dev = scratch + 1;
+    S.part = reinterpret_cast<long long*>(scratch + 2);
+    R.per = std::max(8, ((S.n + blocks - 1) / blocks + 3) & ~3);
+    blocks = (S.n + R.per - 1) / R.per;
+    const void* fn = S.any_eam ? (const void*)k_team_request<true> : (const void*)k_team_request<false>;
+    const size_t dyn = solo_dyn_bytes(kTeamThreads);
+    MDG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    void* argv[2] = {&S, &R};
+    MDG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kTeamThreads), argv, dyn, stream));
+    return MDG_OK;
+}
+
+bool solo_out_started(const void* out_host, uint32_t seq) {
+    return reinterpret_cast<const SoloOut*>(out_host)->started == seq;
 }
 
 size_t solo_args_bytes() { return sizeof(SoloArgs); }
