@@ -2237,6 +2237,12 @@ static double* locked_view(const double* p) {
 // 120 / 109.
 constexpr size_t kTeamOneStep = 28000;
 
+// Up to this many atoms the team kernel reads and writes page-locked host
+// arrays itself: one launch, no copies (three steps of LJ argon, 19,652 atoms:
+// 114 us against 152 with copies; 37,044: 180 against 188; 42,592: 199 against
+// 197).
+constexpr size_t kTeamDirect = 44000;
+
 // Host arrays of a run whose transfers are the team kernel's own.
 struct TeamIo {
     const double *pos = nullptr, *vel = nullptr;
@@ -2710,14 +2716,11 @@ int mdg_run_host(mdg_solver* s, mdg_system* sys, double dt, long steps, double* 
         !(steps == 1 && sys->n >= kTeamOneStep && page_locked(pos) && page_locked(vel) && page_locked(force))) {
         MDG_CUDA(cudaSetDevice(sys->ctx->device));
         mark_stepped(s, sys, ps);
-        // page-locked arrays are read and written by the kernel itself: one
-        // launch, no copies (three steps of LJ argon, 19,652 atoms: 114 us
-        // against 152 with copies; 37,044: 180 against 188)
         TeamIo io;
         io.pos = io.opos = locked_view(pos);
         io.vel = io.ovel = locked_view(vel);
         io.oforce = locked_view(force);
-        const bool direct = io.pos && io.vel && (!force || io.oforce);
+        const bool direct = sys->n <= kTeamDirect && io.pos && io.vel && (!force || io.oforce);
         int rc = MDG_OK;
         bool done = false;
         if (!direct) {

@@ -491,7 +491,7 @@ int alive_blocks(mdg_server* sv, int* alive, int* free_gen) {
 // alive, each request gets a block and a
 // share of the other SMs in proportion to its atom-steps; a cooperative launch
 // makes its blocks resident together. 48 requests of 256 to 8,192 atoms, 100
-// steps: 54.1 ms by a block each, 20.1 ms.
+// steps: 54.1 ms by a block each, 15.6 ms.
 int team_of(const mdg_server* sv, const Request* r, double work, size_t outstanding, int taken) {
     const int most = (int)((r->atoms.size() + 7) / 8);
     const double share = work > 0.0 ? work_of(r) / work : 0.0;

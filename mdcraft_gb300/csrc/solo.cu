@@ -170,7 +170,7 @@ struct SoloShared {
 template <int NT>
 struct LaneShared {
     float part[NT / 32][96];  // lane_sums
-    float sum[3][NT / 8];
+    float sum[3][NT];  // of NT atoms at a time
 };
 
 // Reduces the bounds (BoundKeys) of the block's threads; `busy` false: the
@@ -616,6 +616,15 @@ constexpr int kTeamThreads = 768;
 // may lag by a barrier; the EAM force pass reads its neighbours only through
 // the density pass's copies and takes its cut decisions (k_force_step), so
 // the drift stays in place there. One barrier a step, two with EAM.
+//
+// The mixed passes take eight lanes per atom where a block has fewer than
+// kTeamLanesMost atoms, else one thread: its 768 threads hold 96 atoms by
+// lanes, and an atom's sum takes a thread about as long as three such rounds.
+// Per step, lanes / threads: LJ argon 19,652 atoms (132 a block) 20.0 / 24.1
+// us, 32,000 25.3 / 26.2, 48,668 34.2 / 31.7; EAM Cu 32,000 33.7 / 38.3, 48,668
+// 44.2 / 41.6.
+constexpr int kTeamLanesMost = 272;
+
 template <bool EAM, bool MIXED>
 constexpr bool kFlips = !(EAM && MIXED);
 
@@ -655,36 +664,62 @@ __device__ __forceinline__ bool team_step(Team<NT, true>& tm, const SoloArgs& S,
         }
         return need;
     }
-    // eight lanes per atom, NT / 8 atoms at a time; the sums meet in shared
-    // memory and the first warps finish them, a lane per atom
+    // the sums of up to NT atoms meet in shared memory, then a thread per atom
+    // finishes them (finishing 96 atoms at a time cost a wait for global memory
+    // and two barriers each: LJ argon 32,000 atoms 30.0 us a step against 25.3)
     const int sub = tm.t >> 3;
+    const bool few = R.per < kTeamLanesMost;
     if (EAM) {
-        for (int base = tm.a0; base < tm.a1; base += NT / 8) {
-            const int i = base + sub;
-            const bool in = i < tm.a1, live = in && F.tag[i] != 0;
-            float rho[1];
-            RhoGroup<0, true, false> grp(F, S.ps, in ? i : tm.a0);
-            lane_sums<1>(F, live, in ? i : tm.a0, live ? F.ncnt[i] >> 2 : 0, grp, sh.part[tm.w], rho);
-            if ((tm.t & 7) == 0) sh.sum[0][sub] = rho[0];
+        for (int base = tm.a0; base < tm.a1; base += NT) {
+            const int end = min(base + NT, tm.a1);
+            if (!few) {
+                const int i = base + tm.t;
+                float rho[1] = {0.f};
+                if (i < end && F.tag[i] != 0) {
+                    RhoGroup<0, true, false> grp(F, S.ps, i);
+                    group_sums<1>(F, i, F.ncnt[i] >> 2, grp, rho);
+                }
+                sh.sum[0][tm.t] = rho[0];
+            }
+            for (int k = 0; few && base + k + 4 * tm.w < end; k += NT / 8) {
+                const int i = base + k + sub;
+                const bool in = i < end, live = in && F.tag[i] != 0;
+                float rho[1];
+                RhoGroup<0, true, false> grp(F, S.ps, in ? i : tm.a0);
+                lane_sums<1>(F, live, in ? i : tm.a0, live ? F.ncnt[i] >> 2 : 0, grp, sh.part[tm.w], rho);
+                if (in && (tm.t & 7) == 0) sh.sum[0][k + sub] = rho[0];
+            }
             __syncthreads();
             const int me = base + tm.t;
-            if (tm.t < NT / 8 && me < tm.a1) store_density<false>(F, S.ps, me, F.pos32[me], 0, sh.sum[0][tm.t]);
+            if (me < end) store_density<false>(F, S.ps, me, F.pos32[me], 0, sh.sum[0][tm.t]);
             __syncthreads();
         }
         tm.sync();
         if (tm.dead) return false;
     }
-    for (int base = tm.a0; base < tm.a1; base += NT / 8) {
-        const int i = base + sub;
-        const bool in = i < tm.a1;
-        float f[3];
-        if (EAM) lane_forces<EamGroup<0, true, false>>(F, S.ps, in, in ? i : tm.a0, sh.part[tm.w], f);
-        else lane_forces<LjGroup<false, false>>(F, S.ps, in, in ? i : tm.a0, sh.part[tm.w], f);
-        if ((tm.t & 7) == 0)
-            for (int k = 0; k < 3; ++k) sh.sum[k][sub] = f[k];
+    for (int base = tm.a0; base < tm.a1; base += NT) {
+        const int end = min(base + NT, tm.a1);
+        if (!few) {
+            const int i = base + tm.t;
+            float f[3] = {0.f, 0.f, 0.f};
+            if (i < end) {
+                if (EAM) thread_forces<EamGroup<0, true, false>>(F, S.ps, i, f);
+                else thread_forces<LjGroup<false, false>>(F, S.ps, i, f);
+            }
+            for (int q = 0; q < 3; ++q) sh.sum[q][tm.t] = f[q];
+        }
+        for (int k = 0; few && base + k + 4 * tm.w < end; k += NT / 8) {
+            const int i = base + k + sub;
+            const bool in = i < end;
+            float f[3];
+            if (EAM) lane_forces<EamGroup<0, true, false>>(F, S.ps, in, in ? i : tm.a0, sh.part[tm.w], f);
+            else lane_forces<LjGroup<false, false>>(F, S.ps, in, in ? i : tm.a0, sh.part[tm.w], f);
+            if (in && (tm.t & 7) == 0)
+                for (int q = 0; q < 3; ++q) sh.sum[q][k + sub] = f[q];
+        }
         __syncthreads();
         const int me = base + tm.t;
-        if (tm.t < NT / 8 && me < tm.a1) {
+        if (me < end) {
             const bool live = F.tag[me] != 0;
             const float fx = sh.sum[0][tm.t], fy = sh.sum[1][tm.t], fz = sh.sum[2][tm.t];
             if (R.th) {
@@ -906,16 +941,15 @@ int solo_eligible(const mdg_solver* s, const mdg_system* sys) {
 // Dynamic shared memory of a launch: the list build's state, one per warp.
 static size_t solo_dyn_bytes(int threads) { return (size_t)(threads / 32) * sizeof(NbWarpSmem<kSoloChunks>); }
 
-// Systems (exclusive) whose runs go to a grid's team: below these sizes it
-// beats the graph. A block's 768 threads take 96 atoms at a time, so 152 SMs
-// take 29,184 atoms in two rounds and 43,776 in three. Per step, graph / team:
-// LJ argon mixed 4,000 atoms 20.3 / 12.7 us, 27,436 34.2 / 25.1, 32,000
-// 35.4 / 32.1, 42,592 38.2 / 36.4, 48,668 39.1 / 44.1; EAM Cu mixed 4,000
-// 24.2 / 17.4, 27,436 40.9 / 33.7, 32,000 41.8 / 42.6, 37,044 45.4 / 45.5; FP64
-// (to where 16 lanes per atom end) argon 500 26.4 / 19.2, 4,000 42.4 / 32.2,
-// 19,652 100.9 / 98.7; FP64 Cu 500 32.9 / 27.8, 4,000 62.0 / 51.2, 8,788
-// 98.7 / 96.8.
-constexpr size_t kTeamMostLj = 43776, kTeamMostEam = 30000;
+// Mixed systems (exclusive) whose runs go to a grid's team: as many atoms as
+// its threads on 152 SMs, below which it beats the graph. Per step, graph /
+// team: LJ argon 4,000 atoms 20.3 / 12.2 us, 32,000 33.5 / 25.3, 62,500
+// 38.2 / 33.4, 108,000 48.0 / 45.7, 143,748 55.5 / 65.1; EAM Cu 4,000
+// 24.2 / 16.0, 32,000 44.8 / 33.7, 62,500 50.5 / 43.4, 108,000 64.3 / 56.1,
+// 143,748 79.6 / 91.2. FP64, where 16 or 32 lanes share an atom
+// (some_atoms64): argon 500 26.4 / 19.2, 4,000 42.4 / 32.2, 19,652
+// 100.9 / 98.7; Cu 500 32.9 / 27.8, 4,000 62.0 / 51.1, 8,788 98.7 / 96.8.
+constexpr size_t kTeamMost = 152 * kTeamThreads;
 
 // What both teams need of a system.
 static void fill_system(SoloArgs& S, mdg_system* sys, const PotSet* dps, int any_eam, double pot_rcut, int periodic,
@@ -972,7 +1006,7 @@ bool team_eligible(const mdg_solver* s, const mdg_system* sys) {
     if (type != POT_LJCUT && type != POT_EAM) return false;
     if (!sys->cap_ready || sys->n < 1 || !sys->ctx->num_sms) return false;
     if (s->precision == MDG_PREC_FP64) return sys->n < some_atoms64(type == POT_EAM);
-    return sys->n < (type == POT_EAM ? kTeamMostEam : kTeamMostLj);
+    return sys->n < kTeamMost;
 }
 
 // Enqueues `steps` steps by a grid's team (any host arrays page-locked); the

@@ -73,22 +73,22 @@ def _same(*args, **kw):
     return ra
 
 
-@pytest.mark.parametrize("kind,n", [("lj", 43777), ("lj2", 24001)])
+@pytest.mark.parametrize("kind,n", [("lj", 116737), ("lj2", 24001)])
 @pytest.mark.parametrize("batches", [[1], [2], [3, 1, 2, 4]])
 def test_lj_step_counts(kind, n, batches):
     _same(kind, n, batches)
 
 
-@pytest.mark.parametrize("kind,n", [("lj", 43777), ("lj2", 30011)])
+@pytest.mark.parametrize("kind,n", [("lj", 116737), ("lj2", 30011)])
 def test_lj_rebuilds(kind, n):
     assert _same(kind, n, [9, 16], T=3000.0, skin=0.01) >= 8
 
 
 def test_lj_list_outgrown():
-    _same("lj", 43777, [40], squeeze=0.25, tag0=1 << 30)
+    _same("lj", 116737, [40], squeeze=0.25, tag0=1 << 30)
 
 
-@pytest.mark.parametrize("kind,n", [("eam", 30011), ("lj", 43777), ("lj2", 3001)])
+@pytest.mark.parametrize("kind,n", [("eam", 116737), ("lj", 116737), ("lj2", 3001)])
 @pytest.mark.parametrize("batches", [[1], [2, 3], [20]])
 def test_thermostat_steps(kind, n, batches):
     _same(kind, n, batches, thermo=[LANGEVIN, dict(LANGEVIN, seed=5, heat_y=0, xmin=0.3, xmax=1.9)], T=1500.0,

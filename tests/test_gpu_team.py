@@ -93,7 +93,7 @@ def test_step_counts(kind, batches, precision):
     _check(precision, batches, kind, 2048)
 
 
-@pytest.mark.parametrize("kind,n", [("lj", 29185), ("lj", 43775), ("lj", 43776), ("eam", 29999), ("eam", 30000)])
+@pytest.mark.parametrize("kind,n", [(k, n) for k in ("lj", "eam") for n in (40736, 40737, 116735, 116736)])
 def test_rule_edges_mixed(kind, n):
     _check("mixed", [6], kind, n)
 
@@ -196,7 +196,7 @@ def _pinned(x):
 
 
 @pytest.mark.parametrize("kind", ["lj", "eam"])
-@pytest.mark.parametrize("n,steps", [(500, 30), (16385, 30), (27999, 1), (28000, 1), (28000, 2)])
+@pytest.mark.parametrize("n,steps", [(500, 30), (16385, 30), (27999, 1), (28000, 1), (28000, 2), (44000, 2), (44001, 2)])
 @pytest.mark.parametrize("force", [False, True])
 def test_host_arrays(kind, n, steps, force):
     """Page-locked host arrays, which the kernel reads and writes itself (and
