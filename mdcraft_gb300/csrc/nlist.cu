@@ -406,9 +406,9 @@ __global__ void __launch_bounds__(kExportWarps * 32)
 // Block of NW warps (a system's launch shape, default 4), a warp per bin, on
 // grids without a periodic axis of 2 cells or fewer (GridParams::small_box;
 // those take k_nbuild_atoms, as do systems below kAtomBuildMost atoms).
-constexpr int kNbChunks = 8;
+constexpr int kNbChunks = 16;
 template <int NW>
-__global__ void __launch_bounds__(NW * 32, 32 / NW) k_nbuild_warp(NbArgs A, const GridParams* __restrict__ gp) {
+__global__ void __launch_bounds__(NW * 32, 28 / NW) k_nbuild_warp(NbArgs A, const GridParams* __restrict__ gp) {
     __shared__ GridParams g;
     __shared__ NbWarpSmem<kNbChunks> S[NW];
     if (threadIdx.x == 0) g = *gp;

@@ -657,14 +657,19 @@ __device__ __forceinline__ void nbuild_atom_cells(const NbArgs& A, const GridPar
 // runs.
 //
 // The build is bound by instruction issue, so a test is as few instructions
-// as it takes: the squared distance from the threshold mid as |b|^2 + (|a|^2 - mid) - 2 a.b, three
-// fused operations, two atoms at once in packed FP32 pairs; the rows go to
-// shared memory once per pair of atoms; and appending waits for CH chunks, as
-// the lanes' counts even out (the longest of 19 lanes then has 1.2 times the
-// mean instead of twice it). LJ liquid 500,000 atoms: 405 us with one
-// distance per atom and an append per chunk.
+// as it takes, five for 32 pairs: the squared distance from the threshold mid
+// as |b|^2 + (|a|^2 - mid) - 2 a.b, three fused operations, two atoms at once
+// in packed FP32 pairs, each atom pair read once for two candidates a lane; the
+// signs are shifted into a word per candidate, which the warp transposes once
+// per chunk to a word per atom (a ballot and a store per atom were four
+// instructions more). Appending waits for CH chunks, as the lanes' counts even
+// out, and takes two to four lanes per atom where the cell has no more than 16.
+// Rebuilds: LJ liquid 4,000,000 atoms 3.54 -> 2.77 ms, NiAl 1,018,880
+// 1.16 -> 0.98, EAM Cu 1,000,188 0.87 -> 0.76; with 8 and 24 chunks a turn and
+// 32, 28 and 24 warps an SM no pair was faster on all three than 16 and 28.
 template <int CH>
 struct NbWarpSmem {
+    static_assert(CH % 2 == 0, "chunks are tested two at a time");
     float4 csh[27];          // cell shift (x, y, z) of the image
     float4 oa[32];           // pairs of atoms: (-2ax0, -2ax1, -2ay0, -2ay1), (-2az0, -2az1, m0, m1), m = |a|^2 - mid
     uint32_t row[CH][32];    // accept rows of the turn's chunks: bit = candidate, column = atom
@@ -673,6 +678,21 @@ struct NbWarpSmem {
     uint32_t cpre[28];       // candidate prefix over those cells
     uint32_t ccode[27];      // image code << kJBits
 };
+
+// A 32 x 32 matrix of bits, lane l holding row l, transposed over the warp
+// (five exchanges of half blocks).
+__device__ __forceinline__ unsigned transpose32(unsigned x, int lane) {
+    unsigned keep = 0x0000ffffu;
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, k);
+        const bool low = (lane & k) == 0;
+        const unsigned mine = low ? keep : ~keep;
+        x = (x & mine) | (__funnelshift_l(y, y, low ? k : 32 - k) & ~mine);
+        keep ^= keep << (k >> 1);
+    }
+    return x;
+}
 
 template <int CH>
 __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridParams& g, int bin, int lane,
@@ -722,19 +742,22 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
     const float csm = fmaxf(g.csf[0], fmaxf(g.csf[1], g.csf[2]));
     const float mid = 0.5f * (lo2 + hi2), half_band = fmaf(6e-6f * csm, csm, 0.5f * (hi2 - lo2));
 
-    for (uint32_t base = s0; base < s1; base += 32) {
-        const uint32_t ni = s1 - base < 32u ? s1 - base : 32u;
+    // batches of up to 32 atoms, all of nearly the same size
+    const uint32_t batches = (s1 - s0 + 31) >> 5, per = (s1 - s0 + batches - 1) / batches;
+    for (uint32_t base = s0; base < s1; base += per) {
+        const uint32_t ni = s1 - base < per ? s1 - base : per;
         const bool act = (uint32_t)lane < ni;
         const uint32_t me = base + lane;
         float4 oa = make_float4(0.f, 0.f, 0.f, 0.f);
         if (act) {
             oa = A.o0[me];
         }
-        // an atom whose offset is not exact takes the batch to the exact tests
-        const bool rough = __any_sync(full, oa.w != 0.0f) || !uniform_rns || A.half;
+        const float a2 = fmaf(oa.x, oa.x, fmaf(oa.y, oa.y, oa.z * oa.z));
+        // an atom whose offset is not exact (or not a number) takes the batch
+        // to the exact tests
+        const bool rough = __any_sync(full, oa.w != 0.0f || !(a2 < 1e30f)) || !uniform_rns || A.half;
         {
             // columns past the batch (the second of an odd pair) accept nothing
-            const float a2 = fmaf(oa.x, oa.x, fmaf(oa.y, oa.y, oa.z * oa.z));
             const float m = act ? a2 - mid : 3e38f;
             float* q = reinterpret_cast<float*>(&S.oa[lane & ~1]) + (lane & 1);
             q[0] = -2.0f * oa.x;
@@ -744,63 +767,108 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
         }
         // this atom's own candidate index (it is a candidate of its own cell)
         const uint32_t self_t = act ? S.cpre[home] + (me - s0) : 0xffffffffu;
+        // appending: `lanes` lanes take an atom's chunks in as many parts
+        const int lanes = ni <= 8 ? 4 : ni <= 10 ? 3 : ni <= 16 ? 2 : 1;
+        const int ea = lane / lanes, part = lane - ea * lanes;
+        const bool appends = (uint32_t)ea < ni;
+        const uint32_t mine_e = base + ea;
         __syncwarp();
-        int cnt = 0;  // list length of atom `me`
+        int cnt = 0;  // list length of atom mine_e
         int c = 0;    // neighbour cell of this lane's candidate
-        uint32_t* dst = A.nbr + ((size_t)me << 2);
-        // the lane's candidate of the next chunk, fetched a chunk ahead
-        uint32_t jn = 0;
-        float4 on = make_float4(0.f, 0.f, 0.f, 0.f), shn = on;
-        uint32_t en = 0;
+        // the lane's candidates of the next two chunks, fetched ahead
+        uint32_t jn[2] = {0, 0};
+        int cn[2] = {0, 0};
+        float4 on[2];
+        on[0] = on[1] = make_float4(0.f, 0.f, 0.f, 0.f);
         auto fetch = [&](uint32_t t) {
-            if (t >= T) return;
-            while (S.cpre[c + 1] <= t) ++c;
-            jn = S.cj0[c] + (t - S.cpre[c]);
-            on = A.o0[jn];
-            shn = S.csh[c];
-            en = jn | S.ccode[c];
+#pragma unroll
+            for (int h = 0; h < 2; ++h, t += 32) {
+                if (t >= T) return;
+                while (S.cpre[c + 1] <= t) ++c;
+                cn[h] = c;
+                jn[h] = S.cj0[c] + (t - S.cpre[c]);
+                on[h] = A.o0[jn[h]];
+            }
         };
         fetch(lane);
         for (uint32_t t0 = 0; t0 < T; t0 += CH * 32) {
             const int nch = min((int)((T - t0 + 31) >> 5), CH);
-            for (int ch = 0; ch < nch; ++ch) {
-                const uint32_t t = t0 + 32 * ch + lane;
-                const bool have = t < T;
-                const uint32_t j = jn;
-                // the candidate seen from the cell: offset + image shift
-                const float px = have ? on.x + shn.x : 0.f, py = have ? on.y + shn.y : 0.f, pz = have ? on.z + shn.z : 0.f;
-                const bool pfj = on.w == 0.0f;
-                S.cand[32 * ch + lane] = en;
-                fetch(t + 32);
-                bool exact = rough || __any_sync(full, have && !pfj);
-                if (!exact) {
-                    const float b2 = have ? fmaf(px, px, fmaf(py, py, pz * pz)) : 3e38f;
-                    const unsigned long long bx = pack2(px, px), by = pack2(py, py), bz = pack2(pz, pz),
-                                             bb = pack2(b2, b2);
-                    float near = 3e38f;  // least distance from the threshold
-                    for (uint32_t ii = 0; ii < ni; ii += 2) {
+            for (int ch = 0; ch < nch; ch += 2) {
+                bool have[2], rest = false;
+                uint32_t j[2];
+                float px[2], py[2], pz[2], pw[2], b2[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t t = t0 + 32 * (ch + h) + lane;
+                    have[h] = t < T;
+                    j[h] = jn[h];
+                    // the candidate seen from the cell: offset + image shift
+                    const float4 sh = S.csh[cn[h]];
+                    px[h] = have[h] ? on[h].x + sh.x : 0.f;
+                    py[h] = have[h] ? on[h].y + sh.y : 0.f;
+                    pz[h] = have[h] ? on[h].z + sh.z : 0.f;
+                    pw[h] = on[h].w;
+                    S.cand[32 * (ch + h) + lane] = jn[h] | S.ccode[cn[h]];
+                    b2[h] = fmaf(px[h], px[h], fmaf(py[h], py[h], pz[h] * pz[h]));
+                    rest = rest || (have[h] && (pw[h] != 0.0f || !(b2[h] < 1e30f)));
+                }
+                fetch(t0 + 32 * ch + 64 + lane);
+                bool exact[2];
+                exact[0] = exact[1] = rough || __any_sync(full, rest);
+                if (!exact[0]) {
+                    // a lane tests its two candidates against two atoms at a
+                    // time; the signs go to a bit per atom
+                    unsigned long long bx[2], by[2], bz[2], bb[2];
+                    float near[2];      // least distance from the threshold
+                    unsigned col[2];    // accepting atoms
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float q = have[h] ? b2[h] : 3e38f;
+                        bx[h] = pack2(px[h], px[h]);
+                        by[h] = pack2(py[h], py[h]);
+                        bz[h] = pack2(pz[h], pz[h]);
+                        bb[h] = pack2(q, q);
+                        near[h] = 3e38f;
+                        col[h] = 0;
+                    }
+                    for (int ii = (int)(ni - 1) & ~1; ii >= 0; ii -= 2) {
                         const ulonglong2 u = reinterpret_cast<const ulonglong2*>(S.oa)[ii];
                         const ulonglong2 v = reinterpret_cast<const ulonglong2*>(S.oa)[ii + 1];
-                        float d0, d1;
-                        unpack2(fma2(u.x, bx, fma2(u.y, by, fma2(v.x, bz, add2(bb, v.y)))), d0, d1);
-                        const unsigned m0 = __ballot_sync(full, d0 < 0.0f), m1 = __ballot_sync(full, d1 < 0.0f);
-                        near = fminf(near, fminf(fabsf(d0), fabsf(d1)));
-                        if (lane == 0) *reinterpret_cast<uint2*>(&S.row[ch][ii]) = make_uint2(m0, m1);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            float d0, d1;
+                            unpack2(fma2(u.x, bx[h], fma2(u.y, by[h], fma2(v.x, bz[h], add2(bb[h], v.y)))), d0, d1);
+                            near[h] = fminf(near[h], fminf(fabsf(d0), fabsf(d1)));
+                            col[h] = __funnelshift_l(__float_as_uint(d1), col[h], 1);
+                            col[h] = __funnelshift_l(__float_as_uint(d0), col[h], 1);
+                        }
                     }
-                    exact = __any_sync(full, near <= half_band);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        exact[h] = __any_sync(full, near[h] <= half_band);
+                        if (exact[h]) continue;
+                        // a bit per atom and lane becomes a bit per lane and
+                        // atom; without the atom itself
+                        unsigned row = transpose32(col[h], lane);
+                        const uint32_t own = self_t - (t0 + 32 * (ch + h));
+                        if (own < 32u) row &= ~(1u << own);
+                        S.row[ch + h][lane] = row;
+                    }
                 }
-                if (exact) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (!exact[h]) continue;
                     // pairs within 1e-5 of rns (or of atoms whose offsets are
                     // not exact) are marked in a second row and settled in FP64
                     __syncwarp();
                     unsigned mine = 0, mine_x = 0;
-                    const uint32_t origj = A.half && have ? A.orig[j] : 0u;
+                    const uint32_t origj = A.half && have[h] ? A.orig[j[h]] : 0u;
                     for (uint32_t ii = 0; ii < ni; ++ii) {
                         const float4 oi = A.o0[base + ii];
-                        const float dx = oi.x - px, dy = oi.y - py, dz = oi.z - pz;
+                        const float dx = oi.x - px[h], dy = oi.y - py[h], dz = oi.z - pz[h];
                         const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        const bool pf = uniform_rns && pfj && oi.w == 0.0f;
-                        const bool ok = have && j != base + ii && !(A.half && origj < A.orig[base + ii]);
+                        const bool pf = uniform_rns && pw[h] == 0.0f && oi.w == 0.0f;
+                        const bool ok = have[h] && j[h] != base + ii && !(A.half && origj < A.orig[base + ii]);
                         const unsigned m = __ballot_sync(full, ok && pf && d2 < lo2);
                         const unsigned mx = __ballot_sync(full, ok && !(pf && (d2 < lo2 || d2 > hi2)));
                         if ((uint32_t)lane == ii) {
@@ -811,42 +879,57 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
                     while (mine_x) {
                         const int b = __ffs(mine_x) - 1;
                         mine_x &= mine_x - 1u;
-                        const uint32_t jb = S.cand[32 * ch + b] & kJMask;
+                        const uint32_t jb = S.cand[32 * (ch + h) + b] & kJMask;
                         if (are_neibs_exact(g, A.rx[me], A.ry[me], A.rz[me], A.rns[me], A.rx[jb], A.ry[jb], A.rz[jb],
                                             A.rns[jb], edge))
                             mine |= 1u << b;
                     }
-                    if (act) S.row[ch][lane] = mine;
+                    S.row[ch + h][lane] = mine;
                 }
             }
             __syncwarp();
-            // append this atom's accepted candidates in candidate order
-            if (act) {
-                unsigned w = 0;
-                for (int ch = 0;;) {
-                    while (w == 0 && ch < nch) {
-                        w = S.row[ch][lane];
-                        if (self_t - (t0 + 32 * ch) < 32u) w &= ~(1u << (self_t & 31u));
-                        ++ch;
+            // append the accepted candidates in candidate order
+            if (appends) {
+                int ch = 0, end = nch, at = cnt;
+                if (lanes > 1) {
+                    // this part's chunks, and the entries before and after them
+                    const int from = nch * part / lanes;
+                    end = nch * (part + 1) / lanes;
+                    int all = 0;
+                    for (int q = 0; q < nch; ++q) {
+                        const int k = __popc(S.row[q][ea]);
+                        all += k;
+                        at += q < from ? k : 0;
                     }
+                    cnt += all;
+                    ch = from;
+                }
+                uint32_t* dst = A.nbr + nidx(at, mine_e, A.np);
+                unsigned w = 0;
+                for (;;) {
+                    while (w == 0 && ch < end) w = S.row[ch++][ea];
                     if (w == 0) break;
                     const int b = __ffs(w) - 1;
                     w &= w - 1u;
-                    if (cnt < A.K) *dst = S.cand[32 * (ch - 1) + b];
-                    ++cnt;
-                    dst += (cnt & 3) ? 1 : 4 * (size_t)A.np - 3;
+                    if (at < A.K) *dst = S.cand[32 * (ch - 1) + b];
+                    ++at;
+                    dst += (at & 3) ? 1 : 4 * (size_t)A.np - 3;
                 }
+                if (lanes == 1) cnt = at;
             }
             __syncwarp();
         }
-        if (act) {
+        if (appends && part == 0) {
+            const uint32_t at = mine_e;
             const int padded = (cnt + 3) & ~3;
-            for (int k = cnt; k < padded && k < A.K; ++k) A.nbr[nidx(k, me, A.np)] = me | kSelfCode;
-            A.ncnt[me] = padded < A.K ? padded : A.K;
+            for (int k = cnt; k < padded && k < A.K; ++k) A.nbr[nidx(k, at, A.np)] = at | kSelfCode;
+            A.ncnt[at] = padded < A.K ? padded : A.K;
             if (cnt > A.K) {
                 atomicOr(&A.st->flags, FLAG_OVERFLOW);
                 atomicOr(&A.st->build_flags, FLAG_OVERFLOW);
             }
+        }
+        if (act) {
             A.r0x[me] = A.rx[me];
             A.r0y[me] = A.ry[me];
             A.r0z[me] = A.rz[me];
@@ -855,7 +938,7 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
             A.saved_uid[me] = A.uid[me];
         }
         // the longest list, one atomic per warp
-        const unsigned wmax = __reduce_max_sync(full, act ? (unsigned)cnt : 0u);
+        const unsigned wmax = __reduce_max_sync(full, appends ? (unsigned)cnt : 0u);
         if (lane == 0) atomicMax(&A.st->max_count, wmax);
         __syncwarp();
     }
