@@ -324,7 +324,6 @@ int request_team_prepare(mdg_system* sys, int eam);
 int request_team_launch(const void* args, mdg_system* sys, int blocks, unsigned long long* scratch,
                         cudaStream_t stream);
 bool solo_out_started(const void* out_host, uint32_t seq);
-int solo_eligible(const mdg_solver* s, const mdg_system* sys);
 size_t solo_args_bytes();
 size_t solo_out_bytes();
 // Fills the argument record at `args` (host-mapped) of a fresh system's

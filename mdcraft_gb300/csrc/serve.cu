@@ -257,7 +257,9 @@ void fail(mdg_server* sv, Slot& sl, int rc) {
 bool block_mode(const mdg_server* sv, const Request* r) {
     if (sv->block_threads < 0) return false;
     const mdg_solver* s = r->solver;
-    return r->precision == MDG_PREC_MIXED && !s->multi && s->nstages >= 1 && r->atoms.size() <= 65536 &&
+    // the fused loops carry the LJsCut and EAM bodies only, and no thermostat
+    return r->precision == MDG_PREC_MIXED && !s->multi && s->nstages >= 1 && !s->thermo && s->pot[0][0] &&
+           (s->pot[0][0]->type == POT_LJCUT || s->pot[0][0]->type == POT_EAM) && r->atoms.size() <= 65536 &&
            r->atoms.size() > 0;
 }
 

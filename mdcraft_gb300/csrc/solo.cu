@@ -12,7 +12,7 @@
 //      list build) -> next step.
 // Every pass calls the same per-atom (or per-bin) device code as the
 // per-stage kernels, in the same order, so a system gives the same bits
-// here as through the graph of mdg_run. Two teams:
+// here as through the graph of mdg_run. Three teams:
 //
 //  - one block (the serving loop): a persistent kernel's block takes a whole
 //    request from a queue; many systems run at once, a block each, and no
@@ -20,6 +20,8 @@
 //  - a grid of one block per SM, launched cooperatively (mdg_run and
 //    mdg_run_host of a small system): the blocks share the system's atoms and
 //    meet at barriers in global memory. Every wait is bounded.
+//  - the same with a share of the SMs, for a whole request (the server, while
+//    few requests are outstanding).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -928,14 +930,6 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             S.out->done = S.seq;
         }
     }
-}
-
-int solo_eligible(const mdg_solver* s, const mdg_system* sys) {
-    if (s->precision != MDG_PREC_MIXED || s->multi || s->nstages < 1 || s->thermo) return 0;
-    // the fused loop carries the LJsCut and EAM bodies only
-    if (!s->pot[0][0] || (s->pot[0][0]->type != POT_LJCUT && s->pot[0][0]->type != POT_EAM)) return 0;
-    if (sys->n == 0 || sys->n > (size_t)kSoloMaxAtoms || sys->half || !sys->cap_ready || sys->ctx->timing) return 0;
-    return 1;
 }
 
 // Dynamic shared memory of a launch: the list build's state, one per warp.

@@ -88,3 +88,36 @@ def test_list_outgrown():
     (b, rb), = _serve(reqs, 512, 40)
     assert ra == rb
     assert a.tobytes() == b.tobytes()
+
+
+def test_thermostat_and_tabulated_pair_take_the_graph():
+    """Requests that the fused loops do not carry give the plain API's bits."""
+    from tests import gpu_helpers as H
+    atoms, box, _, p = W.lj_argon_fcc(ncell=5, jitter=0.01)
+    dom = mdg.Domain(*box)
+    for k in range(3):
+        dom.set_periodic(k, True)
+    r = np.linspace(0.0, 1.1 * p["rcut"], 2001)
+    table = r * np.exp(-r / 0.2)
+    pots = [mdg.LJsCut(p["a"], p["s"], p["rcut"]), mdg.Pair(p["rcut"], table, len(r) - 1, r[1])]
+    for pot, thermo in ((pots[0], True), (pots[1], False)):
+        sol = mdg.Single(pot, periodic=True, precision="mixed")
+        if thermo:
+            th = mdg.Langevin(2.0, 300.0, p["dt"], seed=9)
+            sol.set_thermostat(th)
+        server = mdg.Server(slots=4, max_atoms=1024)
+        rid = server.submit(sol, dom, atoms, p["dt"], 20)
+        server.wait(rid, 60.0)
+        got, info = server.result(rid)
+        assert info["status"] == 0
+        server.close()
+        s = mdg.System(H.ctx(), dom, atoms)
+        mdg.VerletList(s).update(-1.0)
+        sol.prepare(s)
+        sol.stages(s)
+        # the request's initial forces count as a thermostat call, as here
+        mdg.Verlet(sol).run(s, p["dt"], 20)
+        want = s.download()
+        for f in ("r", "v"):
+            assert np.array_equal(got[f], want[f]), f
+        s.close()
