@@ -477,13 +477,16 @@ __global__ void __launch_bounds__(kBlock, lane_budget(KINDS))
 }
 
 // Whether a system's mixed passes take eight lanes per atom: below 45,000
-// atoms with EAM tables, 24,000 without (a pair costs less there). One thread
-// per atom leaves the GPU with fewer than nine warps per SM at 45,000 atoms;
-// eight lanes cost about twice the instructions where it is full. Measured per
-// step, one thread / eight lanes: EAM Cu 4,000 atoms 51.3 / 26.8 us, 32,000
-// 51.4 / 43.3, 62,500 54.9 / 68.9; NiAl 31,094 114 / 79; LJ argon 4,000
-// 36.5 / 26.9, 32,000 41.3 / 41.1; LJ liquid 62,500 54.3 / 61.9.
-static bool lanes_mixed(size_t n, const PotSet& ps) { return n < (ps.any_eam ? 45000u : 24000u); }
+// atoms with several EAM tables, 30,000 with one, 24,000 without (a pair costs
+// less there). One thread per atom leaves the GPU with fewer than nine warps
+// per SM at 45,000 atoms; eight lanes cost about twice the instructions where
+// it is full. Measured per step, one thread / eight lanes: EAM Cu 4,000 atoms
+// 37.9 / 22.0 us, 32,000 39.9 / 41.1, 62,500 46.2 / 64.9; NiAl 31,094
+// 92 / 75; LJ argon 4,000 25.6 / 20.6, 32,000 29.2 / 32.4; LJ liquid 62,500
+// 37.1 / 48.9.
+static bool lanes_mixed(size_t n, const PotSet& ps) {
+    return n < (!ps.any_eam ? 24000u : ps.multi ? 45000u : 30000u);
+}
 static int lane_blocks(size_t n) { return (int)((n + kLaneAtoms - 1) / kLaneAtoms); }
 
 // ---- Langevin thermostat (thermo_dev.cuh) -------------------------------------

@@ -298,7 +298,7 @@ __device__ __forceinline__ void group_sums(const FArgs& A, int i, int ng, Group&
 // evaluates groups l, l + 8, ...; after each round of eight groups lane k adds
 // the eight sums of component k in group order (through sh, 32 NC floats per
 // warp). Every lane of the warp calls this; out is the atom's sums, on all
-// eight lanes. A group's sums take about 120 instructions and the ordered
+// eight lanes. A group's sums take about 100 instructions and the ordered
 // additions 4 a group and component, so the eight lanes run about six times
 // as fast as one where the GPU is not full.
 template <int NC, typename Group>

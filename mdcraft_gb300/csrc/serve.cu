@@ -9,20 +9,22 @@
 // run a request:
 //
 // Block mode (mixed precision, one kind, up to 65536 atoms): the request's
-// whole run, set-up included, is one thread block of a persistent kernel
-// (solo.cu). The host allocates the system's buffers (stream-ordered, from
-// the server's pool), sizes its capacities from the atoms and fills the
-// block's argument record in host-mapped memory; once the allocations have
-// passed it publishes the record in a queue. Blocks of the persistent kernel
-// claim queue entries as they finish their previous request, so requests
-// that arrive while others run start as soon as a block is free. Each
-// block writes its result atoms and a completion record into host-mapped
-// memory; the host polls those and never waits for the device. Idle blocks
-// exit after a bounded wait; the host tops the kernel up with a further
-// launch (up to kSoloGens in flight) whenever fewer blocks are alive than
-// the GPU holds and requests wait. Each launch slot's kernel is captured
-// once into a CUDA graph; a top-up sets that graph's grid to the blocks
-// missing and launches it.
+// whole run, set-up included, is in one kernel (solo.cu). The host allocates
+// the system's buffers (stream-ordered, from the server's pool), sizes its
+// capacities from the atoms and fills an argument record in host-mapped
+// memory; the kernel writes the result atoms and a completion record into
+// host-mapped memory; the host polls those and never waits for the device.
+// With many requests outstanding each is one thread block of a persistent
+// kernel: the host publishes the record in a queue once its allocations have
+// passed, and blocks claim entries as they finish their previous request, so
+// requests that arrive while others run start as soon as a block is free.
+// Idle blocks exit after a bounded wait, at once where nothing runs; the host
+// tops the kernel up with a further launch (up to kSoloGens in flight)
+// whenever fewer blocks are alive than the GPU holds and requests wait. Each
+// launch slot's kernel is captured once into a CUDA graph; a top-up sets that
+// graph's grid to the blocks missing and launches it. With few requests
+// outstanding each is a cooperative launch of its own, a team of blocks
+// (team_of).
 //
 // Graph mode (everything else, or when block mode is off): the request's
 // system gets the slot's own stream; set-up and the loop (one graph launch)
@@ -774,10 +776,10 @@ int mdg_server_create(int device, const mdg_server_config* cfg, mdg_server** out
             if (e != cudaSuccess) rc = cuda_status(e, "server queue");
         }
         // persistent kernel: block size, and as many blocks as fit on the GPU
-        // 768 threads (one block per SM, 80 registers) measured fastest on the
-        // serving mix: 2.04-2.08e9 atom-steps/s against 2.06e9 with 896,
-        // 2.00e9 with 640, 1.84e9 with 1024 (64 registers, twice the spills)
-        sv->threads = cfg->block_threads > 0 ? cfg->block_threads : 768;
+        // 640 threads (one block per SM) measured fastest on the serving mix:
+        // 2.49e9 atom-steps/s on a sample of it, against 2.41e9 with 768, 2.25e9
+        // with 896, 2.16e9 with 512, 2.05e9 with 1024 (64 registers, more spills)
+        sv->threads = cfg->block_threads > 0 ? cfg->block_threads : 640;
         int per_sm = 0;
         if (rc == MDG_OK) rc = solo_blocks_per_sm(sv->threads, &per_sm);
         if (rc != MDG_OK) {

@@ -67,7 +67,7 @@ def test_rule_edge_lj(n):
     _check(atoms[:n].copy(), box, _lj(p))
 
 
-@pytest.mark.parametrize("n", [44999, 45000])
+@pytest.mark.parametrize("n", [29999, 30000, 44999, 45000])
 def test_rule_edge_eam(n):
     atoms, box, _, p = W.eam_cu_fcc(ncell=23)
     _check(atoms[:n].copy(), box, _eam(p))
