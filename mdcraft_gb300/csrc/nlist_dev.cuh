@@ -316,6 +316,23 @@ __device__ __forceinline__ void permute_one(const GatherAll& G, uint32_t i, uint
     for (int f = 0; f < 2; ++f) G.h.out[f][d] = G.h.in[f][i];
 }
 
+// The same by eight threads, `part` 0 .. 7 of them.
+__device__ __forceinline__ void permute_part(const GatherAll& G, uint32_t i, uint32_t d, int part) {
+    const bool more = part < 4;
+    const double a = G.a.in[part][i], b = G.b.in[part][i];
+    const double a8 = more ? G.a.in[part + 8][i] : 0.0, b8 = more ? G.b.in[part + 8][i] : 0.0;
+    const float f = part < 3 ? G.fc.in[part][i] : 0.f;
+    const uint32_t u = part == 3 || part == 4 ? G.u.in[part - 3][i] : 0u;
+    const uint16_t h = part == 5 || part == 6 ? G.h.in[part - 5][i] : (uint16_t)0;
+    G.a.out[part][d] = a;
+    G.b.out[part][d] = b;
+    if (more) G.a.out[part + 8][d] = a8;
+    if (more) G.b.out[part + 8][d] = b8;
+    if (part < 3) G.fc.out[part][d] = f;
+    if (part == 3 || part == 4) G.u.out[part - 3][d] = u;
+    if (part == 5 || part == 6) G.h.out[part - 5][d] = h;
+}
+
 struct CellOut {
     uint32_t* cellp;
     double *Rx, *Ry, *Rz;
@@ -349,6 +366,37 @@ __device__ __forceinline__ void settle_one(const GridParams& g, const GatherAll&
     const double r[3] = {x[RX], x[RY], x[RZ]};
     cells_one(g, k, r, cell, orig, kind, C.cellp, C.Rx, C.Ry, C.Rz, C.pos32, C.q0, C.o0, C.slot_of);
     C.trig[k] = trig_of(x[RNS], x[RCUT], g);
+}
+
+// The same by eight threads.
+__device__ __forceinline__ void settle_part(const GridParams& g, const GatherAll& G, int k, uint32_t cell,
+                                            const CellOut& C, int part) {
+    const bool more = part < 4, last = part == 7;
+    const double a = G.a2.in[part][k], b = G.b2.in[part][k];
+    const double a8 = more ? G.a2.in[part + 8][k] : 0.0, b8 = more ? G.b2.in[part + 8][k] : 0.0;
+    const float f = part < 3 ? G.fc2.in[part][k] : 0.f;
+    const uint32_t u = part == 3 || part == 4 ? G.u2.in[part - 3][k] : 0u;
+    const uint16_t h = part == 5 || part == 6 ? G.h2.in[part - 5][k] : (uint16_t)0;
+    double r[3] = {0.0, 0.0, 0.0}, rns = 0.0, rcut = 0.0;
+    uint32_t orig = 0;
+    uint16_t kind = 0;
+    if (last) {
+        for (int q = 0; q < 3; ++q) r[q] = G.a2.in[RX + q][k];
+        rns = G.a2.in[RNS][k];
+        rcut = G.a2.in[RCUT][k];
+        orig = G.u2.in[0][k];
+        kind = G.h2.in[0][k];
+    }
+    G.a2.out[part][k] = a;
+    G.b2.out[part][k] = b;
+    if (more) G.a2.out[part + 8][k] = a8;
+    if (more) G.b2.out[part + 8][k] = b8;
+    if (part < 3) G.fc2.out[part][k] = f;
+    if (part == 3 || part == 4) G.u2.out[part - 3][k] = u;
+    if (part == 5 || part == 6) G.h2.out[part - 5][k] = h;
+    if (!last) return;
+    cells_one(g, k, r, cell, orig, kind, C.cellp, C.Rx, C.Ry, C.Rz, C.pos32, C.q0, C.o0, C.slot_of);
+    C.trig[k] = trig_of(rns, rcut, g);
 }
 
 // Systems (exclusive) whose lists are built by a warp per atom on every grid
@@ -696,12 +744,14 @@ __device__ __forceinline__ unsigned transpose32(unsigned x, int lane) {
 
 template <int CH>
 __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridParams& g, int bin, int lane,
-                                                 bool uniform_rns, NbWarpSmem<CH>& S) {
+                                                 bool uniform_rns, NbWarpSmem<CH>& S, int part = 0, int parts = 1) {
     const unsigned full = 0xffffffffu;
     const float lo2 = (float)(g.max_rns * g.max_rns * (1.0 - 1e-5));
     const float hi2 = (float)(g.max_rns * g.max_rns * (1.0 + 1e-5));
     const uint32_t s0 = A.bin_start[bin], s1 = A.bin_start[bin + 1];
-    if (s0 == s1) return;
+    // this part's atoms of the cell
+    const uint32_t share = (s1 - s0 + parts - 1) / parts, e0 = s0 + share * part, e1 = min(e0 + share, s1);
+    if (e0 >= s1) return;
     int cx, cy, cz;
     unpack_cell(A.cellp[s0], cx, cy, cz);
     int gc[3] = {cx + g.offset[0], cy + g.offset[1], cz + g.offset[2]};
@@ -743,9 +793,9 @@ __device__ __forceinline__ void nbuild_cell_warp(const NbArgs& A, const GridPara
     const float mid = 0.5f * (lo2 + hi2), half_band = fmaf(6e-6f * csm, csm, 0.5f * (hi2 - lo2));
 
     // batches of up to 32 atoms, all of nearly the same size
-    const uint32_t batches = (s1 - s0 + 31) >> 5, per = (s1 - s0 + batches - 1) / batches;
-    for (uint32_t base = s0; base < s1; base += per) {
-        const uint32_t ni = s1 - base < per ? s1 - base : per;
+    const uint32_t batches = (e1 - e0 + 31) >> 5, per = (e1 - e0 + batches - 1) / batches;
+    for (uint32_t base = e0; base < e1; base += per) {
+        const uint32_t ni = e1 - base < per ? e1 - base : per;
         const bool act = (uint32_t)lane < ni;
         const uint32_t me = base + lane;
         float4 oa = make_float4(0.f, 0.f, 0.f, 0.f);

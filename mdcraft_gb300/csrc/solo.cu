@@ -87,6 +87,10 @@ constexpr int kSoloMaxAtoms = 65536;
 // Chunks per turn of the list build here: few, as its shared memory is taken
 // from the L1 that the force passes gather through.
 constexpr int kSoloChunks = 2;
+// A grid's team: of few atoms a block, so more chunks (8 against 2 in LJ argon
+// 13,500 atoms 16.2 -> 15.6 us a step; 16 take L1 from EAM: Cu 87,808 atoms
+// 50.1 -> 53.0).
+constexpr int kTeamParts = 4, kTeamChunks = 8;
 
 // Polls (each an L2 round trip) after which a team's barrier gives up: ten
 // seconds or more, against rebuild phases of microseconds.
@@ -298,7 +302,21 @@ __device__ __noinline__ bool solo_rebuild(Team<NT, WIDE>& tm, const SoloArgs& S,
     }
     tm.sync();
     if (tm.dead) return false;
-    for (int k = tm.a0 + t; k < tm.a1; k += NT) {
+    // (a wide team's blocks have few atoms: eight threads share an atom's 31
+    // fields, whose loads and stores are otherwise one thread's chain)
+    const bool eight = WIDE && tm.a1 - tm.a0 <= 2 * (NT / 8);
+    for (int base = tm.a0; eight && base < tm.a1; base += NT / 8) {
+        const int k = base + (t >> 3), part = t & 7;
+        const bool in = k < tm.a1;
+        const uint32_t i = in ? S.src[k] : 0u;
+        uint32_t d = 0;
+        if (in && part == 0) d = sorted_slot((uint32_t)k, S.key[i], S.bin_start, S.C.cellp);
+        d = __shfl_sync(0xffffffffu, d, tm.lane & ~7);
+        if (!in) continue;
+        permute_part(S.G, i, d, part);
+        if (part == 7) S.rank[d] = S.N.ncnt[i];
+    }
+    for (int k = tm.a0 + t; !eight && k < tm.a1; k += NT) {
         const uint32_t i = S.src[k];
         const uint32_t d = sorted_slot((uint32_t)k, S.key[i], S.bin_start, S.C.cellp);
         permute_one(S.G, i, d);
@@ -306,7 +324,11 @@ __device__ __noinline__ bool solo_rebuild(Team<NT, WIDE>& tm, const SoloArgs& S,
     }
     tm.sync();
     if (tm.dead) return false;
-    for (int k = tm.a0 + t; k < tm.a1; k += NT) settle_one(g, S.G, k, S.rank[k], S.C);
+    for (int base = tm.a0; eight && base < tm.a1; base += NT / 8) {
+        const int k = base + (t >> 3);
+        if (k < tm.a1) settle_part(g, S.G, k, S.rank[k], S.C, t & 7);
+    }
+    for (int k = tm.a0 + t; !eight && k < tm.a1; k += NT) settle_one(g, S.G, k, S.rank[k], S.C);
     tm.sync();
     if (tm.dead) return false;
     {
@@ -318,9 +340,15 @@ __device__ __noinline__ bool solo_rebuild(Team<NT, WIDE>& tm, const SoloArgs& S,
             // build's body); its per-warp state is the launch's dynamic
             // shared memory
             extern __shared__ __align__(16) unsigned char solo_dyn[];
-            NbWarpSmem<kSoloChunks>* nbs = reinterpret_cast<NbWarpSmem<kSoloChunks>*>(solo_dyn);
-            for (int b = tm.gw; b < nb; b += tm.nw)
-                nbuild_cell_warp(S.N, g, b, tm.lane, uniform, nbs[tm.w]);
+            using State = NbWarpSmem<WIDE ? kTeamChunks : kSoloChunks>;
+            State* nbs = reinterpret_cast<State*>(solo_dyn);
+            // up to four warps share a cell where there are more warps than
+            // cells (LJ argon 13,500 atoms, a rebuild every 15 steps: 17.2 us a
+            // step by one, 15.6 by four; EAM Cu 32,000: 34.0 by one, 34.4 by two)
+            const int parts = WIDE ? max(1, min(kTeamParts, 16 * tm.nw / n)) : 1;
+            for (int b = tm.gw; b < nb * parts; b += tm.nw)
+                nbuild_cell_warp(S.N, g, parts > 1 ? b % nb : b, tm.lane, uniform, nbs[tm.w], parts > 1 ? b / nb : 0,
+                                 parts);
         } else {
             // a few cells of many atoms: a warp per atom
             for (int i = tm.gw; i < n; i += tm.nw) nbuild_atom(S.N, g, (uint32_t)i, tm.lane, uniform);
@@ -933,6 +961,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 }
 
 // Dynamic shared memory of a launch: the list build's state, one per warp.
+static size_t team_dyn_bytes() { return (kTeamThreads / 32) * sizeof(NbWarpSmem<kTeamChunks>); }
 static size_t solo_dyn_bytes(int threads) { return (size_t)(threads / 32) * sizeof(NbWarpSmem<kSoloChunks>); }
 
 // Mixed systems (exclusive) whose runs go to a grid's team: as many atoms as
@@ -1066,7 +1095,7 @@ int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam
         MDG_CUDA(cudaMemsetAsync(sys->team_word, 0, sizeof(unsigned long long), ctx->stream));
     }
     R.word = sys->team_word;
-    const size_t dyn = solo_dyn_bytes(kTeamThreads);
+    const size_t dyn = team_dyn_bytes();
     MDG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     void* args[2] = {&S, &R};
     MDG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kTeamThreads), args, dyn, ctx->stream));
@@ -1098,7 +1127,7 @@ int request_team_launch(const void* args, mdg_system* sys, int blocks, unsigned 
     R.per = std::max(8, ((S.n + blocks - 1) / blocks + 3) & ~3);
     blocks = (S.n + R.per - 1) / R.per;
     const void* fn = S.any_eam ? (const void*)k_team_request<true> : (const void*)k_team_request<false>;
-    const size_t dyn = solo_dyn_bytes(kTeamThreads);
+    const size_t dyn = team_dyn_bytes();
     MDG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     void* argv[2] = {&S, &R};
     MDG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kTeamThreads), argv, dyn, stream));
