@@ -2276,6 +2276,14 @@ static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, const Devi
                          pot_rcut_of(s), s->periodic, dt, part, io && first ? io->pos : nullptr,
                          io && first ? io->vel : nullptr, io && last ? io->opos : nullptr,
                          io && last ? io->ovel : nullptr, io && last ? io->oforce : nullptr);
+        if (rc == kTeamTooLarge) {
+            rc = MDG_OK;
+            if (io && first && io->pos) {
+                rc = vec_io(sys, io->opos, RX, 1, 0);
+                if (!rc) rc = vec_io(sys, io->ovel, VX, 1, 0);
+            }
+            return rc ? rc : run_graph(s, sys, ps, dt, left);
+        }
         if (rc) return rc;
         MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
         sys->fp_ok = 0;

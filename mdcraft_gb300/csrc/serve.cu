@@ -377,6 +377,10 @@ bool admit_block(mdg_server* sv, Slot& sl, Request* r, int team) {
         sl.sys->force_prec = MDG_PREC_MIXED;
         sl.team = team;
         if (team) rc = launch_team(sv, sl, ps.any_eam);
+        if (rc == kTeamTooLarge) {  // the persistent kernel takes it
+            sl.team = team = 0;
+            rc = MDG_OK;
+        }
         if (rc == MDG_OK) charge_actual(sv, sl, r);
     }
     r->solver->precision = prec_saved;

@@ -1032,6 +1032,17 @@ bool team_eligible(const mdg_solver* s, const mdg_system* sys) {
     return sys->n < kTeamMost;
 }
 
+// A cooperative launch; kTeamTooLarge, with nothing enqueued, where the context
+// cannot hold the blocks at once.
+static int launch_together(const void* fn, int blocks, void** args, size_t dyn, cudaStream_t stream) {
+    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kTeamThreads), args, dyn, stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return kTeamTooLarge;
+    }
+    return e == cudaSuccess ? MDG_OK : cuda_status(e, "team launch");
+}
+
 // Enqueues `steps` steps by a grid's team (any host arrays page-locked); the
 // steps left and the status words arrive in hcounter and hstat.
 int ensure_cutbits(mdg_system* sys);
@@ -1098,9 +1109,9 @@ int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam
     const size_t dyn = team_dyn_bytes();
     MDG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     void* args[2] = {&S, &R};
-    MDG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kTeamThreads), args, dyn, ctx->stream));
-    MDG_LAUNCHED(ctx);
-    return MDG_OK;
+    int rc = launch_together(fn, blocks, args, dyn, ctx->stream);
+    if (rc == MDG_OK) ctx->launches++;
+    return rc;
 }
 
 // Device scratch of a request's team: the barriers' word, the steps left and 8
@@ -1130,8 +1141,7 @@ int request_team_launch(const void* args, mdg_system* sys, int blocks, unsigned 
     const size_t dyn = team_dyn_bytes();
     MDG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     void* argv[2] = {&S, &R};
-    MDG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kTeamThreads), argv, dyn, stream));
-    return MDG_OK;
+    return launch_together(fn, blocks, argv, dyn, stream);
 }
 
 bool solo_out_started(const void* out_host, uint32_t seq) {
