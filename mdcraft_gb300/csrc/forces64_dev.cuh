@@ -168,10 +168,11 @@ __device__ __forceinline__ double ljs_pair64(const PotParams& P, double r2, doub
     return P.ljs_aVr2 * (Ur * (Ur - 0.5) * FV + (P.ljs_aLJ + P.ljs_bLJ * X) * X);
 }
 
-// r2 <= R2cut and not r2 < 1e-15, on the bits of a non-negative r2; NaN
-// passes, as it fails both of the reference's tests (its force is flagged).
+// r2 <= R2cut and not r2 < 1e-15, on the bits of a non-negative r2; NaN of
+// either sign passes, as it fails both of the reference's tests (its force is
+// flagged).
 __device__ __forceinline__ bool in_cut64(double r2, double R2cut) {
-    const long long b = __double_as_longlong(r2);
+    const long long b = __double_as_longlong(r2) & 0x7fffffffffffffffLL;
     return b >= 0x3cd203af9ee75616LL /* 1e-15 */ &&
            (b <= __double_as_longlong(R2cut) || b > 0x7ff0000000000000LL);
 }
