@@ -214,7 +214,7 @@ struct Screen64 {
     float x, y, z;     // the atom's position
     float L[3], il[3]; // periodic edges and their inverses (0: open)
     float thr;         // (rc + error)^2
-    float rc, Lmin;    // the largest cutoff and the smallest periodic edge
+    float rc, Lmin;    // the largest cutoff; the smallest periodic edge, 0: images by FP64
 
     template <bool MULTI>
     __device__ __forceinline__ void set(const FArgs& A, const PotSet* __restrict__ ps, int ki, double xi, double yi,
@@ -238,6 +238,9 @@ struct Screen64 {
         // largest coordinate an atom within reach can have
         const float reach = fmaf(fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) + far + rc, 9.5367431640625e-7f, rc);
         thr = reach * reach;
+        // nor does an FP32 difference tell the image of a pair in range where
+        // the shorter way round is not longer by that error: no edge will do
+        if (!(Lmin > 2.0f * reach)) Lmin = 0.f;
     }
 };
 
@@ -249,8 +252,9 @@ struct Screen64 {
 // their in-range entries (EAM Cu: 42 of 54 listed pairs are in range).
 // A pair is what the reference visits (Pair::* then Periodic::*_one): the raw
 // difference and, for atoms near a periodic face (bc), its ghost. Where every
-// periodic edge is above 2 rns and rns above the cutoff, a pair is one or the
-// other by the sign and size of its FP32 difference, and the image is one
+// periodic edge is above 2 rns, and above twice the cutoff by more than the
+// FP32 error at these coordinates, and rns above the cutoff, a pair is one or
+// the other by the sign and size of its FP32 difference, and the image is one
 // addition per axis; otherwise ghost64 decides in FP64, and with rns below
 // the cutoff both can count.
 // For every visit: seen(P, kj, k, ghost) (without SCREEN, which skips
