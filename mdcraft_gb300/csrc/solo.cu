@@ -33,6 +33,7 @@
 #include "integrate_dev.cuh"
 #include "mdg_host.h"
 #include "nlist_dev.cuh"
+#include "team_rules.h"
 #include "thermo_dev.cuh"
 
 namespace mdg {
@@ -90,7 +91,7 @@ constexpr int kSoloChunks = 2;
 // A grid's team: of few atoms a block, so more chunks (8 against 2 in LJ argon
 // 13,500 atoms 16.2 -> 15.6 us a step; 16 take L1 from EAM: Cu 87,808 atoms
 // 50.1 -> 53.0).
-constexpr int kTeamParts = 4, kTeamChunks = 8;
+constexpr int kTeamChunks = 8;
 
 // Polls (each an L2 round trip) after which a team's barrier gives up: ten
 // seconds or more, against rebuild phases of microseconds.
@@ -342,13 +343,11 @@ __device__ __noinline__ bool solo_rebuild(Team<NT, WIDE>& tm, const SoloArgs& S,
             extern __shared__ __align__(16) unsigned char solo_dyn[];
             using State = NbWarpSmem<WIDE ? kTeamChunks : kSoloChunks>;
             State* nbs = reinterpret_cast<State*>(solo_dyn);
-            // up to four warps share a cell where there are more warps than
-            // cells (LJ argon 13,500 atoms, a rebuild every 15 steps: 17.2 us a
-            // step by one, 15.6 by four; EAM Cu 32,000: 34.0 by one, 34.4 by two)
-            const int parts = WIDE ? max(1, min(kTeamParts, 16 * tm.nw / n)) : 1;
-            for (int b = tm.gw; b < nb * parts; b += tm.nw)
-                nbuild_cell_warp(S.N, g, parts > 1 ? b % nb : b, tm.lane, uniform, nbs[tm.w], parts > 1 ? b / nb : 0,
-                                 parts);
+            const int parts = WIDE ? team_parts(tm.nw, n) : 1;
+            const long long tasks = team_tasks(nb, parts);
+            for (long long b = tm.gw; b < tasks; b += tm.nw)
+                nbuild_cell_warp(S.N, g, parts > 1 ? task_bin(b, nb) : (int)b, tm.lane, uniform, nbs[tm.w],
+                                 parts > 1 ? task_part(b, nb) : 0, parts);
         } else {
             // a few cells of many atoms: a warp per atom
             for (int i = tm.gw; i < n; i += tm.nw) nbuild_atom(S.N, g, (uint32_t)i, tm.lane, uniform);

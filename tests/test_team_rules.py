@@ -1,0 +1,59 @@
+"""The arithmetic by which a grid's team shares out a rebuild
+(mdcraft_gb300/csrc/team_rules.h), compiled and run on the host."""
+from __future__ import annotations
+
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "mdcraft_gb300", "csrc")
+
+
+def _run(tmp_path, body):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text('#include "team_rules.h"\n#include <cstdio>\n#include <initializer_list>\nusing namespace mdg;\n'
+                   "#define CHECK(x) do { if (!(x)) { std::printf(\"%s\\n\", #x); return 1; } } while (0)\n"
+                   "int main() {\n" + body + "\nreturn 0; }\n")
+    subprocess.run([cxx, "-std=c++17", "-Wall", "-Werror", "-I", CSRC,
+                    str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_tasks_of_the_largest_grids(tmp_path):
+    """Every bin and part once, also where their number exceeds 2^31 (a grid has
+    up to 2^30 bins)."""
+    _run(tmp_path, """
+    for (int bins : {1, 64, 1000, 1 << 20, 600000000, 715827883, 1 << 30})
+        for (int parts = 1; parts <= kTeamParts; ++parts) {
+            const long long tasks = team_tasks(bins, parts);
+            CHECK(tasks / parts == bins && tasks % parts == 0);
+            for (int p = 0; p < parts; ++p)
+                for (long long b : {0LL, 1LL, bins / 2LL, bins - 1LL}) {
+                    if (b >= bins) continue;
+                    const long long t = p * (long long)bins + b;
+                    CHECK(t < tasks);
+                    CHECK(task_part(t, bins) == p && task_bin(t, bins) == (int)b);
+                }
+            CHECK(task_part(tasks - 1, bins) == parts - 1 && task_bin(tasks - 1, bins) == bins - 1);
+        }
+    """)
+
+
+def test_parts(tmp_path):
+    """One to four warps a cell, and more only where there are warps to spare."""
+    _run(tmp_path, """
+    int last = kTeamParts;
+    for (int n = 1; n < 200000; ++n) {
+        const int p = team_parts(152 * 24, n);
+        CHECK(p >= 1 && p <= last);
+        last = p;
+    }
+    CHECK(team_parts(75 * 24, 8000) == 3 && team_parts(152 * 24, 8000) == 4 && team_parts(152 * 24, 58369) == 1);
+    """)
