@@ -423,7 +423,7 @@ constexpr int kLaneAtoms = kBlock / 8;
 
 template <typename Group>
 __device__ __forceinline__ int block_forces(const FArgs& A, const PotSet* __restrict__ ps, float f[3]) {
-    __shared__ float sh[kBlock / 32][96];
+    __shared__ __align__(kLaneAlign) float sh[kBlock / 32][96];
     __shared__ float sum[3][kLaneAtoms];
     const int a = threadIdx.x >> 3, i = blockIdx.x * kLaneAtoms + a;
     const bool in = i < A.n;
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kBlock, MB) k_lane_forces(FArgs A, const PotSe
 
 template <int KINDS, bool REC>
 __global__ void __launch_bounds__(kBlock, lane_budget(KINDS)) k_lane_density(FArgs A, const PotSet* __restrict__ ps) {
-    __shared__ float sh[kBlock / 32][32];
+    __shared__ __align__(kLaneAlign) float sh[kBlock / 32][32];
     __shared__ float sum[kLaneAtoms];
     const int a = threadIdx.x >> 3, i = blockIdx.x * kLaneAtoms + a, w = i < A.n ? i : 0;
     const bool live = i < A.n && A.tag[w] != 0;

@@ -297,10 +297,12 @@ __device__ __forceinline__ void group_sums(const FArgs& A, int i, int ng, Group&
 // Eight lanes per atom (lane = threadIdx.x & 7; `live` false: no atom): lane l
 // evaluates groups l, l + 8, ...; after each round of eight groups lane k adds
 // the eight sums of component k in group order (through sh, 32 NC floats per
-// warp). Every lane of the warp calls this; out is the atom's sums, on all
-// eight lanes. A group's sums take about 100 instructions and the ordered
-// additions 4 a group and component, so the eight lanes run about six times
-// as fast as one where the GPU is not full.
+// warp, read by 16-byte words: on a kLaneAlign boundary, as every row of
+// [warps][32 NC] is when the first is). Every lane of the warp calls this; out
+// is the atom's sums, on all eight lanes. A group's sums take about 100
+// instructions and the ordered additions 4 a group and component, so the eight
+// lanes run about six times as fast as one where the GPU is not full.
+constexpr int kLaneAlign = 16;
 template <int NC, typename Group>
 __device__ __forceinline__ void lane_sums(const FArgs& A, bool live, int i, int ng, Group& grp, float* sh,
                                           float out[NC]) {

@@ -176,7 +176,7 @@ struct SoloShared {
 // leaves its shared memory to L1).
 template <int NT>
 struct LaneShared {
-    float part[NT / 32][96];  // lane_sums
+    alignas(kLaneAlign) float part[NT / 32][96];  // lane_sums
     float sum[3][NT];  // of NT atoms at a time
 };
 
@@ -636,6 +636,7 @@ struct TeamRun {
 };
 
 constexpr int kTeamThreads = 768;
+static_assert(alignof(LaneShared<kTeamThreads>) >= kLaneAlign, "lane_sums reads its exchange by 16-byte words");
 
 // A step's passes by the team: the forces, the thermostat, the second
 // half-kick and, with `next`, the next step's first half-kick and drift;
