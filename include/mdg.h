@@ -35,7 +35,7 @@ extern "C" {
 #define MDG_ERR_NOMEM (-2)    /* device or host allocation failed */
 #define MDG_ERR_OVERFLOW (-3) /* neighbour capacity exceeded (internal retry failed) */
 #define MDG_ERR_RANGE (-4)    /* atom outside the grid, or table range (results flagged) */
-#define MDG_ERR_TIMEOUT (-5)  /* bounded device wait expired */
+#define MDG_ERR_TIMEOUT (-5)  /* bounded device wait expired (a run: the atoms are lost, upload and update again) */
 #define MDG_ERR_CUDA (-6)     /* CUDA runtime error */
 #define MDG_ERR_STATE (-7)    /* object not ready (e.g. forces before a list) */
 #define MDG_ERR_NODEV (-8)    /* no CUDA device */

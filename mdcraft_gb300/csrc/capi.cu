@@ -2257,6 +2257,19 @@ struct TeamIo {
     double *opos = nullptr, *ovel = nullptr, *oforce = nullptr;
 };
 
+// After a team's run that gave up at a barrier: some blocks may have left in the
+// middle of a rebuild, with the list's lengths, the permuted fields and the
+// caller order half written. Nothing reads a list or a capacity from here on,
+// and the caller order is made anew, so that an upload of the atoms and an
+// update put the system right.
+static int team_gave_up(mdg_system* sys) {
+    forget_list(sys);
+    k_iota<<<nblk(sys->n), kBlock, 0, sys->ctx->stream>>>((int)sys->n, sys->u32[ORIG][sys->cur], sys->slot_of);
+    MDG_LAUNCHED(sys->ctx);
+    MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
+    return MDG_OK;
+}
+
 // Steps of one launch of the team kernel (3 to 15 ms).
 constexpr long kTeamSteps = 256;
 
@@ -2297,7 +2310,10 @@ static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, const Devi
         sys->fp_ok = 0;
         sys->force_prec = s->precision;
         if (sys->hstat->pad[1]) {
-            set_error("the step loop's blocks did not meet at a barrier in time");
+            const int lost = team_gave_up(sys);
+            if (lost) return lost;
+            set_error("the step loop's blocks did not meet at a barrier in time; the system's atoms are lost and have "
+                      "to be uploaded again");
             return MDG_ERR_TIMEOUT;
         }
         sys->rebuilds += sys->hstat->pad[0];

@@ -223,6 +223,13 @@ struct mdg_system {
 };
 
 namespace mdg {
+// The list no longer holds, nor what it was sized by: the stages and runs
+// refuse the system until it is built again.
+inline void forget_list(mdg_system* sys) {
+    sys->have_list = 0;
+    sys->cap_ready = 0;
+    sys->dirty = 1;
+}
 // Device buffers of a system (pool-ordered on its stream when it has a pool).
 int sys_malloc(mdg_system* sys, void** p, size_t bytes);
 void sys_free(mdg_system* sys, void* p, size_t bytes);
