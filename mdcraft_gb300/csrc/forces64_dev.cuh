@@ -169,12 +169,12 @@ __device__ __forceinline__ double ljs_pair64(const PotParams& P, double r2, doub
 }
 
 // r2 <= R2cut and not r2 < 1e-15, on the bits of a non-negative r2; NaN of
-// either sign passes, as it fails both of the reference's tests (its force is
-// flagged).
+// either sign passes (unsigned, its bits are above infinity's), as it fails
+// both of the reference's tests (its force is flagged).
 __device__ __forceinline__ bool in_cut64(double r2, double R2cut) {
-    const long long b = __double_as_longlong(r2) & 0x7fffffffffffffffLL;
-    return b >= 0x3cd203af9ee75616LL /* 1e-15 */ &&
-           (b <= __double_as_longlong(R2cut) || b > 0x7ff0000000000000LL);
+    const unsigned long long b = (unsigned long long)__double_as_longlong(r2);
+    return b >= 0x3cd203af9ee75616ULL /* 1e-15 */ &&
+           (b <= (unsigned long long)__double_as_longlong(R2cut) || b > 0x7ff0000000000000ULL);
 }
 
 // Any double as FP32 by integer operations, truncated; NaN from 2^128 up.
