@@ -30,7 +30,7 @@ def test_thin_skin_far_from_the_origin(shift, skin):
     r = (site + 0.5) * (L / 4) + rng.uniform(-0.02, 0.02, (64, 3))
     # pairs two sites apart along an axis lie within a few hundredths of rc
     d = np.abs(r[:, None, 0] - r[None, :, 0])
-    assert ((d > L / 2 - 0.01) & (d < p["rcut"])).any()
+    assert ((d > L / 2 - 0.03) & (d < p["rcut"])).any()
     atoms["r"] = r + shift
     atoms["rns"] = rns
     args = atoms, (shift, shift + L) * 3, (1, 1, 1), _lj(p)
