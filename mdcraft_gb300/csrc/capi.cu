@@ -2221,22 +2221,17 @@ static int graph_prologue(mdg_solver* s, mdg_system* sys) {
     return MDG_OK;
 }
 
-// The device's view of a page-locked host array of `count` doubles; null when a
-// kernel cannot take it: not page-locked to its end, or not on an 8-byte
-// boundary (a copy takes those too).
-static double* locked_view(const double* p, size_t count) {
+// The device's view of a page-locked host array of doubles; null when a kernel
+// cannot take it: not page-locked, or not on an 8-byte boundary (a copy takes
+// those too).
+static double* locked_view(const double* p) {
+    cudaPointerAttributes a;
     if (!p || (uintptr_t)p % alignof(double)) return nullptr;
-    cudaPointerAttributes a[2];
-    const double* ends[2] = {p, p + (count ? count - 1 : 0)};
-    for (int k = 0; k < 2; ++k) {
-        if (cudaPointerGetAttributes(&a[k], ends[k]) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        if (a[k].type != cudaMemoryTypeHost || !a[k].devicePointer) return nullptr;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
     }
-    if ((const double*)a[1].devicePointer - (const double*)a[0].devicePointer != ends[1] - p) return nullptr;
-    return (double*)a[0].devicePointer;
+    return a.type == cudaMemoryTypeHost ? (double*)a.devicePointer : nullptr;
 }
 
 // One step from page-locked arrays of this many atoms and more overlaps its
@@ -2749,9 +2744,9 @@ int mdg_run_host(mdg_solver* s, mdg_system* sys, double dt, long steps, double* 
         MDG_CUDA(cudaSetDevice(sys->ctx->device));
         mark_stepped(s, sys, ps);
         TeamIo io;
-        io.pos = io.opos = locked_view(pos, 3 * sys->n);
-        io.vel = io.ovel = locked_view(vel, 3 * sys->n);
-        io.oforce = locked_view(force, 3 * sys->n);
+        io.pos = io.opos = locked_view(pos);
+        io.vel = io.ovel = locked_view(vel);
+        io.oforce = locked_view(force);
         const bool direct = sys->n <= kTeamDirect && io.pos && io.vel && (!force || io.oforce);
         int rc = MDG_OK;
         bool done = false;
