@@ -31,8 +31,9 @@ constexpr uint32_t kTeamLook = 4096, kTeamPolls = 1u << 30;
 // further). A block's first thread adds and polls. No field may carry into
 // the next one: counts are compared without the field's top bit, and the
 // first block takes that bit out once it is set. (A word per block that
-// every block reads took 4 to 6 us against 2 here: 143 x 143 polls.)
-template <int NT, bool WIDE>
+// every block reads took 4 to 6 us against 2 here: 143 x 143 polls.) WAIT: the
+// barrier's limit in ns.
+template <int NT, bool WIDE, unsigned long long WAIT = kTeamWaitNs>
 struct Team {
     int t, lane, w, rank, size, a0, a1, gt, gn, gw, nw;
     bool dead = false;  // a barrier gave up; the run is void
@@ -40,11 +41,8 @@ struct Team {
     uint32_t cast[2] = {0, 0};      // votes counted so far at even and odd barriers
     unsigned long long* word;       // zero at the kernel's start
     int* said;                      // shared: bit 0 the vote, bit 1 a wait ran out
-    unsigned long long wait_ns;
 
-    __device__ __forceinline__ Team(unsigned long long* wd, int* flag, int n, int per,
-                                    unsigned long long limit = kTeamWaitNs)
-        : word(wd), said(flag), wait_ns(limit) {
+    __device__ __forceinline__ Team(unsigned long long* wd, int* flag, int n, int per) : word(wd), said(flag) {
         t = threadIdx.x;
         lane = t & 31;
         w = t >> 5;
@@ -77,7 +75,7 @@ struct Team {
                 if (wait && ++polls % kTeamLook == 0) {
                     const unsigned long long now = global_ns();
                     if (!since) since = now;
-                    if (now - since > wait_ns || polls >= kTeamPolls) break;
+                    if (now - since > WAIT || polls >= kTeamPolls) break;
                 }
             } while (wait);
             __threadfence();

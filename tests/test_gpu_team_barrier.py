@@ -56,9 +56,9 @@ __global__ void k_votes(unsigned long long* word, unsigned first, unsigned round
     if (tm.dead && tm.t == 0) atomicAdd(dead, 1u);
 }
 // A barrier that waits for one block more than there are.
-__global__ void k_alone(unsigned long long* word, unsigned long long limit, unsigned* dead) {
+__global__ void k_alone(unsigned long long* word, unsigned* dead) {
     __shared__ int said;
-    Team<NT, true> tm(word, &said, NT * gridDim.x, NT, limit);
+    Team<NT, true, 5000000ull> tm(word, &said, NT * gridDim.x, NT);
     tm.size += 1;
     tm.any(false);
     tm.any(true);  // no second wait
@@ -83,10 +83,9 @@ int main() {
         OK(cudaMemcpy(h, out, 8, cudaMemcpyDeviceToHost));
         CHECK(h[0] == 0 && h[1] == 0);
     }
-    unsigned long long limit = 5000000;
     OK(cudaMemset(word, 0, 8));
     OK(cudaMemset(out, 0, 8));
-    void* args[] = {&word, &limit, &out};
+    void* args[] = {&word, &out};
     cudaEvent_t a, b;
     OK(cudaEventCreate(&a));
     OK(cudaEventCreate(&b));
