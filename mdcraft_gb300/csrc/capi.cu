@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "mdg_host.h"
+#include "team_rules.h"
 
 namespace mdg {
 
@@ -938,6 +939,7 @@ int mdg_system_upload_atoms(mdg_system* sys, const mdg_atom* atoms, size_t n) {
     }
     if (n == 0) return MDG_OK;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     int rc = records_in_enqueue(sys, atoms, n);
     if (rc) return rc;
     MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
@@ -957,6 +959,7 @@ int mdg_system_download_atoms(mdg_system* sys, mdg_atom* atoms, size_t n) {
     if (!sys || (!atoms && n) || n != sys->n) return MDG_ERR_INVALID;
     if (n == 0) return MDG_OK;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     // straight into the caller's records: the copy engine reaches pageable
     // host memory at the link's rate here (22 MB in 125 us, as into pinned
     // memory), where a staged copy adds the host's (22 MB in 1.4 ms)
@@ -973,6 +976,7 @@ static int vec_io(mdg_system* sys, double* host, int field, int in, int sync = 1
     size_t n = sys->n;
     if (n == 0) return MDG_OK;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     cudaStream_t st = sys->ctx->stream;
     size_t bytes = n * 3 * sizeof(double);
     void* dbuf;
@@ -1013,6 +1017,7 @@ int mdg_system_get_forces(mdg_system* sys, double* xyz) { return vec_io(sys, xyz
 int mdg_nlist_update(mdg_system* sys, double kbuf, int half) {
     if (!sys) return MDG_ERR_INVALID;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     int rc = nlist_build(sys, kbuf, half ? 1 : 0);  // it also refreshes the rebuild thresholds
     if (rc && rc != MDG_ERR_RANGE) return rc;
     MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
@@ -1026,6 +1031,7 @@ int mdg_nlist_decide(mdg_system* sys, int* need) {
         return MDG_OK;
     }
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     cudaStream_t st = sys->ctx->stream;
     MDG_CUDA(cudaMemsetAsync(&sys->dstat->need_rebuild, 0, sizeof(uint32_t), st));
     int rc = launch_decide(sys);
@@ -1040,6 +1046,7 @@ int mdg_nlist_total(mdg_system* sys, size_t* total) {
     if (!sys || !total) return MDG_ERR_INVALID;
     if (!sys->have_list) return MDG_ERR_STATE;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     std::vector<uint64_t> off;
     int rc = nlist_export_offsets(sys, off);
     if (rc) return rc;
@@ -1051,6 +1058,7 @@ int mdg_nlist_export(mdg_system* sys, uint64_t* offsets, uint64_t* idx, size_t c
     if (!sys || !offsets) return MDG_ERR_INVALID;
     if (!sys->have_list) return MDG_ERR_STATE;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     std::vector<uint64_t> off;
     int rc = nlist_export_offsets(sys, off);
     if (rc) return rc;
@@ -1094,6 +1102,7 @@ int mdg_nlist_list_for(mdg_system* sys, const double x[3], uint64_t* out, size_t
     if (!sys || !x || !count || (!out && cap)) return MDG_ERR_INVALID;
     if (!sys->have_list) return MDG_ERR_STATE;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     std::vector<uint64_t> found;
     int rc = nlist_list_for(sys, x, found);
     if (rc) return rc;
@@ -1106,6 +1115,7 @@ int mdg_nlist_sort(mdg_system* sys, mdg_atom* atoms, size_t n, mdg_atom* sorted)
     if (!sys || ((!atoms || !sorted) && n) || (n && atoms == sorted)) return MDG_ERR_INVALID;
     if (n == 0) return MDG_OK;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     // the atoms go through a scratch system on the same device and domain:
     // its rebuild wraps them and bins them on the grid built from them
     mdg_system* tmp = nullptr;
@@ -1344,6 +1354,7 @@ int mdg_pot_values(mdg_ctx* ctx, mdg_potential* p, const double* r2, size_t n, d
     if (!ctx || !p || ((!r2 || !u) && n)) return MDG_ERR_INVALID;
     if (n == 0) return MDG_OK;
     MDG_CUDA(cudaSetDevice(ctx->device));
+    const DeviceUse use(ctx->device);
     int rc = pot_upload(p, ctx->device);
     if (rc) return rc;
     PotParams P;
@@ -1359,6 +1370,7 @@ int mdg_pot_embedding(mdg_ctx* ctx, mdg_potential* p, const double* rho, size_t 
     }
     if (n == 0) return MDG_OK;
     MDG_CUDA(cudaSetDevice(ctx->device));
+    const DeviceUse use(ctx->device);
     int rc = pot_upload(p, ctx->device);
     if (rc) return rc;
     PotParams P;
@@ -1410,6 +1422,7 @@ int mdg_pot_atom(mdg_ctx* ctx, mdg_potential* p, int what, mdg_atom* atom, mdg_a
         slots[k] = it->second;
     }
     MDG_CUDA(cudaSetDevice(ctx->device));
+    const DeviceUse use(ctx->device);
     int rc = pot_upload(p, ctx->device);
     if (rc) return rc;
     PotParams P;
@@ -1439,6 +1452,7 @@ int mdg_grid_build(mdg_system* sys, int32_t ints[9], double dbls[3]) {
         return MDG_OK;
     }
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     GridParams g;
     int rc = grid_build_only(sys, &g);
     if (rc) return rc;
@@ -1649,6 +1663,7 @@ int mdg_system_get_shape(mdg_system* sys, int what, int* value) {
 int mdg_system_thermo_calls(mdg_system* sys, uint32_t* calls) {
     if (!sys || !calls) return MDG_ERR_INVALID;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     MDG_CUDA(cudaMemcpyAsync(calls, &sys->dstat->therm_calls, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                              sys->ctx->stream));
     MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
@@ -1658,6 +1673,7 @@ int mdg_system_thermo_calls(mdg_system* sys, uint32_t* calls) {
 int mdg_system_set_thermo_calls(mdg_system* sys, uint32_t calls) {
     if (!sys) return MDG_ERR_INVALID;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     sys->hstat->therm_calls = calls;
     MDG_CUDA(cudaMemcpyAsync(&sys->dstat->therm_calls, &sys->hstat->therm_calls, sizeof(uint32_t),
                              cudaMemcpyHostToDevice, sys->ctx->stream));
@@ -1797,6 +1813,7 @@ int mdg_solver_prepare(mdg_solver* s, mdg_system* sys) {
     PotSet ps;
     int rc = check_ready(s, sys, &ps, false);
     if (rc) return rc;
+    const DeviceUse use(sys->ctx->device);
     rc = launch_zero(sys, ps.any_eam || s->multi);
     if (rc) return rc;
     rc = launch_drift(sys, 0.0, MDG_PREC_FP64, pot_rcut_of(s), s->periodic, 0, 0);
@@ -1817,6 +1834,7 @@ int mdg_solver_charge(mdg_solver* s, mdg_system* sys) {
     PotSet ps;
     int rc = check_ready(s, sys, &ps);
     if (rc) return rc;
+    const DeviceUse use(sys->ctx->device);
     rc = stage_impl(s, sys, ps, 0, s->precision);
     if (rc) return rc;
     MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
@@ -1827,6 +1845,7 @@ int mdg_solver_forces(mdg_solver* s, mdg_system* sys) {
     PotSet ps;
     int rc = check_ready(s, sys, &ps);
     if (rc) return rc;
+    const DeviceUse use(sys->ctx->device);
     rc = stage_impl(s, sys, ps, 1, s->precision);
     if (rc) return rc;
     MDG_CUDA(cudaStreamSynchronize(sys->ctx->stream));
@@ -1837,6 +1856,7 @@ int mdg_solver_stages(mdg_solver* s, mdg_system* sys) {
     PotSet ps;
     int rc = check_ready(s, sys, &ps);
     if (rc) return rc;
+    const DeviceUse use(sys->ctx->device);
     for (int k = 0; k < s->nstages; ++k) {
         rc = stage_impl(s, sys, ps, s->stages[k], s->precision);
         if (rc) return rc;
@@ -1851,6 +1871,7 @@ int mdg_solver_virials(mdg_solver* s, mdg_system* sys) {
     PotSet ps;
     int rc = check_ready(s, sys, &ps);
     if (rc) return rc;
+    const DeviceUse use(sys->ctx->device);
     // what the last step's prepare cleared, cleared before the virial pass
     rc = settle_outputs(sys);
     if (rc) return rc;
@@ -1889,6 +1910,7 @@ int mdg_verlet_make_step(mdg_solver* s, mdg_system* sys, double dt) {
     PotSet ps;
     int rc = check_ready(s, sys, &ps);
     if (rc) return rc;
+    const DeviceUse use(sys->ctx->device);
     if (s->precision == MDG_PREC_MIXED) {
         // Pair::prepare's rcut assignment and boundary flags, then the
         // offsets the mixed kernels read
@@ -2265,13 +2287,11 @@ static int team_gave_up(mdg_system* sys) {
     return MDG_OK;
 }
 
-// Steps of one launch of the team kernel (3 to 15 ms).
-constexpr long kTeamSteps = 256;
-
-// `steps` steps by a grid's team (team_eligible), waited for; the graph takes
-// over once something else is in flight on the device. A rebuild that outgrew
-// its capacities ends a launch early: grown here, and resumed. *io (optional):
-// *done tells whether the results went to its arrays.
+// `steps` steps by a grid's team (team_eligible), waited for, in launches of a
+// few milliseconds (kTeamLaunchUs); the graph takes over once something else is
+// in flight on the device. A rebuild that outgrew its capacities ends a launch
+// early too: grown here, and resumed. *io (optional): *done tells whether the
+// results went to its arrays.
 static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, const DeviceUse& use, double dt, long steps,
                     const TeamIo* io, bool* done) {
     int rc = graph_prologue(s, sys);
@@ -2286,12 +2306,15 @@ static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, const Devi
     int grown = 0;
     for (bool first = true; left > 0 && grown < 64; first = false) {
         if (!first && !use.alone()) return run_graph(s, sys, ps, dt, left);
-        const long part = std::min(left, kTeamSteps);
+        const bool mixed = s->precision == MDG_PREC_MIXED;
+        const double guess = team_step_us((long long)sys->n, sys->K, !mixed, ps.any_eam != 0);
+        const long part = team_steps(left, first ? std::max(guess, sys->team_us) : sys->team_us);
         const bool last = part == left;
-        rc = team_launch(sys, ext(s)->d.dev, thermo_of(s), ps.any_eam, s->precision == MDG_PREC_MIXED,
-                         pot_rcut_of(s), s->periodic, dt, part, io && first ? io->pos : nullptr,
-                         io && first ? io->vel : nullptr, io && last ? io->opos : nullptr,
-                         io && last ? io->ovel : nullptr, io && last ? io->oforce : nullptr);
+        const auto t0 = std::chrono::steady_clock::now();
+        rc = team_launch(sys, ext(s)->d.dev, thermo_of(s), ps.any_eam, mixed, pot_rcut_of(s), s->periodic, dt, part,
+                         io && first ? io->pos : nullptr, io && first ? io->vel : nullptr,
+                         io && last ? io->opos : nullptr, io && last ? io->ovel : nullptr,
+                         io && last ? io->oforce : nullptr);
         if (rc == kTeamTooLarge) {
             rc = MDG_OK;
             if (io && first && io->pos) {
@@ -2312,7 +2335,10 @@ static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, const Devi
             return MDG_ERR_TIMEOUT;
         }
         sys->rebuilds += sys->hstat->pad[0];
-        left -= part - (long)*sys->hcounter;
+        const long ran = part - (long)*sys->hcounter;
+        left -= ran;
+        sys->team_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count() /
+                       (double)std::max(ran, 1L);
         if (sys->hstat->build_flags & FLAG_OVERFLOW) {
             ++grown;
             sys->rebuilds--;
@@ -2815,6 +2841,7 @@ int mdg_run_host(mdg_solver* s, mdg_system* sys, double dt, long steps, double* 
 int mdg_system_measure(mdg_system* sys, mdg_state* out) {
     if (!sys || !out) return MDG_ERR_INVALID;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     int rc = settle_outputs(sys);
     if (rc) return rc;
     double r[11];
@@ -2834,6 +2861,7 @@ int mdg_system_measure(mdg_system* sys, mdg_state* out) {
 int mdg_system_flags(mdg_system* sys, uint32_t* flags) {
     if (!sys || !flags) return MDG_ERR_INVALID;
     MDG_CUDA(cudaSetDevice(sys->ctx->device));
+    const DeviceUse use(sys->ctx->device);
     cudaStream_t st = sys->ctx->stream;
     MDG_CUDA(cudaMemcpyAsync(sys->hstat, sys->dstat, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
     MDG_CUDA(cudaStreamSynchronize(st));

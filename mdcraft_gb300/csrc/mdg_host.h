@@ -3,11 +3,11 @@
 
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
 
+#include "device_use.h"
 #include "mdg_internal.cuh"
 
 namespace mdg {
@@ -184,6 +184,7 @@ struct mdg_system {
     int run_pre_kernels = 0;                 // kernels of the graph's prefix
     double graph_build_s = 0.0;              // host seconds spent building run graphs
     unsigned long long* team_word = nullptr; // barrier word of the team kernel (solo.cu)
+    double team_us = 0.0;                    // its last launch's time a step, rebuilds included
 
     // device status + grid
     mdg::DevStatus* dstat = nullptr;
@@ -298,29 +299,6 @@ struct SoloQueue {              // host-mapped
     // yet resident count), 2 running a request
     volatile uint32_t live[kSoloGens][kSoloMaxBlocks];
 };
-// A run or a served request that is in flight on a device, for as long as the
-// object lives. A team of blocks (solo.cu) holds the GPU for its steps, so it
-// takes a run only where nothing else is in flight, a thousandth of a second
-// or a few at a time; a mixed or FP64 step gives the same bits either way. Eight
-// threads with an LJ argon system of 4,000 atoms each, us per step and system:
-// teams in turn 12.5, graphs side by side 4.4.
-class DeviceUse {
-public:
-    explicit DeviceUse(int device) : n_(count(device)) { n_.fetch_add(1); }
-    ~DeviceUse() { n_.fetch_sub(1); }
-    DeviceUse(const DeviceUse&) = delete;
-    DeviceUse& operator=(const DeviceUse&) = delete;
-    bool alone() const { return n_.load() == 1; }
-    static int in_flight(int device) { return count(device).load(); }
-
-private:
-    static std::atomic<int>& count(int device) {
-        static std::atomic<int> in_flight[64];
-        return in_flight[device & 63];
-    }
-    std::atomic<int>& n_;
-};
-
 // The step loop of a small system by a grid of blocks (solo.cu); the launches
 // return kTeamTooLarge where the blocks cannot be resident together.
 constexpr int kTeamTooLarge = 1;

@@ -55,7 +55,7 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 struct Request {
-    std::optional<DeviceUse> use;  // from submission to completion
+    std::optional<DeviceHold> use;  // from submission to completion
     uint64_t id = 0;
     mdg_solver* solver = nullptr;
     mdg_domain dom{};
@@ -581,7 +581,7 @@ int progress(mdg_server* sv) {
         feeding = feeding || ((sl.state == BLOCK || sl.state == ALLOC) && !sl.team);
     }
     const bool teams = sv->team_scratch && !feeding && 2 * outstanding <= (size_t)sv->sms &&
-                       (size_t)DeviceUse::in_flight(sv->device) <= outstanding;
+                       (size_t)DeviceHold::in_flight(sv->device) <= outstanding;
     for (Slot& sl : sv->slots) {
         if (sv->queue.empty()) break;
         if (sl.req) continue;

@@ -57,3 +57,23 @@ def test_parts(tmp_path):
     }
     CHECK(team_parts(75 * 24, 8000) == 3 && team_parts(152 * 24, 8000) == 4 && team_parts(152 * 24, 58369) == 1);
     """)
+
+
+def test_steps_of_a_launch(tmp_path):
+    """About kTeamLaunchUs of steps, never none, never more than are left; the
+    guess before a step was timed grows with the pairs."""
+    _run(tmp_path, """
+    CHECK(team_steps(1, 1e9) == 1 && team_steps(50, 1e9) == 1 && team_steps(7, 0.0) == 7);
+    CHECK(team_steps(1L << 40, 0.0) == 1000000 && team_steps(1L << 40, 1e-12) == 1000000);
+    for (double us : {0.5, 12.2, 98.7, 3999.0, 4001.0})
+        for (long left : {1L, 10L, 1000000L}) {
+            const long k = team_steps(left, us);
+            CHECK(k >= 1 && k <= left && (k == 1 || k * us <= kTeamLaunchUs));
+            CHECK(k == left || (k + 1) * us > kTeamLaunchUs);
+        }
+    // FP64 argon of 19,652 atoms takes 98.7 us a step: 256 steps were 25 ms
+    CHECK(team_steps(256, team_step_us(19652, 100, true, false)) <= 45);
+    CHECK(team_step_us(4000, 100, false, false) < 20.0);
+    for (int k = 0; k < 4; ++k)
+        CHECK(team_step_us(116000, 400, k & 1, k & 2) > team_step_us(116000, 100, k & 1, k & 2));
+    """)
