@@ -2289,9 +2289,9 @@ static int team_gave_up(mdg_system* sys) {
 
 // `steps` steps by a grid's team (team_eligible), waited for, in launches of a
 // few milliseconds (kTeamLaunchUs); the graph takes over once something else is
-// in flight on the device. A rebuild that outgrew its capacities ends a launch
-// early too: grown here, and resumed. *io (optional): *done tells whether the
-// results went to its arrays.
+// in flight on the device, or the grid has outgrown a team. A rebuild that
+// outgrew its capacities ends a launch early too: grown here, and resumed. *io
+// (optional): *done tells whether the results went to its arrays.
 static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, const DeviceUse& use, double dt, long steps,
                     const TeamIo* io, bool* done) {
     int rc = graph_prologue(s, sys);
@@ -2305,7 +2305,7 @@ static int run_team(mdg_solver* s, mdg_system* sys, const PotSet& ps, const Devi
     long left = steps;
     int grown = 0;
     for (bool first = true; left > 0 && grown < 64; first = false) {
-        if (!first && !use.alone()) return run_graph(s, sys, ps, dt, left);
+        if (!first && !(use.alone() && team_eligible(s, sys))) return run_graph(s, sys, ps, dt, left);
         const bool mixed = s->precision == MDG_PREC_MIXED;
         const double guess = team_step_us((long long)sys->n, sys->K, !mixed, ps.any_eam != 0);
         const long part = team_steps(left, first ? std::max(guess, sys->team_us) : sys->team_us);

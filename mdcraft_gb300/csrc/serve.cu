@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "mdg_host.h"
+#include "team_rules.h"
 
 using namespace mdg;
 
@@ -375,6 +376,7 @@ bool admit_block(mdg_server* sv, Slot& sl, Request* r, int team) {
         sl.sys->dirty = 0;
         sl.sys->rebuilds = 1;
         sl.sys->force_prec = MDG_PREC_MIXED;
+        if (!request_team_fits(sl.sys->grid.nbins)) team = 0;
         sl.team = team;
         if (team) rc = launch_team(sv, sl, ps.any_eam);
         if (rc == kTeamTooLarge) {  // the persistent kernel takes it

@@ -943,13 +943,14 @@ void solo_fill(void* args, mdg_system* sys, const PotSet* dps, int any_eam, doub
 }
 
 // Whether a run of this solver on this system goes to a grid's team: LJsCut
-// or EAM, Single, full lists, and few enough atoms that the graph's launches
-// are a good part of a step.
+// or EAM, Single, full lists, few enough atoms that the graph's launches are a
+// good part of a step, and few enough bins (team_fits).
 bool team_eligible(const mdg_solver* s, const mdg_system* sys) {
     if (s->multi || s->nstages < 1 || !s->pot[0][0] || sys->half || sys->pool || sys->ctx->timing) return false;
     const int type = s->pot[0][0]->type;
     if (type != POT_LJCUT && type != POT_EAM) return false;
     if (!sys->cap_ready || sys->n < 1 || !sys->ctx->num_sms) return false;
+    if (!team_fits((long long)sys->n, sys->grid.nbins)) return false;
     if (s->precision == MDG_PREC_FP64) return sys->n < some_atoms64(type == POT_EAM);
     return sys->n < kTeamMost;
 }

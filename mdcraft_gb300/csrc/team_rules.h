@@ -1,8 +1,26 @@
-// team_rules.h — how long a grid's team (solo.cu) holds the GPU and how it shares
-// out a rebuild: plain arithmetic, the same on the host and in the kernels.
+// team_rules.h — what goes to a grid's team (solo.cu), how long it holds the GPU
+// and how it shares out a rebuild: plain arithmetic, the same on the host and in
+// the kernels.
 #pragma once
 
 namespace mdg {
+
+// Whether a run of n atoms on a grid of so many bins goes to a team (besides
+// team_eligible's rule on atoms). A team's rebuild clears and scans every bin,
+// the scan by one block while the others wait; the launched rebuild scans more
+// than 16,384 bins by many. A cluster in vacuum with atoms in the box's corners,
+// a rebuild every 15 steps, us a step by the graph / a team: LJ argon 4,000 atoms
+// with 32,768 bins 25.1 / 14.5, 64,000 25.1 / 16.8, 110,592 25.4 / 23.1, 262,144
+// 24.8 / 28.8, 884,736 25.4 / 134; 19,652 atoms 31.7 / 28.3, 31.3 / 26.1, 32.1 /
+// 34.2, 33.1 / 45.0, 42.2 / 169; 55,296 with 32,768 36.3 / 35.0, 110,592 37.0 /
+// 42.3; 97,556 with 32,768 43.6 / 43.6, 110,592 44.5 / 51.3; EAM Cu 78,732 with
+// 32,768 60.9 / 53.6, 262,144 61.9 / 65.5.
+constexpr bool team_fits(long long n, long long bins) { return bins <= (n < 24000 ? 65536 : 32768); }
+
+// The same for a served request, whose other way is one block that scans the
+// bins alone as well: a team unless its blocks would wait at a barrier for a
+// good part of a second.
+constexpr bool request_team_fits(long long bins) { return bins <= 1LL << 24; }
 
 // Up to this many warps share a cell of a team's list build.
 constexpr int kTeamParts = 4;

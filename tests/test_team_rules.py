@@ -77,3 +77,13 @@ def test_steps_of_a_launch(tmp_path):
     for (int k = 0; k < 4; ++k)
         CHECK(team_step_us(116000, 400, k & 1, k & 2) > team_step_us(116000, 100, k & 1, k & 2));
     """)
+
+
+def test_bins_of_a_team(tmp_path):
+    """Runs: 65,536 bins below 24,000 atoms, 32,768 from there on; requests: as
+    many as the launched scan takes. None where a task would not be an int's."""
+    _run(tmp_path, """
+    CHECK(team_fits(1, 65536) && !team_fits(1, 65537) && team_fits(23999, 65536));
+    CHECK(team_fits(24000, 32768) && !team_fits(24000, 32769) && !team_fits(1, 1 << 30));
+    CHECK(request_team_fits(1 << 24) && !request_team_fits((1 << 24) + 1) && !request_team_fits(1 << 30));
+    """)
