@@ -637,6 +637,15 @@ static void launch_forces_mixed(const mdg_system* sys, const FArgs& A, const Pot
 // neighbours only through the density pass's copies (pos32b, Fp32) and takes
 // each pair's cut decision from the density pass (cutbits), where the
 // unfused pass would settle pairs near the cutoff on the FP64 positions.
+//
+// With one table the pass is bound by L1, so what it gains from packed pairs it
+// can lose by gathers that come too close together (EAM Cu 1,000,188 atoms 220
+// us before, 229 with packed pairs). Blocks of 128 threads, eight an SM, and the
+// library's rsqrtf in place of the bare estimate (EamGroup; the same bits) space
+// them again, 220 us: 229 with neither, 223 with the blocks, 225 with rsqrtf,
+// 227 with unpacked pairs; 442,368 atoms 104 and 103. With several tables: 507
+// us (NiAl 1,018,880), 511 with rsqrtf.
+constexpr int kForceStepThreads = 128, kForceStepBlocks = 8;
 template <int KINDS, int MB, int NT = kBlock>
 __global__ void __launch_bounds__(NT, MB)
     k_force_step(FArgs A, IArgs D, const PotSet* __restrict__ ps, const unsigned long long* __restrict__ left) {
@@ -752,15 +761,14 @@ int launch_forces_step(mdg_system* sys, const PotSet* dps, const PotSet& ps, dou
     const int nb = nblk(sys->n);
     cudaStream_t st = ctx->stream;
     const bool multi = ps.multi != 0;
-    const int mb = force_blocks(sys, multi);
-    // 8: eight 128-thread blocks per SM (the 4-block budget in blocks half
-    // the size, so the launch's last, partly filled wave is shorter)
-    const int nb128 = nblk(sys->n, 128);
+    const int mb = multi || sys->shape[MDG_SHAPE_FORCE_BLOCKS_PER_SM] ? force_blocks(sys, multi) : kForceStepBlocks;
+    const int nb128 = nblk(sys->n, kForceStepThreads);
     with_kinds(ps, [&](auto k) {
         constexpr int K = decltype(k)::value;
         if (lanes_mixed(sys->n, ps)) k_lane_force_step<K><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, D, dps, left);
         else if (mb == 3) k_force_step<K, 3><<<nb, kBlock, 0, st>>>(A, D, dps, left);
-        else if (mb == 8) k_force_step<K, 8, 128><<<nb128, 128, 0, st>>>(A, D, dps, left);
+        else if (mb == kForceStepBlocks)
+            k_force_step<K, kForceStepBlocks, kForceStepThreads><<<nb128, kForceStepThreads, 0, st>>>(A, D, dps, left);
         else k_force_step<K, 4><<<nb, kBlock, 0, st>>>(A, D, dps, left);
     });
     MDG_LAUNCHED(ctx);

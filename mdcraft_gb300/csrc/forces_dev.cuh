@@ -101,7 +101,7 @@ __device__ __forceinline__ float ksum_add(float& s, float& c, float v) {
 // makes an entry's image one shifted and masked word. With the cut test's one
 // branch for several pairs (cut_pairs) and the bare hardware estimates
 // (rcp_approx, rsqrt_approx): LJ liquid 4,000,000 atoms 0.675 -> 0.525 ms,
-// EAM Cu 1,000,188 density 0.153 -> 0.135 and force 0.224 -> 0.228, NiAl
+// EAM Cu 1,000,188 density 0.153 -> 0.135 (force: kForceStepThreads), NiAl
 // 1,018,880 density 0.356 -> 0.332 and force 0.551 -> 0.506.
 template <int N>
 struct PairVecs {
@@ -766,7 +766,11 @@ struct EamGroup {
                 });
             // one reciprocal square root gives both r and 1/r
             const float x0 = fmaxf(v.r2[0], 1e-12f), x1 = fmaxf(v.r2[1], 1e-12f);
-            const unsigned long long rinv = rsqrt_nr2(pack2(x0, x1), pack2(rsqrt_approx(x0), rsqrt_approx(x1)));
+            // (with one table the pass is bound by L1, and the longer way to the
+            // same estimate spaces its gathers: kForceStepThreads)
+            const unsigned long long est = MULTI ? pack2(rsqrt_approx(x0), rsqrt_approx(x1))
+                                                 : pack2(rsqrtf(x0), rsqrtf(x1));
+            const unsigned long long rinv = rsqrt_nr2(pack2(x0, x1), est);
             const unsigned long long r = mul2(pack2(v.r2[0], v.r2[1]), rinv);
             float t[2], W[2], D[2], Fp[2], FF[2];
             if (MULTI) unpack2(r, t[0], t[1]);
