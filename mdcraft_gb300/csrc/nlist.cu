@@ -419,11 +419,11 @@ __global__ void __launch_bounds__(NW * 32, 28 / NW) k_nbuild_warp(NbArgs A, cons
     nbuild_cell_warp(A, g, bin, lane, A.st->nonuniform == 0, S[warp]);
 }
 
-// The list build by a warp per atom: of grids with a periodic axis of 2 cells
-// or fewer (a few cells of many atoms), of small systems (every grid), and of
-// atoms that were clamped into the grid (FLAG_RANGE), whose lists are built
-// again from their unclamped cells (nbuild_atom), over what the other builds
-// wrote. On other grids it returns at once.
+// The list build by atoms: of grids with a periodic axis of 2 cells or fewer, or
+// short of the box, by a thread or a warp each (atoms_by_threads); of small systems
+// (every grid) and of atoms that were clamped into the grid (FLAG_RANGE), whose
+// lists are built again from their unclamped cells (nbuild_atom), over what the
+// other builds wrote, by a warp each. On other grids it returns at once.
 __global__ void __launch_bounds__(kBlock) k_nbuild_atoms(NbArgs A, const GridParams* __restrict__ gp) {
     __shared__ GridParams g;
     if (threadIdx.x == 0) g = *gp;
@@ -432,10 +432,15 @@ __global__ void __launch_bounds__(kBlock) k_nbuild_atoms(NbArgs A, const GridPar
     const bool few = A.n < kAtomBuildMost && !g.small_box, clamped = (A.st->build_flags & FLAG_RANGE) != 0;
     if (!g.small_box && !few && !clamped) return;
     const bool uniform = A.st->nonuniform == 0;
+    if (g.small_box && atoms_by_threads<false>(g, A.n)) {
+        for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < (uint32_t)A.n; i += gridDim.x * kBlock)
+            nbuild_atom<1>(A, g, i, 0, uniform);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (kBlock / 32);
     for (uint32_t i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); i < (uint32_t)A.n; i += warps) {
-        if (g.small_box || A.o0[i].w == 2.0f) nbuild_atom(A, g, i, lane, uniform);
+        if (g.small_box || A.o0[i].w == 2.0f) nbuild_atom<32>(A, g, i, lane, uniform);
         else if (few) nbuild_atom_cells(A, g, i, lane, uniform);
     }
 }
@@ -782,8 +787,11 @@ int nlist_enqueue(mdg_system* sys, bool flips) {
         MDG_LAUNCHED(ctx);
     }
     // a grid-stride launch of at most four blocks per SM: on the large
-    // grids, where it returns at once, its blocks are few
-    k_nbuild_atoms<<<std::min(nblk(n, kBlock / 32), 4 * std::max(ctx->num_sms, 1)), kBlock, 0, st>>>(A, sys->dgrid);
+    // grids, where it returns at once, its blocks are few (the grid of the last
+    // sizing or rebuild tells how many atoms a block will have)
+    const bool threads = sys->grid.small_box && atoms_by_threads<false>(sys->grid, n);
+    k_nbuild_atoms<<<std::min(nblk(n, threads ? kBlock : kBlock / 32), 4 * std::max(ctx->num_sms, 1)), kBlock, 0, st>>>(
+        A, sys->dgrid);
     MDG_LAUNCHED(ctx);
     return MDG_OK;
 }

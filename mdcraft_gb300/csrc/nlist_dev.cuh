@@ -433,7 +433,7 @@ __device__ __forceinline__ bool are_neibs_exact(const GridParams& g, double xa, 
 
 // The grid covers every cell of each periodic axis (no local grid short of
 // the box).
-__device__ __forceinline__ bool grid_whole(const GridParams& g) {
+__host__ __device__ inline bool grid_whole(const GridParams& g) {
     for (int a = 0; a < g.dim; ++a)
         if (g.periodic[a] && (g.offset[a] != 0 || g.num[a] != g.dom_n[a])) return false;
     return true;
@@ -477,11 +477,17 @@ __device__ __forceinline__ float min_image_f(float d, float L) {
     return d;
 }
 
-// The end of atom i's list of cnt entries, by a warp: padding to a multiple of
-// four with self entries, the counts and the rebuild snapshot.
+// The end of atom i's list of cnt entries, by a warp (G = 32) or a thread (1):
+// padding to a multiple of four with self entries, the counts and the rebuild
+// snapshot.
+template <int G>
 __device__ __forceinline__ void end_list(const NbArgs& A, uint32_t i, int lane, int cnt) {
     const int padded = (cnt + 3) & ~3;
-    if (cnt + lane < padded && cnt + lane < A.K) A.nbr[nidx(cnt + lane, i, A.np)] = i | kSelfCode;
+    if (G == 32) {
+        if (cnt + lane < padded && cnt + lane < A.K) A.nbr[nidx(cnt + lane, i, A.np)] = i | kSelfCode;
+    } else {
+        for (int k = cnt; k < padded && k < A.K; ++k) A.nbr[nidx(k, i, A.np)] = i | kSelfCode;
+    }
     if (lane) return;
     A.ncnt[i] = padded < A.K ? padded : A.K;
     if (cnt > A.K) {
@@ -497,23 +503,23 @@ __device__ __forceinline__ void end_list(const NbArgs& A, uint32_t i, int lane, 
     A.saved_uid[i] = A.uid[i];
 }
 
-// The list of atom i by a warp, lanes over the candidates (used for grids
-// with a periodic axis of 2 cells or fewer, which have few cells of many
-// atoms each): its cell's 27 (or fewer, on small periodic axes) neighbour
-// cells in the reference's order, x outer, z inner, each cell's atoms in
-// slot order, 32 at a time; the accepted lanes append in lane order. (A
-// thread per atom walks its ~500 candidates alone: 303 us for 500 LJ atoms.)
-// The FP32 prefilter also holds on periodic axes of
-// one or two cells when the grid covers the whole box: every cell there is
-// an edge cell, so the exact test takes the minimum image, and the FP32
-// minimum image of the neighbour cell's displacement is the same distance
-// to ~1e-6 of r^2, inside the band that goes to FP64. A local grid short of
-// the box keeps the FP64 test for every candidate.
+// The list of atom i, by a warp with its lanes over the candidates (G = 32) or by
+// a thread (1): used for grids with a periodic axis of 2 cells or fewer and for
+// local grids short of a periodic box (atoms_by_threads says which), and for
+// atoms clamped into the grid. Its cell's 27 (or fewer, on small periodic axes)
+// neighbour cells in the reference's order, x outer, z inner, each cell's atoms
+// in slot order; accepted lanes append in lane order, so both give the same list.
+// The FP32 prefilter also holds on periodic axes of one or two cells when the
+// grid covers the whole box: every cell there is an edge cell, so the exact test
+// takes the minimum image, and the FP32 minimum image of the neighbour cell's
+// displacement is the same distance to ~1e-6 of r^2, inside the band that goes to
+// FP64. A local grid short of the box keeps the FP64 test for every candidate.
 // An atom clamped into the grid (a position on the upper face of a periodic
 // axis after the wrap, or outside the grid) is binned in its clamped cell,
 // but, as Grid::adjacent_cells (grid.cxx:138-207) takes the cell of the
 // position itself, its own walk and edge flags come from the unclamped cell;
 // the image codes stay relative to the cell it is binned in.
+template <int G>
 __device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g, uint32_t i, int lane,
                                             bool uniform_rns) {
     // prefilter band: rns^2 (1 -/+ 1e-5), valid when every atom has the same rns
@@ -575,7 +581,7 @@ __device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g
                 // image of the neighbour cell relative to the binned cell
                 const int dl[3] = {x + shift[0], y + shift[1], z + shift[2]};
                 const float sh[3] = {(float)dl[0] * g.csf[0], (float)dl[1] * g.csf[1], (float)dl[2] * g.csf[2]};
-                for (uint32_t jb = j0; jb < j1; jb += 32) {
+                for (uint32_t jb = j0; jb < j1; jb += G) {
                     const uint32_t j = jb + lane;
                     bool acc = j < j1 && j != i && !(A.half && A.orig[j] < origi);
                     float dx = 0.f, dy = 0.f, dz = 0.f;
@@ -592,7 +598,7 @@ __device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g
                         else if (pfi && oj.w == 0.0f && d2 > hi2) acc = false;
                         else acc = are_neibs_exact(g, xi, yi, zi, rni, A.rx[j], A.ry[j], A.rz[j], A.rns[j], edge);
                     }
-                    const unsigned m = __ballot_sync(0xffffffffu, acc);
+                    const unsigned m = G == 32 ? __ballot_sync(0xffffffffu, acc) : (unsigned)acc;
                     if (acc) {
                         // periodic image code: minimum image of j seen from i
                         const uint32_t code = pair_image_code(g, own, lc, dl, dx, dy, dz, A.st);
@@ -604,8 +610,32 @@ __device__ __forceinline__ void nbuild_atom(const NbArgs& A, const GridParams& g
             }
         }
     }
-    end_list(A, i, lane, cnt);
+    end_list<G>(A, i, lane, cnt);
 }
+
+// Whether the atoms of such a grid take a thread each. A warp's lanes are mostly
+// idle in cells of few atoms, but n threads leave the GPU idle where n is small:
+// the line rises with the atoms per cell, and lies lower for a local grid short
+// of the box, whose tests are all FP64. A rebuild, thread / warp: flat boxes (one
+// axis of two cells) with 4 atoms a cell 7,936 155 / 114 us, 31,752 171 / 292,
+// 128,016 294 / 970; 24: 16,416 338 / 185, 63,936 364 / 563; 96: 32,448 1,003 /
+// 572, 65,664 1,093 / 1,164; 192: 31,104 1,962 / 874. Short grids: 4 a cell 4,000
+// 351 / 292, 16,384 368 / 879; 24: 15,552 1,263 / 794, 65,856 2,405 / 3,158; 48:
+// 31,104 2,467 / 2,412, 131,712 8,540 / 10,817. A grid's team (TEAM) has fewer
+// threads; a step with a rebuild in five: flat argon 30,976 88.5 / 73.8 us, 53,824
+// 88.7 / 108; short argon 32,000 191 / 172, 55,296 206 / 263; short copper 16,384
+// 146 / 108, 32,000 156 / 177.
+template <bool TEAM>
+__host__ __device__ inline bool atoms_by_threads(const GridParams& g, long long n) {
+    const long long cells = g.ncells;
+    if (grid_whole(g)) return 2 * n * cells >= (TEAM ? 3 : 2) * (12000 * cells + 950 * n);
+    return 2 * n * cells >= (TEAM ? 5 : 2) * (3000 * cells + 1000 * n);
+}
+// In one block: a thread as soon as half of them have an atom (LJ argon, 100
+// steps: 256 atoms 2.09 / 1.98 ms, 500 3.56 / 4.04, 2,000 45 / 55; EAM Cu 640 6.0 /
+// 9.5).
+template <int NT>
+__device__ __forceinline__ bool block_by_threads(int n) { return 2 * n >= NT; }
 
 // The neighbour cell of lane t < 27, (t / 9 - 1, t / 3 % 3 - 1, t % 3 - 1)
 // from the cell at global index gc (local own): its first slot and count (0:
@@ -689,7 +719,7 @@ __device__ __forceinline__ void nbuild_atom_cells(const NbArgs& A, const GridPar
             cnt += __popc(m);
         }
     }
-    end_list(A, i, lane, cnt);
+    end_list<32>(A, i, lane, cnt);
 }
 
 // ---- list build, a warp per cell with lanes over candidates -------------------

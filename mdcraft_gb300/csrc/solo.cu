@@ -270,16 +270,17 @@ __device__ __noinline__ bool solo_rebuild(Team<NT, WIDE>& tm, const SoloArgs& S,
             for (long long b = tm.gw; b < tasks; b += tm.nw)
                 nbuild_cell_warp(S.N, g, parts > 1 ? task_bin(b, nb) : (int)b, tm.lane, uniform, nbs[tm.w],
                                  parts > 1 ? task_part(b, nb) : 0, parts);
+        } else if (WIDE ? atoms_by_threads<true>(g, n) : block_by_threads<NT>(n)) {
+            for (int i = tm.a0 + t; i < tm.a1; i += NT) nbuild_atom<1>(S.N, g, (uint32_t)i, 0, uniform);
         } else {
-            // a few cells of many atoms: a warp per atom
-            for (int i = tm.gw; i < n; i += tm.nw) nbuild_atom(S.N, g, (uint32_t)i, tm.lane, uniform);
+            for (int i = tm.gw; i < n; i += tm.nw) nbuild_atom<32>(S.N, g, (uint32_t)i, tm.lane, uniform);
         }
         tm.sync();
         if (tm.dead) return false;
         // atoms clamped into the grid: their own lists from their unclamped cells
         if (!g.small_box && (__ldcg(&S.st->build_flags) & FLAG_RANGE)) {
             for (int i = tm.gw; i < n; i += tm.nw)
-                if (S.N.o0[i].w == 2.0f) nbuild_atom(S.N, g, (uint32_t)i, tm.lane, uniform);
+                if (S.N.o0[i].w == 2.0f) nbuild_atom<32>(S.N, g, (uint32_t)i, tm.lane, uniform);
             tm.sync();
         }
     }
