@@ -149,11 +149,14 @@ struct MArgs {
     double* part;
 };
 
-__device__ void block_sum(double* sh, double* vals, int nv) {
+// Sums over the block's threads, of which the first `count` have anything to
+// add (the levels of the tree that would add zeros alone are left out).
+__device__ void block_sum(double* sh, double* vals, int nv, int count = kBlock) {
     int t = threadIdx.x;
     for (int k = 0; k < nv; ++k) sh[k * kBlock + t] = vals[k];
     __syncthreads();
     for (int s = kBlock / 2; s > 0; s >>= 1) {
+        if (s >= count) continue;
         if (t < s)
             for (int k = 0; k < nv; ++k) sh[k * kBlock + t] += sh[k * kBlock + t + s];
         __syncthreads();
@@ -190,7 +193,8 @@ __global__ void k_measure2(MArgs A, const double* __restrict__ com) {
 
 // The blocks' partial sums in one block: a thread per eight columns' worth of
 // rows, then a tree (a fixed order, so deterministic). One thread's chain of
-// nparts FP64 additions took 90 us at 432 parts.
+// nparts FP64 additions took 90 us at 432 parts; a tree over all 256 threads 5 us
+// more than that chain at 2 parts, so the tree has the levels the parts need.
 __global__ void __launch_bounds__(kBlock)
     k_measure_final(const double* __restrict__ part, int nparts, int stage, double* __restrict__ out) {
     __shared__ double sh[7 * kBlock];
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(kBlock)
     const int nv = stage == 1 ? 7 : 1, at = stage == 1 ? 0 : 7;
     for (int b = threadIdx.x; b < nparts; b += kBlock)
         for (int k = 0; k < nv; ++k) v[k] += part[b * 8 + at + k];
-    block_sum(sh, v, nv);
+    block_sum(sh, v, nv, nparts);
     if (threadIdx.x != 0) return;
     if (stage == 1) {
         for (int k = 0; k < 7; ++k) out[k] = sh[k * kBlock];
