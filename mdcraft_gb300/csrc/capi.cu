@@ -334,10 +334,8 @@ int system_alloc(mdg_system* sys) {
 }
 
 void system_free(mdg_system* sys) {
-    if (sys->run_exec) cudaGraphExecDestroy(sys->run_exec);
-    if (sys->run_graph) cudaGraphDestroy(sys->run_graph);
-    sys->run_exec = nullptr;
-    sys->run_graph = nullptr;
+    sys->run.free();
+    sys->run_spare.free();
     sys_free(sys, sys->dcounter, sizeof(unsigned long long));
     for_each_buffer(sys, [&](void** p, size_t b) {
         sys_free(sys, *p, b);
@@ -1984,16 +1982,8 @@ __global__ void k_set_counter(unsigned long long* counter, unsigned long long v,
     }
 }
 
-static void graph_free(mdg_system* sys) {
-    if (sys->run_exec) cudaGraphExecDestroy(sys->run_exec);
-    if (sys->run_graph) cudaGraphDestroy(sys->run_graph);
-    sys->run_exec = nullptr;
-    sys->run_graph = nullptr;
-}
-
-
 static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, double dt) {
-    graph_free(sys);
+    sys->run.free();
     mdg_ctx* ctx = sys->ctx;
     cudaStream_t st = ctx->stream;
     int prec = s->precision;
@@ -2012,7 +2002,7 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
     const bool next = starts_next_step(s, ps, prec) || flips || thermo;
     cudaGraph_t g = nullptr;
     MDG_CUDA(cudaGraphCreate(&g, 0));
-    sys->run_graph = g;
+    sys->run.graph = g;
     cudaGraphConditionalHandle hloop, hrb, hpre = 0;
     MDG_CUDA(cudaGraphConditionalHandleCreate(&hloop, g, 1, cudaGraphCondAssignDefault));
     // a handle must belong to a conditional node: only the mixed form has the pre-rebuild
@@ -2140,7 +2130,7 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
     cudaError_t e2 = cudaStreamEndCapture(st, &out);
     if (rc) return rc;
     if (e2 != cudaSuccess) return cuda_status(e2, "step capture");
-    sys->run_step_kernels = (int)(ctx->launches - l0);
+    sys->run.step_kernels = (int)(ctx->launches - l0);
 
     l0 = ctx->launches;
     MDG_CUDA(cudaStreamBeginCaptureToGraph(st, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
@@ -2152,12 +2142,26 @@ static int build_run_graph(mdg_solver* s, mdg_system* sys, const PotSet& ps, dou
     e2 = cudaStreamEndCapture(st, &out);
     if (rc) return rc;
     if (e2 != cudaSuccess) return cuda_status(e2, "rebuild capture");
-    sys->run_rebuild_kernels = (int)(ctx->launches - l0);
-    sys->run_pre_kernels = pre_kernels;
+    sys->run.rebuild_kernels = (int)(ctx->launches - l0);
+    sys->run.pre_kernels = pre_kernels;
     // counted when run (the pre-rebuild's kernels are counted as one rebuild)
-    ctx->launches -= (uint64_t)sys->run_step_kernels + 2 * (uint64_t)sys->run_rebuild_kernels + pre_kernels;
-    MDG_CUDA(cudaGraphInstantiate(&sys->run_exec, g, 0));
+    ctx->launches -= (uint64_t)sys->run.step_kernels + 2 * (uint64_t)sys->run.rebuild_kernels + pre_kernels;
+    MDG_CUDA(cudaGraphInstantiate(&sys->run.exec, g, 0));
     return MDG_OK;
+}
+
+// Whether the threads that run systems now fill the GPU with systems of this
+// size. Eight lanes an atom (lanes_mixed) and, below 100,000 atoms, the LJ pass that
+// starts the next step (k_lj_step) are for a GPU that a system has to itself; the
+// bits are the same either way. T threads, us a step and system, as alone / as here:
+// EAM Cu 16,384 atoms T = 4 18.1 / 18.8, 6 16.0 / 14.4, 16 15.0 / 9.5; 27,436 3 27.7 /
+// 25.4, 8 23.9 / 15.6; 4,000 16 4.7 / 5.2; NiAl 15,920 4 29.4 / 35.7, 8 29.1 / 23.6;
+// 34,977 8 61.6 / 39.2; LJ argon 16,384 8 9.9 / 8.1, 16 8.6 / 5.6; 62,500 2 33.2 /
+// 26.9; 131,072 4 28.0 / 29.3.
+constexpr long long kCrowd = 70000, kCrowdMost = 100000;
+static bool run_crowded(const mdg_system* sys) {
+    const long long threads = DeviceUse::threads(sys->ctx->device), n = (long long)sys->n;
+    return threads > 1 && n < kCrowdMost && threads * n >= kCrowd;
 }
 
 // Enqueues `left` steps as one graph launch plus the read-back of the
@@ -2169,22 +2173,27 @@ int run_graph_launch(mdg_solver* s, mdg_system* sys, const PotSet& ps, double dt
     uint64_t dtbits;
     memcpy(&dtbits, &dt, sizeof(dtbits));
     const uint64_t shapes = (uint64_t)sys->shape[0] | ((uint64_t)sys->shape[1] << 8) | ((uint64_t)sys->shape[2] << 16);
+    const bool crowded = run_crowded(sys);
     uint64_t key[4] = {(uint64_t)(uintptr_t)s, dtbits,
-                       (uint64_t)s->precision + 2 * (uint64_t)ext(s)->version + (shapes << 40), sys->cap_version};
-    if (!sys->run_exec || memcmp(key, sys->run_key, sizeof(key)) != 0) {
+                       (uint64_t)s->precision + 2 * (uint64_t)ext(s)->version + (shapes << 40) + ((uint64_t)crowded << 63),
+                       sys->cap_version};
+    if (!sys->run.is(key)) std::swap(sys->run, sys->run_spare);
+    if (!sys->run.is(key)) {
         auto t0 = std::chrono::steady_clock::now();
+        sys->crowded = crowded;
         int rc = build_run_graph(s, sys, ps, dt);
+        sys->crowded = 0;
         if (rc) {
-            graph_free(sys);
+            sys->run.free();
             return rc;
         }
-        memcpy(sys->run_key, key, sizeof(key));
+        memcpy(sys->run.key, key, sizeof(key));
         sys->graph_build_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     }
     if (!sys->hcounter) MDG_CUDA(cudaMallocHost((void**)&sys->hcounter, sizeof(unsigned long long)));
     k_set_counter<<<1, 32, 0, st>>>(sys->dcounter, (unsigned long long)left, sys->dstat);
     MDG_LAUNCHED(ctx);
-    MDG_CUDA(cudaGraphLaunch(sys->run_exec, st));
+    MDG_CUDA(cudaGraphLaunch(sys->run.exec, st));
     MDG_CUDA(cudaMemcpyAsync(sys->hcounter, sys->dcounter, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     MDG_CUDA(cudaMemcpyAsync(sys->hstat, sys->dstat, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
     sys->run_launched = left;
@@ -2201,8 +2210,8 @@ int run_graph_finish(mdg_solver* s, mdg_system* sys, long* left) {
     long done = sys->run_launched - rem;
     uint32_t nreb = sys->hstat->pad[0];
     sys->rebuilds += nreb;
-    ctx->launches += (uint64_t)sys->run_pre_kernels + (uint64_t)done * sys->run_step_kernels +
-                     (uint64_t)nreb * sys->run_rebuild_kernels;
+    ctx->launches += (uint64_t)sys->run.pre_kernels + (uint64_t)done * sys->run.step_kernels +
+                     (uint64_t)nreb * sys->run.rebuild_kernels;
     sys->force_prec = s->precision;
     *left = rem;
     if (sys->hstat->build_flags & FLAG_OVERFLOW) {

@@ -32,21 +32,31 @@ protected:
 class DeviceUse {
 public:
     explicit DeviceUse(int device) : device_(device & 63) {
-        if (depth(device_)++ == 0) hold().fetch_add(1);
+        if (depth(device_)++ > 0) return;
+        hold().fetch_add(1);
+        inside(device_).fetch_add(1);
     }
     ~DeviceUse() {
-        if (--depth(device_) == 0) hold().fetch_sub(1);
+        if (--depth(device_) > 0) return;
+        hold().fetch_sub(1);
+        inside(device_).fetch_sub(1);
     }
     DeviceUse(const DeviceUse&) = delete;
     DeviceUse& operator=(const DeviceUse&) = delete;
     // No other thread and no request has work on the device.
     bool alone() const { return DeviceHold::in_flight(device_) == 1; }
+    // Threads inside such calls.
+    static int threads(int device) { return inside(device & 63).load(); }
 
 private:
     struct Counts : DeviceHold {
         using DeviceHold::count;
     };
     std::atomic<int>& hold() const { return Counts::count(device_); }
+    static std::atomic<int>& inside(int device) {
+        static std::atomic<int> n[64];
+        return n[device];
+    }
     static int& depth(int device) {
         static thread_local int d[64] = {};
         return d[device];

@@ -484,8 +484,8 @@ __global__ void __launch_bounds__(kBlock, lane_budget(KINDS))
 // 37.9 / 22.0 us, 32,000 39.9 / 41.1, 62,500 46.2 / 64.9; NiAl 31,094
 // 92 / 75; LJ argon 4,000 25.6 / 20.6, 32,000 29.2 / 32.4; LJ liquid 62,500
 // 37.1 / 48.9.
-static bool lanes_mixed(size_t n, const PotSet& ps) {
-    return n < (!ps.any_eam ? 24000u : ps.multi ? 45000u : 30000u);
+static bool lanes_mixed(const mdg_system* sys, const PotSet& ps) {
+    return !sys->crowded && sys->n < (!ps.any_eam ? 24000u : ps.multi ? 45000u : 30000u);
 }
 static int lane_blocks(size_t n) { return (int)((n + kLaneAtoms - 1) / kLaneAtoms); }
 
@@ -607,7 +607,7 @@ static void launch_forces_mixed(const mdg_system* sys, const FArgs& A, const Pot
                                 cudaStream_t st) {
     const bool multi = ps.multi != 0;
     const int mb = force_blocks(sys, multi);
-    if (lanes_mixed(sys->n, ps)) {
+    if (lanes_mixed(sys, ps)) {
         launch_lane_forces<KICK>(A, dps, ps, lane_blocks(sys->n), st);
     } else if (ps.any_eam) {
         with_kinds(ps, [&](auto k) { launch_eam<decltype(k)::value, KICK>(mb, A, dps, nb, st); });
@@ -724,9 +724,9 @@ PosSet other_positions(mdg_system* sys) {
 }
 
 // Whether a step loop's LJ pass starts the next step: LJsCut alone, one thread
-// per atom.
+// per atom, with the GPU to itself.
 bool lj_starts_next(const mdg_system* sys, const PotSet& ps) {
-    return ps.any_lj && !ps.any_eam && !ps.any_tab && !ps.any_ljs && !lanes_mixed(sys->n, ps);
+    return !sys->crowded && ps.any_lj && !ps.any_eam && !ps.any_tab && !ps.any_ljs && !lanes_mixed(sys, ps);
 }
 
 int launch_lj_step(mdg_system* sys, const PotSet* dps, const PotSet& ps, double dt, const unsigned long long* left) {
@@ -765,7 +765,7 @@ int launch_forces_step(mdg_system* sys, const PotSet* dps, const PotSet& ps, dou
     const int nb128 = nblk(sys->n, kForceStepThreads);
     with_kinds(ps, [&](auto k) {
         constexpr int K = decltype(k)::value;
-        if (lanes_mixed(sys->n, ps)) k_lane_force_step<K><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, D, dps, left);
+        if (lanes_mixed(sys, ps)) k_lane_force_step<K><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, D, dps, left);
         else if (mb == 3) k_force_step<K, 3><<<nb, kBlock, 0, st>>>(A, D, dps, left);
         else if (mb == kForceStepBlocks)
             k_force_step<K, kForceStepBlocks, kForceStepThreads><<<nb128, kForceStepThreads, 0, st>>>(A, D, dps, left);
@@ -790,7 +790,7 @@ int launch_density_rec(mdg_system* sys, const PotSet* dps, const PotSet& ps) {
     const int mb = density_blocks(sys);
     with_kinds(ps, [&](auto k) {
         constexpr int K = decltype(k)::value;
-        if (lanes_mixed(sys->n, ps)) k_lane_density<K, true><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, dps);
+        if (lanes_mixed(sys, ps)) k_lane_density<K, true><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, dps);
         else launch_rec<K>(mb, A, dps, nb, st);
     });
     MDG_LAUNCHED(sys->ctx);
@@ -840,7 +840,7 @@ int launch_stage(mdg_system* sys, const PotSet* dps, const PotSet& ps, int preci
         if (stage == 0) {
             with_kinds(ps, [&](auto k) {
                 constexpr int K = decltype(k)::value;
-                if (lanes_mixed(sys->n, ps)) k_lane_density<K, false><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, dps);
+                if (lanes_mixed(sys, ps)) k_lane_density<K, false><<<lane_blocks(sys->n), kBlock, 0, st>>>(A, dps);
                 else launch_density<K>(density_blocks(sys), A, dps, nb, st);
             });
             sys->fp_ok = 0;  // nc rewritten (FP32 sums); Fp64 no longer matches it

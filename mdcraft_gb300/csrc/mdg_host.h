@@ -103,6 +103,26 @@ struct mdg_solver {
     mdg_thermostat* thermo = nullptr;  // applied after the force stage
 };
 
+namespace mdg {
+struct RunGraph {
+    cudaGraphExec_t exec = nullptr;
+    cudaGraph_t graph = nullptr;
+    uint64_t key[4] = {0, 0, 0, 0};
+    int step_kernels = 0;     // kernels per step / per rebuild in the graph
+    int rebuild_kernels = 0;
+    int pre_kernels = 0;      // kernels of the graph's prefix
+    bool is(const uint64_t k[4]) const {
+        return exec && k[0] == key[0] && k[1] == key[1] && k[2] == key[2] && k[3] == key[3];
+    }
+    void free() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+        exec = nullptr;
+        graph = nullptr;
+    }
+};
+}  // namespace mdg
+
 struct mdg_system {
     mdg_ctx* ctx = nullptr;
     mdg_domain dom{};
@@ -172,16 +192,14 @@ struct mdg_system {
     uint64_t cap_version = 0; // bumped when a capacity buffer is reallocated
 
     // captured step loop (mdg_run): graph of the driver loop, rebuilt when
-    // capacities, the solver, dt or the precision change
-    cudaGraphExec_t run_exec = nullptr;
-    cudaGraph_t run_graph = nullptr;
-    uint64_t run_key[4] = {0, 0, 0, 0};
+    // capacities, the solver, dt or the precision change, and the one before it
+    // (destroying a graph waits for the device, and a system of several threads'
+    // goes back and forth between two, run_crowded)
+    mdg::RunGraph run, run_spare;
+    int crowded = 0;                         // while a graph for a crowded GPU is built
     unsigned long long* dcounter = nullptr;  // steps left (device)
     unsigned long long* hcounter = nullptr;  // its read-back (pinned)
     long run_launched = 0;                   // steps handed to the last graph launch
-    int run_step_kernels = 0;                // kernels per step / per rebuild in the graph
-    int run_rebuild_kernels = 0;
-    int run_pre_kernels = 0;                 // kernels of the graph's prefix
     double graph_build_s = 0.0;              // host seconds spent building run graphs
     unsigned long long* team_word = nullptr; // barrier word of the team kernel (solo.cu)
     double team_us = 0.0;                    // its last launch's time a step, rebuilds included

@@ -232,10 +232,12 @@ void retire(mdg_server* sv, Slot& sl) {
         double t = sv->now();
         // destroying an executable graph waits for the whole device: keep
         // them until no request runs (or the server goes)
-        if (sl.sys->run_exec) sv->spent_execs.push_back(sl.sys->run_exec);
-        if (sl.sys->run_graph) sv->spent_graphs.push_back(sl.sys->run_graph);
-        sl.sys->run_exec = nullptr;
-        sl.sys->run_graph = nullptr;
+        for (RunGraph* g : {&sl.sys->run, &sl.sys->run_spare}) {
+            if (g->exec) sv->spent_execs.push_back(g->exec);
+            if (g->graph) sv->spent_graphs.push_back(g->graph);
+            g->exec = nullptr;
+            g->graph = nullptr;
+        }
         double t1 = sv->now();
         sv->graph_destroy_s += t1 - t;
         system_release(sl.sys);

@@ -19,10 +19,10 @@ PROGRAM = r"""
 using namespace mdg;
 #define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
 int main() {
-    CHECK(DeviceHold::in_flight(0) == 0);
+    CHECK(DeviceHold::in_flight(0) == 0 && DeviceUse::threads(0) == 0);
     {
         const DeviceUse run(0);
-        CHECK(run.alone());
+        CHECK(run.alone() && DeviceUse::threads(0) == 1);
         {
             const DeviceUse inner(0);  // an entry point called by another
             CHECK(inner.alone() && run.alone() && DeviceHold::in_flight(0) == 1);
@@ -33,6 +33,7 @@ int main() {
         bool seen = true, own = true;
         std::thread t([&] {
             const DeviceUse stage(0);
+            if (DeviceUse::threads(0) != 2) return;
             own = stage.alone();
             seen = run.alone();
         });
@@ -40,11 +41,11 @@ int main() {
         CHECK(!seen && !own && run.alone());
         std::optional<DeviceHold> request;
         request.emplace(0);
-        CHECK(!run.alone());
+        CHECK(!run.alone() && DeviceUse::threads(0) == 1);
         request.reset();
         CHECK(run.alone());
     }
-    CHECK(DeviceHold::in_flight(0) == 0 && DeviceHold::in_flight(1) == 0);
+    CHECK(DeviceHold::in_flight(0) == 0 && DeviceHold::in_flight(1) == 0 && DeviceUse::threads(0) == 0);
     return 0;
 }
 """
