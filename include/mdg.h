@@ -263,8 +263,12 @@ int mdg_solver_stages(mdg_solver* s, mdg_system* sys);
  *   MDG_SHAPE_LIST_CELLS_PER_BLOCK   cells (warps) per block of the list build: 2, 4, 8
  *   MDG_SHAPE_FORCE_BLOCKS_PER_SM    register budget of the mixed force pass: 3, 4, or 8
  *                                    (eight 128-thread blocks: the step loop's EAM force
- *                                    pass; the other force passes take 4 then)
- *   MDG_SHAPE_DENSITY_BLOCKS_PER_SM  register budget of the mixed density pass: 3, 4, 5 */
+ *                                    pass, its default with one table; the other force
+ *                                    passes take 4 then)
+ *   MDG_SHAPE_DENSITY_BLOCKS_PER_SM  register budget of the mixed density pass: 3, 4, 5
+ * They shape the launched passes: a small system's mdg_run is one kernel, and the
+ * passes of a few ten thousand atoms take several lanes an atom, which have no
+ * shapes. */
 #define MDG_SHAPE_LIST_CELLS_PER_BLOCK 0
 #define MDG_SHAPE_FORCE_BLOCKS_PER_SM 1
 #define MDG_SHAPE_DENSITY_BLOCKS_PER_SM 2
@@ -372,9 +376,12 @@ typedef struct mdg_server_config {
     int slots;          /* systems on the GPU at once (>= 1) */
     size_t hbm_budget;  /* device bytes the live systems may hold; 0 = half the free memory */
     size_t max_atoms;   /* largest request accepted (sizes the pinned staging) */
-    int block_threads;  /* fused one-block loop per system (mixed precision, one kind,
-                           <= 65536 atoms): its threads (256, 512, 640, 768, 896, 1024), 0 = the default
-                           (640), -1 = off (a graph loop per request instead) */
+    int block_threads;  /* the fused loop (mixed precision, one kind, LJsCut or EAM, no
+                           thermostat, <= 65536 atoms; other requests take a graph loop):
+                           0 = a request runs on several SMs while few are outstanding,
+                           else in one block of 640 threads; 256, 512, 640, 768, 896 or
+                           1024 = every one in one block of so many; -1 = off (a graph
+                           loop per request instead) */
     int order;          /* admission order of waiting requests: MDG_ORDER_FIFO (0, the
                            default), MDG_ORDER_LARGEST (most atom-steps first, which
                            shortens the tail of a backlog at the cost of small requests'

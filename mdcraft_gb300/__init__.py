@@ -679,8 +679,10 @@ class Server:
 
     def __init__(self, device: int = 0, slots: int = 16, hbm_budget: int = 0, max_atoms: int = 1 << 16,
                  block_threads: int = 0, order: str = "fifo"):
-        """block_threads: threads of the fused per-request block (256, 512, 640, 768, 896, 1024; 0 = 640);
-        -1 runs every request as a graph loop on its slot's stream instead. order: "fifo"
+        """block_threads: 0 runs a request of the fused loop (mixed, one kind, LJsCut or EAM, no
+        thermostat) on several SMs while few are outstanding, else in one block of 640 threads;
+        256, 512, 640, 768, 896 or 1024 every one in one block of so many; -1 runs every request
+        as a graph loop on its slot's stream instead. order: "fifo"
         admits waiting requests in arrival order, "largest" the one with the most
         atom-steps first, "balanced" in arrival order except that the largest
         waiting request goes first once its atom-steps reach the waiting

@@ -1,7 +1,8 @@
 // forces.cu — LJsCut and two-pass EAM force stages on the Verlet list.
 //
-// FP64 form: the reference's per-atom arithmetic (LJs-cut.cxx:22-131,
-// EAM.cxx:141-601) including the Periodic boundary's ghost pass
+// FP64 form: the reference's sums (LJs-cut.cxx:22-131, EAM.cxx:141-601) in FP64,
+// with an arithmetic of fewer operations a pair (forces64_dev.cuh; the arrays' and
+// single atoms' calls keep the reference's), including the Periodic boundary's ghost pass
 // (boundary/periodic.cxx:36-102): listed pairs contribute with the raw
 // difference r_j - r_i; for atoms flagged by Periodic::prepare_one, listed
 // pairs at raw distance >= max(rns) contribute again through the shortest
@@ -13,7 +14,8 @@
 // 2*rns), pair math and splines in FP32 (cubic coefficients per table
 // interval), and per-atom sums with Kahan compensation.
 //
-// One thread per atom over the ELL list (entry k of atom i at nbr[k*np+i]),
+// One thread or several lanes per atom over the ELL list (entry k of atom i at
+// nbr[k*np+i]); an atom's sum is the one thread's, or its lanes' in a fixed order,
 // so the per-atom sums need no atomics and are deterministic.
 #include <cuda_runtime.h>
 

@@ -320,6 +320,8 @@ struct SoloQueue {              // host-mapped
 // The step loop of a small system by a grid of blocks (solo.cu); the launches
 // return kTeamTooLarge where the blocks cannot be resident together.
 constexpr int kTeamTooLarge = 1;
+// The largest request of the fused loops.
+constexpr size_t kSoloMaxAtoms = 65536;
 bool team_eligible(const mdg_solver* s, const mdg_system* sys);
 int team_launch(mdg_system* sys, const PotSet* dps, const ThermoDev* th, int eam, int mixed, double pot_rcut,
                 int periodic, double dt, long steps, const double* hpos, const double* hvel, double* opos,

@@ -4,8 +4,9 @@
 // (mdcraft/neibs/verlet-list.cxx:41-55, 306-400) and Grid::build /
 // adjacent_cells (mdcraft/neibs/grid.cxx:43-207) as a device pipeline:
 //   wrap + bounds -> grid parameters -> bin count (bricked Morton keys)
-//   -> exclusive scan -> scatter -> per-bin sort by caller index
-//   -> permutation of every per-atom field -> warp-per-cell list build.
+//   -> exclusive scan -> scatter in arrival order -> permutation of every
+//   per-atom field, each bin ordered by caller index -> list build (a warp per
+//   cell; a warp or a thread per atom where that is faster).
 // The list test is the reference's FP64 expression evaluated without FMA
 // contraction; an FP32 estimate from cell-centred offsets decides the clear
 // cases and sends candidates within 1e-5 (relative) of the radius, or any

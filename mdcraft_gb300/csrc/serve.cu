@@ -264,7 +264,7 @@ bool block_mode(const mdg_server* sv, const Request* r) {
     const mdg_solver* s = r->solver;
     // the fused loops carry the LJsCut and EAM bodies only, and no thermostat
     return r->precision == MDG_PREC_MIXED && !s->multi && s->nstages >= 1 && !s->thermo && s->pot[0][0] &&
-           (s->pot[0][0]->type == POT_LJCUT || s->pot[0][0]->type == POT_EAM) && r->atoms.size() <= 65536 &&
+           (s->pot[0][0]->type == POT_LJCUT || s->pot[0][0]->type == POT_EAM) && r->atoms.size() <= kSoloMaxAtoms &&
            r->atoms.size() > 0;
 }
 

@@ -79,7 +79,6 @@ struct alignas(16) SoloArgs {
     mdg_atom* atoms_out;          // host-mapped: the result records, caller order
 };
 
-constexpr int kSoloMaxAtoms = 65536;
 // Chunks per turn of the list build here: few, as its shared memory is taken
 // from the L1 that the force passes gather through.
 constexpr int kSoloChunks = 2;

@@ -14,6 +14,9 @@ step loop puts around each of its force and density launches, one
 dimension at a time. Whole-step times are not used: a list rebuild (about
 three steps' worth of work) lands in some windows and not others.
 
+Shapes have no effect where `Verlet.run` takes one kernel for all its steps or
+the passes take several lanes an atom (small systems).
+
 Results are cached per (GPU, workload signature) in `_build/tune.json`
 beside the library, so a later run on the same GPU and workload reuses the
 choice without measuring.
