@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -619,15 +620,22 @@ struct SolverDev {
     PotSet host;
     PotSet* dev = nullptr;  // start of the SolverBlob
     int device = -1;
-    int version = -1;
+    uint64_t version = 0;
     ThermoDev th_host{};
     int th_valid = 0;
 };
 
+// A number no solver has had in any state before: what a captured graph is known
+// by (a solver's address is another's once it is gone).
+static uint64_t next_version() {
+    static std::atomic<uint64_t> last{0};
+    return last.fetch_add(1) + 1;
+}
+
 struct mdg_solver_ext {
     mdg_solver s;
     SolverDev d;
-    int version = 0;
+    uint64_t version = next_version();
 };
 
 static SolverBlob* blob_of(SolverDev& d) { return reinterpret_cast<SolverBlob*>(d.dev); }
@@ -647,6 +655,7 @@ int potset_build(mdg_solver* s, mdg_system* sys, PotSet* out) {
         if (e->d.dev) cudaFree(e->d.dev);
         e->d.dev = nullptr;
         e->d.th_valid = 0;
+        e->version = next_version();  // graphs hold the block's address
         MDG_CUDA(cudaMalloc(&e->d.dev, sizeof(SolverBlob)));
         MDG_CUDA(cudaMemset(e->d.dev, 0, sizeof(SolverBlob)));
     }
@@ -1518,7 +1527,7 @@ int mdg_solver_add_potential(mdg_solver* s, int i, int j, mdg_potential* pot) {
     s->pot[i][j] = pot;
     s->pot[j][i] = pot;
     set_stages(s, pot->type, first);
-    ext(s)->version++;
+    ext(s)->version = next_version();
     return MDG_OK;
 }
 
@@ -1605,7 +1614,7 @@ static int thermo_flatten(const mdg_thermostat* t, ThermoDev& out, int depth) {
 int mdg_solver_set_thermostat(mdg_solver* s, mdg_thermostat* t) {
     if (!s) return MDG_ERR_INVALID;
     s->thermo = t;
-    ext(s)->version++;  // captured graphs gain or lose the thermostat pass
+    ext(s)->version = next_version();  // captured graphs gain or lose the thermostat pass
     return MDG_OK;
 }
 
@@ -2174,9 +2183,8 @@ int run_graph_launch(mdg_solver* s, mdg_system* sys, const PotSet& ps, double dt
     memcpy(&dtbits, &dt, sizeof(dtbits));
     const uint64_t shapes = (uint64_t)sys->shape[0] | ((uint64_t)sys->shape[1] << 8) | ((uint64_t)sys->shape[2] << 16);
     const bool crowded = run_crowded(sys);
-    uint64_t key[4] = {(uint64_t)(uintptr_t)s, dtbits,
-                       (uint64_t)s->precision + 2 * (uint64_t)ext(s)->version + (shapes << 40) + ((uint64_t)crowded << 63),
-                       sys->cap_version};
+    const uint64_t key[4] = {ext(s)->version, dtbits,
+                             (uint64_t)s->precision + 2 * (uint64_t)crowded + (shapes << 8), sys->cap_version};
     if (!sys->run.is(key)) std::swap(sys->run, sys->run_spare);
     if (!sys->run.is(key)) {
         auto t0 = std::chrono::steady_clock::now();
