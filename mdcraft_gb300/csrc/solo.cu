@@ -119,6 +119,17 @@ __device__ __forceinline__ void block_bounds8(long long v[8], bool busy, SoloSha
     }
 }
 
+// The lists of flat and short grids (a function of its own: the rebuild's
+// registers are for the other grids).
+template <int NT, bool WIDE>
+__device__ __noinline__ void small_box_lists(const Team<NT, WIDE>& tm, const NbArgs& N, const GridParams& g, bool uniform) {
+    if (WIDE ? atoms_by_threads<true>(g, N.n) : block_by_threads<NT>(N.n)) {
+        for (int i = tm.a0 + tm.t; i < tm.a1; i += NT) nbuild_atom<1>(N, g, (uint32_t)i, 0, uniform);
+    } else {
+        for (int i = tm.gw; i < N.n; i += tm.nw) nbuild_atom<32>(N, g, (uint32_t)i, tm.lane, uniform);
+    }
+}
+
 // One rebuild by the team (the pipeline of nlist_enqueue). Team-uniform
 // result: false when a capacity overflowed (the loop stops and the host grows
 // the capacities).
@@ -269,10 +280,8 @@ __device__ __noinline__ bool solo_rebuild(Team<NT, WIDE>& tm, const SoloArgs& S,
             for (long long b = tm.gw; b < tasks; b += tm.nw)
                 nbuild_cell_warp(S.N, g, parts > 1 ? task_bin(b, nb) : (int)b, tm.lane, uniform, nbs[tm.w],
                                  parts > 1 ? task_part(b, nb) : 0, parts);
-        } else if (WIDE ? atoms_by_threads<true>(g, n) : block_by_threads<NT>(n)) {
-            for (int i = tm.a0 + t; i < tm.a1; i += NT) nbuild_atom<1>(S.N, g, (uint32_t)i, 0, uniform);
         } else {
-            for (int i = tm.gw; i < n; i += tm.nw) nbuild_atom<32>(S.N, g, (uint32_t)i, tm.lane, uniform);
+            small_box_lists(tm, S.N, g, uniform);
         }
         tm.sync();
         if (tm.dead) return false;
